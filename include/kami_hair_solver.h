@@ -406,30 +406,22 @@ typedef enum KhsxSolveMode {
 KHS_API KhsResult khsxSetSolveMode(KhsSolver *solver, uint32_t mode);
 KHS_API uint32_t khsxGetSolveMode(const KhsSolver *solver);
 
-/* Launch shape of the FP64 block-tridiagonal solve.  By default it is tuned
-   once per solver by timing each shape on the first system; this pins it:
-   strands_per_warp 5 (6 lanes per strand), 2 (12 lanes per strand, half
-   the instructions on each strand's sequential chain) or 1 (18 lanes),
-   blocks_per_sm 1-8; long_strands > 0 first gives that many longest
-   strands one warp of 18 lanes each (with strands_per_warp 5) or a pair of
-   warps each (with strands_per_warp 1: one warp runs the pivot steps on the
-   diagonal blocks, the other applies them to the coupling blocks and the
-   right-hand side), the rest five per warp.  strands_per_warp 0 restores
-   the tuning.  Every shape gives bit-identical directions.
-   Requires a built solver. */
+/* Launch shape of the FP64 block-tridiagonal solve.  By default a rule on the
+   strands' lengths chooses it; this pins it: strands_per_warp 5 (6 lanes per
+   strand), or 1 or 2 (a warp for every strand: the shortest sequential
+   chain), blocks_per_sm 1-8 (four warps each); long_strands > 0 (with
+   strands_per_warp 5 or 1) gives that many longest strands a warp each and
+   the rest five per warp.  strands_per_warp 0 restores the rule.  Every shape
+   gives bit-identical directions.  Requires a built solver. */
 KHS_API KhsResult khsxSetBlockSolveSchedule(KhsSolver *solver, uint32_t strands_per_warp, uint32_t blocks_per_sm,
                                             uint32_t long_strands);
 
-/* Tiered launch shape of the FP64 block-tridiagonal solve (the tuner also
-   considers it): the `quads` longest strands each on four warps of one
-   block (one warp runs the pivot steps on the diagonal blocks, three apply
-   them to two columns each of the coupling blocks and the right-hand side
-   and form the next Schur complement), the next `singles` strands one per
-   warp (18 lanes), the next `doubles` two per warp (12 lanes each), the rest
-   five per warp; blocks_per_sm 1-8; quads + singles + doubles must not
-   exceed the strand count.  Every shape gives bit-identical directions.
-   No counterpart in the reference (its solve is one thread per strand,
-   src/cuda_backend.cu:866-881).  Requires a built solver. */
+/* The same launch shape by tiers of strand length: the quads + singles +
+   doubles longest strands a warp each, the rest five per warp; blocks_per_sm
+   1-8; quads + singles + doubles must not exceed the strand count.  Every
+   shape gives bit-identical directions.  No counterpart in the reference (its
+   solve is one thread per strand, src/cuda_backend.cu:866-881).  Requires a
+   built solver. */
 KHS_API KhsResult khsxSetBlockSolveTiers(KhsSolver *solver, uint32_t quads, uint32_t singles, uint32_t doubles,
                                          uint32_t blocks_per_sm);
 

@@ -702,29 +702,31 @@ KHS_HD V rotation_vector(const M &r)
 // ---- correctly rounded reciprocal on the integer pipes -----------------
 //
 // 1/x rounded to nearest, computed without FP64 instructions: on GB300 one
-// FP64 warp instruction occupies a sub-partition's pipe for ~64 cycles, and
-// the block solve's pivot warp is bound by its FP64 instruction count.
+// FP64 warp instruction occupies a sub-partition's pipe for ~64 cycles, and a
+// reciprocal is on the chain of every pivot step of the block solve.
 // For x = (-1)^s * M * 2^(E-1075) with M the 53-bit significand,
-// 1/x = (-1)^s * (2^105 / M) * 2^(970-E).  T = 2^105 / M lies in
-// (2^52, 2^53]:
-// * seed: an FP32 reciprocal of the top 24 bits of M, scaled to T0 ~ T
-//   (relative error below 2^-21);
-// * one residual step of order three: e = (2^105 - T0 M) / 2^105 in 64-bit
-//   fixed point, T1 = T0 (1 + e + e^2), error of order e^3 plus truncation
-//   (a few units);
-// * exact remainder R = 2^105 - T1 M (the low 64 bits suffice: |R| < 2^63)
-//   brings T1 to floor(T) with 0 <= R < M; the nearest integer is floor(T)
-//   + (2R > M) (no ties: M > 1 is odd or a power of two);
-// * reciprocals below the normal range (|x| >= 2^1022) are rounded from
-//   floor(T) and R to nearest-even.
-// The result equals the IEEE division 1.0 / x for every finite nonzero x
-// (checked bit for bit against __drcp_rn on 2^31 values on GB300 and
-// against 1.0 / x on the host, tests/native/test_recip.cpp); zero,
-// subnormal and non-finite inputs give an unspecified finite bit pattern
-// (the block solve fails such pivots before using the result).
+// 1/x = (-1)^s * T * 2^(970-E) with T = 2^105 / M in (2^52, 2^53]:
+// * seed: an FP32 reciprocal of the top 24 bits of M as the integer
+//   t ~ 2^23 * 2^52 / M, so T0 = 2^30 t; its relative error e = 1 - T0 / T
+//   is below 2^-20 (one ulp of the seed, the bits of M cut off, the rounding
+//   of t, and three further ulps of the seed to spare);
+// * residual: d = 2^75 - t M = 2^75 e, exact in 64 bits modulo 2^64 (2^75
+//   vanishes, |d| < 2^55), so one 24 x 53 bit product;
+// * Q = T0 (1 + e + e^2), rounded to an integer: e carried to 2^-62, e^2
+//   from the top 27 bits of d; with the cubic term left out the sum is within
+//   0.01 of T before the rounding, so Q is the nearest integer or next to it;
+// * the remainder R = 2^105 - Q M (exact modulo 2^64, |R| < 2^53) moves Q by
+//   one where |R| > M / 2.  No ties: M is odd times a power of two and T
+//   has more bits than a midpoint, or M = 2^52 and R = 0.
+// The steps are chosen for latency: 156 cycles of dependent instructions
+// (the FP64 reciprocal takes 352, the 128-bit form this replaces 382).  Reciprocals below the normal range (|x| >= 2^1022) are rounded from
+// floor(T) and its remainder to nearest-even on a branch of their own.
+// The result equals the IEEE division 1.0 / x for every finite normal x
+// (against 1.0 / x on the host, tests/native/test_recip.cpp); zero,
+// subnormal and non-finite inputs give an unspecified bit pattern (the block
+// solve fails such pivots before using the result).
 #if defined(__CUDA_ARCH__)
-KHS_HD uint64_t umulhi64(uint64_t a, uint64_t b) { return __umul64hi(a, b); }
-KHS_HD int64_t smulhi64(int64_t a, int64_t b) { return __mul64hi(a, b); }
+KHS_HD int32_t smulhi32(int32_t a, int32_t b) { return __mulhi(a, b); }
 KHS_HD float recip_seed(float m)
 {
     float r;
@@ -736,8 +738,7 @@ KHS_HD double double_of(uint64_t b) { return __longlong_as_double((long long)b);
 KHS_HD uint32_t bits_of(float x) { return __float_as_uint(x); }
 KHS_HD float float_of(uint32_t b) { return __uint_as_float(b); }
 #else
-KHS_HD uint64_t umulhi64(uint64_t a, uint64_t b) { return uint64_t((unsigned __int128)a * b >> 64); }
-KHS_HD int64_t smulhi64(int64_t a, int64_t b) { return int64_t((__int128)a * b >> 64); }
+KHS_HD int32_t smulhi32(int32_t a, int32_t b) { return int32_t((int64_t(a) * b) >> 32); }
 // Host seed: the correctly rounded float reciprocal (tests may substitute a
 // perturbed one through KHS_RECIP_SEED_HOST).
 #ifndef KHS_RECIP_SEED_HOST
@@ -750,49 +751,56 @@ KHS_HD uint32_t bits_of(float x) { uint32_t b; std::memcpy(&b, &x, 4); return b;
 KHS_HD float float_of(uint32_t b) { float x; std::memcpy(&x, &b, 4); return x; }
 #endif
 
-KHS_HD double recip_rn(double x)
+// The reciprocal where it is normal too (2^-1022 <= |x| < 2^1022), without
+// a branch.  Q and nR: the rounded T and minus its remainder.
+KHS_HD double recip_normal(double x, uint64_t &Q, int64_t &nR)
 {
     const uint64_t b = bits_of(x);
-    const uint64_t sign = b & 0x8000000000000000ull;
+    const uint32_t hi = uint32_t(b >> 32), mlo = uint32_t(b);
+    const uint32_t E = (hi >> 20) & 0x7ff, mhi = (hi & 0xfffffu) | 0x100000u;
+    const uint64_t M = (uint64_t(mhi) << 32) | mlo, half = M >> 1;
+    const float seed = recip_seed(float_of((127u << 23) | ((hi << 3 | mlo >> 29) & 0x7fffffu)));
+    // 2^23 * seed as an integer: the bits of 1 + seed count it from those of 1.
+    const uint32_t t = bits_of(1.0f + seed) - 0x3f800000u;
+    // -d, and s = 2^62 (e + e^2) from it.
+    const uint64_t tm = uint64_t(t) * mlo;
+    const int64_t nd = int64_t((uint64_t(uint32_t(tm >> 32) + t * mhi) << 32) | uint32_t(tm));
+    const int32_t dh = int32_t(nd >> 28);
+    const int64_t s = int64_t(smulhi32(dh, dh)) - (nd >> 13);
+    // Q = round(2^30 t + t s / 2^32), the low and high words of s apart.
+    const uint64_t low = uint64_t(t) * uint32_t(s) + 0x80000000u;
+    Q = (uint64_t(t) << 30) + uint64_t(int64_t(int32_t(t)) * int32_t(s >> 32)) + (low >> 32);
+    nR = int64_t(Q * M);
+    // Q counts its implicit bit into the exponent field (Q = 2^53 as well).
+    const uint64_t out = (b & 0x8000000000000000ull) | ((uint64_t(2044 - E) << 52) + Q);
+    const uint64_t above = out + 1, below = out - 1;
+    return double_of(nR < -int64_t(half) ? above : (nR > int64_t(half) ? below : out));
+}
+KHS_HD double recip_normal(double x)
+{
+    uint64_t Q;
+    int64_t nR;
+    return recip_normal(x, Q, nR);
+}
+
+KHS_HD double recip_rn(double x)
+{
+    uint64_t F;
+    int64_t nR;
+    const double normal = recip_normal(x, F, nR);
+    const uint64_t b = bits_of(x);
     const int E = int((b >> 52) & 0x7ff);
-    const uint64_t M = (b & 0xfffffffffffffull) | (1ull << 52);
-    const uint32_t rb = bits_of(recip_seed(float_of((127u << 23) | uint32_t((M >> 29) & 0x7fffff))));
-    const int er = int((rb >> 23) & 0xff) - 127;  // the seed lies in (0.5, 1]: -1 or 0
-    const uint64_t T0 = uint64_t((rb & 0x7fffff) | 0x800000) << (30 + er);
-    const uint64_t Plo = T0 * M, Phi = umulhi64(T0, M);
-    const uint64_t Rlo = 0 - Plo;
-    const uint64_t Rhi = (1ull << 41) - Phi - uint64_t(Plo != 0);
-    const int64_t e = int64_t((Rhi << 23) | (Rlo >> 41));  // (2^105 - T0 M) / 2^41
-    const uint64_t ae = e < 0 ? uint64_t(-e) : uint64_t(e);
-    const int64_t s = e + int64_t(umulhi64(ae, ae));
-    uint64_t T1 = T0 + uint64_t(smulhi64(int64_t(T0), s));
-    int64_t R = int64_t(0 - T1 * M);
-    for (int k = 0; k < 2; ++k) {
-        const bool low = R < 0;
-        T1 -= uint64_t(low);
-        R += low ? int64_t(M) : 0;
-    }
-    for (int k = 0; k < 2; ++k) {
-        const bool high = R >= int64_t(M);
-        T1 += uint64_t(high);
-        R -= high ? int64_t(M) : 0;
-    }
-    int bexp = 2045 - E;
-    uint64_t out;
-    if (bexp >= 1) {
-        uint64_t Q = T1 + uint64_t(2 * uint64_t(R) > M);
-        const bool carry = (Q >> 53) != 0;
-        Q = carry ? Q >> 1 : Q;
-        bexp += int(carry);
-        out = sign | (uint64_t(bexp) << 52) | (Q & 0xfffffffffffffull);
-    } else {
-        const int k = 1 - bexp < 63 ? 1 - bexp : 63;
-        const uint64_t mant = T1 >> k;
-        const uint64_t dropped = T1 & ((1ull << k) - 1), half = 1ull << (k - 1);
-        const bool up = dropped > half || (dropped == half && (R > 0 || (mant & 1)));
-        out = sign | (mant + uint64_t(up));
-    }
-    return double_of(out);
+    if (E < 2045) return normal;
+    // floor(T) and the remainder below M, then the subnormal's bits.
+    const int64_t M = int64_t((b & 0xfffffffffffffull) | (1ull << 52));
+    int64_t R = -nR;
+    if (R < 0) { --F; R += M; }
+    if (R >= M) { ++F; R -= M; }
+    const int k = E - 2044;
+    const uint64_t mant = F >> k;
+    const uint64_t dropped = F & ((1ull << k) - 1), mid = 1ull << (k - 1);
+    const bool up = dropped > mid || (dropped == mid && (R > 0 || (mant & 1)));
+    return double_of((b & 0x8000000000000000ull) | (mant + uint64_t(up)));
 }
 
 }  // namespace dm

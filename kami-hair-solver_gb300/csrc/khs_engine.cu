@@ -26,8 +26,8 @@
 //                 FP32 survivor), k_contact_select], k_elem_eval, k_node_sum
 //                 (thread per block entry), k_reduce_eval (both levels: the
 //                 last block to finish reduces the partials)
-//   direction     k_block_solve_aug<H> / k_block_solve_hybrid (persistent
-//                 warps, strand groups from a longest-first queue),
+//   direction     k_block_solve (blocks of one warp, a strand or five at a
+//                 time from a longest-first queue),
 //                 [float-float form: k_ff_factor, k_ff_residual, k_ff_correct],
 //                 k_steepest, k_scale, k_reduce_dir, k_final_dir
 //   CCD           k_ccd (plain), k_ccd_collect + k_ccd_pairs (mixed)
@@ -40,6 +40,7 @@
 #include "khs_engine.hpp"
 #include "khs_device_math.cuh"
 #include "khs_ff.cuh"
+#include "khs_block_solve.cuh"
 
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -183,6 +184,7 @@ struct View {
     uint32_t *near_list;  // elements with cached leaves, one warp each in k_contact_near
     uint8_t *surv_n;
     double *surv_res;
+    const uint32_t *solve_items;  // work items of the block solve, at most one per strand
     const uint32_t *besc, *bfirst, *bcount, *border, *bleaves;
     const int32_t *bparent;
     const uint32_t *bleft, *bright;
@@ -1643,743 +1645,24 @@ __global__ void __launch_bounds__(kBlock) k_reduce_eval(View d, int gradient)
 // the solve start first.
 constexpr int kSolveGroup = 6, kSolveGroupsPerWarp = 5;  // float-float kernels: 6 lanes per strand, 5 per warp
 
-// Block Thomas solve with Gauss-Jordan elimination on the augmented block
-// [B_n | U_n | rhs_n]: the elimination leaves C_n = B_n^-1 U_n and
-// d'_n = B_n^-1 rhs_n in place of U_n and rhs_n (the reference forms
-// B_n^-1 first and multiplies; the operations per result entry differ in
-// order only).  Finished pivot columns are not updated.  A group of 6 H lanes
-// owns one strand: lane (r, h) holds row r, columns [6h/H, 6(h+1)/H) of B_n
-// and U_n; every lane of row r holds rhs_n[r].  H = 1 puts 5 strands in a
-// warp, H = 2 puts 2 strands in a warp and halves the instructions on each
-// strand's sequential chain, H = 3 gives one strand 18 lanes.  Every entry is computed by the same sequence
-// of operations in both layouts, so the results are identical bit for bit
-// and the launch tuner may pick either.
-template<int H> struct AugLayout {
-    static constexpr int kCols = 6 / H;              // columns per lane
-    static constexpr int kLanes = 6 * H;             // lanes per strand
-    static constexpr int kStrands = 32 / kLanes;     // strands per warp
-};
+// The work items of the solve (Engine::plan_block_solve): places in the
+// solve order, marked where the strand has a warp of its own, else the first
+// of five; longest expected time first.  Blocks of one warp take them from a
+// queue, so the block scheduler spreads few items over as many SMs.
+constexpr uint32_t kSolveAlone = 0x80000000u;
+constexpr uint32_t kSolveByRule = 0xffffffffu;  // plan_block_solve chooses the split
 
-// Group g of the strands in solve order [first, end) (end 0: to the last).
-template<int H> __device__ __forceinline__ void solve_group_aug(const View &d, uint32_t g, uint32_t first = 0,
-                                                                uint32_t end = 0)
+__global__ void __launch_bounds__(32) k_block_solve(View d, uint32_t items)
 {
-    using L = AugLayout<H>;
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const int grp = lane / L::kLanes, gl = lane % L::kLanes, r = gl % 6, h = gl / 6;
-    const int base = grp * L::kLanes;
-    const int c0 = h * L::kCols;  // first column of this lane
-    const uint32_t k = first + g * L::kStrands + uint32_t(grp);
-    const bool member = grp < L::kStrands && k < (end ? end : d.S);
-    uint32_t begin = 0, len = 0;
-    if (member) {
-        const uint32_t s = d.sorder[k];
-        begin = d.sfirst[s] + d.sfixed[s];
-        const uint32_t end = d.sfirst[s] + d.scount[s];
-        len = end > begin ? end - begin : 0;
-    }
-    uint32_t maxlen = len;
-    for (int o = 16; o > 0; o >>= 1) maxlen = max(maxlen, __shfl_xor_sync(FULL, maxlen, o));
-    double nd[L::kCols], nu[L::kCols], nuc[6], ng = 0.0;
-    auto fetch = [&](uint32_t t) {
-        const bool on = t < len;
-        const size_t n = begin + t;
-#pragma unroll
-        for (int j = 0; j < L::kCols; ++j) nd[j] = on ? d.diag[36 * n + 6 * r + c0 + j] : 0.0;
-        ng = on ? d.grad[6 * n + r] : 0.0;
-        const bool up = on && t + 1 < len;
-#pragma unroll
-        for (int j = 0; j < L::kCols; ++j) nu[j] = up ? d.upper[36 * n + 6 * r + c0 + j] : 0.0;
-#pragma unroll
-        for (int q = 0; q < 6; ++q) nuc[q] = (on && t > 0) ? d.upper[36 * (n - 1) + 6 * q + r] : 0.0;
-    };
-    fetch(0);
-    double Cprev[L::kCols], dprev = 0.0;
-#pragma unroll
-    for (int j = 0; j < L::kCols; ++j) Cprev[j] = 0.0;
-    bool failed = false;
-    for (uint32_t t = 0; t < maxlen; ++t) {
-        const bool on = t < len && !failed;
-        const size_t n = begin + t;
-        double a[L::kCols], u[L::kCols], ucol[6], rhs = -ng;
-#pragma unroll
-        for (int j = 0; j < L::kCols; ++j) { a[j] = nd[j]; u[j] = nu[j]; }
-#pragma unroll
-        for (int q = 0; q < 6; ++q) ucol[q] = nuc[q];
-        if (t + 1 < maxlen) fetch(t + 1);
-        if (t > 0) {
-            // B = D - U_{n-1}^T C_{n-1}, rhs = -g - U_{n-1}^T d'_{n-1}
-#pragma unroll
-            for (int q = 0; q < 6; ++q) {
-#pragma unroll
-                for (int j = 0; j < L::kCols; ++j) a[j] = __fma_rn(-ucol[q], __shfl_sync(FULL, Cprev[j], base + 6 * h + q), a[j]);
-                rhs = __fma_rn(-ucol[q], __shfl_sync(FULL, dprev, base + q), rhs);
-            }
-        }
-        // Relative diagonal shift max(1e-12 max|b_ii|, 1e-24).
-        double diag_r = 0.0;
-#pragma unroll
-        for (int j = 0; j < L::kCols; ++j) if (c0 + j == r) diag_r = a[j];
-        unsigned long long smax = 0ull;
-#pragma unroll
-        for (int q = 0; q < 6; ++q) {
-            const int owner = base + 6 * (q / L::kCols) + q;
-            const unsigned long long b = (unsigned long long)__double_as_longlong(__shfl_sync(FULL, diag_r, owner)) & 0x7fffffffffffffffull;
-            smax = b > smax ? b : smax;
-        }
-        const double shift = fmax(__dmul_rn(1.0e-12, __longlong_as_double((long long)smax)), 1.0e-24);
-#pragma unroll
-        for (int j = 0; j < L::kCols; ++j) if (c0 + j == r) a[j] = __dadd_rn(a[j], shift);
-        // Gauss-Jordan with the pivot rows left unscaled: row r is divided
-        // by its pivot (the value at column r when it became the pivot row)
-        // once at the end, so each column costs one reciprocal, one product
-        // and one fused multiply-add per live entry.
-        bool ok = true;
-        double ipiv = 1.0;
-#pragma unroll
-        for (int col = 0; col < 6; ++col) {
-            const int hc = col / L::kCols, jc = col % L::kCols;
-            const int owner_half = base + 6 * hc;
-            double acol = 0.0;
-#pragma unroll
-            for (int j = 0; j < L::kCols; ++j) if (j == jc && h == hc) acol = a[j];
-            const unsigned long long mb = (unsigned long long)__double_as_longlong(acol) & 0x7fffffffffffffffull;
-            int pivot = col;
-            unsigned long long best = __shfl_sync(FULL, mb, owner_half + col);
-#pragma unroll
-            for (int row = col + 1; row < 6; ++row) {
-                const unsigned long long vrow = __shfl_sync(FULL, mb, owner_half + row);
-                if (vrow > best) { best = vrow; pivot = row; }
-            }
-            // best < 1e-30 or not finite (exponent all ones) => failure.
-            if (best < 0x39b4484bfeebc2a0ull || best >= 0x7ff0000000000000ull) ok = false;
-            const int partner = r == col ? pivot : (r == pivot ? col : r);
-            const int src = base + 6 * h + partner;
-#pragma unroll
-            for (int j = 0; j < L::kCols; ++j) {
-                a[j] = __shfl_sync(FULL, a[j], src);
-                u[j] = __shfl_sync(FULL, u[j], src);
-            }
-            rhs = __shfl_sync(FULL, rhs, src);
-            acol = 0.0;
-#pragma unroll
-            for (int j = 0; j < L::kCols; ++j) if (j == jc && h == hc) acol = a[j];
-            const double ip = __drcp_rn(__shfl_sync(FULL, acol, owner_half + col));
-            const double fp = __dmul_rn(__shfl_sync(FULL, acol, owner_half + r), ip);
-            if (r == col) ipiv = ip;
-            const int prow = base + 6 * h + col;
-#pragma unroll
-            for (int j = 0; j < L::kCols; ++j) {
-                if (L::kCols * (H - 1) + j <= col) continue;  // finished in every lane
-                const double x = __shfl_sync(FULL, a[j], prow);
-                a[j] = (r == col) ? a[j] : __fma_rn(-fp, x, a[j]);
-            }
-#pragma unroll
-            for (int j = 0; j < L::kCols; ++j) {
-                const double x = __shfl_sync(FULL, u[j], prow);
-                u[j] = (r == col) ? u[j] : __fma_rn(-fp, x, u[j]);
-            }
-            const double xr = __shfl_sync(FULL, rhs, prow);
-            rhs = (r == col) ? rhs : __fma_rn(-fp, xr, rhs);
-        }
-#pragma unroll
-        for (int j = 0; j < L::kCols; ++j) u[j] = __dmul_rn(u[j], ipiv);
-        rhs = __dmul_rn(rhs, ipiv);
-        if (on && !ok) {
-            failed = true;
-            if (gl == 0) atomicExch(&d.sc->solve_failed, 1);
-        }
-        // u now holds row r of C_n (zero at the strand tip), rhs = d'_n[r].
-#pragma unroll
-        for (int j = 0; j < L::kCols; ++j) Cprev[j] = u[j];
-        dprev = rhs;
-        if (on && !failed) {
-#pragma unroll
-            for (int j = 0; j < L::kCols; ++j) d.cprime[36 * n + 6 * r + c0 + j] = u[j];
-            if (h == 0) d.dprime[6 * n + r] = rhs;
-        }
-    }
-    // Back substitution d_n = d'_n - C_n d_{n+1} (full C row in every lane).
-    double next = 0.0;
-    double pc[6], pd = 0.0;
-    auto fetch_back = [&](uint32_t t) {
-        const bool on = t < len && !failed;
-        const size_t n = begin + t;
-        pd = on ? d.dprime[6 * n + r] : 0.0;
-#pragma unroll
-        for (int q = 0; q < 6; ++q) pc[q] = on ? d.cprime[36 * n + 6 * r + q] : 0.0;
-    };
-    if (maxlen) fetch_back(maxlen - 1);
-    for (uint32_t t = maxlen; t-- > 0;) {
-        const bool on = t < len && !failed;
-        const size_t n = begin + t;
-        double value = pd, crow[6];
-#pragma unroll
-        for (int q = 0; q < 6; ++q) crow[q] = pc[q];
-        if (t > 0) fetch_back(t - 1);
-        const bool coupled = on && t + 1 < len;
-#pragma unroll
-        for (int q = 0; q < 6; ++q) {
-            const double dq = __shfl_sync(FULL, next, base + q);
-            if (coupled) value = __fma_rn(-crow[q], dq, value);
-        }
-        if (on && h == 0) d.dir[6 * n + r] = value;
-        next = on ? value : 0.0;
-    }
-}
-
-// Hybrid schedule: the `long_strands` longest strands one per warp with
-// 18 lanes each (the shortest chain per node), then the rest five per warp
-// with 6 lanes each (the fewest instructions per node overall).  Both
-// layouts compute every entry identically, so the split point does not
-// change the result.
-__global__ void __launch_bounds__(128) k_block_solve_hybrid(View d, uint32_t long_strands)
-{
-    const uint32_t rest = d.S > long_strands ? d.S - long_strands : 0;
-    const uint32_t groups = long_strands + (rest + AugLayout<1>::kStrands - 1) / AugLayout<1>::kStrands;
+    __shared__ __align__(16) BackRing ring;
     for (;;) {
         uint32_t g = 0;
-        if ((threadIdx.x & 31) == 0) g = atomicAdd(&d.sc->solve_next, 1u);
+        if (threadIdx.x == 0) g = atomicAdd(&d.sc->solve_next, 1u);
         g = __shfl_sync(0xffffffffu, g, 0);
-        if (g >= groups) break;
-        if (g < long_strands) solve_group_aug<3>(d, g);
-        else solve_group_aug<1>(d, g - long_strands, long_strands);
-    }
-}
-
-// ---- long strands on a pair of warps ------------------------------------
-//
-// On GB300 one FP64 warp instruction holds a sub-partition's FP64 pipe for
-// about 64 cycles whatever the number of active lanes, so a strand solved by
-// one warp is bound by the FP64 instructions of its per-node chain (about 110
-// per node with 18 lanes).  Here the longest strands are solved by two warps
-// of one block, which the SM places on two sub-partitions:
-// * the B warp holds the Schur complement B_n (lane (r, h): row r, columns
-//   2h, 2h+1), adds the relative shift and runs the six pivot steps --
-//   pivot search, row swap, pivot reciprocal, row factors, update of the
-//   remaining columns -- and publishes each step's pivot row, reciprocal
-//   and row factors in shared memory;
-// * the U warp holds [U_n | rhs_n] in the same lane layout, applies each
-//   published step to it one step behind, scales the rows, stores C_n and
-//   d'_n, and forms the next Schur complement B_{n+1} = D_{n+1} - U_n^T C_n
-//   and right-hand side, which it hands to the B warp; it also runs the back
-//   substitution.
-// Every entry goes through the same operations in the same order as in
-// solve_group_aug<3>, so the directions are identical bit for bit.  The two
-// warps meet at a named barrier (bar.sync, 64 threads) once per pivot step
-// and once per node; both execute the same number of barriers by
-// construction (same strand length, six steps per node, no early exit).
-struct PairShared {
-    double B[36];      // B_n, row-major, from the U warp to the B warp
-    double fp[2][6];   // row factors a[r][col] * (1 / pivot) of a step (double-buffered by step parity)
-    double ip[2];      // the step's pivot reciprocal
-    int pivot[2];      // the step's pivot row
-    int ok[2];         // no pivot failure in this node up to and including the step
-    uint32_t item;     // work item, from the B warp to the U warp
-};
-
-__device__ __forceinline__ void pair_barrier(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
-
-__device__ __forceinline__ void pair_strand_range(const View &d, uint32_t k, uint32_t &begin, uint32_t &len)
-{
-    const uint32_t s = d.sorder[k];
-    begin = d.sfirst[s] + d.sfixed[s];
-    const uint32_t end = d.sfirst[s] + d.scount[s];
-    len = end > begin ? end - begin : 0;
-}
-
-// B warp of a pair (see above): pivot steps on the Schur complements.
-__device__ void solve_pair_b(const View &d, uint32_t k, PairShared &sh, int bar)
-{
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const int gl = lane < 18 ? lane : lane - 18;  // lanes 18-31 shadow lanes 0-13 and write nothing
-    const int r = gl % 6, h = gl / 6, c0 = 2 * h;
-    uint32_t begin, len;
-    pair_strand_range(d, k, begin, len);
-    for (uint32_t t = 0; t < len; ++t) {
-        pair_barrier(bar);  // B_t is in shared memory
-        double a[2] = {sh.B[6 * r + c0], sh.B[6 * r + c0 + 1]};
-        double diag_r = 0.0;
-#pragma unroll
-        for (int j = 0; j < 2; ++j) if (c0 + j == r) diag_r = a[j];
-        unsigned long long smax = 0ull;
-#pragma unroll
-        for (int q = 0; q < 6; ++q) {
-            const unsigned long long b = (unsigned long long)__double_as_longlong(__shfl_sync(FULL, diag_r, 6 * (q / 2) + q)) &
-                                         0x7fffffffffffffffull;
-            smax = b > smax ? b : smax;
-        }
-        const double shift = fmax(__dmul_rn(1.0e-12, __longlong_as_double((long long)smax)), 1.0e-24);
-#pragma unroll
-        for (int j = 0; j < 2; ++j) if (c0 + j == r) a[j] = __dadd_rn(a[j], shift);
-        bool ok = true;
-#pragma unroll
-        for (int col = 0; col < 6; ++col) {
-            const int hc = col / 2, jc = col % 2, owner_half = 6 * hc;
-            double acol = 0.0;
-#pragma unroll
-            for (int j = 0; j < 2; ++j) if (j == jc && h == hc) acol = a[j];
-            const unsigned long long mb = (unsigned long long)__double_as_longlong(acol) & 0x7fffffffffffffffull;
-            int pivot = col;
-            unsigned long long best = __shfl_sync(FULL, mb, owner_half + col);
-#pragma unroll
-            for (int row = col + 1; row < 6; ++row) {
-                const unsigned long long vrow = __shfl_sync(FULL, mb, owner_half + row);
-                if (vrow > best) { best = vrow; pivot = row; }
-            }
-            if (best < 0x39b4484bfeebc2a0ull || best >= 0x7ff0000000000000ull) ok = false;
-            const int partner = r == col ? pivot : (r == pivot ? col : r);
-#pragma unroll
-            for (int j = 0; j < 2; ++j) a[j] = __shfl_sync(FULL, a[j], 6 * h + partner);
-            acol = 0.0;
-#pragma unroll
-            for (int j = 0; j < 2; ++j) if (j == jc && h == hc) acol = a[j];
-            const double ip = __drcp_rn(__shfl_sync(FULL, acol, owner_half + col));
-            const double fp = __dmul_rn(__shfl_sync(FULL, acol, owner_half + r), ip);
-            const int prow = 6 * h + col;
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                if (2 * 2 + j <= col) continue;  // finished in every lane
-                const double x = __shfl_sync(FULL, a[j], prow);
-                a[j] = (r == col) ? a[j] : __fma_rn(-fp, x, a[j]);
-            }
-            const int slot = col & 1;
-            if (lane < 6) sh.fp[slot][lane] = fp;
-            if (lane == 0) {
-                sh.ip[slot] = ip;
-                sh.pivot[slot] = pivot;
-                sh.ok[slot] = ok ? 1 : 0;
-            }
-            pair_barrier(bar);  // step published
-        }
-    }
-}
-
-// U warp of a pair (see above): the published steps applied to [U_n | rhs_n],
-// the next Schur complement, and the back substitution.
-__device__ void solve_pair_u(const View &d, uint32_t k, PairShared &sh, int bar)
-{
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const int gl = lane < 18 ? lane : lane - 18;
-    const int r = gl % 6, h = gl / 6, c0 = 2 * h;
-    const bool writer = lane < 18;
-    uint32_t begin, len;
-    pair_strand_range(d, k, begin, len);
-    double nd[2], nu[2], nuc[6], ng = 0.0;
-    auto fetch = [&](uint32_t t) {
-        const bool on = t < len;
-        const size_t n = begin + t;
-#pragma unroll
-        for (int j = 0; j < 2; ++j) nd[j] = on ? d.diag[36 * n + 6 * r + c0 + j] : 0.0;
-        ng = on ? d.grad[6 * n + r] : 0.0;
-        const bool up = on && t + 1 < len;
-#pragma unroll
-        for (int j = 0; j < 2; ++j) nu[j] = up ? d.upper[36 * n + 6 * r + c0 + j] : 0.0;
-#pragma unroll
-        for (int q = 0; q < 6; ++q) nuc[q] = (on && t > 0) ? d.upper[36 * (n - 1) + 6 * q + r] : 0.0;
-    };
-    fetch(0);
-    double Cprev[2] = {0.0, 0.0}, dprev = 0.0;
-    bool failed = false;
-    for (uint32_t t = 0; t < len; ++t) {
-        const bool on = !failed;
-        const size_t n = begin + t;
-        double a[2] = {nd[0], nd[1]}, u[2] = {nu[0], nu[1]}, ucol[6], rhs = -ng;
-#pragma unroll
-        for (int q = 0; q < 6; ++q) ucol[q] = nuc[q];
-        if (t + 1 < len) fetch(t + 1);
-        if (t > 0) {
-#pragma unroll
-            for (int q = 0; q < 6; ++q) {
-#pragma unroll
-                for (int j = 0; j < 2; ++j) a[j] = __fma_rn(-ucol[q], __shfl_sync(FULL, Cprev[j], 6 * h + q), a[j]);
-                rhs = __fma_rn(-ucol[q], __shfl_sync(FULL, dprev, q), rhs);
-            }
-        }
-        if (writer) {
-            sh.B[6 * r + c0] = a[0];
-            sh.B[6 * r + c0 + 1] = a[1];
-        }
-        pair_barrier(bar);  // hand B_t over
-        double ipiv = 1.0;
-        bool ok = true;
-#pragma unroll
-        for (int col = 0; col < 6; ++col) {
-            pair_barrier(bar);  // step published
-            const int slot = col & 1;
-            const int pivot = sh.pivot[slot];
-            const double fp = sh.fp[slot][r], ip = sh.ip[slot];
-            ok = sh.ok[slot] != 0;
-            const int partner = r == col ? pivot : (r == pivot ? col : r);
-            const int src = 6 * h + partner;
-#pragma unroll
-            for (int j = 0; j < 2; ++j) u[j] = __shfl_sync(FULL, u[j], src);
-            rhs = __shfl_sync(FULL, rhs, src);
-            if (r == col) ipiv = ip;
-            const int prow = 6 * h + col;
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const double x = __shfl_sync(FULL, u[j], prow);
-                u[j] = (r == col) ? u[j] : __fma_rn(-fp, x, u[j]);
-            }
-            const double xr = __shfl_sync(FULL, rhs, prow);
-            rhs = (r == col) ? rhs : __fma_rn(-fp, xr, rhs);
-        }
-#pragma unroll
-        for (int j = 0; j < 2; ++j) u[j] = __dmul_rn(u[j], ipiv);
-        rhs = __dmul_rn(rhs, ipiv);
-        if (on && !ok) {
-            failed = true;
-            if (lane == 0) atomicExch(&d.sc->solve_failed, 1);
-        }
-        Cprev[0] = u[0];
-        Cprev[1] = u[1];
-        dprev = rhs;
-        if (on && !failed && writer) {
-#pragma unroll
-            for (int j = 0; j < 2; ++j) d.cprime[36 * n + 6 * r + c0 + j] = u[j];
-            if (h == 0) d.dprime[6 * n + r] = rhs;
-        }
-    }
-    __syncwarp();  // C_n and d'_n written by the other lanes of this warp
-    double next = 0.0, pc[6], pd = 0.0;
-    auto fetch_back = [&](uint32_t t) {
-        const bool on = t < len && !failed;
-        const size_t n = begin + t;
-        pd = on ? d.dprime[6 * n + r] : 0.0;
-#pragma unroll
-        for (int q = 0; q < 6; ++q) pc[q] = on ? d.cprime[36 * n + 6 * r + q] : 0.0;
-    };
-    if (len) fetch_back(len - 1);
-    for (uint32_t t = len; t-- > 0;) {
-        const bool on = !failed;
-        const size_t n = begin + t;
-        double value = pd, crow[6];
-#pragma unroll
-        for (int q = 0; q < 6; ++q) crow[q] = pc[q];
-        if (t > 0) fetch_back(t - 1);
-        const bool coupled = on && t + 1 < len;
-#pragma unroll
-        for (int q = 0; q < 6; ++q) {
-            const double dq = __shfl_sync(FULL, next, q);
-            if (coupled) value = __fma_rn(-crow[q], dq, value);
-        }
-        if (on && h == 0 && writer) d.dir[6 * n + r] = value;
-        next = on ? value : 0.0;
-    }
-}
-
-// Pair schedule: the `long_strands` longest strands each on a pair of
-// warps (solve_pair_b / solve_pair_u), then the rest five per warp.  Blocks
-// of four warps hold two pairs.  A pair takes work items together while
-// they are long strands; at the first item past them both warps go on alone
-// through the five-strand groups.
-__global__ void __launch_bounds__(128) k_block_solve_pairs(View d, uint32_t long_strands)
-{
-    __shared__ PairShared shared[2];
-    const int warp = threadIdx.x >> 5, pair = warp >> 1, role = warp & 1;
-    const int bar = 1 + pair;
-    PairShared &sh = shared[pair];
-    const uint32_t rest = d.S > long_strands ? d.S - long_strands : 0;
-    const uint32_t items = long_strands + (rest + AugLayout<1>::kStrands - 1) / AugLayout<1>::kStrands;
-    bool paired = true;
-    for (;;) {
-        uint32_t g = 0;
-        if (paired) {
-            if (role == 0 && (threadIdx.x & 31) == 0) sh.item = atomicAdd(&d.sc->solve_next, 1u);
-            pair_barrier(bar);
-            g = sh.item;
-            if (g < long_strands) {
-                if (role == 0) solve_pair_b(d, g, sh, bar);
-                else solve_pair_u(d, g, sh, bar);
-                continue;
-            }
-            paired = false;  // every later item is a five-strand group
-            if (role == 1) {
-                if ((threadIdx.x & 31) == 0) g = atomicAdd(&d.sc->solve_next, 1u);
-                g = __shfl_sync(0xffffffffu, g, 0);
-            }
-        } else {
-            if ((threadIdx.x & 31) == 0) g = atomicAdd(&d.sc->solve_next, 1u);
-            g = __shfl_sync(0xffffffffu, g, 0);
-        }
         if (g >= items) break;
-        solve_group_aug<1>(d, g - long_strands, long_strands);
-    }
-}
-
-// ---- long strands on four warps ------------------------------------------
-//
-// One warp issues at most one FP64 instruction per ~64 cycles, so a strand
-// is bound by the FP64 instructions its busiest warp issues per node (about
-// 84 with 18 lanes, 45 on the pair's pivot warp, plus its reciprocals).  A
-// quad spreads a strand over the four warps of a block (four sub-partitions):
-// * the pivot warp (warp 0) holds B_n in the 18-lane layout, adds the shift
-//   and runs the six pivot steps; the reciprocal of every candidate of the
-//   step's column is taken on the integer pipes (dm::recip_rn, equal to the
-//   FP64 division) while the pivot search runs, so the step's FP64 work is
-//   one product and the update of the remaining columns;
-// * column warps 1-3 hold columns 2(w-1), 2(w-1)+1 of [U_n], one entry per
-//   lane (slots 0-11), and the right-hand side (slots 12-17, used in warp
-//   3); they apply each published step one behind, scale the rows, store
-//   C_n and d'_n, and form their two columns of the next Schur complement
-//   B_{n+1} = D_{n+1} - U_n^T C_n (column c of B needs column c of C only)
-//   and, in warp 3, the next right-hand side; warp 1 then runs the back
-//   substitution.
-// Each entry goes through the same operations in the same order as in
-// solve_group_aug<3>, so the directions are identical bit for bit.  The four
-// warps meet at a named barrier (128 threads) once per pivot step and once
-// per node; all execute the same number by construction (same strand, six
-// steps per node, no early exit).  Lanes 18-31 shadow lanes 0-13 (full-warp
-// shuffles; they write nothing).
-struct QuadShared {
-    double B[36];      // B_n, row-major, from the column warps to the pivot warp
-    double fp[2][6];   // row factors of a step (double-buffered by step parity)
-    double ip[2];      // the step's pivot reciprocal
-    int pivot[2];      // the step's pivot row
-    int ok[2];         // no pivot failure in this node up to and including the step
-    uint32_t item[2];  // work item (double-buffered by fetch parity)
-};
-
-__device__ __forceinline__ void quad_barrier(int id) { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
-
-__device__ void solve_quad_pivot(const View &d, uint32_t k, QuadShared &sh, int bar)
-{
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const int gl = lane < 18 ? lane : lane - 18;
-    const int r = gl % 6, h = gl / 6, c0 = 2 * h;
-    uint32_t begin, len;
-    pair_strand_range(d, k, begin, len);
-    for (uint32_t t = 0; t < len; ++t) {
-        quad_barrier(bar);  // B_t is in shared memory
-        double a[2] = {sh.B[6 * r + c0], sh.B[6 * r + c0 + 1]};
-        double diag_r = 0.0;
-#pragma unroll
-        for (int j = 0; j < 2; ++j) if (c0 + j == r) diag_r = a[j];
-        unsigned long long smax = 0ull;
-#pragma unroll
-        for (int q = 0; q < 6; ++q) {
-            const unsigned long long b = (unsigned long long)__double_as_longlong(__shfl_sync(FULL, diag_r, 6 * (q / 2) + q)) &
-                                         0x7fffffffffffffffull;
-            smax = b > smax ? b : smax;
-        }
-        const double shift = fmax(__dmul_rn(1.0e-12, __longlong_as_double((long long)smax)), 1.0e-24);
-#pragma unroll
-        for (int j = 0; j < 2; ++j) if (c0 + j == r) a[j] = __dadd_rn(a[j], shift);
-        bool ok = true;
-#pragma unroll
-        for (int col = 0; col < 6; ++col) {
-            const int hc = col / 2, jc = col % 2, owner_half = 6 * hc;
-            double acol = 0.0;
-#pragma unroll
-            for (int j = 0; j < 2; ++j) if (j == jc && h == hc) acol = a[j];
-            // Every candidate's reciprocal, alongside the pivot search; the
-            // pivot's is the one the 18-lane layout takes after the swap.
-            const double rc = dm::recip_rn(acol);
-            const unsigned long long mb = (unsigned long long)__double_as_longlong(acol) & 0x7fffffffffffffffull;
-            int pivot = col;
-            unsigned long long best = __shfl_sync(FULL, mb, owner_half + col);
-#pragma unroll
-            for (int row = col + 1; row < 6; ++row) {
-                const unsigned long long vrow = __shfl_sync(FULL, mb, owner_half + row);
-                if (vrow > best) { best = vrow; pivot = row; }
-            }
-            if (best < 0x39b4484bfeebc2a0ull || best >= 0x7ff0000000000000ull) ok = false;
-            const double ip = __shfl_sync(FULL, rc, owner_half + pivot);
-            const int partner = r == col ? pivot : (r == pivot ? col : r);
-#pragma unroll
-            for (int j = 0; j < 2; ++j) a[j] = __shfl_sync(FULL, a[j], 6 * h + partner);
-            acol = 0.0;
-#pragma unroll
-            for (int j = 0; j < 2; ++j) if (j == jc && h == hc) acol = a[j];
-            const double fp = __dmul_rn(__shfl_sync(FULL, acol, owner_half + r), ip);
-            const int prow = 6 * h + col;
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                if (2 * 2 + j <= col) continue;  // finished in every lane
-                const double x = __shfl_sync(FULL, a[j], prow);
-                a[j] = (r == col) ? a[j] : __fma_rn(-fp, x, a[j]);
-            }
-            const int slot = col & 1;
-            if (lane < 6) sh.fp[slot][lane] = fp;
-            if (lane == 0) {
-                sh.ip[slot] = ip;
-                sh.pivot[slot] = pivot;
-                sh.ok[slot] = ok ? 1 : 0;
-            }
-            quad_barrier(bar);  // step published
-        }
-    }
-}
-
-__device__ void solve_quad_columns(const View &d, uint32_t k, QuadShared &sh, int bar, int w)
-{
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const int s = lane < 18 ? lane : lane - 18;
-    const int r = s % 6, jj = s / 6;                 // jj 0, 1: a column of U; 2: the right-hand side
-    const int c = 2 * (w - 1) + (jj < 2 ? jj : 0);
-    const bool writer = lane < 18;
-    uint32_t begin, len;
-    pair_strand_range(d, k, begin, len);
-    double nd = 0.0, nu = 0.0, nuc[6], ng = 0.0;
-    auto fetch = [&](uint32_t t) {
-        const bool on = t < len;
-        const size_t n = begin + t;
-        nd = on ? d.diag[36 * n + 6 * r + c] : 0.0;
-        ng = on ? d.grad[6 * n + r] : 0.0;
-        nu = (on && t + 1 < len) ? d.upper[36 * n + 6 * r + c] : 0.0;
-#pragma unroll
-        for (int q = 0; q < 6; ++q) nuc[q] = (on && t > 0) ? d.upper[36 * (n - 1) + 6 * q + r] : 0.0;
-    };
-    fetch(0);
-    double prev = 0.0;  // C_{t-1}[r][c] or d'_{t-1}[r]
-    bool failed = false;
-    for (uint32_t t = 0; t < len; ++t) {
-        const bool on = !failed;
-        const size_t n = begin + t;
-        double acc = jj < 2 ? nd : -ng, ucol[6];
-        const double u_next = nu;
-#pragma unroll
-        for (int q = 0; q < 6; ++q) ucol[q] = nuc[q];
-        if (t + 1 < len) fetch(t + 1);
-        if (t > 0) {
-            // B = D - U_{t-1}^T C_{t-1} (column c), rhs = -g - U_{t-1}^T d'_{t-1}
-#pragma unroll
-            for (int q = 0; q < 6; ++q) {
-                acc = __fma_rn(-ucol[q], __shfl_sync(FULL, prev, 6 * jj + q), acc);
-            }
-        }
-        if (writer && jj < 2) sh.B[6 * r + c] = acc;
-        double v = jj < 2 ? u_next : acc;
-        quad_barrier(bar);  // hand B_t over
-        double ipiv = 1.0;
-        bool ok = true;
-#pragma unroll
-        for (int col = 0; col < 6; ++col) {
-            quad_barrier(bar);  // step published
-            const int slot = col & 1;
-            const int pivot = sh.pivot[slot];
-            const double fp = sh.fp[slot][r], ip = sh.ip[slot];
-            ok = sh.ok[slot] != 0;
-            const int partner = r == col ? pivot : (r == pivot ? col : r);
-            v = __shfl_sync(FULL, v, 6 * jj + partner);
-            if (r == col) ipiv = ip;
-            const double x = __shfl_sync(FULL, v, 6 * jj + col);
-            v = (r == col) ? v : __fma_rn(-fp, x, v);
-        }
-        v = __dmul_rn(v, ipiv);
-        if (on && !ok) {
-            failed = true;
-            if (w == 1 && lane == 0) atomicExch(&d.sc->solve_failed, 1);
-        }
-        prev = v;
-        if (on && !failed && writer) {
-            if (jj < 2) d.cprime[36 * n + 6 * r + c] = v;
-            else if (w == 3) d.dprime[6 * n + r] = v;
-        }
-    }
-    // Back substitution d_n = d'_n - C_n d_{n+1} in warp 1, once the three
-    // column warps have stored C and d' (barrier bar + 1, 96 threads).
-    asm volatile("bar.sync %0, 96;" ::"r"(bar + 1) : "memory");
-    if (w != 1) return;
-    double next = 0.0, pc[6], pd = 0.0;
-    auto fetch_back = [&](uint32_t t) {
-        const bool on = t < len && !failed;
-        const size_t n = begin + t;
-        pd = on ? d.dprime[6 * n + r] : 0.0;
-#pragma unroll
-        for (int q = 0; q < 6; ++q) pc[q] = on ? d.cprime[36 * n + 6 * r + q] : 0.0;
-    };
-    if (len) fetch_back(len - 1);
-    for (uint32_t t = len; t-- > 0;) {
-        const bool on = !failed;
-        const size_t n = begin + t;
-        double value = pd, crow[6];
-#pragma unroll
-        for (int q = 0; q < 6; ++q) crow[q] = pc[q];
-        if (t > 0) fetch_back(t - 1);
-        const bool coupled = on && t + 1 < len;
-#pragma unroll
-        for (int q = 0; q < 6; ++q) {
-            const double dq = __shfl_sync(FULL, next, q);
-            if (coupled) value = __fma_rn(-crow[q], dq, value);
-        }
-        if (on && lane < 6) d.dir[6 * n + r] = value;
-        next = on ? value : 0.0;
-    }
-}
-
-// Tiered schedule over one longest-first queue: the `quads` longest strands
-// on a block of four warps each, the next `singles` one per warp (18 lanes),
-// the next `doubles` two per warp (12 lanes each), the rest five per warp.
-// A block takes queue items together while they are quads; at the first
-// item past them its warps go on alone.  Every tier computes each entry
-// with the same operations, so the split changes no result.
-// The tiers are inlined: as separate functions they would take the View by
-// reference, which places the kernel's parameter block in local memory.
-__device__ __forceinline__ void tier_quad(const View &d, uint32_t g, QuadShared &sh, int warp)
-{
-    if (warp == 0) solve_quad_pivot(d, g, sh, 1);
-    else solve_quad_columns(d, g, sh, 1, warp);
-}
-__device__ __forceinline__ void tier_single(const View &d, uint32_t g, uint32_t first) { solve_group_aug<3>(d, g, first); }
-__device__ __forceinline__ void tier_double(const View &d, uint32_t g, uint32_t first, uint32_t end)
-{
-    solve_group_aug<2>(d, g, first, end);
-}
-__device__ __forceinline__ void tier_five(const View &d, uint32_t g, uint32_t first) { solve_group_aug<1>(d, g, first); }
-
-__global__ void __launch_bounds__(128) k_block_solve_tiers(View d, uint32_t quads, uint32_t singles, uint32_t doubles)
-{
-    __shared__ QuadShared sh;
-    const int warp = threadIdx.x >> 5;
-    const uint32_t end1 = quads + singles, end2 = end1 + doubles;
-    const uint32_t i2 = end1 + (doubles + 1) / 2;  // first five-strand item
-    const uint32_t rest = d.S > end2 ? d.S - end2 : 0;
-    const uint32_t items = i2 + (rest + AugLayout<1>::kStrands - 1) / AugLayout<1>::kStrands;
-    bool together = quads > 0;
-    uint32_t parity = 0;
-    for (;;) {
-        uint32_t g = 0;
-        if (together) {
-            if (threadIdx.x == 0) sh.item[parity] = atomicAdd(&d.sc->solve_next, 1u);
-            quad_barrier(1);
-            g = sh.item[parity];
-            parity ^= 1u;
-            if (g < quads) {
-                tier_quad(d, g, sh, warp);
-                continue;
-            }
-            together = false;  // every later item is a one-warp item
-            if (warp != 0) {
-                if ((threadIdx.x & 31) == 0) g = atomicAdd(&d.sc->solve_next, 1u);
-                g = __shfl_sync(0xffffffffu, g, 0);
-            }
-        } else {
-            if ((threadIdx.x & 31) == 0) g = atomicAdd(&d.sc->solve_next, 1u);
-            g = __shfl_sync(0xffffffffu, g, 0);
-        }
-        if (g >= items) break;
-        if (g < end1) tier_single(d, g - quads, quads);
-        else if (g < i2) tier_double(d, g - end1, end1, end2);
-        else tier_five(d, g - i2, end2);
-    }
-}
-
-template<int H> __global__ void __launch_bounds__(128) k_block_solve_aug(View d)
-{
-    const uint32_t groups = (d.S + AugLayout<H>::kStrands - 1) / AugLayout<H>::kStrands;
-    for (;;) {
-        uint32_t g = 0;
-        if ((threadIdx.x & 31) == 0) g = atomicAdd(&d.sc->solve_next, 1u);
-        g = __shfl_sync(0xffffffffu, g, 0);
-        if (g >= groups) break;
-        solve_group_aug<H>(d, g);
+        const uint32_t item = d.solve_items[g];
+        if (item & kSolveAlone) solve_strand_warp(d, item & ~kSolveAlone, ring);
+        else solve_strands_five(d, item);
     }
 }
 
@@ -3214,7 +2497,8 @@ struct Engine::Impl {
     struct KernelStat { const char *name; uint64_t launches; double ms; };
     bool profiling = false;
     uint64_t launches = 0;
-    unsigned solve_blocks = 0;  // launch shape of the FP64 block solve (0 = not tuned yet)
+    // Launch shape of the FP64 block solve: work items, blocks of one warp.
+    unsigned solve_items = 0, solve_blocks = 0;
     // Rollback ring: q and v of the last ring_frame.size() animation frames,
     // slot k holding frame ring_frame[k] (-1 = empty), [slots][2][N][6] FP64.
     double *ring = nullptr;
@@ -3244,11 +2528,6 @@ struct Engine::Impl {
         out_frame.clear();
         out_next = 0;
     }
-    void (*solve_kernel)(View) = nullptr;
-    uint32_t solve_long = 0;  // > 0: k_block_solve_hybrid / k_block_solve_pairs with this many long strands
-    bool solve_pairs = false; // the long strands on warp pairs (k_block_solve_pairs)
-    bool solve_tiers = false; // k_block_solve_tiers with tier_quads / tier_singles / tier_doubles
-    uint32_t tier_quads = 0, tier_singles = 0, tier_doubles = 0;
     std::vector<uint32_t> sorted_len;  // free nodes per strand, in the solve order
     unsigned ff_blocks = 0;     // launch shape of the float-float kernels
     std::vector<KernelStat> kstats;
@@ -3372,7 +2651,7 @@ void Engine::initialize(const Model &m, const KhsSolverDesc &desc, const KhsHair
     bytes += 3 * padded<uint32_t>(N) + padded<double>(N);  // root bindings, node strand
     bytes += 3 * padded<uint32_t>(E) + padded<uint8_t>(E) + padded<double>(E) + 2 * padded<double>(3 * E);
     bytes += 3 * padded<double>(E) + 2 * padded<uint32_t>(E) + padded<uint8_t>(E);
-    bytes += 4 * padded<uint32_t>(S);
+    bytes += 5 * padded<uint32_t>(S);
     bytes += padded<uint32_t>(3 * T) + 5 * padded<double>(3 * Vn) + padded<float>(3 * Vn);
     bytes += 2 * padded<float>(3 * B) + padded<float4>(2 * B);
     const size_t pair_capacity = std::min<size_t>(std::max<size_t>(size_t(1) << 20, 8 * E), size_t(16) << 20);
@@ -3422,6 +2701,7 @@ void Engine::initialize(const Model &m, const KhsSolverDesc &desc, const KhsHair
     v.e_el = a.take<double>(E); v.e_co = a.take<double>(E); v.c_gap = a.take<double>(E);
     v.c_cand = a.take<uint32_t>(E); v.c_tri = a.take<uint32_t>(E); v.c_flags = a.take<uint8_t>(E);
     uint32_t *sf = a.take<uint32_t>(S), *sc = a.take<uint32_t>(S), *sx = a.take<uint32_t>(S), *so = a.take<uint32_t>(S);
+    v.solve_items = a.take<uint32_t>(S);
     uint32_t *tri = a.take<uint32_t>(3 * T);
     v.col_cur = a.take<double>(3 * Vn); v.col_old = a.take<double>(3 * Vn);
     v.col32 = a.take<float>(3 * Vn);
@@ -3551,6 +2831,7 @@ void Engine::initialize(const Model &m, const KhsSolverDesc &desc, const KhsHair
     max_rest_length_ = 0.0;
     for (double L : m.rest_length) max_rest_length_ = std::fmax(max_rest_length_, L);
     update_runtime(desc, material, m.mass, m.rotational_mass);
+    plan_block_solve(kSolveByRule, 0);
     I.sync();
     clear_failure();
     step_stats_ = {};
@@ -3819,180 +3100,103 @@ bool Engine::make_steepest()
     return limit_direction(I.mail_host->max_translation);
 }
 
-// Launch shape of the persistent FP64 block solve: the layout (H = 1: five
-// strands of 6 lanes per warp; H = 2: two strands of 12 lanes; H = 3: one
-// strand of 18 lanes) and 1-4
-// blocks of four warps per SM, chosen once by timing each on the first
-// system.  The choice does not change the result: both layouts compute every
-// entry with the same operations, and each strand is solved by one group.
-KhsResult Engine::set_block_solve_schedule(uint32_t strands_per_warp, uint32_t blocks_per_sm, uint32_t long_strands)
+// Work items of the FP64 block solve: the `alone` longest strands on a warp
+// each, the rest five to a warp, longest expected time first.  The split does
+// not change the result (k_block_solve).
+//
+// The rule's model, in cycles measured on GB300 (160-node strands on random
+// blocks): a node of a strand alone takes 4,950 with one warp on a
+// sub-partition and 6,400 beside a second one; a node of five strands 14,700
+// and 20,200; the machine is full at two warps on each of its 608
+// sub-partitions, where a node of either kind costs 3,200 and 2,020 of a
+// sub-partition's time.  The expected time of a split is its longest chain
+// or, if larger, the total work plus half of the shortest item (the uneven
+// end of the queue).  Against a sweep of the split on GB300 it picks the best
+// or is within 4% of it: 100 strands of 16-160 nodes all alone (384 us a
+// solve, all by fives 992); 2,000 all alone (491, 1,159); the body scene's
+// 6,757 strands of 8-200 nodes with a quarter alone (575, all alone 654, all
+// by fives 1,650; 831 with the timed shapes this replaces).
+void Engine::plan_block_solve(uint32_t alone, uint32_t blocks_per_sm)
 {
     Impl &I = *d_;
+    const std::vector<uint32_t> &len = I.sorted_len;
+    const uint32_t S = uint32_t(len.size());
+    int sms = 0;
+    KHS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, kDevice));
+    constexpr double kAlone[2] = {4950.0, 6400.0}, kFive[2] = {14700.0, 20200.0};
+    if (alone == kSolveByRule) {
+        std::vector<double> sum(S + 1, 0.0);
+        for (uint32_t k = 0; k < S; ++k) sum[k + 1] = sum[k] + len[k];
+        const double parts = 4.0 * sms;
+        double best = std::numeric_limits<double>::infinity();
+        for (uint32_t step = 0; step <= 20; ++step) {
+            const uint32_t w = uint32_t(uint64_t(S) * step / 20);
+            const double items = w + (S - w + kStrandsPerWarp - 1) / kStrandsPerWarp;
+            const double crowd = std::min(1.0, std::max(0.0, items / parts - 1.0));
+            auto node = [&](const double cost[2]) { return cost[0] + crowd * (cost[1] - cost[0]); };
+            double chain = 0.0, shortest = std::numeric_limits<double>::infinity();
+            if (w) { chain = len[0] * node(kAlone); shortest = len[w - 1] * kAlone[1]; }
+            if (w < S) {
+                chain = std::max(chain, len[w] * node(kFive));
+                shortest = std::min(shortest, len[w + (S - w - 1) / kStrandsPerWarp * kStrandsPerWarp] * kFive[1]);
+            }
+            const double work = (sum[w] * 3200.0 + (sum[S] - sum[w]) * 2020.0) / parts;
+            const double time = std::max(chain, items > 2.0 * parts ? work + 0.5 * shortest : 0.0);
+            if (time <= best) { best = time; alone = w; }
+        }
+    }
+    struct Item { double cost; uint32_t code; };
+    std::vector<Item> items;
+    for (uint32_t k = 0; k < alone; ++k) items.push_back({len[k] * kAlone[1], k | kSolveAlone});
+    for (uint32_t k = alone; k < S; k += kStrandsPerWarp) items.push_back({len[k] * kFive[1], k});
+    std::stable_sort(items.begin(), items.end(), [](const Item &a, const Item &b) { return a.cost > b.cost; });
+    std::vector<uint32_t> codes;
+    for (const Item &i : items) codes.push_back(i.code);
+    KHS_CUDA(cudaMemcpyAsync(const_cast<uint32_t *>(I.v.solve_items), codes.data(), codes.size() * 4, cudaMemcpyHostToDevice,
+                             I.stream));
+    I.sync();
+    I.solve_items = unsigned(items.size());
+    I.solve_blocks = std::min(I.solve_items, 4 * (blocks_per_sm ? blocks_per_sm : 2u) * unsigned(sms));
+    const unsigned ff_groups = unsigned((S + kSolveGroupsPerWarp - 1) / kSolveGroupsPerWarp);
+    I.ff_blocks = std::min(std::max(1u, (ff_groups + 3) / 4), 2u * unsigned(sms));
+}
+
+// 5: the long_strands longest on a warp each, the rest five to a warp; 2 and
+// 1: every strand on a warp of its own, or with long_strands as 5 does.
+KhsResult Engine::set_block_solve_schedule(uint32_t strands_per_warp, uint32_t blocks_per_sm, uint32_t long_strands)
+{
+    const uint32_t S = d_->v.S;
     if (strands_per_warp == 0) {
-        I.solve_blocks = 0; I.solve_kernel = nullptr; I.solve_long = 0; I.solve_pairs = false; I.solve_tiers = false;
+        plan_block_solve(kSolveByRule, 0);
         return KHS_OK;
     }
     if ((strands_per_warp != 5 && strands_per_warp != 2 && strands_per_warp != 1) || blocks_per_sm < 1 || blocks_per_sm > 8 ||
-        (long_strands && ((strands_per_warp != 5 && strands_per_warp != 1) || long_strands >= I.v.S)))
+        (long_strands && ((strands_per_warp != 5 && strands_per_warp != 1) || long_strands >= S)))
         return KHS_ERROR_INVALID_ARGUMENT;
-    int sms = 0;
-    KHS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, kDevice));
-    const unsigned groups = long_strands ? long_strands + unsigned((I.v.S - long_strands + 4) / 5)
-                                         : unsigned((I.v.S + strands_per_warp - 1) / strands_per_warp);
-    I.solve_kernel = long_strands ? nullptr
-                     : strands_per_warp == 5 ? k_block_solve_aug<1>
-                     : strands_per_warp == 2 ? k_block_solve_aug<2>
-                                             : k_block_solve_aug<3>;
-    I.solve_long = long_strands;
-    I.solve_pairs = long_strands && strands_per_warp == 1;
-    I.solve_tiers = false;
-    I.solve_blocks = std::min(std::max(1u, (groups + 3) / 4), blocks_per_sm * unsigned(sms));
-    const unsigned ff_groups = unsigned((I.v.S + kSolveGroupsPerWarp - 1) / kSolveGroupsPerWarp);
-    I.ff_blocks = std::min(std::max(1u, (ff_groups + 3) / 4), 2u * unsigned(sms));
+    plan_block_solve(strands_per_warp == 5 || long_strands ? long_strands : S, blocks_per_sm);
     return KHS_OK;
 }
 
-// Queue items of the tiered schedule: one per quad strand and per single,
-// one per two doubles, one per five of the rest.
-static unsigned tier_items(uint32_t S, uint32_t quads, uint32_t singles, uint32_t doubles)
-{
-    const uint32_t head = quads + singles + doubles;
-    return quads + singles + (doubles + 1) / 2 + (S > head ? (S - head + 4) / 5 : 0);
-}
-
-// Tiered launch shape (k_block_solve_tiers): the `quads` longest strands on
-// four warps each, the next `singles` on one warp of 18 lanes, the next
-// `doubles` two per warp, the rest five per warp; blocks_per_sm 1-8.  The
-// shape does not change the result.
+// The quads + singles + doubles longest strands on a warp each, the rest five
+// to a warp.
 KhsResult Engine::set_block_solve_tiers(uint32_t quads, uint32_t singles, uint32_t doubles, uint32_t blocks_per_sm)
 {
-    Impl &I = *d_;
-    if (blocks_per_sm < 1 || blocks_per_sm > 8 || uint64_t(quads) + singles + doubles > I.v.S)
+    if (blocks_per_sm < 1 || blocks_per_sm > 8 || uint64_t(quads) + singles + doubles > d_->v.S)
         return KHS_ERROR_INVALID_ARGUMENT;
-    int sms = 0;
-    KHS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, kDevice));
-    I.solve_kernel = nullptr;
-    I.solve_long = 0;
-    I.solve_pairs = false;
-    I.solve_tiers = true;
-    I.tier_quads = quads; I.tier_singles = singles; I.tier_doubles = doubles;
-    const unsigned items = tier_items(I.v.S, quads, singles, doubles);
-    I.solve_blocks = std::min(std::max(1u, (items + 3) / 4), blocks_per_sm * unsigned(sms));
-    const unsigned ff_groups = unsigned((I.v.S + kSolveGroupsPerWarp - 1) / kSolveGroupsPerWarp);
-    I.ff_blocks = std::min(std::max(1u, (ff_groups + 3) / 4), 2u * unsigned(sms));
+    plan_block_solve(quads + singles + doubles, blocks_per_sm);
     return KHS_OK;
-}
-
-void Engine::tune_block_solve()
-{
-    Impl &I = *d_;
-    int sms = 0;
-    KHS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, kDevice));
-    cudaEvent_t ev[2];
-    KHS_CUDA(cudaEventCreate(&ev[0]));
-    KHS_CUDA(cudaEventCreate(&ev[1]));
-    auto time_it = [&](void (*kernel)(View), unsigned blocks, uint32_t nlong, bool pairs = false,
-                       const uint32_t *tiers = nullptr) {
-        float best = 3.0e38f;
-        for (int rep = 0; rep < 2; ++rep) {
-            KHS_CUDA(cudaMemsetAsync(&I.v.sc->solve_next, 0, sizeof(uint32_t), I.stream));
-            KHS_CUDA(cudaEventRecord(ev[0], I.stream));
-            if (tiers) k_block_solve_tiers<<<blocks, 128, 0, I.stream>>>(I.v, tiers[0], tiers[1], tiers[2]);
-            else if (kernel) kernel<<<blocks, 128, 0, I.stream>>>(I.v);
-            else if (pairs) k_block_solve_pairs<<<blocks, 128, 0, I.stream>>>(I.v, nlong);
-            else k_block_solve_hybrid<<<blocks, 128, 0, I.stream>>>(I.v, nlong);
-            ++I.launches;
-            KHS_CUDA(cudaEventRecord(ev[1], I.stream));
-            KHS_CUDA(cudaEventSynchronize(ev[1]));
-            float ms = 0.0f;
-            KHS_CUDA(cudaEventElapsedTime(&ms, ev[0], ev[1]));
-            best = std::min(best, ms);
-        }
-        return best;
-    };
-    struct Candidate { void (*kernel)(View); unsigned strands_per_warp; };
-    const Candidate layouts[3] = {{k_block_solve_aug<1>, 5u}, {k_block_solve_aug<2>, 2u}, {k_block_solve_aug<3>, 1u}};
-    float best_ms = 3.0e38f;
-    for (const Candidate &c : layouts) {
-        const unsigned groups = unsigned((I.v.S + c.strands_per_warp - 1) / c.strands_per_warp);
-        const unsigned most = std::max(1u, (groups + 3) / 4);
-        for (unsigned per_sm = 1; per_sm <= 4; ++per_sm) {
-            const unsigned blocks = std::min(most, per_sm * unsigned(sms));
-            const float ms = time_it(c.kernel, blocks, 0);
-            if (ms < best_ms) {
-                best_ms = ms; I.solve_kernel = c.kernel; I.solve_blocks = blocks; I.solve_long = 0; I.solve_pairs = false;
-                I.solve_tiers = false;
-            }
-            if (blocks == most) break;
-        }
-    }
-    // Hybrid: the strands of at least `cut` free nodes one per warp (18
-    // lanes) or on a pair of warps, the rest five per warp.
-    uint32_t last_long = 0;
-    for (uint32_t cut : {160u, 128u, 96u, 64u, 48u}) {
-        const uint32_t nlong = uint32_t(std::count_if(I.sorted_len.begin(), I.sorted_len.end(),
-                                                       [&](uint32_t len) { return len >= cut; }));
-        if (nlong == 0 || nlong == last_long || nlong >= I.v.S) continue;
-        last_long = nlong;
-        const unsigned groups = nlong + unsigned((I.v.S - nlong + 4) / 5);
-        const unsigned most = std::max(1u, (groups + 3) / 4);
-        for (unsigned per_sm = 1; per_sm <= 3; ++per_sm) {
-            const unsigned blocks = std::min(most, per_sm * unsigned(sms));
-            for (bool pairs : {false, true}) {
-                const float ms = time_it(nullptr, blocks, nlong, pairs);
-                if (ms < best_ms) {
-                    best_ms = ms; I.solve_kernel = nullptr; I.solve_blocks = blocks; I.solve_long = nlong; I.solve_pairs = pairs;
-                    I.solve_tiers = false;
-                }
-            }
-            if (blocks == most) break;
-        }
-    }
-    // Tiered: quads for the longest ~0.5-2% of the strands, then singles,
-    // doubles and five per warp, two blocks per SM (its 255 registers per
-    // thread leave no room for a third).
-    for (uint32_t qd : {110u, 75u, 55u})
-        for (uint32_t sd : {70u, 35u, 25u})
-            for (uint32_t dd : {34u, 17u}) {
-                const uint32_t tiers[3] = {I.v.S / qd, I.v.S / sd, (I.v.S / dd) & ~1u};
-                if (tiers[0] == 0 || uint64_t(tiers[0]) + tiers[1] + tiers[2] >= I.v.S) continue;
-                const unsigned items = tier_items(I.v.S, tiers[0], tiers[1], tiers[2]);
-                const unsigned most = std::max(1u, (items + 3) / 4);
-                const unsigned blocks = std::min(most, 2u * unsigned(sms));
-                const float ms = time_it(nullptr, blocks, 0, false, tiers);
-                if (ms < best_ms) {
-                    best_ms = ms; I.solve_kernel = nullptr; I.solve_blocks = blocks; I.solve_long = 0;
-                    I.solve_pairs = false; I.solve_tiers = true;
-                    I.tier_quads = tiers[0]; I.tier_singles = tiers[1]; I.tier_doubles = tiers[2];
-                }
-            }
-    // Float-float kernels (5 strands of 6 lanes per warp).
-    {
-        const unsigned groups = unsigned((I.v.S + kSolveGroupsPerWarp - 1) / kSolveGroupsPerWarp);
-        I.ff_blocks = std::min(std::max(1u, (groups + 3) / 4), 2u * unsigned(sms));
-    }
-    cudaEventDestroy(ev[0]);
-    cudaEventDestroy(ev[1]);
-    KHS_CUDA(cudaMemsetAsync(&I.v.sc->solve_next, 0, sizeof(uint32_t), I.stream));
-    KHS_CUDA(cudaMemsetAsync(&I.v.sc->solve_failed, 0, sizeof(int), I.stream));
 }
 
 void Engine::launch_block_solve()
 {
     Impl &I = *d_;
-    if (I.solve_kernel) I.launch("k_block_solve", I.solve_kernel, I.solve_blocks, 128, I.v);
-    else if (I.solve_tiers)
-        I.launch("k_block_solve", k_block_solve_tiers, I.solve_blocks, 128, I.v, I.tier_quads, I.tier_singles,
-                 I.tier_doubles);
-    else if (I.solve_pairs) I.launch("k_block_solve", k_block_solve_pairs, I.solve_blocks, 128, I.v, I.solve_long);
-    else I.launch("k_block_solve", k_block_solve_hybrid, I.solve_blocks, 128, I.v, I.solve_long);
+    I.launch("k_block_solve", k_block_solve, I.solve_blocks, 32, I.v, uint32_t(I.solve_items));
 }
 
 bool Engine::make_direction(KhsxSubstepRecord &rec, double grad_norm2)
 {
     Impl &I = *d_;
     (void)grad_norm2;
-    if (!I.solve_blocks) tune_block_solve();
     const Mailbox &mb = *I.mail_host;
     bool fp64 = mode_ != KHSX_MODE_MIXED_FF;
     if (!fp64) {
@@ -4099,7 +3303,6 @@ KhsResult Engine::optimize_substep(double dt, KhsxSubstepRecord &rec)
         EvalStats first{};
         double first_alpha = 1.0, first_slope = 0.0;
         if (mode_ != KHSX_MODE_MIXED_FF) {
-            if (!I.solve_blocks) tune_block_solve();
             launch_block_solve();
             I.launch("k_reduce_dir", k_reduce_dir, kPartials, kBlock, v);
             I.launch("k_final_dir", k_final_dir, 1, kBlock, v, 0);

@@ -88,9 +88,10 @@ public:
     void set_mode(uint32_t mode) { mode_ = mode; }
     // Ends every frame after its first `substeps` substeps (0: whole frames).
     void set_substep_limit(uint32_t substeps) { substep_limit_ = substeps; }
-    // Block-solve launch shape: 5, 2 or 1 strands per warp and blocks of four
-    // warps per SM (long_strands > 0 with 5: the longest strands one per
-    // warp first); 0 strands per warp restores the one-time tuning.
+    // Block-solve launch shape: 5 strands per warp, or 1 or 2 for a warp each
+    // (long_strands > 0: that many longest strands a warp each, the rest five
+    // per warp) and 4 blocks_per_sm warps per SM; 0 strands per warp restores
+    // the rule.
     KhsResult set_block_solve_schedule(uint32_t strands_per_warp, uint32_t blocks_per_sm, uint32_t long_strands);
     KhsResult set_block_solve_tiers(uint32_t quads, uint32_t singles, uint32_t doubles, uint32_t blocks_per_sm);
     uint32_t mode() const { return mode_; }
@@ -127,7 +128,7 @@ private:
     KhsResult optimize_substep(double dt, KhsxSubstepRecord &rec);
     EvalStats evaluate(bool gradient, double dt, double alpha_for_trial, const double *alpha_dev = nullptr);
     bool make_direction(KhsxSubstepRecord &rec, double grad_norm2);
-    void tune_block_solve();
+    void plan_block_solve(uint32_t alone, uint32_t blocks_per_sm);
     void launch_block_solve();
     void launch_ccd_bound();
     void push_ring(uint32_t frame);

@@ -24,7 +24,7 @@ INCLUDE = REPO / "include"
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 CUDA_UNITS = ["khs_engine.cu", "khs_peaks.cu"]
 HOST_UNITS = ["khs_model.cpp", "khs_api.cpp"]
-HEADERS = ["khs_engine.hpp", "khs_model.hpp", "khs_device_math.cuh"]
+HEADERS = ["khs_engine.hpp", "khs_model.hpp", "khs_device_math.cuh", "khs_ff.cuh", "khs_block_solve.cuh"]
 
 
 def _nvcc() -> str:
