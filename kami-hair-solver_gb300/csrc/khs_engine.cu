@@ -100,7 +100,7 @@ struct Scalars {
     uint32_t sweep_fail;
     int solve_failed;
     uint32_t pair_count;
-    uint32_t surv_count;  // entries of the mixed contact pass's FP64 work list
+    uint32_t surv_count;  // pairs of the contact pass's FP64 pool handed out
     uint32_t solve_next;  // next strand group of the block-solve work queue
     uint32_t refine_bits; // largest relative refinement correction (FP32 bits)
     uint32_t near_count;  // elements queued for the warp-cooperative contact pass
@@ -151,7 +151,6 @@ struct View {
     double *col_cur, *col_old;
     float *col32;  // FP32 copy of col_cur for the mixed form's filters
     double *blo, *bhi;
-    float *blo32, *bhi32;  // outward-rounded copies for the mixed form
     // Mixed form: each BVH node packed in 32 bytes (FP32 outward-rounded box,
     // escape index, leaf range), the per-element contact result of the
     // separate contact pass, and the CCD (element, triangle) work list.
@@ -170,22 +169,23 @@ struct View {
     uint32_t *leaf_pool;
     uint32_t leaf_pool_capacity;
     float *cache_x32;  // FP32 node positions when the leaves were collected [E][6]
-    // Mixed contact pass in three launches: FP32 vertex records of every
-    // triangle in leaf order (a, b, c as three float4, the triangle index in
-    // the first .w), the survivors of the FP32 filter per element (at most
-    // kSurvivors, in traversal order), their FP64 closest pairs (distance,
-    // t, barycentrics) and the (element, slot) work list of the FP64 pass.
+    // Contact pass in several launches: FP32 vertex records of every triangle
+    // in leaf order (a, b, c as three float4, the triangle index in the first
+    // .w), and a pool of (element, triangle) pairs for the FP64 pass with
+    // their closest pairs (distance, t, barycentrics).  An element's pairs
+    // are surv_n from surv_off on, in traversal order.
     float4 *tri32, *tri32_old;  // FP32 records of col_cur and col_old
     // Mixed-form factors in float-float (hi, lo): B_n^-1 and C_n rows [N][36],
     // d'_n [N][6], and the diagonal shift used at each node.
     float2 *ff_inv, *ff_c, *ff_d;
     float *ff_shift;
-    uint32_t *surv_tri, *surv_list;
+    uint32_t *surv_elem, *surv_tri;
+    uint32_t surv_capacity;
+    uint32_t *surv_off, *surv_n;
     uint32_t *near_list;  // elements with cached leaves, one warp each in k_contact_near
-    uint8_t *surv_n;
     double *surv_res;
     const uint32_t *solve_items;  // work items of the block solve, at most one per strand
-    const uint32_t *besc, *bfirst, *bcount, *border, *bleaves;
+    const uint32_t *bfirst, *bcount, *border, *bleaves;
     const int32_t *bparent;
     const uint32_t *bleft, *bright;
     uint32_t *brefit;
@@ -233,47 +233,6 @@ __device__ __forceinline__ V tri_vertex(const View &d, uint32_t t, int c) { retu
 // always greater than i; anything else (a corrupted or uninitialised tree)
 // ends the walk instead of restarting it.
 __device__ __forceinline__ uint32_t escape_from(uint32_t i, uint32_t escape) { return escape > i ? escape : 0xffffffffu; }
-
-// Stackless BVH walk in the reference's visiting order.
-template<class F> __device__ void bvh_query(const View &d, V lo, V hi, double pad, F &&f)
-{
-    uint32_t i = 0;
-    while (i < d.B) {
-        const V nl = load3(d.blo + 3 * size_t(i)), nh = load3(d.bhi + 3 * size_t(i));
-        if (!dm::boxes_overlap(lo, hi, nl, nh, pad)) { i = escape_from(i, d.besc[i]); continue; }
-        const uint32_t cnt = d.bcount[i];
-        if (cnt == 0) { ++i; continue; }
-        const uint32_t first = d.bfirst[i];
-        for (uint32_t k = first; k < first + cnt; ++k) f(d.border[k]);
-        i = escape_from(i, d.besc[i]);
-    }
-}
-
-// Mixed-form walk: internal nodes are tested on outward-rounded FP32 boxes
-// against the outward-rounded FP32 query box (a superset of the FP64 test,
-// and an FP64 overlap of a leaf implies FP64 overlap of every ancestor);
-// leaves passing the FP32 test are re-tested exactly in FP64.  The
-// candidates and their order are therefore exactly those of bvh_query.
-template<class F> __device__ void bvh_query_mixed(const View &d, V lo, V hi, double pad, F &&f)
-{
-    const float lx = __double2float_rd(lo.x), ly = __double2float_rd(lo.y), lz = __double2float_rd(lo.z);
-    const float hx = __double2float_ru(hi.x), hy = __double2float_ru(hi.y), hz = __double2float_ru(hi.z);
-    const float p = __double2float_ru(pad);
-    uint32_t i = 0;
-    while (i < d.B) {
-        const float *nl = d.blo32 + 3 * size_t(i), *nh = d.bhi32 + 3 * size_t(i);
-        const bool hit = lx <= __fadd_ru(nh[0], p) && nl[0] <= __fadd_ru(hx, p) && ly <= __fadd_ru(nh[1], p) &&
-                         nl[1] <= __fadd_ru(hy, p) && lz <= __fadd_ru(nh[2], p) && nl[2] <= __fadd_ru(hz, p);
-        if (!hit) { i = escape_from(i, d.besc[i]); continue; }
-        const uint32_t cnt = d.bcount[i];
-        if (cnt == 0) { ++i; continue; }
-        if (dm::boxes_overlap(lo, hi, load3(d.blo + 3 * size_t(i)), load3(d.bhi + 3 * size_t(i)), pad)) {
-            const uint32_t first = d.bfirst[i];
-            for (uint32_t k = first; k < first + cnt; ++k) f(d.border[k]);
-        }
-        i = escape_from(i, d.besc[i]);
-    }
-}
 
 // Exact FP64 leaf test of the reference (al <= bu + p && bl <= au + p per
 // axis) decided in FP32 when possible: if the query box rounded inwards
@@ -347,10 +306,14 @@ __device__ __forceinline__ bool leaf_overlap_exact(const View &d, uint32_t node,
     return dm::boxes_overlap(q.lo, q.hi, load3(d.blo + 3 * size_t(node)), load3(d.bhi + 3 * size_t(node)), q.pad);
 }
 
-// Same walk over the packed 32-byte nodes: one pair of 16-byte loads per
-// visited node (box + escape, box + leaf range (first << 4 | count)).
-// f receives the position of each candidate in leaf order (index into
-// border and tri32).
+// Stackless BVH walk in the reference's visiting order over packed 32-byte
+// nodes: one pair of 16-byte loads per visited node (box + escape, box + leaf
+// range (first << 4 | count)).  Nodes are tested on outward-rounded FP32 boxes
+// (a superset of the FP64 test, and an FP64 overlap of a leaf implies FP64
+// overlap of every ancestor), leaves exactly, so the candidates and their
+// order are those of a walk over FP64 boxes; an FP64 comparison costs as much
+// as a multiply-add, twelve of them a node.  f receives the position of each
+// candidate in leaf order (index into border and tri32).
 template<class F> __device__ void bvh_positions_packed(const View &d, const QueryBox &q, F &&f)
 {
     uint32_t i = 0;
@@ -406,33 +369,6 @@ __device__ __forceinline__ const uint32_t *cached_leaves(const View &d, uint32_t
     if (nl == kCacheBig) { count = slots[1]; return d.leaf_pool + slots[0]; }
     count = nl;
     return slots;
-}
-
-// Candidates of leaves given as a list (the cached leaves), with the exact
-// per-leaf test: the same candidates in the same order as the full walk,
-// provided the list holds every leaf that test can accept.  f receives
-// leaf-order positions.
-template<class F> __device__ void leaves_positions(const View &d, const uint32_t *leaves, uint32_t n, const QueryBox &q,
-                                                   F &&f)
-{
-    for (uint32_t k = 0; k < n; ++k) {
-        const uint32_t i = leaves[k];
-        const float4 a = __ldg(d.bnode + 2 * size_t(i)), b = __ldg(d.bnode + 2 * size_t(i) + 1);
-        if (!maybe_overlap(q, a, b) || !leaf_overlap_exact(d, i, a, b, q)) continue;
-        const uint32_t leaf = __float_as_uint(b.w), first = leaf >> 4, cnt = leaf & 15u;
-        for (uint32_t t = first; t < first + cnt; ++t) f(t);
-    }
-}
-
-template<class F> __device__ void leaves_query(const View &d, const uint32_t *leaves, uint32_t n, V lo, V hi, double pad, F &&f)
-{
-    leaves_positions(d, leaves, n, make_query(lo, hi, pad), [&](uint32_t k) { f(d.border[k]); });
-}
-
-template<bool MIXED, class F> __device__ __forceinline__ void bvh_walk(const View &d, V lo, V hi, double pad, F &&f)
-{
-    if (MIXED) bvh_query_packed(d, lo, hi, pad, f);
-    else bvh_query(d, lo, hi, pad, f);
 }
 
 // FP32 distance of a candidate from the FP32 vertex copy, relative to an
@@ -495,6 +431,15 @@ __global__ void __launch_bounds__(kBlock) k_collider_interp(View d, const double
     d.col32[3 * size_t(i)] = float(nv.x); d.col32[3 * size_t(i) + 1] = float(nv.y); d.col32[3 * size_t(i) + 2] = float(nv.z);
 }
 
+// The outward-rounded FP32 box of a packed node (its escape index and leaf
+// range, the .w words, are the build's).
+__device__ __forceinline__ void put_box(const View &d, uint32_t node, V lo, V hi)
+{
+    float4 *pn = d.bnode + 2 * size_t(node);
+    pn[0].x = __double2float_rd(lo.x); pn[0].y = __double2float_rd(lo.y); pn[0].z = __double2float_rd(lo.z);
+    pn[1].x = __double2float_ru(hi.x); pn[1].y = __double2float_ru(hi.y); pn[1].z = __double2float_ru(hi.z);
+}
+
 // Bottom-up refit in one launch: each leaf thread computes its box and walks
 // up; the second child to arrive at a parent (atomic counter) merges the two
 // children, resets the counter for the next launch and continues.
@@ -517,15 +462,7 @@ __global__ void __launch_bounds__(kBlock) k_refit(View d, int swept)
     }
     store3(d.blo + 3 * size_t(node), lo);
     store3(d.bhi + 3 * size_t(node), hi);
-    d.blo32[3 * size_t(node)] = __double2float_rd(lo.x); d.blo32[3 * size_t(node) + 1] = __double2float_rd(lo.y);
-    d.blo32[3 * size_t(node) + 2] = __double2float_rd(lo.z);
-    d.bhi32[3 * size_t(node)] = __double2float_ru(hi.x); d.bhi32[3 * size_t(node) + 1] = __double2float_ru(hi.y);
-    d.bhi32[3 * size_t(node) + 2] = __double2float_ru(hi.z);
-    if (d.bnode) {
-        float4 *pn = d.bnode + 2 * size_t(node);
-        pn[0].x = d.blo32[3 * size_t(node)]; pn[0].y = d.blo32[3 * size_t(node) + 1]; pn[0].z = d.blo32[3 * size_t(node) + 2];
-        pn[1].x = d.bhi32[3 * size_t(node)]; pn[1].y = d.bhi32[3 * size_t(node) + 1]; pn[1].z = d.bhi32[3 * size_t(node) + 2];
-    }
+    put_box(d, node, lo, hi);
     for (;;) {
         const int32_t p = d.bparent[node];
         if (p < 0) return;
@@ -542,15 +479,7 @@ __global__ void __launch_bounds__(kBlock) k_refit(View d, int swept)
         store3(d.bhi + 3 * size_t(p), phi);
         // Rounding is monotone, so rounding the merged FP64 box equals the
         // merge of the rounded children.
-        d.blo32[3 * size_t(p)] = __double2float_rd(plo.x); d.blo32[3 * size_t(p) + 1] = __double2float_rd(plo.y);
-        d.blo32[3 * size_t(p) + 2] = __double2float_rd(plo.z);
-        d.bhi32[3 * size_t(p)] = __double2float_ru(phi.x); d.bhi32[3 * size_t(p) + 1] = __double2float_ru(phi.y);
-        d.bhi32[3 * size_t(p) + 2] = __double2float_ru(phi.z);
-        if (d.bnode) {
-            float4 *pn = d.bnode + 2 * size_t(p);
-            pn[0].x = d.blo32[3 * size_t(p)]; pn[0].y = d.blo32[3 * size_t(p) + 1]; pn[0].z = d.blo32[3 * size_t(p) + 2];
-            pn[1].x = d.bhi32[3 * size_t(p)]; pn[1].y = d.bhi32[3 * size_t(p) + 1]; pn[1].z = d.bhi32[3 * size_t(p) + 2];
-        }
+        put_box(d, p, plo, phi);
         node = uint32_t(p);
     }
 }
@@ -600,7 +529,7 @@ template<bool MIXED> __device__ bool sweep_element(const View &d, uint32_t e, Sw
     const double target = d.radius + d.offset + d.min_gap;
     const dm::F3 f0 = dm::f3(0.f, 0.f, 0.f), f1 = dm::to_local(p1, p0);
     bool failed = false;
-    bvh_walk<MIXED>(d, dm::vmin(p0, p1), dm::vmax(p0, p1), target, [&](uint32_t t) {
+    bvh_query_packed(d, dm::vmin(p0, p1), dm::vmax(p0, p1), target, [&](uint32_t t) {
         if (failed) return;
         const V oa = load3(d.col_old + 3 * size_t(d.tri[3 * t])), ob = load3(d.col_old + 3 * size_t(d.tri[3 * t + 1])),
                 oc = load3(d.col_old + 3 * size_t(d.tri[3 * t + 2]));
@@ -858,7 +787,7 @@ __device__ __forceinline__ uint32_t closest_triangle(const View &d, V xi, V xj, 
     pair.distance = 1.0e300; pair.t = 0.0; pair.bary = dm::v(1, 0, 0);
     const V lo = dm::vmin(xi, xj), hi = dm::vmax(xi, xj);
     if (!MIXED) {
-        bvh_query(d, lo, hi, pad, [&](uint32_t t) {
+        bvh_query_packed(d, lo, hi, pad, [&](uint32_t t) {
             ++cand;
             const dm::ClosestPair c = dm::closest_segment_triangle(xi, xj, tri_vertex(d, t, 0), tri_vertex(d, t, 1), tri_vertex(d, t, 2));
             if (c.distance < pair.distance) { pair = c; closest = t; }
@@ -903,21 +832,27 @@ template<bool MIXED> __global__ void __launch_bounds__(kBlock) k_contact(View d,
     store3(d.c_bary + 3 * size_t(e), pair.bary);
 }
 
-// ---- mixed contact pass in three launches ---------------------------------
+// ---- contact pass of an evaluation ------------------------------------------
 //
-// k_contact_filter (per element): candidate count and the FP32 filter over
-// the triangle records in leaf order; the survivors (every candidate whose
-// FP32 lower bound does not exceed the smallest FP32 upper bound, in
-// traversal order) go to per-element slots and to a compact work list.
-// k_contact_exact (per survivor): the FP64 closest pair, with every lane of
-// a warp on the same code path.  k_contact_select (per element): the first
-// strictly closest survivor in traversal order.  Candidates that are not
-// survivors are strictly farther in FP64 than the minimum, so the result,
-// tie-break included, equals k_contact's and the all-FP64 search.
+// k_contact_filter (thread per element): the element's cached leaves are still
+// valid, or are collected again; elements with leaves are queued.
+// k_contact_near (warp per queued element): lane l tests leaf l exactly, so
+// the candidates are counted in traversal order; in the mixed form an FP32
+// filter over the triangle records keeps every candidate whose lower bound
+// does not exceed the smallest upper bound, in the plain form all stay.  They
+// go to a pool of (element, triangle) pairs.  k_contact_exact (thread per
+// pair): the FP64 closest pair.  k_contact_select (thread per element): the
+// first strictly closest of the element's pairs.  Candidates the mixed form
+// drops are strictly farther in FP64 than the minimum, so either way the
+// result, tie-break included, equals k_contact's.
+//
+// The plain form used to search inside the element kernel, one thread walking
+// the FP64 boxes and evaluating every candidate in turn: on 80 strands among
+// contacts that took 2.0 ms an evaluation; the pairs are few (7,000 there) and
+// independent.
 
-constexpr int kSurvivors = 8;
 constexpr int kLeafTriangles = 8;  // BVH leaves hold at most 8 triangles (cuda_backend.cu:305)
-constexpr uint8_t kSurvOverflow = 0xff;
+constexpr uint32_t kSurvOverflow = 0xffffffffu;  // surv_n: no room in a pool, k_contact_select searches
 
 // FP32 vertex records of every triangle in leaf order, of col_cur and of
 // col_old; run whenever they change (after k_collider_interp and at set-up).
@@ -957,37 +892,6 @@ __device__ __forceinline__ float record_distance_f(const View &d, uint32_t p, dm
     return df;
 }
 
-// Filter of one element over a position source; returns the survivor count
-// (kSurvivors + 1 or more on overflow; the first kSurvivors are stored).
-template<class Source>
-__device__ __forceinline__ uint32_t filter_survivors(const View &d, uint32_t e, dm::F3 xi32, dm::F3 xj32, uint32_t &cand,
-                                                     Source &&source)
-{
-    const dm::F3 origin = xi32;
-    const dm::F3 p0 = dm::f3(0.f, 0.f, 0.f), p1 = dm::f3(xj32.x - origin.x, xj32.y - origin.y, xj32.z - origin.z);
-    float bound = 3.0e38f;
-    cand = 0;
-    source([&](uint32_t p) {
-        ++cand;
-        float m;
-        uint32_t t;
-        const float df = record_distance_f(d, p, origin, p0, p1, m, t);
-        bound = fminf(bound, df + m);
-    });
-    if (cand == 0) return 0;
-    uint32_t n = 0;
-    uint32_t *slots = d.surv_tri + size_t(kSurvivors) * e;
-    source([&](uint32_t p) {
-        float m;
-        uint32_t t;
-        const float df = record_distance_f(d, p, origin, p0, p1, m, t);
-        if (df - m > bound) return;
-        if (n < uint32_t(kSurvivors)) slots[n] = t;
-        ++n;
-    });
-    return n;
-}
-
 __device__ __forceinline__ void write_contact(const View &d, uint32_t e, uint32_t closest, const dm::ClosestPair &pair)
 {
     uint8_t flags = 0;
@@ -1006,121 +910,74 @@ __device__ __forceinline__ void write_contact(const View &d, uint32_t e, uint32_
     store3(d.c_bary + 3 * size_t(e), pair.bary);
 }
 
-// Slack test of the leaf cache on the FP32 copies: the copies differ from
-// the FP64 positions by at most 2^-24 of a coordinate's magnitude, so the
-// margin of 1e-5 m keeps every accepted displacement within kCacheSlack
-// for coordinates below a few hundred metres.
+// Slack test of the leaf cache on the FP32 copies: below kCacheReach metres
+// they differ from the FP64 positions by at most 2^-24 of that, 4e-6 m, so the
+// margin of 1e-5 m keeps every accepted displacement within kCacheSlack.
+// Elements further out collect their leaves at every evaluation.
+constexpr float kCacheReach = 64.0f;
 __device__ __forceinline__ bool within_cache_slack(const float *c, dm::F3 xi, dm::F3 xj)
 {
     const float s = float(kCacheSlack) - 1.0e-5f;
-    return fabsf(xi.x - c[0]) <= s && fabsf(xi.y - c[1]) <= s && fabsf(xi.z - c[2]) <= s && fabsf(xj.x - c[3]) <= s &&
-           fabsf(xj.y - c[4]) <= s && fabsf(xj.z - c[5]) <= s;
+    const float far = fmaxf(fmaxf(fmaxf(fabsf(xi.x), fabsf(xi.y)), fmaxf(fabsf(xi.z), fabsf(xj.x))), fmaxf(fabsf(xj.y), fabsf(xj.z)));
+    return far <= kCacheReach && fabsf(xi.x - c[0]) <= s && fabsf(xi.y - c[1]) <= s && fabsf(xi.z - c[2]) <= s &&
+           fabsf(xj.x - c[3]) <= s && fabsf(xj.y - c[4]) <= s && fabsf(xj.z - c[5]) <= s;
 }
 
-// q must be d.q (its FP32 copy d.q32 is read).
+// q must be d.q (its FP32 copy d.q32 is read).  cache 1: collect every
+// element's leaves; 0: only where the element has left its slack.
 __global__ void __launch_bounds__(kBlock) k_contact_filter(View d, const double *q, int cache)
 {
     const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool live = e < d.E;
-    uint32_t append = 0;
-    if (live) {
-        const uint32_t i = d.ei[e], j = d.ej[e];
-        uint32_t cand = 0, n = 0;
-        bool deferred = false;  // finished by k_contact_near
-        const bool enabled = d.has_collider && !d.fixed[i] && d.econtact[e];
-        if (enabled) {
-            const dm::F3 xi32 = dm::f3(d.q32[3 * size_t(i)], d.q32[3 * size_t(i) + 1], d.q32[3 * size_t(i) + 2]);
-            const dm::F3 xj32 = dm::f3(d.q32[3 * size_t(j)], d.q32[3 * size_t(j) + 1], d.q32[3 * size_t(j) + 2]);
+    if (e >= d.E) return;
+    const uint32_t i = d.ei[e], j = d.ej[e];
+    if (!d.fixed[i] && d.econtact[e]) {
+        const dm::F3 xi32 = dm::f3(d.q32[3 * size_t(i)], d.q32[3 * size_t(i) + 1], d.q32[3 * size_t(i) + 2]);
+        const dm::F3 xj32 = dm::f3(d.q32[3 * size_t(j)], d.q32[3 * size_t(j) + 1], d.q32[3 * size_t(j) + 2]);
+        float *c32 = d.cache_x32 + 6 * size_t(e);
+        uint8_t nl = d.cache_n[e];
+        if (cache == 1 || nl == kCacheInvalid || !within_cache_slack(c32, xi32, xj32)) {
+            // (Re)collect the leaves around the element box grown by the
+            // slack, so that the passes of many evaluations read a short list.
+            const V xi = load3(q + 6 * size_t(i)), xj = load3(q + 6 * size_t(j));
             const double pad = d.radius + d.offset + d.dhat;
-            float *c32 = d.cache_x32 + 6 * size_t(e);
-            uint8_t nl = cache >= 0 ? d.cache_n[e] : kCacheInvalid;
-            bool inside = cache == 0 && nl != kCacheInvalid && within_cache_slack(c32, xi32, xj32);
-            // FP64 positions only where a walk is needed.
-            V xi = dm::v(0, 0, 0), xj = xi;
-            if (!inside) { xi = load3(q + 6 * size_t(i)); xj = load3(q + 6 * size_t(j)); }
-            if (cache == 1 || (cache == 0 && !inside)) {
-                // (Re)collect the leaves around the element box grown by the
-                // slack: one walk, after which both filter passes read the
-                // short leaf list (an element that left its slack would
-                // otherwise walk the tree twice in every evaluation).
-                const V s3 = dm::v(kCacheSlack, kCacheSlack, kCacheSlack);
-                const V clo = dm::vmin(xi, xj) - s3, chi = dm::vmax(xi, xj) + s3;
-                uint32_t *slots = d.cache_leaf + size_t(kCacheLeaves) * e;
-                const uint32_t c = collect_leaves(d, clo, chi, pad, slots, kCacheLeaves);
-                if (c <= uint32_t(kCacheLeaves)) {
-                    nl = uint8_t(c);
-                } else {
-                    // A dense patch of the collider (a mesh pole, a seam):
-                    // the list goes to the pool, and k_contact_near works
-                    // through it 32 leaves at a time.
-                    const uint32_t off = atomicAdd(&d.sc->pool_used, c);
-                    nl = kCacheInvalid;
-                    if (size_t(off) + c <= d.leaf_pool_capacity) {
-                        collect_leaves(d, clo, chi, pad, d.leaf_pool + off, c);
-                        slots[0] = off;
-                        slots[1] = c;
-                        nl = kCacheBig;
-                    }
-                }
-                d.cache_n[e] = nl;
-                c32[0] = xi32.x; c32[1] = xi32.y; c32[2] = xi32.z; c32[3] = xj32.x; c32[4] = xj32.y; c32[5] = xj32.z;
-                inside = nl != kCacheInvalid;
-            }
-            if (inside) {
-                if (nl > 0) {
-                    // k_contact_near finishes the element, one warp over its leaves.
-                    d.near_list[append_slot(&d.sc->near_count)] = e;
-                    deferred = true;
-                }
+            const V s3 = dm::v(kCacheSlack, kCacheSlack, kCacheSlack);
+            const V clo = dm::vmin(xi, xj) - s3, chi = dm::vmax(xi, xj) + s3;
+            uint32_t *slots = d.cache_leaf + size_t(kCacheLeaves) * e;
+            const uint32_t c = collect_leaves(d, clo, chi, pad, slots, kCacheLeaves);
+            if (c <= uint32_t(kCacheLeaves)) {
+                nl = uint8_t(c);
             } else {
-                // More than kCacheLeaves leaves around the element: walk.
-                const float lo32[3] = {fminf(xi32.x, xj32.x), fminf(xi32.y, xj32.y), fminf(xi32.z, xj32.z)};
-                const float hi32[3] = {fmaxf(xi32.x, xj32.x), fmaxf(xi32.y, xj32.y), fmaxf(xi32.z, xj32.z)};
-                const QueryBox qb = make_query_f(lo32, hi32, dm::vmin(xi, xj), dm::vmax(xi, xj), pad);
-                n = filter_survivors(d, e, xi32, xj32, cand, [&](auto &&fn) { bvh_positions_packed(d, qb, fn); });
+                // A dense patch of the collider (a mesh pole, a seam): the
+                // list goes to the pool, and k_contact_near works through it
+                // 32 leaves at a time.
+                const uint32_t off = atomicAdd(&d.sc->pool_used, c);
+                nl = kCacheInvalid;
+                if (size_t(off) + c <= d.leaf_pool_capacity) {
+                    collect_leaves(d, clo, chi, pad, d.leaf_pool + off, c);
+                    slots[0] = off;
+                    slots[1] = c;
+                    nl = kCacheBig;
+                }
             }
+            d.cache_n[e] = nl;
+            c32[0] = xi32.x; c32[1] = xi32.y; c32[2] = xi32.z; c32[3] = xj32.x; c32[4] = xj32.y; c32[5] = xj32.z;
         }
-        if (!deferred) {
-            d.c_cand[e] = cand;
-            if (n > uint32_t(kSurvivors)) {
-                // Rare: more near-equal candidates than slots; k_contact_select
-                // finishes the element with the in-thread search.
-                d.surv_n[e] = kSurvOverflow;
-            } else {
-                d.surv_n[e] = uint8_t(n);
-                append = n;
-                if (n == 0) {
-                    dm::ClosestPair pair;
-                    pair.distance = 1.0e300; pair.t = 0.0; pair.bary = dm::v(1, 0, 0);
-                    write_contact(d, e, kNone, pair);
-                }
-            }
+        if (nl == kCacheInvalid) {  // the leaf pool is full
+            d.surv_n[e] = kSurvOverflow;
+            return;
+        }
+        if (nl > 0) {
+            d.near_list[append_slot(&d.sc->near_count)] = e;
+            return;
         }
     }
-    // Warp-aggregated append of (element, slot) entries to the work list.
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    uint32_t incl = append;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(FULL, incl, o);
-        if (lane >= o) incl += v;
-    }
-    const uint32_t total = __shfl_sync(FULL, incl, 31);
-    uint32_t base = 0;
-    if (lane == 31 && total) base = atomicAdd(&d.sc->surv_count, total);
-    base = __shfl_sync(FULL, base, 31);
-    const uint32_t start = base + incl - append;
-    for (uint32_t k = 0; k < append; ++k) d.surv_list[start + k] = uint32_t(kSurvivors) * e + k;
+    d.c_cand[e] = 0;
+    d.surv_n[e] = 0;
+    dm::ClosestPair pair;
+    pair.distance = 1.0e300; pair.t = 0.0; pair.bary = dm::v(1, 0, 0);
+    write_contact(d, e, kNone, pair);
 }
 
-// One warp per element with cached leaves: lane l tests cached leaf l
-// (DFS order) and evaluates the FP32 distances of that leaf's triangles, so
-// the element's candidates are examined in parallel instead of one after
-// another by a single lane.  The candidate order is leaf order, then
-// triangle order within the leaf, as in the single-lane filter; survivors
-// are compacted in that order (a prefix over lanes, then ascending within a
-// lane), so slots, the FP64 pass and the ordered selection are unchanged.
 // Triangle range (first, cnt) of cached leaf k of a list of `count` when
 // its box passes the query's exact per-leaf test; cnt = 0 otherwise.
 __device__ __forceinline__ void near_leaf(const View &d, const uint32_t *leaves, uint32_t k, uint32_t count, const QueryBox &qb,
@@ -1148,35 +1005,42 @@ __device__ __forceinline__ uint32_t warp_inclusive_sum(uint32_t v, int lane)
     return v;
 }
 
-// Result of one element of the warp-cooperative contact pass (lane 0
-// writes): candidate count, survivor count or overflow, the no-contact
-// record, and the survivors' entries in the FP64 work list.
-__device__ __forceinline__ void near_finish(const View &d, uint32_t e, uint32_t total, uint32_t n, int lane)
+// The pool range of an element's n pairs of total candidates (lane 0 writes
+// the element's record): its offset, or kNone without room or pairs.
+__device__ __forceinline__ uint32_t near_claim(const View &d, uint32_t e, uint32_t total, uint32_t n, int lane)
 {
-    uint32_t base = 0;
+    uint32_t off = kNone;
     if (lane == 0) {
         d.c_cand[e] = total;
-        if (n > uint32_t(kSurvivors)) {
-            d.surv_n[e] = kSurvOverflow;
+        uint32_t held = n;
+        if (n == 0) {
+            dm::ClosestPair pair;
+            pair.distance = 1.0e300; pair.t = 0.0; pair.bary = dm::v(1, 0, 0);
+            write_contact(d, e, kNone, pair);
         } else {
-            d.surv_n[e] = uint8_t(n);
-            if (n == 0) {
-                dm::ClosestPair pair;
-                pair.distance = 1.0e300; pair.t = 0.0; pair.bary = dm::v(1, 0, 0);
-                write_contact(d, e, kNone, pair);
-            } else {
-                base = atomicAdd(&d.sc->surv_count, n);
+            off = atomicAdd(&d.sc->surv_count, n);
+            if (uint64_t(off) + n > d.surv_capacity) {
+                off = kNone;
+                held = kSurvOverflow;
             }
+            d.surv_off[e] = off;
         }
+        d.surv_n[e] = held;
     }
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (n <= uint32_t(kSurvivors) && uint32_t(lane) < n) d.surv_list[base + lane] = uint32_t(kSurvivors) * e + lane;
+    return __shfl_sync(0xffffffffu, off, 0);
+}
+
+__device__ __forceinline__ void put_pair(const View &d, uint32_t slot, uint32_t e, uint32_t t)
+{
+    d.surv_elem[slot] = e;
+    d.surv_tri[slot] = t;
 }
 
 // An element whose cached leaves live in the leaf pool (more than 32): the
-// list is taken 32 leaves at a time, once for the FP32 bound and once more
-// for the survivors, which are written in leaf order.  Kept out of line so
-// the common one-round path keeps its registers.
+// list is taken 32 leaves at a time, for the FP32 bound (FILTER), to count
+// the pairs and to write them, in leaf order.  Kept out of line so the common
+// one-round path keeps its registers.
+template<bool FILTER>
 __device__ __noinline__ void near_pool_element(const View &d, uint32_t e, const QueryBox &qb, dm::F3 origin, dm::F3 p1)
 {
     const unsigned FULL = 0xffffffffu;
@@ -1189,49 +1053,61 @@ __device__ __noinline__ void near_pool_element(const View &d, uint32_t e, const 
     for (uint32_t r0 = 0; r0 < nleaves; r0 += 32) {
         uint32_t first, cnt;
         near_leaf(d, leaves, r0 + lane, nleaves, qb, first, cnt);
-        for (uint32_t r = 0; r < cnt; ++r) {
+        for (uint32_t r = 0; FILTER && r < cnt; ++r) {
             float m;
             uint32_t t;
             const float df = record_distance_f(d, first + r, origin, p0, p1, m, t);
             ub = fminf(ub, df + m);
         }
-        total += __shfl_sync(FULL, warp_inclusive_sum(cnt, lane), 31);
+        total += __reduce_add_sync(FULL, cnt);
     }
+    uint32_t n = total;
+    if (FILTER) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ub = fminf(ub, __shfl_xor_sync(FULL, ub, o));
-    uint32_t *slots = d.surv_tri + size_t(kSurvivors) * e;
-    uint32_t n = 0;
-    for (uint32_t r0 = 0; r0 < nleaves; r0 += 32) {
-        uint32_t first, cnt;
-        near_leaf(d, leaves, r0 + lane, nleaves, qb, first, cnt);
-        uint32_t mine = 0;
-        for (uint32_t r = 0; r < cnt; ++r) {
-            float m;
-            uint32_t t;
-            const float df = record_distance_f(d, first + r, origin, p0, p1, m, t);
-            mine += !(df - m > ub) ? 1u : 0u;
+        for (int o = 16; o > 0; o >>= 1) ub = fminf(ub, __shfl_xor_sync(FULL, ub, o));
+        n = 0;
+        for (uint32_t r0 = 0; r0 < nleaves; r0 += 32) {
+            uint32_t first, cnt, mine = 0;
+            near_leaf(d, leaves, r0 + lane, nleaves, qb, first, cnt);
+            for (uint32_t r = 0; r < cnt; ++r) {
+                float m;
+                uint32_t t;
+                const float df = record_distance_f(d, first + r, origin, p0, p1, m, t);
+                mine += !(df - m > ub) ? 1u : 0u;
+            }
+            n += __reduce_add_sync(FULL, mine);
         }
-        const uint32_t sincl = warp_inclusive_sum(mine, lane);
-        uint32_t slot = n + sincl - mine;
-        for (uint32_t r = 0; r < cnt && mine; ++r) {
-            float m;
-            uint32_t t;
-            const float df = record_distance_f(d, first + r, origin, p0, p1, m, t);
-            if (df - m > ub) continue;
-            if (slot < uint32_t(kSurvivors)) slots[slot] = t;
-            ++slot;
-        }
-        n += __shfl_sync(FULL, sincl, 31);
     }
-    near_finish(d, e, total, n, lane);
+    uint32_t slot = near_claim(d, e, total, n, lane);
+    if (slot == kNone) return;
+    for (uint32_t r0 = 0; r0 < nleaves; r0 += 32) {
+        uint32_t first, cnt, mine = 0;
+        near_leaf(d, leaves, r0 + lane, nleaves, qb, first, cnt);
+        uint32_t keep = 0;  // bit r: triangle first + r stays
+        for (uint32_t r = 0; r < cnt; ++r) {
+            bool stays = true;
+            if (FILTER) {
+                float m;
+                uint32_t t;
+                const float df = record_distance_f(d, first + r, origin, p0, p1, m, t);
+                stays = !(df - m > ub);
+            }
+            keep |= uint32_t(stays) << r;
+        }
+        mine = __popc(keep);
+        const uint32_t sincl = warp_inclusive_sum(mine, lane);
+        uint32_t at = slot + sincl - mine;
+        for (uint32_t r = 0; r < cnt; ++r)
+            if (keep >> r & 1u) put_pair(d, at++, e, __float_as_uint(__ldg(d.tri32 + 3 * size_t(first + r)).w));
+        slot += __shfl_sync(FULL, sincl, 31);
+    }
 }
 
-// One warp per element queued by k_contact_filter (leaves cached and the
-// element within its slack): lane l tests cached leaf l and the FP32
-// distances of its triangles; the smallest upper bound is reduced across
-// the warp and the survivors are written in traversal order (leaf, then
-// triangle), so the first-found tie-break is kept.
-__global__ void __launch_bounds__(kBlock) k_contact_near(View d)
+// One warp per element queued by k_contact_filter: lane l tests cached leaf l
+// and, with FILTER, the FP32 distances of its triangles; the smallest upper
+// bound is reduced across the warp.  The pairs are written in traversal order
+// (leaf, then triangle), so the first-found tie-break is kept.
+template<bool FILTER> __global__ void __launch_bounds__(kBlock) k_contact_near(View d)
 {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -1251,60 +1127,58 @@ __global__ void __launch_bounds__(kBlock) k_contact_near(View d)
         const dm::F3 p1 = dm::f3(xj32.x - origin.x, xj32.y - origin.y, xj32.z - origin.z);
         const uint8_t nl = d.cache_n[e];
         if (nl == kCacheBig) {
-            near_pool_element(d, e, qb, origin, p1);
+            near_pool_element<FILTER>(d, e, qb, origin, p1);
             continue;
         }
         uint32_t first, cnt;
         near_leaf(d, d.cache_leaf + size_t(kCacheLeaves) * e, lane, nl, qb, first, cnt);
-        const uint32_t total = __shfl_sync(FULL, warp_inclusive_sum(cnt, lane), 31);
+        const uint32_t total = __reduce_add_sync(FULL, cnt);
         float lb[kLeafTriangles];
-        uint32_t tri[kLeafTriangles];
         float ub = 3.0e38f;
+        uint32_t keep = cnt ? (1u << cnt) - 1u : 0u;  // bit r: triangle first + r stays
+        if (FILTER) {
 #pragma unroll
-        for (int r = 0; r < kLeafTriangles; ++r) {
-            lb[r] = 3.0e38f;
-            tri[r] = 0;
-            if (uint32_t(r) < cnt) {
-                float m;
-                const float df = record_distance_f(d, first + r, origin, p0, p1, m, tri[r]);
-                lb[r] = df - m;
-                ub = fminf(ub, df + m);
+            for (int r = 0; r < kLeafTriangles; ++r) {
+                lb[r] = 3.0e38f;
+                if (uint32_t(r) < cnt) {
+                    float m;
+                    uint32_t t;
+                    const float df = record_distance_f(d, first + r, origin, p0, p1, m, t);
+                    lb[r] = df - m;
+                    ub = fminf(ub, df + m);
+                }
             }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) ub = fminf(ub, __shfl_xor_sync(FULL, ub, o));
+#pragma unroll
+            for (int r = 0; r < kLeafTriangles; ++r)
+                if (lb[r] > ub) keep &= ~(1u << r);
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) ub = fminf(ub, __shfl_xor_sync(FULL, ub, o));
-        uint32_t mine = 0;
-#pragma unroll
-        for (int r = 0; r < kLeafTriangles; ++r) mine += (uint32_t(r) < cnt && !(lb[r] > ub)) ? 1u : 0u;
+        const uint32_t mine = __popc(keep);
         const uint32_t sincl = warp_inclusive_sum(mine, lane);
         const uint32_t n = __shfl_sync(FULL, sincl, 31);
-        uint32_t slot = sincl - mine;
-        uint32_t *slots = d.surv_tri + size_t(kSurvivors) * e;
-#pragma unroll
-        for (int r = 0; r < kLeafTriangles; ++r) {
-            if (uint32_t(r) < cnt && !(lb[r] > ub)) {
-                if (slot < uint32_t(kSurvivors)) slots[slot] = tri[r];
-                ++slot;
-            }
-        }
-        near_finish(d, e, total, n, lane);
+        const uint32_t base = near_claim(d, e, total, n, lane);
+        if (base == kNone) continue;
+        uint32_t at = base + sincl - mine;
+        for (; keep; keep &= keep - 1)
+            put_pair(d, at++, e, __float_as_uint(__ldg(d.tri32 + 3 * size_t(first + uint32_t(__ffs(keep) - 1))).w));
     }
 }
 
 __global__ void __launch_bounds__(kBlock) k_contact_exact(View d, const double *q)
 {
-    const uint32_t count = d.sc->surv_count;
+    const uint32_t count = min(d.sc->surv_count, d.surv_capacity);
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
-        const uint32_t slot = d.surv_list[k], e = slot / uint32_t(kSurvivors), t = d.surv_tri[slot];
+        const uint32_t e = d.surv_elem[k], t = d.surv_tri[k];
         const uint32_t i = d.ei[e], j = d.ej[e];
         const V xi = load3(q + 6 * size_t(i)), xj = load3(q + 6 * size_t(j));
         const dm::ClosestPair c = dm::closest_segment_triangle(xi, xj, tri_vertex(d, t, 0), tri_vertex(d, t, 1), tri_vertex(d, t, 2));
-        double *r = d.surv_res + 5 * size_t(slot);
+        double *r = d.surv_res + 5 * size_t(k);
         r[0] = c.distance; r[1] = c.t; r[2] = c.bary.x; r[3] = c.bary.y; r[4] = c.bary.z;
     }
 }
 
-__global__ void __launch_bounds__(kBlock) k_contact_select(View d, const double *q)
+template<bool FILTER> __global__ void __launch_bounds__(kBlock) k_contact_select(View d, const double *q)
 {
     const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e == 0) {  // k_contact_near and k_contact_exact, their only readers, have completed
@@ -1314,38 +1188,30 @@ __global__ void __launch_bounds__(kBlock) k_contact_select(View d, const double 
     if (e >= d.E) return;
     const uint32_t n = d.surv_n[e];
     if (n == 0) return;
-    if (n == kSurvOverflow) {
-        // The two-pass search over the same candidates (the cached leaves
-        // when the filter used them, else the full walk).
-        const uint32_t i = d.ei[e], j = d.ej[e];
-        const V xi = load3(q + 6 * size_t(i)), xj = load3(q + 6 * size_t(j));
-        const double pad = d.radius + d.offset + d.dhat;
-        const uint8_t nl = d.cache_n[e];
-        const dm::F3 xi32 = dm::f3(d.q32[3 * size_t(i)], d.q32[3 * size_t(i) + 1], d.q32[3 * size_t(i) + 2]);
-        const dm::F3 xj32 = dm::f3(d.q32[3 * size_t(j)], d.q32[3 * size_t(j) + 1], d.q32[3 * size_t(j) + 2]);
-        const bool inside = nl != kCacheInvalid && within_cache_slack(d.cache_x32 + 6 * size_t(e), xi32, xj32);
-        uint32_t nleaves = 0;
-        const uint32_t *leaves = cached_leaves(d, e, nl, nleaves);
-        const V lo = dm::vmin(xi, xj), hi = dm::vmax(xi, xj);
-        uint32_t c2 = 0;
-        dm::ClosestPair pair;
-        const uint32_t closest =
-            inside ? closest_triangle_in(d, xi, xj, c2, pair, [&](auto &&fn) { leaves_query(d, leaves, nleaves, lo, hi, pad, fn); })
-                   : closest_triangle<true>(d, xi, xj, pad, c2, pair);
-        write_contact(d, e, closest, pair);
-        return;
-    }
-    uint32_t best = 0;
-    double bd = 1.0e300;
-    for (uint32_t k = 0; k < n; ++k) {
-        const double dist = d.surv_res[5 * (size_t(kSurvivors) * e + k)];
-        if (dist < bd) { bd = dist; best = k; }
-    }
-    const size_t slot = size_t(kSurvivors) * e + best;
-    const double *r = d.surv_res + 5 * slot;
     dm::ClosestPair pair;
-    pair.distance = r[0]; pair.t = r[1]; pair.bary = dm::v(r[2], r[3], r[4]);
-    write_contact(d, e, d.surv_tri[slot], pair);
+    pair.distance = 1.0e300; pair.t = 0.0; pair.bary = dm::v(1, 0, 0);
+    uint32_t closest = kNone;
+    if (n == kSurvOverflow) {
+        // A pool is full: the search over all candidates by one thread.
+        const uint32_t i = d.ei[e], j = d.ej[e];
+        uint32_t cand = 0;
+        closest = closest_triangle<FILTER>(d, load3(q + 6 * size_t(i)), load3(q + 6 * size_t(j)), d.radius + d.offset + d.dhat,
+                                           cand, pair);
+        d.c_cand[e] = cand;
+    } else {
+        const uint32_t off = d.surv_off[e];
+        uint32_t best = kNone;
+        for (uint32_t k = off; k < off + n; ++k) {
+            const double dist = d.surv_res[5 * size_t(k)];
+            if (dist < pair.distance) { pair.distance = dist; best = k; }
+        }
+        if (best != kNone) {
+            const double *r = d.surv_res + 5 * size_t(best);
+            pair.t = r[1]; pair.bary = dm::v(r[2], r[3], r[4]);
+            closest = d.surv_tri[best];
+        }
+    }
+    write_contact(d, e, closest, pair);
 }
 
 // ---- contact query without allocation -------------------------------------
@@ -1389,7 +1255,7 @@ template<bool MIXED> __global__ void __launch_bounds__(kBlock) k_contact_query_r
 
 // Per element: elastic energy (+ gradient and GN blocks) and barrier contact
 // against the closest BVH candidate (cuda_backend.cu:899-939).
-template<bool MIXED> __global__ void __launch_bounds__(kBlock) k_elem_eval(View d, int gradient)
+__global__ void __launch_bounds__(kBlock) k_elem_eval(View d, int gradient)
 {
     const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= d.E) return;
@@ -1437,20 +1303,10 @@ template<bool MIXED> __global__ void __launch_bounds__(kBlock) k_elem_eval(View 
     uint8_t flags = 0;
     double gap = 0.0, ce = 0.0;
     if (d.has_collider && !fi && d.econtact[e]) {
+        // Result of the contact pass at this same state.
         dm::ClosestPair pair;
-        if (MIXED) {
-            // Result of the contact pass at this same state.
-            cand = d.c_cand[e]; closest = d.c_tri[e]; flags = d.c_flags[e]; gap = d.c_gap[e];
-            pair.t = d.c_t[e]; pair.distance = d.c_dist[e]; pair.bary = load3(d.c_bary + 3 * size_t(e));
-        } else {
-            closest = closest_triangle<false>(d, xi, xj, d.radius + d.offset + d.dhat, cand, pair);
-            if (closest != kNone) {
-                flags |= kFlagClosest;
-                gap = pair.distance - d.radius - d.offset;
-                if (gap <= d.min_gap) flags |= kFlagInfeasible;
-                else if (gap < d.dhat) flags |= kFlagActive;
-            }
-        }
+        cand = d.c_cand[e]; closest = d.c_tri[e]; flags = d.c_flags[e]; gap = d.c_gap[e];
+        pair.t = d.c_t[e]; pair.distance = d.c_dist[e]; pair.bary = load3(d.c_bary + 3 * size_t(e));
         if (closest != kNone) {
             if (flags & kFlagActive) {
                 const V a = tri_vertex(d, closest, 0), b = tri_vertex(d, closest, 1), c = tri_vertex(d, closest, 2);
@@ -2091,7 +1947,7 @@ template<bool MIXED> __global__ void __launch_bounds__(kBlock) k_ccd(View d)
     const double target = d.radius + d.offset + d.min_gap;
     double local = 1.0;
     const dm::F3 f0 = dm::f3(0.f, 0.f, 0.f), f1 = dm::to_local(p1, p0);
-    bvh_walk<MIXED>(d, lo, hi, target, [&](uint32_t t) {
+    bvh_query_packed(d, lo, hi, target, [&](uint32_t t) {
         const double speed = fmax(dm::gnorm(d0), dm::gnorm(d1));
         if (speed < 1e-30) return;
         const V a = tri_vertex(d, t, 0), b = tri_vertex(d, t, 1), c = tri_vertex(d, t, 2);
@@ -2124,13 +1980,14 @@ template<bool MIXED> __global__ void __launch_bounds__(kBlock) k_ccd(View d)
     if (local < 1.0) atomicMin(&d.sc->ccd_bits, (unsigned long long)__double_as_longlong(local));
 }
 
-// Mixed-form CCD, load balanced: k_ccd_collect lists every (element,
-// triangle) candidate whose FP32 lower-bound clearance does not already let
-// the first advancement step reach alpha = 1; k_ccd_pairs runs the exact FP64
-// conservative advancement of cuda_backend.cu:989-1000 per listed pair and
-// stops a pair once 0.9 alpha reaches the global minimum found so far (every
-// limit the pair could still produce is >= 0.9 alpha).  The minimum equals
-// the per-element kernel's.
+// CCD bound, load balanced: k_ccd_collect and k_ccd_near list every (element,
+// triangle) candidate, in the mixed form (FILTER) without those whose FP32
+// lower-bound clearance already lets the first advancement step reach
+// alpha = 1; k_ccd_pairs runs the exact FP64 conservative advancement of
+// cuda_backend.cu:989-1000 per listed pair and stops a pair once 0.9 alpha
+// reaches the global minimum found so far (every limit the pair could still
+// produce is >= 0.9 alpha).  The minimum equals the per-element kernel's
+// (k_ccd), which remains for a full pair list.
 // Candidates of the swept element box (positions at step 0 and 1) whose
 // FP32 lower-bound distance does not rule out a limit below 1: a pair is
 // skipped only when even the lower bound of 0.8 (dist - target) reaches the
@@ -2139,7 +1996,7 @@ template<bool MIXED> __global__ void __launch_bounds__(kBlock) k_ccd(View d)
 // slack of the element's leaf cache, the cached leaves (collected with the
 // contact padding, which is at least the CCD target) hold every leaf the
 // swept box can touch and replace the tree walk.
-__global__ void __launch_bounds__(kBlock) k_ccd_collect(View d)
+template<bool FILTER> __global__ void __launch_bounds__(kBlock) k_ccd_collect(View d)
 {
     const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= d.E) return;
@@ -2161,10 +2018,14 @@ __global__ void __launch_bounds__(kBlock) k_ccd_collect(View d)
     const float speed_ru = __fmul_ru(__double2float_ru(speed), 1.000002f);
     const QueryBox qb = make_query(lo, hi, target);
     auto test = [&](uint32_t p) {
-        float m;
         uint32_t t;
-        const float df = record_distance_f(d, p, origin, f0, f1, m, t);
-        if (__fmul_rd(0.8f, __fsub_rd(__fsub_rd(df, m), target_ru)) >= speed_ru) return;
+        if (FILTER) {
+            float m;
+            const float df = record_distance_f(d, p, origin, f0, f1, m, t);
+            if (__fmul_rd(0.8f, __fsub_rd(__fsub_rd(df, m), target_ru)) >= speed_ru) return;
+        } else {
+            t = __float_as_uint(__ldg(d.tri32 + 3 * size_t(p)).w);
+        }
         const uint32_t slot = append_slot(&d.sc->pair_count);
         if (slot < d.pair_capacity) { d.pair_elem[slot] = e; d.pair_tri[slot] = t; }
     };
@@ -2187,7 +2048,7 @@ __global__ void __launch_bounds__(kBlock) k_ccd_collect(View d)
 // One warp per element queued by k_ccd_collect: lane l tests cached leaf l
 // against the swept box and applies the same FP32 skip bound to that leaf's
 // triangles (the pair order does not matter: the bound is a minimum).
-__global__ void __launch_bounds__(kBlock) k_ccd_near(View d)
+template<bool FILTER> __global__ void __launch_bounds__(kBlock) k_ccd_near(View d)
 {
     const int lane = threadIdx.x & 31;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -2218,10 +2079,14 @@ __global__ void __launch_bounds__(kBlock) k_ccd_near(View d)
             if (!maybe_overlap(qb, a, b) || !leaf_overlap_exact(d, node, a, b, qb)) continue;
             const uint32_t leaf = __float_as_uint(b.w), first = leaf >> 4, cnt = leaf & 15u;
             for (uint32_t p = first; p < first + cnt; ++p) {
-                float m;
                 uint32_t t;
-                const float df = record_distance_f(d, p, origin, f0, f1, m, t);
-                if (__fmul_rd(0.8f, __fsub_rd(__fsub_rd(df, m), target_ru)) >= speed_ru) continue;
+                if (FILTER) {
+                    float m;
+                    const float df = record_distance_f(d, p, origin, f0, f1, m, t);
+                    if (__fmul_rd(0.8f, __fsub_rd(__fsub_rd(df, m), target_ru)) >= speed_ru) continue;
+                } else {
+                    t = __float_as_uint(__ldg(d.tri32 + 3 * size_t(p)).w);
+                }
                 const uint32_t slot = append_slot(&d.sc->pair_count);
                 if (slot < d.pair_capacity) { d.pair_elem[slot] = e; d.pair_tri[slot] = t; }
             }
@@ -2281,7 +2146,7 @@ template<bool MIXED> __global__ void __launch_bounds__(kBlock) k_friction(View d
         const V p0 = load3(d.q + 6 * size_t(i)), p1 = load3(d.q + 6 * size_t(j));
         uint32_t cand = 0, closest;
         dm::ClosestPair pair;
-        if (MIXED && !fi) {
+        if (!fi) {
             // The last gradient evaluation ran the contact pass at this q and
             // this collider state: reuse its closest pair.
             closest = d.c_tri[e];
@@ -2653,7 +2518,11 @@ void Engine::initialize(const Model &m, const KhsSolverDesc &desc, const KhsHair
     bytes += 3 * padded<double>(E) + 2 * padded<uint32_t>(E) + padded<uint8_t>(E);
     bytes += 5 * padded<uint32_t>(S);
     bytes += padded<uint32_t>(3 * T) + 5 * padded<double>(3 * Vn) + padded<float>(3 * Vn);
-    bytes += 2 * padded<float>(3 * B) + padded<float4>(2 * B);
+    bytes += padded<float4>(2 * B);
+    // Pairs of the contact pass: the mixed form keeps one or two candidates of
+    // an element near the surface, the plain form all of them, hundreds at a
+    // mesh pole; a full pool falls back to the search by one thread.
+    const size_t surv_capacity = std::max<size_t>(size_t(1) << 18, 8 * E);
     const size_t pair_capacity = std::min<size_t>(std::max<size_t>(size_t(1) << 20, 8 * E), size_t(16) << 20);
     bytes += 2 * padded<double>(E) + padded<double>(3 * E) + 2 * padded<uint32_t>(pair_capacity);
     bytes += padded<uint32_t>(size_t(kCacheLeaves) * E) + padded<uint8_t>(E);
@@ -2662,8 +2531,8 @@ void Engine::initialize(const Model &m, const KhsSolverDesc &desc, const KhsHair
     bytes += padded<float>(3 * N) + padded<float>(6 * E);
     bytes += padded<uint32_t>(E);
     bytes += 2 * padded<float2>(36 * N) + padded<float2>(6 * N) + padded<float>(N);
-    bytes += 2 * padded<float4>(3 * T) + 2 * padded<uint32_t>(size_t(kSurvivors) * E) + padded<uint8_t>(E) +
-             padded<double>(5 * size_t(kSurvivors) * E);
+    bytes += 2 * padded<float4>(3 * T) + 2 * padded<uint32_t>(surv_capacity) + 2 * padded<uint32_t>(E) +
+             padded<double>(5 * surv_capacity);
     bytes += 2 * padded<double>(3 * B) + 4 * padded<uint32_t>(B) + padded<int32_t>(B) + 2 * padded<uint32_t>(B) +
              padded<uint32_t>(L) + padded<uint32_t>(T);
     bytes += padded<Partial>(kPartials) + padded<DirPartial>(kPartials) + padded<Scalars>(1);
@@ -2707,7 +2576,6 @@ void Engine::initialize(const Model &m, const KhsSolverDesc &desc, const KhsHair
     v.col32 = a.take<float>(3 * Vn);
     I.col_frame_start = a.take<double>(3 * Vn); I.col_pending = a.take<double>(3 * Vn); I.col_a_copy = a.take<double>(3 * Vn);
     v.blo = a.take<double>(3 * B); v.bhi = a.take<double>(3 * B);
-    v.blo32 = a.take<float>(3 * B); v.bhi32 = a.take<float>(3 * B);
     v.bnode = B ? a.take<float4>(2 * B) : nullptr;
     v.c_t = a.take<double>(E); v.c_dist = a.take<double>(E); v.c_bary = a.take<double>(3 * E);
     v.pair_elem = a.take<uint32_t>(pair_capacity); v.pair_tri = a.take<uint32_t>(pair_capacity);
@@ -2718,11 +2586,12 @@ void Engine::initialize(const Model &m, const KhsSolverDesc &desc, const KhsHair
     v.tri32 = a.take<float4>(3 * T); v.tri32_old = a.take<float4>(3 * T);
     v.ff_inv = a.take<float2>(36 * N); v.ff_c = a.take<float2>(36 * N); v.ff_d = a.take<float2>(6 * N);
     v.ff_shift = a.take<float>(N);
-    v.surv_tri = a.take<uint32_t>(size_t(kSurvivors) * E); v.surv_list = a.take<uint32_t>(size_t(kSurvivors) * E);
-    v.surv_n = a.take<uint8_t>(E); v.surv_res = a.take<double>(5 * size_t(kSurvivors) * E);
+    v.surv_elem = a.take<uint32_t>(surv_capacity); v.surv_tri = a.take<uint32_t>(surv_capacity);
+    v.surv_off = a.take<uint32_t>(E); v.surv_n = a.take<uint32_t>(E); v.surv_res = a.take<double>(5 * surv_capacity);
+    v.surv_capacity = uint32_t(surv_capacity);
     v.near_list = a.take<uint32_t>(E);
     if (E) KHS_CUDA(cudaMemsetAsync(v.cache_n, kCacheInvalid, E, I.stream));
-    uint32_t *besc = a.take<uint32_t>(B), *bfirst = a.take<uint32_t>(B), *bcount = a.take<uint32_t>(B);
+    uint32_t *bfirst = a.take<uint32_t>(B), *bcount = a.take<uint32_t>(B);
     v.brefit = a.take<uint32_t>(B);
     int32_t *bparent = a.take<int32_t>(B);
     uint32_t *bleft = a.take<uint32_t>(B), *bright = a.take<uint32_t>(B), *bleaves = a.take<uint32_t>(L);
@@ -2797,7 +2666,6 @@ void Engine::initialize(const Model &m, const KhsSolverDesc &desc, const KhsHair
             lo32[k] = std::nextafter(float(m.bvh.lower[k]), -std::numeric_limits<float>::infinity());
             hi32[k] = std::nextafter(float(m.bvh.upper[k]), std::numeric_limits<float>::infinity());
         }
-        up(v.blo32, lo32.data(), 3 * B * 4); up(v.bhi32, hi32.data(), 3 * B * 4);
         std::vector<float4> packed(2 * B);
         for (size_t k = 0; k < B; ++k) {
             const uint32_t leaf = m.bvh.count[k] ? (m.bvh.first[k] << 4) | m.bvh.count[k] : 0u;
@@ -2809,7 +2677,7 @@ void Engine::initialize(const Model &m, const KhsSolverDesc &desc, const KhsHair
             packed[2 * k + 1] = make_float4(hi32[3 * k], hi32[3 * k + 1], hi32[3 * k + 2], l_f);
         }
         up(v.bnode, packed.data(), 2 * B * sizeof(float4));
-        up(besc, m.bvh.escape.data(), B * 4); up(bfirst, m.bvh.first.data(), B * 4); up(bcount, m.bvh.count.data(), B * 4);
+        up(bfirst, m.bvh.first.data(), B * 4); up(bcount, m.bvh.count.data(), B * 4);
         up(bparent, m.bvh.parent.data(), B * 4); up(bleft, m.bvh.left_child.data(), B * 4);
         up(bright, m.bvh.right_child.data(), B * 4); up(bleaves, m.bvh.leaves.data(), L * 4);
         up(border, m.bvh.order.data(), T * 4);
@@ -2818,7 +2686,7 @@ void Engine::initialize(const Model &m, const KhsSolverDesc &desc, const KhsHair
     v.ref = ref; v.mass = mass; v.rmass = rmass; v.fixed = fixed; v.elem_left = eleft; v.elem_right = eright;
     v.ei = ei; v.ej = ej; v.estrand = es; v.econtact = ec; v.L0 = L0; v.gamma0 = g0; v.kappa0 = k0;
     v.sfirst = sf; v.scount = sc; v.sfixed = sx; v.sorder = so; v.tri = tri;
-    v.besc = besc; v.bfirst = bfirst; v.bcount = bcount; v.border = border; v.bleaves = bleaves; v.bparent = bparent;
+    v.bfirst = bfirst; v.bcount = bcount; v.border = border; v.bleaves = bleaves; v.bparent = bparent;
     v.bleft = bleft; v.bright = bright;
     KHS_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void **>(&v.mail), I.mail_host, 0));
     KHS_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void **>(&v.sweep), I.sweep_host, 0));
@@ -3037,11 +2905,10 @@ EvalStats Engine::evaluate(bool gradient, double dt, double alpha, const double 
     const View &v = I.v;
     const bool trial = alpha >= 0.0 || alpha_dev;
     const double a = alpha >= 0.0 ? alpha : 0.0;
-    if (mode_ && v.has_collider) {
-        // The mixed form's contact passes read only q and its FP32 copy: once
-        // k_positions has written them, the passes run on a second stream
-        // beside the node kernel (on one stream while kernels are timed one by
-        // one).  The same kernels see the same inputs either way.
+    if (v.has_collider) {
+        // The contact passes read only q and its FP32 copy: once k_positions
+        // has written them, the passes run on a second stream beside the node
+        // kernel (on one stream while kernels are timed one by one).  The same kernels see the same inputs either way.
         I.launch("k_positions", k_positions, grid_for(v.N), kBlock, v, trial ? 1 : 0, a, alpha_dev);
         const bool side = !I.profiling;
         const cudaStream_t cs = side ? I.side : I.stream;
@@ -3053,9 +2920,10 @@ EvalStats Engine::evaluate(bool gradient, double dt, double alpha, const double 
         if (rebuild_cache_) KHS_CUDA(cudaMemsetAsync(&v.sc->pool_used, 0, sizeof(uint32_t), cs));
         I.launch_on(cs, rebuild_cache_ ? "k_contact_filter_rebuild" : trial ? "k_contact_filter_trial" : "k_contact_filter",
                     k_contact_filter, grid_for(v.E), kBlock, v, q, rebuild_cache_ ? 1 : 0);
-        I.launch_on(cs, "k_contact_near", k_contact_near, 152 * 8, kBlock, v);
+        I.launch_on(cs, "k_contact_near", mode_ ? k_contact_near<true> : k_contact_near<false>, 152 * 8, kBlock, v);
         I.launch_on(cs, "k_contact_exact", k_contact_exact, 152 * 4, kBlock, v, q);
-        I.launch_on(cs, "k_contact_select", k_contact_select, grid_for(v.E), kBlock, v, q);
+        I.launch_on(cs, "k_contact_select", mode_ ? k_contact_select<true> : k_contact_select<false>, grid_for(v.E),
+                    kBlock, v, q);
         if (side) KHS_CUDA(cudaEventRecord(I.join, I.side));
         I.launch(gradient ? "k_node_eval_grad" : "k_node_eval_energy", k_node_eval, grid_for(v.N), kBlock, v,
                  gradient ? 1 : 0, trial ? 1 : 0, a, dt, alpha_dev, 1);
@@ -3065,8 +2933,7 @@ EvalStats Engine::evaluate(bool gradient, double dt, double alpha, const double 
                  gradient ? 1 : 0, trial ? 1 : 0, a, dt, alpha_dev, 0);
     }
     rebuild_cache_ = false;
-    I.launch(gradient ? "k_elem_eval_grad" : "k_elem_eval_energy", mode_ ? k_elem_eval<true> : k_elem_eval<false>, grid_for(v.E),
-             kBlock, v, gradient ? 1 : 0);
+    I.launch(gradient ? "k_elem_eval_grad" : "k_elem_eval_energy", k_elem_eval, grid_for(v.E), kBlock, v, gradient ? 1 : 0);
     if (gradient) I.launch("k_node_sum", k_node_sum, grid_for(42 * size_t(v.N)), kBlock, v);
     I.launch("k_reduce_eval", k_reduce_eval, kPartials, kBlock, v, gradient ? 1 : 0);
     I.check();
@@ -3238,19 +3105,14 @@ bool Engine::make_direction(KhsxSubstepRecord &rec, double grad_norm2)
     return true;
 }
 
-// The line-search CCD bound of the current direction (the mixed form's
-// FP32-filtered pair list, or the per-element FP64 kernel).
+// The line-search CCD bound of the current direction.
 void Engine::launch_ccd_bound()
 {
     Impl &I = *d_;
     const View &v = I.v;
-    if (mode_) {
-        I.launch("k_ccd_collect", k_ccd_collect, grid_for(v.E), kBlock, v);
-        I.launch("k_ccd_near", k_ccd_near, 152u * 8u, kBlock, v);
-        I.launch("k_ccd_pairs", k_ccd_pairs, 152u * 8u, kBlock, v);
-    } else {
-        I.launch("k_ccd", k_ccd<false>, grid_for(v.E), kBlock, v);
-    }
+    I.launch("k_ccd_collect", mode_ ? k_ccd_collect<true> : k_ccd_collect<false>, grid_for(v.E), kBlock, v);
+    I.launch("k_ccd_near", mode_ ? k_ccd_near<true> : k_ccd_near<false>, 152u * 8u, kBlock, v);
+    I.launch("k_ccd_pairs", k_ccd_pairs, 152u * 8u, kBlock, v);
 }
 
 KhsResult Engine::optimize_substep(double dt, KhsxSubstepRecord &rec)
@@ -3323,7 +3185,7 @@ KhsResult Engine::optimize_substep(double dt, KhsxSubstepRecord &rec)
                 first_alpha = lim;
                 if (first_alpha < 1.0) first_alpha *= 0.9;
             }
-            const bool overflow = mode_ && v.has_collider && mb.pair_count > v.pair_capacity;
+            const bool overflow = v.has_collider && mb.pair_count > v.pair_capacity;
             // The direction was limited to the trust radius on the device.
             const bool scaled = max_translation > trust_radius_;
             pipelined = used && !overflow && first_alpha >= desc_.minimum_line_search_step;
@@ -3369,9 +3231,9 @@ KhsResult Engine::optimize_substep(double dt, KhsxSubstepRecord &rec)
                 I.launch("k_final_dir", k_final_dir, 1, kBlock, v, 0);
                 I.check();
                 I.sync();
-                if (mode_ && v.has_collider && I.mail_host->pair_count > v.pair_capacity) {
+                if (v.has_collider && I.mail_host->pair_count > v.pair_capacity) {
                     // Work list overflow: redo the bound with the per-element kernel.
-                    I.launch("k_ccd", k_ccd<true>, grid_for(v.E), kBlock, v);
+                    I.launch("k_ccd", mode_ ? k_ccd<true> : k_ccd<false>, grid_for(v.E), kBlock, v);
                     I.launch("k_final_dir", k_final_dir, 1, kBlock, v, 0);
                     I.check();
                     I.sync();
