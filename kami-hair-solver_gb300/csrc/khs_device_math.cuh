@@ -17,8 +17,10 @@
 
 #if defined(__CUDACC__)
 #define KHS_HD __host__ __device__ __forceinline__
+#define KHS_HD_SLOW inline __host__ __device__ __noinline__  // a rare path, kept out of line
 #else
 #define KHS_HD inline
+#define KHS_HD_SLOW inline
 #endif
 
 namespace khs {
@@ -347,32 +349,71 @@ struct ClosestPair {
     V bary;
 };
 
-KHS_HD V closest_point_triangle(V p, V a, V b, V c, V &bary)
+#if defined(__CUDA_ARCH__)
+KHS_HD uint64_t bits_of(double x) { return uint64_t(__double_as_longlong(x)); }
+KHS_HD double double_of(uint64_t b) { return __longlong_as_double((long long)b); }
+KHS_HD uint32_t bits_of(float x) { return __float_as_uint(x); }
+KHS_HD float float_of(uint32_t b) { return __uint_as_float(b); }
+#else
+KHS_HD uint64_t bits_of(double x) { uint64_t b; std::memcpy(&b, &x, 8); return b; }
+KHS_HD double double_of(uint64_t b) { double x; std::memcpy(&x, &b, 8); return x; }
+KHS_HD uint32_t bits_of(float x) { uint32_t b; std::memcpy(&b, &x, 4); return b; }
+KHS_HD float float_of(uint32_t b) { float x; std::memcpy(&x, &b, 4); return x; }
+#endif
+
+// Comparisons of the closest-point code.  On GB300 an FP64 comparison takes an
+// FP64 issue slot (64 cycles) like a multiply-add, and fmin / fmax several, so
+// FAST decides on the bits with integer instructions.  The answers are those
+// of the floating comparisons for everything but NaN (zeros of either sign
+// and infinities included); callers take FAST only for coordinates that
+// sane_coordinate admits, which cannot produce a NaN before the last division.
+template<bool FAST> KHS_HD bool le0(double x) { return FAST ? int64_t(bits_of(x)) <= 0 : x <= 0; }
+template<bool FAST> KHS_HD bool ge0(double x) { return FAST ? bits_of(x) <= 0x8000000000000000ull : x >= 0; }
+template<bool FAST> KHS_HD bool lt0(double x) { return FAST ? bits_of(x) > 0x8000000000000000ull : x < 0; }
+// x <= y for y >= 0.
+template<bool FAST> KHS_HD bool le_nonneg(double x, double y)
+{
+    return FAST ? int64_t(bits_of(x)) <= int64_t(bits_of(y) & 0x7fffffffffffffffull) : x <= y;
+}
+template<bool FAST> KHS_HD bool nonzero(double x) { return FAST ? (bits_of(x) << 1) != 0 : x != 0; }
+template<bool FAST> KHS_HD bool gt1(double x) { return FAST ? int64_t(bits_of(x)) > 0x3ff0000000000000ll : x > 1; }
+// fmin(1, fmax(0, x)).
+template<bool FAST> KHS_HD double clamp01(double x)
+{
+    if (!FAST) return fmin(1.0, fmax(0.0, x));
+    return int64_t(bits_of(x)) <= 0 ? 0.0 : (gt1<true>(x) ? 1.0 : x);
+}
+// Finite and below 2^200: sums of products of four differences stay finite.
+KHS_HD bool sane_coordinate(double x) { return (uint32_t(bits_of(x) >> 32) & 0x7fffffffu) < ((1023u + 200u) << 20); }
+KHS_HD bool sane(V a) { return sane_coordinate(a.x) && sane_coordinate(a.y) && sane_coordinate(a.z); }
+
+template<bool FAST> KHS_HD V closest_point_triangle(V p, V a, V b, V c, V &bary)
 {
     const V ab = gsub(b, a), ac = gsub(c, a), ap = gsub(p, a);
     const double d1 = gdot(ab, ap), d2 = gdot(ac, ap);
-    if (d1 <= 0 && d2 <= 0) { bary = v(1, 0, 0); return a; }
+    if (le0<FAST>(d1) && le0<FAST>(d2)) { bary = v(1, 0, 0); return a; }
     const V bp = gsub(p, b);
     const double d3 = gdot(ab, bp), d4 = gdot(ac, bp);
-    if (d3 >= 0 && d4 <= d3) { bary = v(0, 1, 0); return b; }
+    if (ge0<FAST>(d3) && le_nonneg<FAST>(d4, d3)) { bary = v(0, 1, 0); return b; }
     const double vc = xs(xm(d1, d4), xm(d3, d2));
-    if (vc <= 0 && d1 >= 0 && d3 <= 0) {
+    if (le0<FAST>(vc) && ge0<FAST>(d1) && le0<FAST>(d3)) {
         const double w = d1 / xs(d1, d3);
         bary = v(xs(1.0, w), w, 0);
         return gadd(a, gmul(ab, w));
     }
     const V cp = gsub(p, c);
     const double d5 = gdot(ab, cp), d6 = gdot(ac, cp);
-    if (d6 >= 0 && d5 <= d6) { bary = v(0, 0, 1); return c; }
+    if (ge0<FAST>(d6) && le_nonneg<FAST>(d5, d6)) { bary = v(0, 0, 1); return c; }
     const double vb = xs(xm(d5, d2), xm(d1, d6));
-    if (vb <= 0 && d2 >= 0 && d6 <= 0) {
+    if (le0<FAST>(vb) && ge0<FAST>(d2) && le0<FAST>(d6)) {
         const double w = d2 / xs(d2, d6);
         bary = v(xs(1.0, w), 0, w);
         return gadd(a, gmul(ac, w));
     }
     const double va = xs(xm(d3, d6), xm(d5, d4));
-    if (va <= 0 && xs(d4, d3) >= 0 && xs(d5, d6) >= 0) {
-        const double w = xs(d4, d3) / xa(xs(d4, d3), xs(d5, d6));
+    const double d43 = xs(d4, d3), d56 = xs(d5, d6);
+    if (le0<FAST>(va) && ge0<FAST>(d43) && ge0<FAST>(d56)) {
+        const double w = d43 / xa(d43, d56);
         bary = v(0, xs(1.0, w), w);
         return gadd(b, gmul(gsub(c, b), w));
     }
@@ -381,54 +422,101 @@ KHS_HD V closest_point_triangle(V p, V a, V b, V c, V &bary)
     return gadd(gadd(a, gmul(ab, vv)), gmul(ac, ww));
 }
 
-KHS_HD void segment_segment_params(V p1, V q1, V p2, V q2, double &s, double &t)
+template<bool FAST> KHS_HD void segment_segment_params(V p1, V q1, V p2, V q2, double &s, double &t)
 {
     const V d1 = gsub(q1, p1), d2 = gsub(q2, p2), r = gsub(p1, p2);
     const double a = gdot(d1, d1), e = gdot(d2, d2), f = gdot(d2, r);
     s = 0.0; t = 0.0;
-    if (a <= 1e-14 && e <= 1e-14) return;
-    if (a <= 1e-14) { t = fmin(1.0, fmax(0.0, f / e)); return; }
+    const bool point1 = le_nonneg<FAST>(a, 1e-14), point2 = le_nonneg<FAST>(e, 1e-14);
+    if (point1 && point2) return;
+    if (point1) { t = clamp01<FAST>(f / e); return; }
     const double c = gdot(d1, r);
-    if (e <= 1e-14) { s = fmin(1.0, fmax(0.0, -c / a)); return; }
+    if (point2) { s = clamp01<FAST>(-c / a); return; }
     const double b = gdot(d1, d2), den = xs(xm(a, e), xm(b, b));
-    if (den != 0) s = fmin(1.0, fmax(0.0, xs(xm(b, f), xm(c, e)) / den));
+    if (nonzero<FAST>(den)) s = clamp01<FAST>(xs(xm(b, f), xm(c, e)) / den);
     t = xa(xm(b, s), f) / e;
-    if (t < 0) { t = 0; s = fmin(1.0, fmax(0.0, -c / a)); }
-    else if (t > 1) { t = 1; s = fmin(1.0, fmax(0.0, xs(b, c) / a)); }
+    if (lt0<FAST>(t)) { t = 0; s = clamp01<FAST>(-c / a); }
+    else if (gt1<FAST>(t)) { t = 1; s = clamp01<FAST>(xs(b, c) / a); }
 }
 
 // Closest pair between segment p0-p1 and triangle abc: end points against
 // the face, then the segment against the three edges, keeping the first
 // strictly smaller distance.  No interior-crossing test (device semantics of
 // the reference).
+//
+// The five tests as parts of their own, so that threads can share a pair:
+// part 0 and 1 the end points, 2 ... 4 the edges.  dist2 is the squared
+// distance before the square root.
+struct PairPart {
+    double dist2, t;
+    V bary;
+};
+
+template<bool FAST> KHS_HD PairPart point_part(V p, double t, V a, V b, V c)
+{
+    PairPart out;
+    const V cp = closest_point_triangle<FAST>(p, a, b, c, out.bary);
+    const V w = gsub(p, cp);
+    out.dist2 = gdot(w, w);
+    out.t = t;
+    return out;
+}
+
+template<bool FAST> KHS_HD PairPart edge_part(int e, V p0, V p1, V a, V b, V c)
+{
+    const V p2 = e == 0 ? a : (e == 1 ? b : c);
+    const V q2 = e == 0 ? b : (e == 1 ? c : a);
+    PairPart out;
+    double t;
+    segment_segment_params<FAST>(p0, p1, p2, q2, out.t, t);
+    const V w = gsub(gadd(p0, gmul(gsub(p1, p0), out.t)), gadd(p2, gmul(gsub(q2, p2), t)));
+    out.dist2 = gdot(w, w);
+    const double u = xs(1.0, t);
+    out.bary = e == 0 ? v(u, t, 0) : (e == 1 ? v(0, u, t) : v(t, 0, u));
+    return out;
+}
+
+template<bool FAST> KHS_HD PairPart pair_part(int part, V p0, V p1, V a, V b, V c)
+{
+    return part < 2 ? point_part<FAST>(part ? p1 : p0, part ? 1.0 : 0.0, a, b, c) : edge_part<FAST>(part - 2, p0, p1, a, b, c);
+}
+
+// sqrt(x) < sqrt(best) of two squared distances, or NaN (never smaller), for
+// best >= 0 and not NaN.  The rounded square root does not decrease, and more
+// than 16 units in the last place apart it differs; closer ones are compared
+// as roots.
+KHS_HD bool root_less(double x, double best)
+{
+    const uint64_t bx = bits_of(x), bb = bits_of(best);
+    if (bx >= bb) return false;  // NaN included
+    return bb - bx > 16 || sqrt(x) < sqrt(best);
+}
+
+template<bool FAST> KHS_HD ClosestPair closest_of_parts(V p0, V p1, V a, V b, V c)
+{
+    // No part found: the distance stays at 1e300, whose square is infinite.
+    PairPart best;
+    best.dist2 = double_of(0x7ff0000000000000ull); best.t = 0.0; best.bary = v(1, 0, 0);
+#pragma unroll
+    for (int part = 0; part < 5; ++part) {
+        const PairPart x = pair_part<FAST>(part, p0, p1, a, b, c);
+        if (root_less(x.dist2, best.dist2)) best = x;
+    }
+    ClosestPair out;
+    out.distance = bits_of(best.dist2) < 0x7ff0000000000000ull ? sqrt(best.dist2) : 1.0e300;
+    out.t = best.t;
+    out.bary = best.bary;
+    return out;
+}
+KHS_HD_SLOW ClosestPair closest_of_parts_slow(V p0, V p1, V a, V b, V c) { return closest_of_parts<false>(p0, p1, a, b, c); }
+KHS_HD_SLOW PairPart pair_part_slow(int part, V p0, V p1, V a, V b, V c) { return pair_part<false>(part, p0, p1, a, b, c); }
+
+KHS_HD bool sane_pair(V p0, V p1, V a, V b, V c) { return sane(p0) && sane(p1) && sane(a) && sane(b) && sane(c); }
+
 KHS_HD ClosestPair closest_segment_triangle(V p0, V p1, V a, V b, V c)
 {
-    ClosestPair out;
-    out.distance = 1.0e300; out.t = 0.0; out.bary = v(1, 0, 0);
-    V bary;
-    V cp = closest_point_triangle(p0, a, b, c, bary);
-    double d = gnorm(gsub(p0, cp));
-    if (d < out.distance) { out.distance = d; out.t = 0.0; out.bary = bary; }
-    cp = closest_point_triangle(p1, a, b, c, bary);
-    d = gnorm(gsub(p1, cp));
-    if (d < out.distance) { out.distance = d; out.t = 1.0; out.bary = bary; }
-    const V d1 = gsub(p1, p0);
-#pragma unroll
-    for (int e = 0; e < 3; ++e) {
-        const V p2 = e == 0 ? a : (e == 1 ? b : c);
-        const V q2 = e == 0 ? b : (e == 1 ? c : a);
-        double s, t;
-        segment_segment_params(p0, p1, p2, q2, s, t);
-        const double dd = gnorm(gsub(gadd(p0, gmul(d1, s)), gadd(p2, gmul(gsub(q2, p2), t))));
-        if (dd < out.distance) {
-            out.distance = dd;
-            out.t = s;
-            if (e == 0) out.bary = v(xs(1.0, t), t, 0);
-            else if (e == 1) out.bary = v(0, xs(1.0, t), t);
-            else out.bary = v(t, 0, xs(1.0, t));
-        }
-    }
-    return out;
+    if (!sane_pair(p0, p1, a, b, c)) return closest_of_parts_slow(p0, p1, a, b, c);
+    return closest_of_parts<true>(p0, p1, a, b, c);
 }
 
 // ---- FP32 filters for the mixed form -----------------------------------
@@ -733,10 +821,6 @@ KHS_HD float recip_seed(float m)
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(m));
     return r;
 }
-KHS_HD uint64_t bits_of(double x) { return uint64_t(__double_as_longlong(x)); }
-KHS_HD double double_of(uint64_t b) { return __longlong_as_double((long long)b); }
-KHS_HD uint32_t bits_of(float x) { return __float_as_uint(x); }
-KHS_HD float float_of(uint32_t b) { return __uint_as_float(b); }
 #else
 KHS_HD int32_t smulhi32(int32_t a, int32_t b) { return int32_t((int64_t(a) * b) >> 32); }
 // Host seed: the correctly rounded float reciprocal (tests may substitute a
@@ -745,10 +829,6 @@ KHS_HD int32_t smulhi32(int32_t a, int32_t b) { return int32_t((int64_t(a) * b) 
 #define KHS_RECIP_SEED_HOST(m) (1.0f / (m))
 #endif
 KHS_HD float recip_seed(float m) { return KHS_RECIP_SEED_HOST(m); }
-KHS_HD uint64_t bits_of(double x) { uint64_t b; std::memcpy(&b, &x, 8); return b; }
-KHS_HD double double_of(uint64_t b) { double x; std::memcpy(&x, &b, 8); return x; }
-KHS_HD uint32_t bits_of(float x) { uint32_t b; std::memcpy(&b, &x, 4); return b; }
-KHS_HD float float_of(uint32_t b) { float x; std::memcpy(&x, &b, 4); return x; }
 #endif
 
 // The reciprocal where it is normal too (2^-1022 <= |x| < 2^1022), without

@@ -359,6 +359,28 @@ __device__ uint32_t collect_leaves(const View &d, V lo, V hi, double pad, uint32
     return n;
 }
 
+// Collects the leaves around (lo, hi) into the element's cache slots; returns
+// its cache_n.  More than kCacheLeaves, at a dense patch of the collider (a
+// mesh pole, a seam), go to the pool, which the warp passes take 32 at a time.
+__device__ __forceinline__ uint8_t leaves_to_cache(const View &d, uint32_t e, V lo, V hi, double pad)
+{
+    uint32_t *slots = d.cache_leaf + size_t(kCacheLeaves) * e;
+    const uint32_t c = collect_leaves(d, lo, hi, pad, slots, kCacheLeaves);
+    uint8_t nl = uint8_t(c);
+    if (c > uint32_t(kCacheLeaves)) {
+        const uint32_t off = atomicAdd(&d.sc->pool_used, c);
+        nl = kCacheInvalid;
+        if (size_t(off) + c <= d.leaf_pool_capacity) {
+            collect_leaves(d, lo, hi, pad, d.leaf_pool + off, c);
+            slots[0] = off;
+            slots[1] = c;
+            nl = kCacheBig;
+        }
+    }
+    d.cache_n[e] = nl;
+    return nl;
+}
+
 // The cached leaf list of element e with cache state nl (its cache_n):
 // the element's own slots, or its range of the leaf pool; nullptr without
 // a cache.
@@ -487,9 +509,6 @@ __global__ void __launch_bounds__(kBlock) k_refit(View d, int swept)
 // Conservative advancement of each moving triangle against the stationary
 // hair at the start of the substep (cuda_backend.cu:975-987).  Returns the
 // first failing triangle of this element in traversal order.
-// Mixed form: a candidate whose FP32 lower-bound clearance already lets the
-// first advancement step reach alpha = 1 cannot fail and is skipped (the
-// 1e-6 relative slack dwarfs the FP64 rounding of that one step).
 // FP32 pre-test of the mixed sweep for the candidate at leaf-order position
 // p: true when the first conservative-advancement step of the exact pass is
 // certain to reach the end of the substep (no failure from this triangle).
@@ -522,12 +541,11 @@ __device__ __forceinline__ bool sweep_skip_f(const View &d, uint32_t p, dm::F3 o
     return __fmul_rd(0.8f, __fsub_rd(__fsub_rd(df, m), target_ru)) >= __fmul_ru(speed_ub, 1.000002f);
 }
 
-template<bool MIXED> __device__ bool sweep_element(const View &d, uint32_t e, SweepRecord *rec)
+__device__ bool sweep_element(const View &d, uint32_t e, SweepRecord *rec)
 {
     const uint32_t i = d.ei[e], j = d.ej[e];
     const V p0 = load3(d.q + 6 * size_t(i)), p1 = load3(d.q + 6 * size_t(j));
     const double target = d.radius + d.offset + d.min_gap;
-    const dm::F3 f0 = dm::f3(0.f, 0.f, 0.f), f1 = dm::to_local(p1, p0);
     bool failed = false;
     bvh_query_packed(d, dm::vmin(p0, p1), dm::vmax(p0, p1), target, [&](uint32_t t) {
         if (failed) return;
@@ -537,12 +555,6 @@ template<bool MIXED> __device__ bool sweep_element(const View &d, uint32_t e, Sw
                 dc = dm::gsub(tri_vertex(d, t, 2), oc);
         const double speed = fmax(dm::gnorm(da), fmax(dm::gnorm(db), dm::gnorm(dc)));
         if (speed < 1e-30) return;
-        if (MIXED) {
-            float m;
-            const float df = dm::segment_triangle_distance_f(f0, f1, dm::to_local(oa, p0), dm::to_local(ob, p0),
-                                                              dm::to_local(oc, p0), m);
-            if (0.8 * (double(df) - double(m) - target) >= speed * (1.0 + 1e-6)) return;
-        }
         double alpha = 0.0;
         bool end = false;
         dm::ClosestPair pair;
@@ -569,64 +581,12 @@ template<bool MIXED> __device__ bool sweep_element(const View &d, uint32_t e, Sw
     return failed;
 }
 
-// Mixed sweep of one element: the same candidates in the same order as
-// sweep_element, with sweep_skip_f deciding first from FP32 copies, so only
-// the triangles that could fail are loaded and advanced in FP64.
-__device__ bool sweep_element_f(const View &d, uint32_t e)
-{
-    const uint32_t i = d.ei[e], j = d.ej[e];
-    const V p0 = load3(d.q + 6 * size_t(i)), p1 = load3(d.q + 6 * size_t(j));
-    const double target = d.radius + d.offset + d.min_gap;
-    const float target_ru = __double2float_ru(target);
-    const dm::F3 origin = dm::f3(float(p0.x), float(p0.y), float(p0.z));
-    const dm::F3 f1 = dm::f3(float(p1.x) - origin.x, float(p1.y) - origin.y, float(p1.z) - origin.z);
-    bool failed = false;
-    bvh_positions_packed(d, make_query(dm::vmin(p0, p1), dm::vmax(p0, p1), target), [&](uint32_t p) {
-        if (failed || sweep_skip_f(d, p, origin, f1, target_ru)) return;
-        const uint32_t t = __float_as_uint(__ldg(d.tri32 + 3 * size_t(p)).w);
-        const V oa = load3(d.col_old + 3 * size_t(d.tri[3 * t])), ob = load3(d.col_old + 3 * size_t(d.tri[3 * t + 1])),
-                oc = load3(d.col_old + 3 * size_t(d.tri[3 * t + 2]));
-        const V da = dm::gsub(tri_vertex(d, t, 0), oa), db = dm::gsub(tri_vertex(d, t, 1), ob),
-                dc = dm::gsub(tri_vertex(d, t, 2), oc);
-        const double speed = fmax(dm::gnorm(da), fmax(dm::gnorm(db), dm::gnorm(dc)));
-        if (speed < 1e-30) return;
-        double alpha = 0.0;
-        bool end = false;
-        for (int k = 0; k < 80; ++k) {
-            const V a = dm::gadd(oa, dm::gmul(da, alpha)), b = dm::gadd(ob, dm::gmul(db, alpha)), c = dm::gadd(oc, dm::gmul(dc, alpha));
-            const double clearance = dm::closest_segment_triangle(p0, p1, a, b, c).distance - target;
-            if (clearance <= 0) { failed = true; break; }
-            const double advance = 0.8 * clearance / speed;
-            if (alpha + advance >= 1) { end = true; break; }
-            if (advance < 1e-12) { failed = true; break; }
-            alpha += advance;
-        }
-        if (!end) failed = true;
-    });
-    return failed;
-}
-
-template<bool MIXED> __global__ void __launch_bounds__(kBlock) k_sweep(View d)
+__global__ void __launch_bounds__(kBlock) k_sweep(View d)
 {
     const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= d.E) return;
     if (d.fixed[d.ei[e]] || !d.econtact[e]) return;
-    const bool failed = MIXED ? sweep_element_f(d, e) : sweep_element<false>(d, e, nullptr);
-    if (failed) atomicMin(&d.sc->sweep_fail, e);
-}
-
-// Publishes the lowest failing element of k_sweep (with its first failing
-// triangle in traversal order) and re-arms the atomic.
-__global__ void k_sweep_record(View d)
-{
-    if (threadIdx.x || blockIdx.x) return;
-    const uint32_t e = d.sc->sweep_fail;
-    d.sc->sweep_fail = kNone;
-    d.mail->sweep_fail = e;
-    if (e == kNone) return;
-    SweepRecord rec{};
-    sweep_element<false>(d, e, &rec);
-    *d.sweep = rec;
+    if (sweep_element(d, e, nullptr)) atomicMin(&d.sc->sweep_fail, e);
 }
 
 // Diagonal preconditioner (cuda_backend.cu:815-841): node term then the
@@ -923,45 +883,33 @@ __device__ __forceinline__ bool within_cache_slack(const float *c, dm::F3 xi, dm
            fabsf(xj.x - c[3]) <= s && fabsf(xj.y - c[4]) <= s && fabsf(xj.z - c[5]) <= s;
 }
 
-// q must be d.q (its FP32 copy d.q32 is read).  cache 1: collect every
-// element's leaves; 0: only where the element has left its slack.
+// The element's cached leaves: collected around its box grown by the slack
+// (always with force, else where it has left the slack), so that the passes of
+// many evaluations read a short list.  Returns cache_n.  q must be d.q (its
+// FP32 copy d.q32 is read).
+__device__ __forceinline__ uint8_t refresh_leaves(const View &d, const double *q, uint32_t e, uint32_t i, uint32_t j, bool force)
+{
+    const dm::F3 xi32 = dm::f3(d.q32[3 * size_t(i)], d.q32[3 * size_t(i) + 1], d.q32[3 * size_t(i) + 2]);
+    const dm::F3 xj32 = dm::f3(d.q32[3 * size_t(j)], d.q32[3 * size_t(j) + 1], d.q32[3 * size_t(j) + 2]);
+    float *c32 = d.cache_x32 + 6 * size_t(e);
+    uint8_t nl = d.cache_n[e];
+    if (!force && nl != kCacheInvalid && within_cache_slack(c32, xi32, xj32)) return nl;
+    const V xi = load3(q + 6 * size_t(i)), xj = load3(q + 6 * size_t(j));
+    const V s3 = dm::v(kCacheSlack, kCacheSlack, kCacheSlack);
+    nl = leaves_to_cache(d, e, dm::vmin(xi, xj) - s3, dm::vmax(xi, xj) + s3, d.radius + d.offset + d.dhat);
+    c32[0] = xi32.x; c32[1] = xi32.y; c32[2] = xi32.z; c32[3] = xj32.x; c32[4] = xj32.y; c32[5] = xj32.z;
+    return nl;
+}
+
+// cache 1: collect every element's leaves (the first evaluation of a
+// substep); 0: only where the element has left its slack.
 __global__ void __launch_bounds__(kBlock) k_contact_filter(View d, const double *q, int cache)
 {
     const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= d.E) return;
     const uint32_t i = d.ei[e], j = d.ej[e];
     if (!d.fixed[i] && d.econtact[e]) {
-        const dm::F3 xi32 = dm::f3(d.q32[3 * size_t(i)], d.q32[3 * size_t(i) + 1], d.q32[3 * size_t(i) + 2]);
-        const dm::F3 xj32 = dm::f3(d.q32[3 * size_t(j)], d.q32[3 * size_t(j) + 1], d.q32[3 * size_t(j) + 2]);
-        float *c32 = d.cache_x32 + 6 * size_t(e);
-        uint8_t nl = d.cache_n[e];
-        if (cache == 1 || nl == kCacheInvalid || !within_cache_slack(c32, xi32, xj32)) {
-            // (Re)collect the leaves around the element box grown by the
-            // slack, so that the passes of many evaluations read a short list.
-            const V xi = load3(q + 6 * size_t(i)), xj = load3(q + 6 * size_t(j));
-            const double pad = d.radius + d.offset + d.dhat;
-            const V s3 = dm::v(kCacheSlack, kCacheSlack, kCacheSlack);
-            const V clo = dm::vmin(xi, xj) - s3, chi = dm::vmax(xi, xj) + s3;
-            uint32_t *slots = d.cache_leaf + size_t(kCacheLeaves) * e;
-            const uint32_t c = collect_leaves(d, clo, chi, pad, slots, kCacheLeaves);
-            if (c <= uint32_t(kCacheLeaves)) {
-                nl = uint8_t(c);
-            } else {
-                // A dense patch of the collider (a mesh pole, a seam): the
-                // list goes to the pool, and k_contact_near works through it
-                // 32 leaves at a time.
-                const uint32_t off = atomicAdd(&d.sc->pool_used, c);
-                nl = kCacheInvalid;
-                if (size_t(off) + c <= d.leaf_pool_capacity) {
-                    collect_leaves(d, clo, chi, pad, d.leaf_pool + off, c);
-                    slots[0] = off;
-                    slots[1] = c;
-                    nl = kCacheBig;
-                }
-            }
-            d.cache_n[e] = nl;
-            c32[0] = xi32.x; c32[1] = xi32.y; c32[2] = xi32.z; c32[3] = xj32.x; c32[4] = xj32.y; c32[5] = xj32.z;
-        }
+        const uint8_t nl = refresh_leaves(d, q, e, i, j, cache == 1);
         if (nl == kCacheInvalid) {  // the leaf pool is full
             d.surv_n[e] = kSurvOverflow;
             return;
@@ -970,6 +918,8 @@ __global__ void __launch_bounds__(kBlock) k_contact_filter(View d, const double 
             d.near_list[append_slot(&d.sc->near_count)] = e;
             return;
         }
+    } else if (cache == 1 && !d.fixed[j] && d.econtact[e]) {
+        refresh_leaves(d, q, e, i, j, true);  // for k_friction_collect
     }
     d.c_cand[e] = 0;
     d.surv_n[e] = 0;
@@ -1165,17 +1115,75 @@ template<bool FILTER> __global__ void __launch_bounds__(kBlock) k_contact_near(V
     }
 }
 
-__global__ void __launch_bounds__(kBlock) k_contact_exact(View d, const double *q)
+// FP64 passes over pairs: a block of five warps takes 32 pairs, warp w part w
+// of each (the segment's ends against the face, the segment against an edge),
+// so the parts of a pair run on as many sub-partitions and no lane waits for
+// another's kind of part.  A whole pair in one thread is a chain of some 600
+// FP64 instructions of 64 cycles (54 us for however few pairs); a part is
+// about 80, with its comparisons on the integer pipes.
+constexpr int kPairWarps = 5, kPairBlock = 32 * kPairWarps;
+constexpr unsigned kPairGrid = 152 * 4;
+
+__device__ __forceinline__ dm::PairPart part_of(bool fast, int part, V p0, V p1, V a, V b, V c)
 {
+    return fast ? dm::pair_part<true>(part, p0, p1, a, b, c) : dm::pair_part_slow(part, p0, p1, a, b, c);
+}
+
+__global__ void __launch_bounds__(kPairBlock) k_contact_exact(View d, const double *q)
+{
+    __shared__ double sh[kPairWarps][5][32];
+    const int part = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t count = min(d.sc->surv_count, d.surv_capacity);
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
-        const uint32_t e = d.surv_elem[k], t = d.surv_tri[k];
-        const uint32_t i = d.ei[e], j = d.ej[e];
-        const V xi = load3(q + 6 * size_t(i)), xj = load3(q + 6 * size_t(j));
-        const dm::ClosestPair c = dm::closest_segment_triangle(xi, xj, tri_vertex(d, t, 0), tri_vertex(d, t, 1), tri_vertex(d, t, 2));
-        double *r = d.surv_res + 5 * size_t(k);
-        r[0] = c.distance; r[1] = c.t; r[2] = c.bary.x; r[3] = c.bary.y; r[4] = c.bary.z;
+    for (uint32_t base = 32 * blockIdx.x; base < count; base += 32 * gridDim.x) {
+        const uint32_t k = base + lane;
+        if (k < count) {
+            const uint32_t e = d.surv_elem[k], t = d.surv_tri[k];
+            const V xi = load3(q + 6 * size_t(d.ei[e])), xj = load3(q + 6 * size_t(d.ej[e]));
+            const V a = tri_vertex(d, t, 0), b = tri_vertex(d, t, 1), c = tri_vertex(d, t, 2);
+            const dm::PairPart x = part_of(dm::sane_pair(xi, xj, a, b, c), part, xi, xj, a, b, c);
+            sh[part][0][lane] = x.dist2; sh[part][1][lane] = x.t;
+            sh[part][2][lane] = x.bary.x; sh[part][3][lane] = x.bary.y; sh[part][4][lane] = x.bary.z;
+        }
+        __syncthreads();
+        if (part == 0 && k < count) {
+            double best = __longlong_as_double(0x7ff0000000000000ll);
+            int from = -1;
+#pragma unroll
+            for (int w = 0; w < kPairWarps; ++w)
+                if (dm::root_less(sh[w][0][lane], best)) { best = sh[w][0][lane]; from = w; }
+            double *r = d.surv_res + 5 * size_t(k);
+            r[0] = from < 0 ? 1.0e300 : sqrt(best);
+#pragma unroll
+            for (int f = 1; f < 5; ++f) r[f] = from < 0 ? (f == 2 ? 1.0 : 0.0) : sh[from][f][lane];
+        }
+        __syncthreads();
     }
+}
+
+// The first strictly closest of element e's n pairs, or the search by one
+// thread where a pool was full (which also counts the candidates).
+template<bool FILTER>
+__device__ __forceinline__ uint32_t select_pair(const View &d, const double *q, uint32_t e, uint32_t n, dm::ClosestPair &pair)
+{
+    pair.distance = 1.0e300; pair.t = 0.0; pair.bary = dm::v(1, 0, 0);
+    if (n == kSurvOverflow) {
+        const uint32_t i = d.ei[e], j = d.ej[e];
+        uint32_t cand = 0;
+        const uint32_t closest = closest_triangle<FILTER>(d, load3(q + 6 * size_t(i)), load3(q + 6 * size_t(j)),
+                                                          d.radius + d.offset + d.dhat, cand, pair);
+        d.c_cand[e] = cand;
+        return closest;
+    }
+    const uint32_t off = n ? d.surv_off[e] : 0;
+    uint32_t best = kNone;
+    for (uint32_t k = off; k < off + n; ++k) {
+        const double dist = d.surv_res[5 * size_t(k)];
+        if (dist < pair.distance) { pair.distance = dist; best = k; }
+    }
+    if (best == kNone) return kNone;
+    const double *r = d.surv_res + 5 * size_t(best);
+    pair.t = r[1]; pair.bary = dm::v(r[2], r[3], r[4]);
+    return d.surv_tri[best];
 }
 
 template<bool FILTER> __global__ void __launch_bounds__(kBlock) k_contact_select(View d, const double *q)
@@ -1189,28 +1197,7 @@ template<bool FILTER> __global__ void __launch_bounds__(kBlock) k_contact_select
     const uint32_t n = d.surv_n[e];
     if (n == 0) return;
     dm::ClosestPair pair;
-    pair.distance = 1.0e300; pair.t = 0.0; pair.bary = dm::v(1, 0, 0);
-    uint32_t closest = kNone;
-    if (n == kSurvOverflow) {
-        // A pool is full: the search over all candidates by one thread.
-        const uint32_t i = d.ei[e], j = d.ej[e];
-        uint32_t cand = 0;
-        closest = closest_triangle<FILTER>(d, load3(q + 6 * size_t(i)), load3(q + 6 * size_t(j)), d.radius + d.offset + d.dhat,
-                                           cand, pair);
-        d.c_cand[e] = cand;
-    } else {
-        const uint32_t off = d.surv_off[e];
-        uint32_t best = kNone;
-        for (uint32_t k = off; k < off + n; ++k) {
-            const double dist = d.surv_res[5 * size_t(k)];
-            if (dist < pair.distance) { pair.distance = dist; best = k; }
-        }
-        if (best != kNone) {
-            const double *r = d.surv_res + 5 * size_t(best);
-            pair.t = r[1]; pair.bary = dm::v(r[2], r[3], r[4]);
-            closest = d.surv_tri[best];
-        }
-    }
+    const uint32_t closest = select_pair<FILTER>(d, q, e, n, pair);
     write_contact(d, e, closest, pair);
 }
 
@@ -1983,10 +1970,8 @@ template<bool MIXED> __global__ void __launch_bounds__(kBlock) k_ccd(View d)
 // CCD bound, load balanced: k_ccd_collect and k_ccd_near list every (element,
 // triangle) candidate, in the mixed form (FILTER) without those whose FP32
 // lower-bound clearance already lets the first advancement step reach
-// alpha = 1; k_ccd_pairs runs the exact FP64 conservative advancement of
-// cuda_backend.cu:989-1000 per listed pair and stops a pair once 0.9 alpha
-// reaches the global minimum found so far (every limit the pair could still
-// produce is >= 0.9 alpha).  The minimum equals the per-element kernel's
+// alpha = 1; k_advance_pairs runs the exact FP64 conservative advancement
+// of cuda_backend.cu:989-1000 per listed pair.  The minimum equals the per-element kernel's
 // (k_ccd), which remains for a full pair list.
 // Candidates of the swept element box (positions at step 0 and 1) whose
 // FP32 lower-bound distance does not rule out a limit below 1: a pair is
@@ -2094,34 +2079,191 @@ template<bool FILTER> __global__ void __launch_bounds__(kBlock) k_ccd_near(View 
     }
 }
 
-__global__ void __launch_bounds__(kBlock) k_ccd_pairs(View d)
+// Conservative advancement of the listed pairs, 32 to a block of five warps as
+// in k_contact_exact: in each of at most 80 steps the warps take the parts of
+// the distance at the pair's alpha, and warp 0 moves it on.  SWEEP: the
+// triangle moves from its old position and the hair stands (the pair's element
+// fails unless alpha reaches 1); else the hair moves by its direction and the
+// triangle stands (the pair's limit bounds the step).
+template<bool SWEEP> __global__ void __launch_bounds__(kPairBlock) k_advance_pairs(View d)
 {
+    __shared__ double sh_d2[kPairWarps][32], sh_alpha[32];
+    __shared__ uint32_t sh_active;
+    const int part = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t count = min(d.sc->pair_count, d.pair_capacity);
     const double target = d.radius + d.offset + d.min_gap;
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
-        const uint32_t e = d.pair_elem[k], t = d.pair_tri[k];
-        const uint32_t i = d.ei[e], j = d.ej[e];
-        const V p0 = load3(d.q + 6 * size_t(i)), p1 = load3(d.q + 6 * size_t(j));
-        const V d0 = load3(d.dir + 6 * size_t(i)), d1 = load3(d.dir + 6 * size_t(j));
-        const double speed = fmax(dm::gnorm(d0), dm::gnorm(d1));
-        const V a = tri_vertex(d, t, 0), b = tri_vertex(d, t, 1), c = tri_vertex(d, t, 2);
-        double limit = 2.0;  // no limit
-        double alpha = 0.0;
-        const double bound = __longlong_as_double(*reinterpret_cast<volatile long long *>(&d.sc->ccd_bits));
-        bool done = false;
-        for (int it = 0; it < 80 && !done; ++it) {
-            if (0.9 * alpha >= bound) { done = true; break; }
-            const double dist = dm::closest_segment_triangle(dm::gadd(p0, dm::gmul(d0, alpha)), dm::gadd(p1, dm::gmul(d1, alpha)), a, b, c).distance;
-            const double clear = dist - target;
-            if (clear <= 0) { limit = fmax(0.0, alpha * 0.9); done = true; break; }
-            const double advance = 0.8 * clear / speed;
-            if (alpha + advance >= 1) { done = true; break; }
-            if (advance < 1e-12) { limit = alpha; done = true; break; }
-            alpha += advance;
+    for (uint32_t base = 32 * blockIdx.x; base < count; base += 32 * gridDim.x) {
+        const uint32_t k = base + lane;
+        uint32_t e = 0;
+        V p0 = dm::v(0, 0, 0), p1 = p0, a = p0, b = p0, c = p0;  // at alpha 0
+        V m0 = p0, m1 = p0, m2 = p0;                             // what alpha moves: p0, p1 or a, b, c
+        bool fast = false;
+        double speed = 0.0;
+        if (k < count) {
+            e = d.pair_elem[k];
+            const uint32_t t = d.pair_tri[k], i = d.ei[e], j = d.ej[e];
+            p0 = load3(d.q + 6 * size_t(i)); p1 = load3(d.q + 6 * size_t(j));
+            a = tri_vertex(d, t, 0); b = tri_vertex(d, t, 1); c = tri_vertex(d, t, 2);
+            if (SWEEP) {
+                const V oa = load3(d.col_old + 3 * size_t(d.tri[3 * t])), ob = load3(d.col_old + 3 * size_t(d.tri[3 * t + 1])),
+                        oc = load3(d.col_old + 3 * size_t(d.tri[3 * t + 2]));
+                fast = dm::sane_pair(p0, p1, a, b, c) && dm::sane(oa) && dm::sane(ob) && dm::sane(oc);
+                m0 = dm::gsub(a, oa); m1 = dm::gsub(b, ob); m2 = dm::gsub(c, oc);
+                a = oa; b = ob; c = oc;
+            } else {
+                m0 = load3(d.dir + 6 * size_t(i)); m1 = load3(d.dir + 6 * size_t(j));
+                fast = dm::sane_pair(p0, p1, a, b, c) && dm::sane(m0) && dm::sane(m1);
+            }
         }
-        if (!done) limit = alpha;
-        if (limit < 1.0) atomicMin(&d.sc->ccd_bits, (unsigned long long)__double_as_longlong(limit));
+        double alpha = 0.0;
+        if (part == 0) {
+            speed = SWEEP ? fmax(dm::gnorm(m0), fmax(dm::gnorm(m1), dm::gnorm(m2))) : fmax(dm::gnorm(m0), dm::gnorm(m1));
+            bool on = k < count;
+            // Every limit a pair can still produce is >= 0.9 alpha, so it
+            // stops as soon as that reaches the smallest limit found so far.
+            if (SWEEP) on = on && !(speed < 1e-30);
+            else on = on && __longlong_as_double(*reinterpret_cast<volatile long long *>(&d.sc->ccd_bits)) > 0.0;
+            const uint32_t active = __ballot_sync(0xffffffffu, on);
+            sh_alpha[lane] = 0.0;
+            if (lane == 0) sh_active = active;
+        }
+        __syncthreads();
+        for (int it = 0; it < 80; ++it) {
+            const uint32_t active = sh_active;
+            if (active == 0) break;
+            const bool on = active >> lane & 1u;
+            double bound = 0.0;
+            if (!SWEEP && part == 0) bound = __longlong_as_double(*reinterpret_cast<volatile long long *>(&d.sc->ccd_bits));
+            if (on) {
+                alpha = sh_alpha[lane];
+                dm::PairPart x;
+                if (SWEEP)
+                    x = part_of(fast, part, p0, p1, dm::gadd(a, dm::gmul(m0, alpha)), dm::gadd(b, dm::gmul(m1, alpha)),
+                                dm::gadd(c, dm::gmul(m2, alpha)));
+                else
+                    x = part_of(fast, part, dm::gadd(p0, dm::gmul(m0, alpha)), dm::gadd(p1, dm::gmul(m1, alpha)), a, b, c);
+                sh_d2[part][lane] = x.dist2;
+            }
+            __syncthreads();
+            if (part == 0) {
+                bool more = false;
+                if (on) {
+                    unsigned long long least = 0x7ff0000000000000ull;  // smallest squared distance; NaN never is
+#pragma unroll
+                    for (int w = 0; w < kPairWarps; ++w) {
+                        const unsigned long long x = (unsigned long long)__double_as_longlong(sh_d2[w][lane]);
+                        least = x < least ? x : least;
+                    }
+                    const double dist = least == 0x7ff0000000000000ull ? 1.0e300 : sqrt(__longlong_as_double((long long)least));
+                    const double clear = dist - target;
+                    double limit = 2.0;  // none
+                    bool failed = false;
+                    if (clear <= 0) {
+                        limit = fmax(0.0, alpha * 0.9);
+                        failed = true;
+                    } else {
+                        const double advance = 0.8 * clear / speed;
+                        if (alpha + advance >= 1) {
+                        } else if (advance < 1e-12) {
+                            limit = alpha;
+                            failed = true;
+                        } else {
+                            alpha += advance;
+                            more = it < 79 && (SWEEP || !(0.9 * alpha >= bound));
+                            if (it == 79) {
+                                limit = alpha;
+                                failed = true;
+                            }
+                        }
+                    }
+                    if (SWEEP) {
+                        if (failed) atomicMin(&d.sc->sweep_fail, e);
+                    } else if (limit < 1.0) {
+                        atomicMin(&d.sc->ccd_bits, (unsigned long long)__double_as_longlong(limit));
+                    }
+                    sh_alpha[lane] = alpha;
+                }
+                const uint32_t next = __ballot_sync(0xffffffffu, more);
+                if (lane == 0) sh_active = next;
+            }
+            __syncthreads();
+        }
+        __syncthreads();
     }
+}
+
+// ---- moving-collider sweep ------------------------------------------------
+//
+// k_sweep_collect (thread per element): the leaves of the swept BVH (boxes of
+// old and new positions) around the standing element, into its cache slots,
+// which the substep's first evaluation fills anew.  k_sweep_near (warp per
+// element with leaves): exact leaf tests; every candidate, in the mixed form
+// without those that sweep_skip_f clears, goes to the pair list.
+// k_advance_pairs<true>: the FP64 advancement a pair.  k_sweep_record publishes
+// the lowest failing element.  k_sweep, one thread per element for all of it
+// (1.3 ms on 67,000 elements, 3.0 ms on 3,200 among contacts in the plain
+// form), remains for a full pair list.
+__global__ void __launch_bounds__(kBlock) k_sweep_collect(View d)
+{
+    const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= d.E) return;
+    const uint32_t i = d.ei[e], j = d.ej[e];
+    if (d.fixed[i] || !d.econtact[e]) return;
+    const V p0 = load3(d.q + 6 * size_t(i)), p1 = load3(d.q + 6 * size_t(j));
+    const uint8_t nl = leaves_to_cache(d, e, dm::vmin(p0, p1), dm::vmax(p0, p1), d.radius + d.offset + d.min_gap);
+    if (nl == kCacheInvalid) {  // the leaf pool is full
+        if (sweep_element(d, e, nullptr)) atomicMin(&d.sc->sweep_fail, e);
+    } else if (nl > 0) {
+        d.near_list[append_slot(&d.sc->ccd_near)] = e;
+    }
+}
+
+template<bool FILTER> __global__ void __launch_bounds__(kBlock) k_sweep_near(View d)
+{
+    const int lane = threadIdx.x & 31;
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t count = d.sc->ccd_near;
+    const double target = d.radius + d.offset + d.min_gap;
+    const float target_ru = __double2float_ru(target);
+    for (uint32_t k = warp; k < count; k += nwarps) {
+        const uint32_t e = d.near_list[k];
+        uint32_t nleaves = 0;
+        const uint32_t *leaves = cached_leaves(d, e, d.cache_n[e], nleaves);
+        if (uint32_t(lane) >= nleaves) continue;
+        const V p0 = load3(d.q + 6 * size_t(d.ei[e])), p1 = load3(d.q + 6 * size_t(d.ej[e]));
+        const QueryBox qb = make_query(dm::vmin(p0, p1), dm::vmax(p0, p1), target);
+        const dm::F3 origin = dm::f3(float(p0.x), float(p0.y), float(p0.z));
+        const dm::F3 f1 = dm::f3(float(p1.x) - origin.x, float(p1.y) - origin.y, float(p1.z) - origin.z);
+        for (uint32_t c = lane; c < nleaves; c += 32) {
+            uint32_t first, cnt;
+            near_leaf(d, leaves, c, nleaves, qb, first, cnt);
+            for (uint32_t p = first; p < first + cnt; ++p) {
+                if (FILTER && sweep_skip_f(d, p, origin, f1, target_ru)) continue;
+                const uint32_t slot = append_slot(&d.sc->pair_count);
+                if (slot < d.pair_capacity) {
+                    d.pair_elem[slot] = e;
+                    d.pair_tri[slot] = __float_as_uint(__ldg(d.tri32 + 3 * size_t(p)).w);
+                }
+            }
+        }
+    }
+}
+
+// Publishes the lowest failing element of the sweep (with its first failing
+// triangle in traversal order) and the length of the pair list, and re-arms.
+__global__ void k_sweep_record(View d)
+{
+    if (threadIdx.x || blockIdx.x) return;
+    const uint32_t e = d.sc->sweep_fail;
+    d.mail->pair_count = d.sc->pair_count;
+    d.sc->pair_count = 0;
+    d.sc->ccd_near = 0;
+    d.sc->sweep_fail = kNone;
+    d.mail->sweep_fail = e;
+    if (e == kNone) return;
+    SweepRecord rec{};
+    sweep_element(d, e, &rec);
+    *d.sweep = rec;
 }
 
 // ---- end of substep -------------------------------------------------------
@@ -2133,18 +2275,42 @@ __global__ void __launch_bounds__(kBlock) k_update_velocity(View d, double inv_d
     for (int k = 0; k < 6; ++k) d.v[6 * size_t(n) + k] = (d.q[6 * size_t(n) + k] - d.q_old[6 * size_t(n) + k]) * inv_dt;
 }
 
-// Coulomb friction impulse (cuda_backend.cu:941-964); each element writes
-// its velocity change into its left/right node slots.
-template<bool MIXED> __global__ void __launch_bounds__(kBlock) k_friction(View d, double dt)
+// The elements between a fixed and a free node take part in friction but not
+// in the evaluations' contact pass: their leaves (collected with the others')
+// are queued here for k_contact_near and k_contact_exact, and k_friction
+// selects their pairs and clears their records.
+__device__ __forceinline__ bool friction_root(const View &d, uint32_t e, uint32_t i, uint32_t j)
+{
+    return d.fixed[i] && !d.fixed[j] && d.econtact[e];
+}
+
+__global__ void __launch_bounds__(kBlock) k_friction_collect(View d)
 {
     const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= d.E) return;
+    const uint32_t i = d.ei[e], j = d.ej[e];
+    if (!friction_root(d, e, i, j)) return;
+    const uint8_t nl = refresh_leaves(d, d.q, e, i, j, false);
+    d.surv_n[e] = nl == kCacheInvalid ? kSurvOverflow : 0;
+    if (nl != kCacheInvalid && nl > 0) d.near_list[append_slot(&d.sc->near_count)] = e;
+}
+
+// Coulomb friction impulse (cuda_backend.cu:941-964); each element writes
+// its velocity change into its left/right node slots.
+template<bool FILTER> __global__ void __launch_bounds__(kBlock) k_friction(View d, double dt)
+{
+    const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e == 0) {  // k_contact_near and k_contact_exact, their only readers, have completed
+        d.sc->surv_count = 0;
+        d.sc->near_count = 0;
+    }
     if (e >= d.E) return;
     const uint32_t i = d.ei[e], j = d.ej[e];
     double di[3] = {0, 0, 0}, dj[3] = {0, 0, 0};
     const bool fi = d.fixed[i], fj = d.fixed[j];
     if (d.econtact[e] && !(fi && fj)) {
         const V p0 = load3(d.q + 6 * size_t(i)), p1 = load3(d.q + 6 * size_t(j));
-        uint32_t cand = 0, closest;
+        uint32_t closest;
         dm::ClosestPair pair;
         if (!fi) {
             // The last gradient evaluation ran the contact pass at this q and
@@ -2152,7 +2318,8 @@ template<bool MIXED> __global__ void __launch_bounds__(kBlock) k_friction(View d
             closest = d.c_tri[e];
             pair.t = d.c_t[e]; pair.distance = d.c_dist[e]; pair.bary = load3(d.c_bary + 3 * size_t(e));
         } else {
-            closest = closest_triangle<MIXED>(d, p0, p1, d.radius + d.offset + d.dhat, cand, pair);
+            closest = select_pair<FILTER>(d, d.q, e, d.surv_n[e], pair);
+            d.c_cand[e] = 0; d.c_tri[e] = kNone; d.c_flags[e] = 0; d.c_gap[e] = 0.0;
         }
         const double gap = pair.distance - d.radius - d.offset;
         if (closest != kNone && gap > 0.0 && gap < d.dhat) {
@@ -2921,7 +3088,7 @@ EvalStats Engine::evaluate(bool gradient, double dt, double alpha, const double 
         I.launch_on(cs, rebuild_cache_ ? "k_contact_filter_rebuild" : trial ? "k_contact_filter_trial" : "k_contact_filter",
                     k_contact_filter, grid_for(v.E), kBlock, v, q, rebuild_cache_ ? 1 : 0);
         I.launch_on(cs, "k_contact_near", mode_ ? k_contact_near<true> : k_contact_near<false>, 152 * 8, kBlock, v);
-        I.launch_on(cs, "k_contact_exact", k_contact_exact, 152 * 4, kBlock, v, q);
+        I.launch_on(cs, "k_contact_exact", k_contact_exact, kPairGrid, kPairBlock, v, q);
         I.launch_on(cs, "k_contact_select", mode_ ? k_contact_select<true> : k_contact_select<false>, grid_for(v.E),
                     kBlock, v, q);
         if (side) KHS_CUDA(cudaEventRecord(I.join, I.side));
@@ -3112,7 +3279,7 @@ void Engine::launch_ccd_bound()
     const View &v = I.v;
     I.launch("k_ccd_collect", mode_ ? k_ccd_collect<true> : k_ccd_collect<false>, grid_for(v.E), kBlock, v);
     I.launch("k_ccd_near", mode_ ? k_ccd_near<true> : k_ccd_near<false>, 152u * 8u, kBlock, v);
-    I.launch("k_ccd_pairs", k_ccd_pairs, 152u * 8u, kBlock, v);
+    I.launch("k_ccd_pairs", k_advance_pairs<false>, kPairGrid, kPairBlock, v);
 }
 
 KhsResult Engine::optimize_substep(double dt, KhsxSubstepRecord &rec)
@@ -3359,10 +3526,20 @@ KhsResult Engine::run_frame(double frame_dt, const double *root_a, const double 
                 I.launch("k_tri32", k_tri32, grid_for(v.T), kBlock, v);
                 I.launch("k_refit", k_refit, grid_for(v.L), kBlock, v, 1);
                 progress_phase_.store(KHS_PHASE_CCD);
-                I.launch("k_sweep", mode_ ? k_sweep<true> : k_sweep<false>, grid_for(v.E), kBlock, v);
+                KHS_CUDA(cudaMemsetAsync(&v.sc->pool_used, 0, sizeof(uint32_t), I.stream));
+                I.launch("k_sweep_collect", k_sweep_collect, grid_for(v.E), kBlock, v);
+                I.launch("k_sweep_near", mode_ ? k_sweep_near<true> : k_sweep_near<false>, 152u * 8u, kBlock, v);
+                I.launch("k_sweep_pairs", k_advance_pairs<true>, kPairGrid, kPairBlock, v);
                 I.launch("k_sweep_record", k_sweep_record, 1, 1, v);
                 I.check();
                 I.sync();
+                if (I.mail_host->pair_count > v.pair_capacity) {
+                    // Pair list overflow: every element by one thread.
+                    I.launch("k_sweep", k_sweep, grid_for(v.E), kBlock, v);
+                    I.launch("k_sweep_record", k_sweep_record, 1, 1, v);
+                    I.check();
+                    I.sync();
+                }
                 if (I.mail_host->sweep_fail != kNone) {
                     const SweepRecord &sr = *I.sweep_host;
                     set_failure_context(KHS_FAILURE_MOVING_COLLIDER_SWEEP, frame, sub, substeps, maximum, attempts);
@@ -3394,6 +3571,9 @@ KhsResult Engine::run_frame(double frame_dt, const double *root_a, const double 
                 break;
             }
             if (v.has_collider && material_.friction > 0.0) {
+                I.launch("k_friction_collect", k_friction_collect, grid_for(v.E), kBlock, v);
+                I.launch("k_contact_near", mode_ ? k_contact_near<true> : k_contact_near<false>, 152 * 8, kBlock, v);
+                I.launch("k_contact_exact", k_contact_exact, kPairGrid, kPairBlock, v, v.q);
                 I.launch("k_friction", mode_ ? k_friction<true> : k_friction<false>, grid_for(v.E), kBlock, v, dt);
                 I.launch("k_friction_apply", k_friction_apply, grid_for(v.N), kBlock, v);
             }
