@@ -79,6 +79,126 @@ KHS_HD V mvec(const M &a, V x)
              a.m[6] * x.x + a.m[7] * x.y + a.m[8] * x.z);
 }
 
+#if defined(__CUDA_ARCH__)
+KHS_HD uint64_t bits_of(double x) { return uint64_t(__double_as_longlong(x)); }
+KHS_HD double double_of(uint64_t b) { return __longlong_as_double((long long)b); }
+KHS_HD uint32_t bits_of(float x) { return __float_as_uint(x); }
+KHS_HD float float_of(uint32_t b) { return __uint_as_float(b); }
+#else
+KHS_HD uint64_t bits_of(double x) { uint64_t b; std::memcpy(&b, &x, 8); return b; }
+KHS_HD double double_of(uint64_t b) { double x; std::memcpy(&x, &b, 8); return x; }
+KHS_HD uint32_t bits_of(float x) { uint32_t b; std::memcpy(&b, &x, 4); return b; }
+KHS_HD float float_of(uint32_t b) { float x; std::memcpy(&x, &b, 4); return x; }
+#endif
+
+// ---- correctly rounded reciprocal on the integer pipes -----------------
+//
+// 1/x rounded to nearest, computed without FP64 instructions: on GB300 one
+// FP64 warp instruction occupies a sub-partition's pipe for ~64 cycles, and a
+// reciprocal is on the chain of every pivot step of the block solve.
+// For x = (-1)^s * M * 2^(E-1075) with M the 53-bit significand,
+// 1/x = (-1)^s * T * 2^(970-E) with T = 2^105 / M in (2^52, 2^53]:
+// * seed: an FP32 reciprocal of the top 24 bits of M as the integer
+//   t ~ 2^23 * 2^52 / M, so T0 = 2^30 t; its relative error e = 1 - T0 / T
+//   is below 2^-20 (one ulp of the seed, the bits of M cut off, the rounding
+//   of t, and three further ulps of the seed to spare);
+// * residual: d = 2^75 - t M = 2^75 e, exact in 64 bits modulo 2^64 (2^75
+//   vanishes, |d| < 2^55), so one 24 x 53 bit product;
+// * Q = T0 (1 + e + e^2), rounded to an integer: e carried to 2^-62, e^2
+//   from the top 27 bits of d; with the cubic term left out the sum is within
+//   0.01 of T before the rounding, so Q is the nearest integer or next to it;
+// * the remainder R = 2^105 - Q M (exact modulo 2^64, |R| < 2^53) moves Q by
+//   one where |R| > M / 2.  No ties: M is odd times a power of two and T
+//   has more bits than a midpoint, or M = 2^52 and R = 0.
+// The steps are chosen for latency: 156 cycles of dependent instructions
+// (the FP64 reciprocal takes 352, the 128-bit form this replaces 382).  Reciprocals below the normal range (|x| >= 2^1022) are rounded from
+// floor(T) and its remainder to nearest-even on a branch of their own.
+// The result equals the IEEE division 1.0 / x for every finite normal x
+// (against 1.0 / x on the host, tests/native/test_recip.cpp); zero,
+// subnormal and non-finite inputs give an unspecified bit pattern (the block
+// solve fails such pivots before using the result).
+#if defined(__CUDA_ARCH__)
+KHS_HD int32_t smulhi32(int32_t a, int32_t b) { return __mulhi(a, b); }
+KHS_HD float recip_seed(float m)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(m));
+    return r;
+}
+#else
+KHS_HD int32_t smulhi32(int32_t a, int32_t b) { return int32_t((int64_t(a) * b) >> 32); }
+// Host seed: the correctly rounded float reciprocal (tests may substitute a
+// perturbed one through KHS_RECIP_SEED_HOST).
+#ifndef KHS_RECIP_SEED_HOST
+#define KHS_RECIP_SEED_HOST(m) (1.0f / (m))
+#endif
+KHS_HD float recip_seed(float m) { return KHS_RECIP_SEED_HOST(m); }
+#endif
+
+// The reciprocal where it is normal too (2^-1022 <= |x| < 2^1022), without
+// a branch.  Q and nR: the rounded T and minus its remainder.
+KHS_HD double recip_normal(double x, uint64_t &Q, int64_t &nR)
+{
+    const uint64_t b = bits_of(x);
+    const uint32_t hi = uint32_t(b >> 32), mlo = uint32_t(b);
+    const uint32_t E = (hi >> 20) & 0x7ff, mhi = (hi & 0xfffffu) | 0x100000u;
+    const uint64_t M = (uint64_t(mhi) << 32) | mlo, half = M >> 1;
+    const float seed = recip_seed(float_of((127u << 23) | ((hi << 3 | mlo >> 29) & 0x7fffffu)));
+    // 2^23 * seed as an integer: the bits of 1 + seed count it from those of 1.
+    const uint32_t t = bits_of(1.0f + seed) - 0x3f800000u;
+    // -d, and s = 2^62 (e + e^2) from it.
+    const uint64_t tm = uint64_t(t) * mlo;
+    const int64_t nd = int64_t((uint64_t(uint32_t(tm >> 32) + t * mhi) << 32) | uint32_t(tm));
+    const int32_t dh = int32_t(nd >> 28);
+    const int64_t s = int64_t(smulhi32(dh, dh)) - (nd >> 13);
+    // Q = round(2^30 t + t s / 2^32), the low and high words of s apart.
+    const uint64_t low = uint64_t(t) * uint32_t(s) + 0x80000000u;
+    Q = (uint64_t(t) << 30) + uint64_t(int64_t(int32_t(t)) * int32_t(s >> 32)) + (low >> 32);
+    nR = int64_t(Q * M);
+    // Q counts its implicit bit into the exponent field (Q = 2^53 as well).
+    const uint64_t out = (b & 0x8000000000000000ull) | ((uint64_t(2044 - E) << 52) + Q);
+    const uint64_t above = out + 1, below = out - 1;
+    return double_of(nR < -int64_t(half) ? above : (nR > int64_t(half) ? below : out));
+}
+KHS_HD double recip_normal(double x)
+{
+    uint64_t Q;
+    int64_t nR;
+    return recip_normal(x, Q, nR);
+}
+
+KHS_HD double recip_rn(double x)
+{
+    uint64_t F;
+    int64_t nR;
+    const double normal = recip_normal(x, F, nR);
+    const uint64_t b = bits_of(x);
+    const int E = int((b >> 52) & 0x7ff);
+    if (E < 2045) return normal;
+    // floor(T) and the remainder below M, then the subnormal's bits.
+    const int64_t M = int64_t((b & 0xfffffffffffffull) | (1ull << 52));
+    int64_t R = -nR;
+    if (R < 0) { --F; R += M; }
+    if (R >= M) { ++F; R -= M; }
+    const int k = E - 2044;
+    const uint64_t mant = F >> k;
+    const uint64_t dropped = F & ((1ull << k) - 1), mid = 1ull << (k - 1);
+    const bool up = dropped > mid || (dropped == mid && (R > 0 || (mant & 1)));
+    return double_of((b & 0x8000000000000000ull) | (mant + uint64_t(up)));
+}
+
+// 1 / x with the integer-pipe reciprocal where it is exact and the division
+// elsewhere (zero, subnormal, not finite, a result below the normal range).
+KHS_HD double recip_any(double x)
+{
+#if defined(__CUDA_ARCH__)
+    const uint32_t E = uint32_t(bits_of(x) >> 52) & 0x7ffu;
+    return E - 1u < 2044u ? recip_normal(x) : 1.0 / x;
+#else
+    return 1.0 / x;
+#endif
+}
+
 // Rotation R = exp([u]x) Ref with the reference's Rodrigues coefficients and
 // small-angle Taylor branch below theta^2 = 1e-10 (cuda_backend.cu:130-136).
 // Also returns the left Jacobian Jl(u), defined by
@@ -89,7 +209,7 @@ KHS_HD void rotation_and_jacobian(V u, const double *ref, M &R, M *Jl)
 {
     const double t2 = dot(u, u);
     double a, b;
-    double s;
+    double s, t = 0.0, it = 0.0;
     if (t2 < 1.0e-10) {
         a = 1.0 - t2 / 6.0 + t2 * t2 / 120.0;
         b = 0.5 - t2 / 24.0 + t2 * t2 / 720.0;
@@ -97,7 +217,8 @@ KHS_HD void rotation_and_jacobian(V u, const double *ref, M &R, M *Jl)
     } else {
         // Half-angle form: one sincos, and 1 - cos t = 2 sin^2(t/2) without
         // cancellation (it is also the left Jacobian's coefficient p).
-        const double t = sqrt(t2), it = 1.0 / t;
+        t = sqrt(t2);
+        it = recip_any(t);
         double sh, ch;
         sincos(0.5 * t, &sh, &ch);
         s = 2.0 * sh * ch;
@@ -123,7 +244,6 @@ KHS_HD void rotation_and_jacobian(V u, const double *ref, M &R, M *Jl)
             p = 0.5 - t2 / 24.0 + t2 * t2 / 720.0 - t2 * t2 * t2 / 40320.0;
             r = 1.0 / 6.0 - t2 / 120.0 + t2 * t2 / 5040.0 - t2 * t2 * t2 / 362880.0;
         } else {
-            const double t = sqrt(t2), it = 1.0 / t;
             p = b;
             r = (t - s) * (it * it * it);
         }
@@ -165,14 +285,18 @@ KHS_HD Weights strain_weights(double radius, double young, double poisson, doubl
 //   with K = ((tr Q) I - Q) / s + 2 c c^T / s^2, Q = Ri^T Rj, c = axial(Q),
 //   s = 1 + (tr Q - 1) / 2 + 1e-12 (differential of the regularised Cayley
 //   map along dQ = [w]x Q).
+// The Jacobian blocks, A, S and T with the factors of a half left out: a
+// product with a power of two is exact, so the sums that use them take it up
+// in their other factor without a change of rounding (A2 = 2 A, S2 = 2 d gamma
+// / d u).
 struct ElementJacobian {
-    M A, Sgi, Sgj, Kki, Kkj;
+    M A2, S2i, S2j, Kki, Kkj;
 };
 
-KHS_HD void element_strain(const M &Ri, const M &Rj, V xi, V xj, double L0, V gamma0, V kappa0, double eps[6],
-                           ElementJacobian *J, const M *Jli, const M *Jlj)
+// invL = 1 / L0.
+KHS_HD void element_strain_inv(const M &Ri, const M &Rj, V xi, V xj, double invL, V gamma0, V kappa0, double eps[6],
+                               ElementJacobian *J, const M *Jli, const M *Jlj)
 {
-    const double invL = 1.0 / L0;
     const V t = (xj - xi) * invL;
     M S;  // Ri^T + Rj^T
 #pragma unroll
@@ -181,21 +305,19 @@ KHS_HD void element_strain(const M &Ri, const M &Rj, V xi, V xj, double L0, V ga
         for (int c = 0; c < 3; ++c) S.m[3 * r + c] = Ri.m[3 * c + r] + Rj.m[3 * c + r];
     const V shear = mvec(S, t) * 0.5;
     const M Q = mtmul(Ri, Rj);
-    const V ax = v((Q.m[7] - Q.m[5]) * 0.5, (Q.m[2] - Q.m[6]) * 0.5, (Q.m[3] - Q.m[1]) * 0.5);
+    const V ax2 = v(Q.m[7] - Q.m[5], Q.m[2] - Q.m[6], Q.m[3] - Q.m[1]);  // 2 axial(Q)
     const double trQ = Q.m[0] + Q.m[4] + Q.m[8];
     const double s = 1.0 + (trQ - 1.0) * 0.5 + 1.0e-12;
-    const double f = 2.0 / s;
+    const double is = recip_any(s);
     eps[0] = shear.x - gamma0.x;
     eps[1] = shear.y - gamma0.y;
     eps[2] = shear.z - gamma0.z;
-    eps[3] = ax.x * f * invL - kappa0.x;
-    eps[4] = ax.y * f * invL - kappa0.y;
-    eps[5] = ax.z * f * invL - kappa0.z;
+    eps[3] = ax2.x * is * invL - kappa0.x;
+    eps[4] = ax2.y * is * invL - kappa0.y;
+    eps[5] = ax2.z * is * invL - kappa0.z;
     if (!J) return;
-    // A = 0.5 (Ri + Rj)^T / L0
-    const double hl = 0.5 * invL;
 #pragma unroll
-    for (int k = 0; k < 9; ++k) J->A.m[k] = S.m[k] * hl;
+    for (int k = 0; k < 9; ++k) J->A2.m[k] = S.m[k] * invL;
     // [t]x Jl: column k = t x Jl_col(k)
     M TJi, TJj;
 #pragma unroll
@@ -205,14 +327,12 @@ KHS_HD void element_strain(const M &Ri, const M &Rj, V xi, V xj, double L0, V ga
         TJi.m[k] = ci.x; TJi.m[3 + k] = ci.y; TJi.m[6 + k] = ci.z;
         TJj.m[k] = cj.x; TJj.m[3 + k] = cj.y; TJj.m[6 + k] = cj.z;
     }
-    J->Sgi = mtmul(Ri, TJi);
-    J->Sgj = mtmul(Rj, TJj);
-#pragma unroll
-    for (int k = 0; k < 9; ++k) { J->Sgi.m[k] *= 0.5; J->Sgj.m[k] *= 0.5; }
-    // K
+    J->S2i = mtmul(Ri, TJi);
+    J->S2j = mtmul(Rj, TJj);
+    // K = ((tr Q) I - Q) / s + 2 c c^T / s^2 with c = ax2 / 2
     M K;
-    const double is = 1.0 / s, is2 = 2.0 * is * is;
-    const double axv[3] = {ax.x, ax.y, ax.z};
+    const double is2 = 0.5 * is * is;
+    const double axv[3] = {ax2.x, ax2.y, ax2.z};
 #pragma unroll
     for (int r = 0; r < 3; ++r)
 #pragma unroll
@@ -224,12 +344,32 @@ KHS_HD void element_strain(const M &Ri, const M &Rj, V xi, V xj, double L0, V ga
     for (int k = 0; k < 9; ++k) { J->Kki.m[k] *= -invL; J->Kkj.m[k] *= invL; }
 }
 
+KHS_HD void element_strain(const M &Ri, const M &Rj, V xi, V xj, double L0, V gamma0, V kappa0, double eps[6],
+                           ElementJacobian *J, const M *Jli, const M *Jlj)
+{
+    element_strain_inv(Ri, Rj, xi, xj, 1.0 / L0, gamma0, kappa0, eps, J, Jli, Jlj);
+}
+
+// Half the weights times the length; the first two strains' weights are equal
+// and so are the fourth's and fifth's (strain_weights).
+struct HalfWeights {
+    double shear, stretch, bend, twist;
+};
+KHS_HD HalfWeights half_weights(const Weights &w, double L0)
+{
+    HalfWeights h;
+    h.shear = 0.5 * L0 * w.w[0]; h.stretch = 0.5 * L0 * w.w[2]; h.bend = 0.5 * L0 * w.w[3]; h.twist = 0.5 * L0 * w.w[5];
+    return h;
+}
+
 // Elastic energy 0.5 L0 sum w eps^2.
 KHS_HD double element_energy(const double eps[6], const Weights &w, double L0)
 {
+    const HalfWeights h = half_weights(w, L0);
+    const double hw[6] = {h.shear, h.shear, h.stretch, h.bend, h.bend, h.twist};
     double e = 0.0;
 #pragma unroll
-    for (int s = 0; s < 6; ++s) e += (0.5 * L0 * w.w[s]) * eps[s] * eps[s];
+    for (int s = 0; s < 6; ++s) e += hw[s] * eps[s] * eps[s];
     return e;
 }
 
@@ -238,32 +378,21 @@ KHS_HD double element_energy(const double eps[6], const Weights &w, double L0)
 KHS_HD void element_gradient(const ElementJacobian &J, const double eps[6], const Weights &w, double L0, double gi[6],
                              double gj[6])
 {
-    double se[3], ke[3];
+    const HalfWeights h = half_weights(w, L0);
+    const double hs[3] = {h.shear, h.shear, h.stretch}, hb[3] = {h.bend, h.bend, h.twist};
+    double se[3], ke[3];  // se: half of L0 w eps, for A2 and S2
 #pragma unroll
-    for (int k = 0; k < 3; ++k) { se[k] = L0 * w.w[k] * eps[k]; ke[k] = L0 * w.w[3 + k] * eps[3 + k]; }
+    for (int k = 0; k < 3; ++k) { se[k] = hs[k] * eps[k]; ke[k] = 2.0 * (hb[k] * eps[3 + k]); }
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        const double ax = J.A.m[c] * se[0] + J.A.m[3 + c] * se[1] + J.A.m[6 + c] * se[2];
+        const double ax = J.A2.m[c] * se[0] + J.A2.m[3 + c] * se[1] + J.A2.m[6 + c] * se[2];
         gi[c] = -ax;
         gj[c] = ax;
-        gi[3 + c] = J.Sgi.m[c] * se[0] + J.Sgi.m[3 + c] * se[1] + J.Sgi.m[6 + c] * se[2] +
+        gi[3 + c] = J.S2i.m[c] * se[0] + J.S2i.m[3 + c] * se[1] + J.S2i.m[6 + c] * se[2] +
                     J.Kki.m[c] * ke[0] + J.Kki.m[3 + c] * ke[1] + J.Kki.m[6 + c] * ke[2];
-        gj[3 + c] = J.Sgj.m[c] * se[0] + J.Sgj.m[3 + c] * se[1] + J.Sgj.m[6 + c] * se[2] +
+        gj[3 + c] = J.S2j.m[c] * se[0] + J.S2j.m[3 + c] * se[1] + J.S2j.m[6 + c] * se[2] +
                     J.Kkj.m[c] * ke[0] + J.Kkj.m[3 + c] * ke[1] + J.Kkj.m[6 + c] * ke[2];
     }
-}
-
-// X^T diag(d) Y for 3x3 X, Y.
-KHS_HD void xtdy(const M &X, const double d[3], const M &Y, double *out, int ld, bool accumulate, double sign)
-{
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const double h = X.m[r] * d[0] * Y.m[c] + X.m[3 + r] * d[1] * Y.m[3 + c] + X.m[6 + r] * d[2] * Y.m[6 + c];
-            if (accumulate) out[ld * r + c] += sign * h;
-            else out[ld * r + c] = sign * h;
-        }
 }
 
 // Gauss-Newton Hessian blocks L0 J^T diag(w) J of one element, as 6x6
@@ -275,6 +404,7 @@ KHS_HD void xtdy(const M &X, const double d[3], const M &Y, double *out, int ld,
 //   Rii = Sgi^T Wg Sgi + Kki^T Wk Kki, Rjj likewise, Rij = Sgi^T Wg Sgj + Kki^T Wk Kkj,
 //   Hii = [P, -Xi; -Xi^T, Rii], Hjj = [P, Xj; Xj^T, Rjj], Hij = [-P, -Xj; Xi^T, Rij],
 // with the symmetric ones (P, Rii, Rjj) evaluated on one triangle and mirrored.
+// (On the doubled A2, S2 with a quarter of the weights.)
 KHS_HD double dot3w(const M &X, int r, const M &WY, int c)
 {
     return X.m[r] * WY.m[c] + X.m[3 + r] * WY.m[3 + c] + X.m[6 + r] * WY.m[6 + c];
@@ -282,15 +412,17 @@ KHS_HD double dot3w(const M &X, int r, const M &WY, int c)
 
 KHS_HD void element_hessian(const ElementJacobian &J, const Weights &w, double L0, double *Hii, double *Hjj, double *Hij)
 {
-    M WA, WSi, WSj, WKi, WKj;  // rows scaled by L0 w
+    M WA, WSi, WSj, WKi, WKj;  // rows scaled by L0 w / 4 and, for K, L0 w
+    const HalfWeights h = half_weights(w, L0);
+    const double hs[3] = {h.shear, h.shear, h.stretch}, hb[3] = {h.bend, h.bend, h.twist};
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        const double g = L0 * w.w[k], kk = L0 * w.w[3 + k];
+        const double g = 0.5 * hs[k], kk = 2.0 * hb[k];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            WA.m[3 * k + c] = g * J.A.m[3 * k + c];
-            WSi.m[3 * k + c] = g * J.Sgi.m[3 * k + c];
-            WSj.m[3 * k + c] = g * J.Sgj.m[3 * k + c];
+            WA.m[3 * k + c] = g * J.A2.m[3 * k + c];
+            WSi.m[3 * k + c] = g * J.S2i.m[3 * k + c];
+            WSj.m[3 * k + c] = g * J.S2j.m[3 * k + c];
             WKi.m[3 * k + c] = kk * J.Kki.m[3 * k + c];
             WKj.m[3 * k + c] = kk * J.Kkj.m[3 * k + c];
         }
@@ -299,18 +431,18 @@ KHS_HD void element_hessian(const ElementJacobian &J, const Weights &w, double L
     for (int r = 0; r < 3; ++r) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const double xi = dot3w(J.A, r, WSi, c), xj = dot3w(J.A, r, WSj, c);
+            const double xi = dot3w(J.A2, r, WSi, c), xj = dot3w(J.A2, r, WSj, c);
             Hii[6 * r + 3 + c] = -xi;
             Hii[6 * (3 + c) + r] = -xi;
             Hjj[6 * r + 3 + c] = xj;
             Hjj[6 * (3 + c) + r] = xj;
             Hij[6 * r + 3 + c] = -xj;
             Hij[6 * (3 + c) + r] = xi;
-            Hij[6 * (3 + r) + 3 + c] = dot3w(J.Sgi, r, WSj, c) + dot3w(J.Kki, r, WKj, c);
+            Hij[6 * (3 + r) + 3 + c] = dot3w(J.S2i, r, WSj, c) + dot3w(J.Kki, r, WKj, c);
             if (c < r) continue;
-            const double p = dot3w(J.A, r, WA, c);
-            const double rii = dot3w(J.Sgi, r, WSi, c) + dot3w(J.Kki, r, WKi, c);
-            const double rjj = dot3w(J.Sgj, r, WSj, c) + dot3w(J.Kkj, r, WKj, c);
+            const double p = dot3w(J.A2, r, WA, c);
+            const double rii = dot3w(J.S2i, r, WSi, c) + dot3w(J.Kki, r, WKi, c);
+            const double rjj = dot3w(J.S2j, r, WSj, c) + dot3w(J.Kkj, r, WKj, c);
             Hii[6 * r + c] = p; Hii[6 * c + r] = p;
             Hjj[6 * r + c] = p; Hjj[6 * c + r] = p;
             Hij[6 * r + c] = -p; Hij[6 * c + r] = -p;
@@ -348,18 +480,6 @@ struct ClosestPair {
     double distance, t;
     V bary;
 };
-
-#if defined(__CUDA_ARCH__)
-KHS_HD uint64_t bits_of(double x) { return uint64_t(__double_as_longlong(x)); }
-KHS_HD double double_of(uint64_t b) { return __longlong_as_double((long long)b); }
-KHS_HD uint32_t bits_of(float x) { return __float_as_uint(x); }
-KHS_HD float float_of(uint32_t b) { return __uint_as_float(b); }
-#else
-KHS_HD uint64_t bits_of(double x) { uint64_t b; std::memcpy(&b, &x, 8); return b; }
-KHS_HD double double_of(uint64_t b) { double x; std::memcpy(&x, &b, 8); return x; }
-KHS_HD uint32_t bits_of(float x) { uint32_t b; std::memcpy(&b, &x, 4); return b; }
-KHS_HD float float_of(uint32_t b) { float x; std::memcpy(&x, &b, 4); return x; }
-#endif
 
 // Comparisons of the closest-point code.  On GB300 an FP64 comparison takes an
 // FP64 issue slot (64 cycles) like a multiply-add, and fmin / fmax several, so
@@ -785,102 +905,6 @@ KHS_HD V rotation_vector(const M &r)
     if (!gfinite(angle) || !gfinite(axis.x) || !gfinite(axis.y) || !gfinite(axis.z)) return v(0.0, 0.0, 0.0);
     if (angle > kPi) angle = xs(angle, xm(2.0, kPi));
     return gmul(axis, angle);
-}
-
-// ---- correctly rounded reciprocal on the integer pipes -----------------
-//
-// 1/x rounded to nearest, computed without FP64 instructions: on GB300 one
-// FP64 warp instruction occupies a sub-partition's pipe for ~64 cycles, and a
-// reciprocal is on the chain of every pivot step of the block solve.
-// For x = (-1)^s * M * 2^(E-1075) with M the 53-bit significand,
-// 1/x = (-1)^s * T * 2^(970-E) with T = 2^105 / M in (2^52, 2^53]:
-// * seed: an FP32 reciprocal of the top 24 bits of M as the integer
-//   t ~ 2^23 * 2^52 / M, so T0 = 2^30 t; its relative error e = 1 - T0 / T
-//   is below 2^-20 (one ulp of the seed, the bits of M cut off, the rounding
-//   of t, and three further ulps of the seed to spare);
-// * residual: d = 2^75 - t M = 2^75 e, exact in 64 bits modulo 2^64 (2^75
-//   vanishes, |d| < 2^55), so one 24 x 53 bit product;
-// * Q = T0 (1 + e + e^2), rounded to an integer: e carried to 2^-62, e^2
-//   from the top 27 bits of d; with the cubic term left out the sum is within
-//   0.01 of T before the rounding, so Q is the nearest integer or next to it;
-// * the remainder R = 2^105 - Q M (exact modulo 2^64, |R| < 2^53) moves Q by
-//   one where |R| > M / 2.  No ties: M is odd times a power of two and T
-//   has more bits than a midpoint, or M = 2^52 and R = 0.
-// The steps are chosen for latency: 156 cycles of dependent instructions
-// (the FP64 reciprocal takes 352, the 128-bit form this replaces 382).  Reciprocals below the normal range (|x| >= 2^1022) are rounded from
-// floor(T) and its remainder to nearest-even on a branch of their own.
-// The result equals the IEEE division 1.0 / x for every finite normal x
-// (against 1.0 / x on the host, tests/native/test_recip.cpp); zero,
-// subnormal and non-finite inputs give an unspecified bit pattern (the block
-// solve fails such pivots before using the result).
-#if defined(__CUDA_ARCH__)
-KHS_HD int32_t smulhi32(int32_t a, int32_t b) { return __mulhi(a, b); }
-KHS_HD float recip_seed(float m)
-{
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(m));
-    return r;
-}
-#else
-KHS_HD int32_t smulhi32(int32_t a, int32_t b) { return int32_t((int64_t(a) * b) >> 32); }
-// Host seed: the correctly rounded float reciprocal (tests may substitute a
-// perturbed one through KHS_RECIP_SEED_HOST).
-#ifndef KHS_RECIP_SEED_HOST
-#define KHS_RECIP_SEED_HOST(m) (1.0f / (m))
-#endif
-KHS_HD float recip_seed(float m) { return KHS_RECIP_SEED_HOST(m); }
-#endif
-
-// The reciprocal where it is normal too (2^-1022 <= |x| < 2^1022), without
-// a branch.  Q and nR: the rounded T and minus its remainder.
-KHS_HD double recip_normal(double x, uint64_t &Q, int64_t &nR)
-{
-    const uint64_t b = bits_of(x);
-    const uint32_t hi = uint32_t(b >> 32), mlo = uint32_t(b);
-    const uint32_t E = (hi >> 20) & 0x7ff, mhi = (hi & 0xfffffu) | 0x100000u;
-    const uint64_t M = (uint64_t(mhi) << 32) | mlo, half = M >> 1;
-    const float seed = recip_seed(float_of((127u << 23) | ((hi << 3 | mlo >> 29) & 0x7fffffu)));
-    // 2^23 * seed as an integer: the bits of 1 + seed count it from those of 1.
-    const uint32_t t = bits_of(1.0f + seed) - 0x3f800000u;
-    // -d, and s = 2^62 (e + e^2) from it.
-    const uint64_t tm = uint64_t(t) * mlo;
-    const int64_t nd = int64_t((uint64_t(uint32_t(tm >> 32) + t * mhi) << 32) | uint32_t(tm));
-    const int32_t dh = int32_t(nd >> 28);
-    const int64_t s = int64_t(smulhi32(dh, dh)) - (nd >> 13);
-    // Q = round(2^30 t + t s / 2^32), the low and high words of s apart.
-    const uint64_t low = uint64_t(t) * uint32_t(s) + 0x80000000u;
-    Q = (uint64_t(t) << 30) + uint64_t(int64_t(int32_t(t)) * int32_t(s >> 32)) + (low >> 32);
-    nR = int64_t(Q * M);
-    // Q counts its implicit bit into the exponent field (Q = 2^53 as well).
-    const uint64_t out = (b & 0x8000000000000000ull) | ((uint64_t(2044 - E) << 52) + Q);
-    const uint64_t above = out + 1, below = out - 1;
-    return double_of(nR < -int64_t(half) ? above : (nR > int64_t(half) ? below : out));
-}
-KHS_HD double recip_normal(double x)
-{
-    uint64_t Q;
-    int64_t nR;
-    return recip_normal(x, Q, nR);
-}
-
-KHS_HD double recip_rn(double x)
-{
-    uint64_t F;
-    int64_t nR;
-    const double normal = recip_normal(x, F, nR);
-    const uint64_t b = bits_of(x);
-    const int E = int((b >> 52) & 0x7ff);
-    if (E < 2045) return normal;
-    // floor(T) and the remainder below M, then the subnormal's bits.
-    const int64_t M = int64_t((b & 0xfffffffffffffull) | (1ull << 52));
-    int64_t R = -nR;
-    if (R < 0) { --F; R += M; }
-    if (R >= M) { ++F; R -= M; }
-    const int k = E - 2044;
-    const uint64_t mant = F >> k;
-    const uint64_t dropped = F & ((1ull << k) - 1), mid = 1ull << (k - 1);
-    const bool up = dropped > mid || (dropped == mid && (R > 0 || (mant & 1)));
-    return double_of((b & 0x8000000000000000ull) | (mant + uint64_t(up)));
 }
 
 }  // namespace dm

@@ -65,12 +65,16 @@ using dm::V;
 using dm::M;
 
 constexpr int kBlock = 256;
+// Element and node evaluation: FP64 bound with few registers to spare, so one
+// or two warps keep a sub-partition's FP64 pipe busy and small blocks spread a
+// small scene over all of them.
+constexpr int kEvalBlock = 64;
 constexpr int kPartials = 304;  // 2 reduction blocks per SM on a 152-SM GB300
 constexpr uint32_t kNone = 0xffffffffu;
 constexpr uint64_t kCheckpointMagic = 0x3154504348534bULL;  // same blob header as the reference
 constexpr uint8_t kFlagActive = 1, kFlagInfeasible = 2, kFlagEnergy = 4, kFlagClosest = 8;
 
-inline unsigned grid_for(size_t n) { return unsigned((n + kBlock - 1) / kBlock); }
+inline unsigned grid_for(size_t n, int block = kBlock) { return unsigned((n + block - 1) / block); }
 // Every solver runs on device 0 (Engine::initialize selects it).
 constexpr int kDevice = 0;
 
@@ -142,7 +146,7 @@ struct View {
     const int32_t *elem_left, *elem_right;
     const uint32_t *ei, *ej, *estrand;
     const uint8_t *econtact;
-    const double *L0, *gamma0, *kappa0;
+    const double *L0, *invL, *gamma0, *kappa0;  // invL = 1 / L0
     double *e_el, *e_co, *c_gap;
     uint32_t *c_cand, *c_tri;
     uint8_t *c_flags;
@@ -648,7 +652,7 @@ __global__ void __launch_bounds__(kBlock) k_positions(View d, int trial, double 
 }
 
 // positions_done: k_positions has written q and the FP32 copy.
-__global__ void __launch_bounds__(kBlock) k_node_eval(View d, int gradient, int trial, double alpha, double dt,
+__global__ void __launch_bounds__(kEvalBlock) k_node_eval(View d, int gradient, int trial, double alpha, double dt,
                                                       const double *alpha_dev, int positions_done)
 {
     const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1242,7 +1246,7 @@ template<bool MIXED> __global__ void __launch_bounds__(kBlock) k_contact_query_r
 
 // Per element: elastic energy (+ gradient and GN blocks) and barrier contact
 // against the closest BVH candidate (cuda_backend.cu:899-939).
-__global__ void __launch_bounds__(kBlock) k_elem_eval(View d, int gradient)
+__global__ void __launch_bounds__(kEvalBlock) k_elem_eval(View d, int gradient)
 {
     const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= d.E) return;
@@ -1257,8 +1261,8 @@ __global__ void __launch_bounds__(kBlock) k_elem_eval(View d, int gradient)
     if (gradient) {
         const M Jli = load9(d.jl + 9 * size_t(i)), Jlj = load9(d.jl + 9 * size_t(j));
         dm::ElementJacobian J;
-        dm::element_strain(Ri, Rj, xi, xj, L0, load3(d.gamma0 + 3 * size_t(e)), load3(d.kappa0 + 3 * size_t(e)), eps, &J,
-                           &Jli, &Jlj);
+        dm::element_strain_inv(Ri, Rj, xi, xj, d.invL[e], load3(d.gamma0 + 3 * size_t(e)), load3(d.kappa0 + 3 * size_t(e)), eps,
+                               &J, &Jli, &Jlj);
         double a[6], b[6];
         dm::element_gradient(J, eps, d.w, L0, a, b);
         // 16-byte stores: every block starts on a 16-byte boundary (36 and
@@ -1281,8 +1285,8 @@ __global__ void __launch_bounds__(kBlock) k_elem_eval(View d, int gradient)
             Hij2[k] = fij ? make_double2(0.0, 0.0) : make_double2(hij[2 * k], hij[2 * k + 1]);
         }
     } else {
-        dm::element_strain(Ri, Rj, xi, xj, L0, load3(d.gamma0 + 3 * size_t(e)), load3(d.kappa0 + 3 * size_t(e)), eps,
-                           nullptr, nullptr, nullptr);
+        dm::element_strain_inv(Ri, Rj, xi, xj, d.invL[e], load3(d.gamma0 + 3 * size_t(e)), load3(d.kappa0 + 3 * size_t(e)), eps,
+                               nullptr, nullptr, nullptr);
     }
     d.e_el[e] = dm::element_energy(eps, d.w, L0);
 
@@ -2681,7 +2685,7 @@ void Engine::initialize(const Model &m, const KhsSolverDesc &desc, const KhsHair
     bytes += padded<uint8_t>(N) + 2 * padded<int32_t>(N);
     bytes += 4 * padded<double>(3 * N);      // root cur/pending x r
     bytes += 3 * padded<uint32_t>(N) + padded<double>(N);  // root bindings, node strand
-    bytes += 3 * padded<uint32_t>(E) + padded<uint8_t>(E) + padded<double>(E) + 2 * padded<double>(3 * E);
+    bytes += 3 * padded<uint32_t>(E) + padded<uint8_t>(E) + 2 * padded<double>(E) + 2 * padded<double>(3 * E);
     bytes += 3 * padded<double>(E) + 2 * padded<uint32_t>(E) + padded<uint8_t>(E);
     bytes += 5 * padded<uint32_t>(S);
     bytes += padded<uint32_t>(3 * T) + 5 * padded<double>(3 * Vn) + padded<float>(3 * Vn);
@@ -2733,7 +2737,7 @@ void Engine::initialize(const Model &m, const KhsSolverDesc &desc, const KhsHair
     I.bind_t = a.take<double>(N);
     uint32_t *ei = a.take<uint32_t>(E), *ej = a.take<uint32_t>(E), *es = a.take<uint32_t>(E);
     uint8_t *ec = a.take<uint8_t>(E);
-    double *L0 = a.take<double>(E), *g0 = a.take<double>(3 * E), *k0 = a.take<double>(3 * E);
+    double *L0 = a.take<double>(E), *invL = a.take<double>(E), *g0 = a.take<double>(3 * E), *k0 = a.take<double>(3 * E);
     v.e_el = a.take<double>(E); v.e_co = a.take<double>(E); v.c_gap = a.take<double>(E);
     v.c_cand = a.take<uint32_t>(E); v.c_tri = a.take<uint32_t>(E); v.c_flags = a.take<uint8_t>(E);
     uint32_t *sf = a.take<uint32_t>(S), *sc = a.take<uint32_t>(S), *sx = a.take<uint32_t>(S), *so = a.take<uint32_t>(S);
@@ -2818,6 +2822,9 @@ void Engine::initialize(const Model &m, const KhsSolverDesc &desc, const KhsHair
     I.root.sfirst = sf; I.root.scount = sc; I.root.sorder = so; I.root.ref = ref;
     up(ei, m.elem_i.data(), E * 4); up(ej, m.elem_j.data(), E * 4); up(es, m.elem_strand.data(), E * 4);
     up(ec, m.elem_contact.data(), E);
+    std::vector<double> hinv(E);
+    for (size_t e = 0; e < E; ++e) hinv[e] = 1.0 / m.rest_length[e];
+    up(invL, hinv.data(), E * 8);
     up(L0, m.rest_length.data(), E * 8); up(g0, hg0.data(), 3 * E * 8); up(k0, hk0.data(), 3 * E * 8);
     up(sf, m.strand_first.data(), S * 4); up(sc, m.strand_count.data(), S * 4); up(sx, m.strand_fixed.data(), S * 4);
     up(so, order.data(), S * 4);
@@ -2851,7 +2858,7 @@ void Engine::initialize(const Model &m, const KhsSolverDesc &desc, const KhsHair
     }
     up(I.mapping_dev, m.mapping.data(), O * 4);
     v.ref = ref; v.mass = mass; v.rmass = rmass; v.fixed = fixed; v.elem_left = eleft; v.elem_right = eright;
-    v.ei = ei; v.ej = ej; v.estrand = es; v.econtact = ec; v.L0 = L0; v.gamma0 = g0; v.kappa0 = k0;
+    v.ei = ei; v.ej = ej; v.estrand = es; v.econtact = ec; v.L0 = L0; v.invL = invL; v.gamma0 = g0; v.kappa0 = k0;
     v.sfirst = sf; v.scount = sc; v.sfixed = sx; v.sorder = so; v.tri = tri;
     v.bfirst = bfirst; v.bcount = bcount; v.border = border; v.bleaves = bleaves; v.bparent = bparent;
     v.bleft = bleft; v.bright = bright;
@@ -3092,15 +3099,15 @@ EvalStats Engine::evaluate(bool gradient, double dt, double alpha, const double 
         I.launch_on(cs, "k_contact_select", mode_ ? k_contact_select<true> : k_contact_select<false>, grid_for(v.E),
                     kBlock, v, q);
         if (side) KHS_CUDA(cudaEventRecord(I.join, I.side));
-        I.launch(gradient ? "k_node_eval_grad" : "k_node_eval_energy", k_node_eval, grid_for(v.N), kBlock, v,
+        I.launch(gradient ? "k_node_eval_grad" : "k_node_eval_energy", k_node_eval, grid_for(v.N, kEvalBlock), kEvalBlock, v,
                  gradient ? 1 : 0, trial ? 1 : 0, a, dt, alpha_dev, 1);
         if (side) KHS_CUDA(cudaStreamWaitEvent(I.stream, I.join, 0));
     } else {
-        I.launch(gradient ? "k_node_eval_grad" : "k_node_eval_energy", k_node_eval, grid_for(v.N), kBlock, v,
+        I.launch(gradient ? "k_node_eval_grad" : "k_node_eval_energy", k_node_eval, grid_for(v.N, kEvalBlock), kEvalBlock, v,
                  gradient ? 1 : 0, trial ? 1 : 0, a, dt, alpha_dev, 0);
     }
     rebuild_cache_ = false;
-    I.launch(gradient ? "k_elem_eval_grad" : "k_elem_eval_energy", k_elem_eval, grid_for(v.E), kBlock, v, gradient ? 1 : 0);
+    I.launch(gradient ? "k_elem_eval_grad" : "k_elem_eval_energy", k_elem_eval, grid_for(v.E, kEvalBlock), kEvalBlock, v, gradient ? 1 : 0);
     if (gradient) I.launch("k_node_sum", k_node_sum, grid_for(42 * size_t(v.N)), kBlock, v);
     I.launch("k_reduce_eval", k_reduce_eval, kPartials, kBlock, v, gradient ? 1 : 0);
     I.check();
