@@ -245,7 +245,7 @@ __device__ __forceinline__ uint32_t escape_from(uint32_t i, uint32_t escape) { r
 // outward FP32 test failed it is false; only inside the rounding band is
 // the FP64 test evaluated.
 struct QueryBox {
-    V lo, hi;
+    V lo, hi;  // two opposite corners, or (make_query_f) the segment's ends
     double pad;
     float olx, oly, olz, ohx, ohy, ohz, opad;  // outward-rounded box and padding
     float ilx, ily, ilz, ihx, ihy, ihz, ipad;  // inward-rounded box and padding
@@ -268,12 +268,12 @@ __device__ __forceinline__ QueryBox make_query(V lo, V hi, double pad)
 // componentwise min / max of the rounded coordinates): rounding to nearest
 // moved each coordinate by at most 2^-24 of its magnitude, so widening by
 // 2^-23 of the magnitude (plus 1e-30) bounds the FP64 box from outside and
-// narrowing by the same bounds it from inside.  lo and hi (FP64) serve the
-// exact leaf test.
-__device__ __forceinline__ QueryBox make_query_f(const float lo32[3], const float hi32[3], V lo, V hi, double pad)
+// narrowing by the same bounds it from inside.  The FP64 ends p and q serve
+// the exact leaf test, which the FP32 bounds nearly always decide.
+__device__ __forceinline__ QueryBox make_query_f(const float lo32[3], const float hi32[3], V p, V q, double pad)
 {
     QueryBox qb;
-    qb.lo = lo; qb.hi = hi; qb.pad = pad;
+    qb.lo = p; qb.hi = q; qb.pad = pad;
     const float k = 1.1920929e-7f;  // 2^-23
     qb.olx = __fsub_rd(lo32[0], __fmaf_ru(fabsf(lo32[0]), k, 1e-30f));
     qb.oly = __fsub_rd(lo32[1], __fmaf_ru(fabsf(lo32[1]), k, 1e-30f));
@@ -307,7 +307,8 @@ __device__ __forceinline__ bool leaf_overlap_exact(const View &d, uint32_t node,
                         q.ilz <= __fadd_rd(nextafterf(b.z, -INFINITY), q.ipad) &&
                         nextafterf(a.z, INFINITY) <= __fadd_rd(q.ihz, q.ipad);
     if (surely) return true;
-    return dm::boxes_overlap(q.lo, q.hi, load3(d.blo + 3 * size_t(node)), load3(d.bhi + 3 * size_t(node)), q.pad);
+    return dm::boxes_overlap(dm::vmin(q.lo, q.hi), dm::vmax(q.lo, q.hi), load3(d.blo + 3 * size_t(node)),
+                             load3(d.bhi + 3 * size_t(node)), q.pad);
 }
 
 // Stackless BVH walk in the reference's visiting order over packed 32-byte
@@ -990,81 +991,32 @@ __device__ __forceinline__ void put_pair(const View &d, uint32_t slot, uint32_t 
     d.surv_tri[slot] = t;
 }
 
-// An element whose cached leaves live in the leaf pool (more than 32): the
-// list is taken 32 leaves at a time, for the FP32 bound (FILTER), to count
-// the pairs and to write them, in leaf order.  Kept out of line so the common
-// one-round path keeps its registers.
-template<bool FILTER>
-__device__ __noinline__ void near_pool_element(const View &d, uint32_t e, const QueryBox &qb, dm::F3 origin, dm::F3 p1)
+// Candidates of up to 32 leaves, spread over the warp: lane l brings leaf l's
+// triangle range (first, cnt <= kLeafTriangles); pos lists the leaf-order
+// positions of all of them in traversal order.  Returns their number.  A leaf
+// a lane would leave most lanes idle: one or two leaves pass of thirty.
+constexpr int kNearList = 32 * kLeafTriangles;
+__device__ __forceinline__ uint32_t spread_candidates(uint32_t first, uint32_t cnt, uint32_t *pos, int lane)
 {
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const dm::F3 p0 = dm::f3(0.f, 0.f, 0.f);
-    uint32_t nleaves = 0;
-    const uint32_t *leaves = cached_leaves(d, e, kCacheBig, nleaves);
-    uint32_t total = 0;
-    float ub = 3.0e38f;
-    for (uint32_t r0 = 0; r0 < nleaves; r0 += 32) {
-        uint32_t first, cnt;
-        near_leaf(d, leaves, r0 + lane, nleaves, qb, first, cnt);
-        for (uint32_t r = 0; FILTER && r < cnt; ++r) {
-            float m;
-            uint32_t t;
-            const float df = record_distance_f(d, first + r, origin, p0, p1, m, t);
-            ub = fminf(ub, df + m);
-        }
-        total += __reduce_add_sync(FULL, cnt);
-    }
-    uint32_t n = total;
-    if (FILTER) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) ub = fminf(ub, __shfl_xor_sync(FULL, ub, o));
-        n = 0;
-        for (uint32_t r0 = 0; r0 < nleaves; r0 += 32) {
-            uint32_t first, cnt, mine = 0;
-            near_leaf(d, leaves, r0 + lane, nleaves, qb, first, cnt);
-            for (uint32_t r = 0; r < cnt; ++r) {
-                float m;
-                uint32_t t;
-                const float df = record_distance_f(d, first + r, origin, p0, p1, m, t);
-                mine += !(df - m > ub) ? 1u : 0u;
-            }
-            n += __reduce_add_sync(FULL, mine);
-        }
-    }
-    uint32_t slot = near_claim(d, e, total, n, lane);
-    if (slot == kNone) return;
-    for (uint32_t r0 = 0; r0 < nleaves; r0 += 32) {
-        uint32_t first, cnt, mine = 0;
-        near_leaf(d, leaves, r0 + lane, nleaves, qb, first, cnt);
-        uint32_t keep = 0;  // bit r: triangle first + r stays
-        for (uint32_t r = 0; r < cnt; ++r) {
-            bool stays = true;
-            if (FILTER) {
-                float m;
-                uint32_t t;
-                const float df = record_distance_f(d, first + r, origin, p0, p1, m, t);
-                stays = !(df - m > ub);
-            }
-            keep |= uint32_t(stays) << r;
-        }
-        mine = __popc(keep);
-        const uint32_t sincl = warp_inclusive_sum(mine, lane);
-        uint32_t at = slot + sincl - mine;
-        for (uint32_t r = 0; r < cnt; ++r)
-            if (keep >> r & 1u) put_pair(d, at++, e, __float_as_uint(__ldg(d.tri32 + 3 * size_t(first + r)).w));
-        slot += __shfl_sync(FULL, sincl, 31);
-    }
+    const uint32_t incl = warp_inclusive_sum(cnt, lane);
+    __syncwarp();  // the list's last readers are done
+    for (uint32_t r = 0; r < cnt; ++r) pos[incl - cnt + r] = first + r;
+    __syncwarp();
+    return __shfl_sync(0xffffffffu, incl, 31);
 }
 
-// One warp per element queued by k_contact_filter: lane l tests cached leaf l
-// and, with FILTER, the FP32 distances of its triangles; the smallest upper
-// bound is reduced across the warp.  The pairs are written in traversal order
-// (leaf, then triangle), so the first-found tie-break is kept.
+// One warp per element queued by k_contact_filter: the leaves are tested 32 at
+// a time, lane by lane, their candidates taken 32 at a time, lane by lane: with
+// FILTER once for the smallest upper bound, once to count the survivors, and
+// once to write the pairs, in traversal order (leaf, then triangle), so the
+// first-found tie-break is kept.  With at most 32 candidates, the common case,
+// the first round's bounds are kept instead.
 template<bool FILTER> __global__ void __launch_bounds__(kBlock) k_contact_near(View d)
 {
+    __shared__ uint32_t lists[kBlock / 32][kNearList];
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
+    uint32_t *pos = lists[threadIdx.x >> 5];
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
     const uint32_t count = d.sc->near_count;
     const double pad = d.radius + d.offset + d.dhat;
@@ -1076,46 +1028,79 @@ template<bool FILTER> __global__ void __launch_bounds__(kBlock) k_contact_near(V
         const V xi = load3(d.q + 6 * size_t(i)), xj = load3(d.q + 6 * size_t(j));
         const float lo32[3] = {fminf(xi32.x, xj32.x), fminf(xi32.y, xj32.y), fminf(xi32.z, xj32.z)};
         const float hi32[3] = {fmaxf(xi32.x, xj32.x), fmaxf(xi32.y, xj32.y), fmaxf(xi32.z, xj32.z)};
-        const QueryBox qb = make_query_f(lo32, hi32, dm::vmin(xi, xj), dm::vmax(xi, xj), pad);
+        const QueryBox qb = make_query_f(lo32, hi32, xi, xj, pad);
         const dm::F3 origin = xi32, p0 = dm::f3(0.f, 0.f, 0.f);
         const dm::F3 p1 = dm::f3(xj32.x - origin.x, xj32.y - origin.y, xj32.z - origin.z);
-        const uint8_t nl = d.cache_n[e];
-        if (nl == kCacheBig) {
-            near_pool_element<FILTER>(d, e, qb, origin, p1);
-            continue;
+        uint32_t nleaves = 0;
+        const uint32_t *leaves = cached_leaves(d, e, d.cache_n[e], nleaves);
+        auto bounds = [&](uint32_t p, float &lb, uint32_t &t) {  // returns the upper bound
+            float m;
+            const float df = record_distance_f(d, p, origin, p0, p1, m, t);
+            lb = df - m;
+            return df + m;
+        };
+        uint32_t total = 0, here = 0, tri0 = 0;
+        float ub = 3.0e38f, lb0 = 3.0e38f;
+        for (uint32_t r0 = 0; r0 < nleaves; r0 += 32) {
+            uint32_t first, cnt;
+            near_leaf(d, leaves, r0 + lane, nleaves, qb, first, cnt);
+            here = spread_candidates(first, cnt, pos, lane);
+            if (FILTER)
+                for (uint32_t c = lane; c < here; c += 32) ub = fminf(ub, bounds(pos[c], lb0, tri0));
+            total += here;
         }
-        uint32_t first, cnt;
-        near_leaf(d, d.cache_leaf + size_t(kCacheLeaves) * e, lane, nl, qb, first, cnt);
-        const uint32_t total = __reduce_add_sync(FULL, cnt);
-        float lb[kLeafTriangles];
-        float ub = 3.0e38f;
-        uint32_t keep = cnt ? (1u << cnt) - 1u : 0u;  // bit r: triangle first + r stays
         if (FILTER) {
 #pragma unroll
-            for (int r = 0; r < kLeafTriangles; ++r) {
-                lb[r] = 3.0e38f;
-                if (uint32_t(r) < cnt) {
-                    float m;
-                    uint32_t t;
-                    const float df = record_distance_f(d, first + r, origin, p0, p1, m, t);
-                    lb[r] = df - m;
-                    ub = fminf(ub, df + m);
+            for (int o = 16; o > 0; o >>= 1) ub = fminf(ub, __shfl_xor_sync(FULL, ub, o));
+        }
+        if (nleaves <= 32 && total <= 32) {
+            const bool stays = uint32_t(lane) < total && !(FILTER && lb0 > ub);
+            const uint32_t mask = __ballot_sync(FULL, stays);
+            const uint32_t base = near_claim(d, e, total, __popc(mask), lane);
+            if (base != kNone && stays) {
+                if (!FILTER) tri0 = __float_as_uint(__ldg(d.tri32 + 3 * size_t(pos[lane])).w);
+                put_pair(d, base + __popc(mask & ((1u << lane) - 1u)), e, tri0);
+            }
+            continue;
+        }
+        // More candidates: count the survivors, then write them.
+        uint32_t n = total, at = 0;
+        for (int pass = FILTER ? 0 : 1; pass < 2; ++pass) {
+            if (pass == 1) {
+                at = near_claim(d, e, total, n, lane);
+                if (at == kNone) break;
+            } else {
+                n = 0;
+            }
+            for (uint32_t r0 = 0; r0 < nleaves; r0 += 32) {
+                if (nleaves > 32) {
+                    uint32_t first, cnt;
+                    near_leaf(d, leaves, r0 + lane, nleaves, qb, first, cnt);
+                    here = spread_candidates(first, cnt, pos, lane);
+                }
+                for (uint32_t c0 = 0; c0 < here; c0 += 32) {
+                    const uint32_t c = c0 + lane;
+                    bool stays = c < here;
+                    uint32_t t = 0;
+                    if (stays) {
+                        float lb;
+                        if (FILTER) {
+                            bounds(pos[c], lb, t);
+                            stays = !(lb > ub);
+                        } else {
+                            t = __float_as_uint(__ldg(d.tri32 + 3 * size_t(pos[c])).w);
+                        }
+                    }
+                    const uint32_t mask = __ballot_sync(FULL, stays);
+                    if (pass == 0) {
+                        n += __popc(mask);
+                    } else {
+                        if (stays) put_pair(d, at + __popc(mask & ((1u << lane) - 1u)), e, t);
+                        at += __popc(mask);
+                    }
                 }
             }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) ub = fminf(ub, __shfl_xor_sync(FULL, ub, o));
-#pragma unroll
-            for (int r = 0; r < kLeafTriangles; ++r)
-                if (lb[r] > ub) keep &= ~(1u << r);
         }
-        const uint32_t mine = __popc(keep);
-        const uint32_t sincl = warp_inclusive_sum(mine, lane);
-        const uint32_t n = __shfl_sync(FULL, sincl, 31);
-        const uint32_t base = near_claim(d, e, total, n, lane);
-        if (base == kNone) continue;
-        uint32_t at = base + sincl - mine;
-        for (; keep; keep &= keep - 1)
-            put_pair(d, at++, e, __float_as_uint(__ldg(d.tri32 + 3 * size_t(first + uint32_t(__ffs(keep) - 1))).w));
     }
 }
 
@@ -1977,108 +1962,97 @@ template<bool MIXED> __global__ void __launch_bounds__(kBlock) k_ccd(View d)
 // alpha = 1; k_advance_pairs runs the exact FP64 conservative advancement
 // of cuda_backend.cu:989-1000 per listed pair.  The minimum equals the per-element kernel's
 // (k_ccd), which remains for a full pair list.
-// Candidates of the swept element box (positions at step 0 and 1) whose
-// FP32 lower-bound distance does not rule out a limit below 1: a pair is
-// skipped only when even the lower bound of 0.8 (dist - target) reaches the
-// speed, so the first advancement step of the exact pass would leave the
-// step unlimited anyway.  When all four swept end points stay within the
-// slack of the element's leaf cache, the cached leaves (collected with the
-// contact padding, which is at least the CCD target) hold every leaf the
-// swept box can touch and replace the tree walk.
+// The swept element box covers the positions at step 0 and 1.  When all four
+// swept end points stay within the slack of the element's leaf cache, the
+// cached leaves (collected with the contact padding, which is at least the
+// CCD target) hold every leaf the swept box can touch and replace the tree
+// walk; most elements have none and are done.  FILTER skips a pair only when
+// even the lower bound of 0.8 (dist - target) reaches the speed, so the first
+// advancement step of the exact pass would leave the step unlimited anyway.
+struct SweptElement {
+    QueryBox qb;
+    dm::F3 origin, f1;
+    float target_ru, speed_ru;
+    bool moves;
+};
+
+__device__ __forceinline__ SweptElement swept_element(const View &d, uint32_t i, uint32_t j)
+{
+    SweptElement w;
+    const V p0 = load3(d.q + 6 * size_t(i)), p1 = load3(d.q + 6 * size_t(j));
+    const V d0 = load3(d.dir + 6 * size_t(i)), d1 = load3(d.dir + 6 * size_t(j));
+    const double speed = fmax(dm::gnorm(d0), dm::gnorm(d1));
+    w.moves = !(speed < 1e-30);
+    const V e0 = p0 + d0, e1 = p1 + d1;
+    const double target = d.radius + d.offset + d.min_gap;
+    w.qb = make_query(dm::vmin(dm::vmin(p0, p1), dm::vmin(e0, e1)), dm::vmax(dm::vmax(p0, p1), dm::vmax(e0, e1)), target);
+    w.origin = dm::f3(d.q32[3 * size_t(i)], d.q32[3 * size_t(i) + 1], d.q32[3 * size_t(i) + 2]);
+    w.f1 = dm::f3(d.q32[3 * size_t(j)] - w.origin.x, d.q32[3 * size_t(j) + 1] - w.origin.y, d.q32[3 * size_t(j) + 2] - w.origin.z);
+    w.target_ru = __double2float_ru(target);
+    w.speed_ru = __fmul_ru(__double2float_ru(speed), 1.000002f);
+    return w;
+}
+
+template<bool FILTER> __device__ __forceinline__ void list_swept_pair(const View &d, const SweptElement &w, uint32_t e, uint32_t p)
+{
+    uint32_t t;
+    if (FILTER) {
+        float m;
+        const float df = record_distance_f(d, p, w.origin, dm::f3(0.f, 0.f, 0.f), w.f1, m, t);
+        if (__fmul_rd(0.8f, __fsub_rd(__fsub_rd(df, m), w.target_ru)) >= w.speed_ru) return;
+    } else {
+        t = __float_as_uint(__ldg(d.tri32 + 3 * size_t(p)).w);
+    }
+    const uint32_t slot = append_slot(&d.sc->pair_count);
+    if (slot < d.pair_capacity) { d.pair_elem[slot] = e; d.pair_tri[slot] = t; }
+}
+
 template<bool FILTER> __global__ void __launch_bounds__(kBlock) k_ccd_collect(View d)
 {
     const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= d.E) return;
     const uint32_t i = d.ei[e], j = d.ej[e];
     if (d.fixed[i] || !d.econtact[e]) return;
-    const V p0 = load3(d.q + 6 * size_t(i)), p1 = load3(d.q + 6 * size_t(j));
-    const V d0 = load3(d.dir + 6 * size_t(i)), d1 = load3(d.dir + 6 * size_t(j));
-    const double speed = fmax(dm::gnorm(d0), dm::gnorm(d1));
-    if (speed < 1e-30) return;
-    const V e0 = p0 + d0, e1 = p1 + d1;
-    const V lo = dm::vmin(dm::vmin(p0, p1), dm::vmin(e0, e1));
-    const V hi = dm::vmax(dm::vmax(p0, p1), dm::vmax(e0, e1));
-    const double target = d.radius + d.offset + d.min_gap;
-    const dm::F3 origin = dm::f3(d.q32[3 * size_t(i)], d.q32[3 * size_t(i) + 1], d.q32[3 * size_t(i) + 2]);
-    const dm::F3 f0 = dm::f3(0.f, 0.f, 0.f);
-    const dm::F3 f1 = dm::f3(d.q32[3 * size_t(j)] - origin.x, d.q32[3 * size_t(j) + 1] - origin.y,
-                             d.q32[3 * size_t(j) + 2] - origin.z);
-    const float target_ru = __double2float_ru(target);
-    const float speed_ru = __fmul_ru(__double2float_ru(speed), 1.000002f);
-    const QueryBox qb = make_query(lo, hi, target);
-    auto test = [&](uint32_t p) {
-        uint32_t t;
-        if (FILTER) {
-            float m;
-            const float df = record_distance_f(d, p, origin, f0, f1, m, t);
-            if (__fmul_rd(0.8f, __fsub_rd(__fsub_rd(df, m), target_ru)) >= speed_ru) return;
-        } else {
-            t = __float_as_uint(__ldg(d.tri32 + 3 * size_t(p)).w);
-        }
-        const uint32_t slot = append_slot(&d.sc->pair_count);
-        if (slot < d.pair_capacity) { d.pair_elem[slot] = e; d.pair_tri[slot] = t; }
-    };
     const uint8_t nl = d.cache_n[e];
-    bool cached = nl != kCacheInvalid && d.dhat >= d.min_gap;
-    if (cached) {
+    if (nl != kCacheInvalid && d.dhat >= d.min_gap) {
         const float *c = d.cache_x32 + 6 * size_t(e);
+        const dm::F3 xi32 = dm::f3(d.q32[3 * size_t(i)], d.q32[3 * size_t(i) + 1], d.q32[3 * size_t(i) + 2]);
         const dm::F3 xj32 = dm::f3(d.q32[3 * size_t(j)], d.q32[3 * size_t(j) + 1], d.q32[3 * size_t(j) + 2]);
+        const V e0 = load3(d.q + 6 * size_t(i)) + load3(d.dir + 6 * size_t(i));
+        const V e1 = load3(d.q + 6 * size_t(j)) + load3(d.dir + 6 * size_t(j));
         const dm::F3 a0 = dm::f3(float(e0.x), float(e0.y), float(e0.z)), a1 = dm::f3(float(e1.x), float(e1.y), float(e1.z));
-        cached = within_cache_slack(c, origin, xj32) && within_cache_slack(c, a0, a1);
+        if (within_cache_slack(c, xi32, xj32) && within_cache_slack(c, a0, a1)) {
+            // k_ccd_near tests the cached leaves, one warp per element.
+            if (nl > 0) d.near_list[append_slot(&d.sc->ccd_near)] = e;
+            return;
+        }
     }
-    if (cached) {
-        // k_ccd_near tests the cached leaves, one warp per element.
-        if (nl > 0) d.near_list[append_slot(&d.sc->ccd_near)] = e;
-    } else {
-        bvh_positions_packed(d, qb, test);
-    }
+    const SweptElement w = swept_element(d, i, j);
+    if (!w.moves) return;
+    bvh_positions_packed(d, w.qb, [&](uint32_t p) { list_swept_pair<FILTER>(d, w, e, p); });
 }
 
-// One warp per element queued by k_ccd_collect: lane l tests cached leaf l
-// against the swept box and applies the same FP32 skip bound to that leaf's
-// triangles (the pair order does not matter: the bound is a minimum).
+// One warp per element queued by k_ccd_collect: its leaves are tested 32 at a
+// time against the swept box and their candidates spread over the warp (the
+// pair order does not matter: the bound is a minimum).
 template<bool FILTER> __global__ void __launch_bounds__(kBlock) k_ccd_near(View d)
 {
+    __shared__ uint32_t lists[kBlock / 32][kNearList];
     const int lane = threadIdx.x & 31;
+    uint32_t *pos = lists[threadIdx.x >> 5];
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
     const uint32_t count = d.sc->ccd_near;
-    const double target = d.radius + d.offset + d.min_gap;
-    const float target_ru = __double2float_ru(target);
     for (uint32_t k = warp; k < count; k += nwarps) {
         const uint32_t e = d.near_list[k];
         uint32_t nleaves = 0;
         const uint32_t *leaves = cached_leaves(d, e, d.cache_n[e], nleaves);
-        if (uint32_t(lane) >= nleaves) continue;
-        const uint32_t i = d.ei[e], j = d.ej[e];
-        const V p0 = load3(d.q + 6 * size_t(i)), p1 = load3(d.q + 6 * size_t(j));
-        const V d0 = load3(d.dir + 6 * size_t(i)), d1 = load3(d.dir + 6 * size_t(j));
-        const double speed = fmax(dm::gnorm(d0), dm::gnorm(d1));
-        const V e0 = p0 + d0, e1 = p1 + d1;
-        const QueryBox qb = make_query(dm::vmin(dm::vmin(p0, p1), dm::vmin(e0, e1)), dm::vmax(dm::vmax(p0, p1), dm::vmax(e0, e1)),
-                                       target);
-        const dm::F3 origin = dm::f3(d.q32[3 * size_t(i)], d.q32[3 * size_t(i) + 1], d.q32[3 * size_t(i) + 2]);
-        const dm::F3 f0 = dm::f3(0.f, 0.f, 0.f);
-        const dm::F3 f1 = dm::f3(d.q32[3 * size_t(j)] - origin.x, d.q32[3 * size_t(j) + 1] - origin.y,
-                                 d.q32[3 * size_t(j) + 2] - origin.z);
-        const float speed_ru = __fmul_ru(__double2float_ru(speed), 1.000002f);
-        // Lane l takes leaves l, l + 32, ... of the cached list.
-        for (uint32_t c = lane; c < nleaves; c += 32) {
-            const uint32_t node = leaves[c];
-            const float4 a = __ldg(d.bnode + 2 * size_t(node)), b = __ldg(d.bnode + 2 * size_t(node) + 1);
-            if (!maybe_overlap(qb, a, b) || !leaf_overlap_exact(d, node, a, b, qb)) continue;
-            const uint32_t leaf = __float_as_uint(b.w), first = leaf >> 4, cnt = leaf & 15u;
-            for (uint32_t p = first; p < first + cnt; ++p) {
-                uint32_t t;
-                if (FILTER) {
-                    float m;
-                    const float df = record_distance_f(d, p, origin, f0, f1, m, t);
-                    if (__fmul_rd(0.8f, __fsub_rd(__fsub_rd(df, m), target_ru)) >= speed_ru) continue;
-                } else {
-                    t = __float_as_uint(__ldg(d.tri32 + 3 * size_t(p)).w);
-                }
-                const uint32_t slot = append_slot(&d.sc->pair_count);
-                if (slot < d.pair_capacity) { d.pair_elem[slot] = e; d.pair_tri[slot] = t; }
-            }
+        const SweptElement w = swept_element(d, d.ei[e], d.ej[e]);
+        if (!w.moves) continue;
+        for (uint32_t r0 = 0; r0 < nleaves; r0 += 32) {
+            uint32_t first, cnt;
+            near_leaf(d, leaves, r0 + lane, nleaves, w.qb, first, cnt);
+            const uint32_t here = spread_candidates(first, cnt, pos, lane);
+            for (uint32_t c = lane; c < here; c += 32) list_swept_pair<FILTER>(d, w, e, pos[c]);
         }
     }
 }
@@ -2224,7 +2198,9 @@ __global__ void __launch_bounds__(kBlock) k_sweep_collect(View d)
 
 template<bool FILTER> __global__ void __launch_bounds__(kBlock) k_sweep_near(View d)
 {
+    __shared__ uint32_t lists[kBlock / 32][kNearList];
     const int lane = threadIdx.x & 31;
+    uint32_t *pos = lists[threadIdx.x >> 5];
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
     const uint32_t count = d.sc->ccd_near;
     const double target = d.radius + d.offset + d.min_gap;
@@ -2233,15 +2209,16 @@ template<bool FILTER> __global__ void __launch_bounds__(kBlock) k_sweep_near(Vie
         const uint32_t e = d.near_list[k];
         uint32_t nleaves = 0;
         const uint32_t *leaves = cached_leaves(d, e, d.cache_n[e], nleaves);
-        if (uint32_t(lane) >= nleaves) continue;
         const V p0 = load3(d.q + 6 * size_t(d.ei[e])), p1 = load3(d.q + 6 * size_t(d.ej[e]));
         const QueryBox qb = make_query(dm::vmin(p0, p1), dm::vmax(p0, p1), target);
         const dm::F3 origin = dm::f3(float(p0.x), float(p0.y), float(p0.z));
         const dm::F3 f1 = dm::f3(float(p1.x) - origin.x, float(p1.y) - origin.y, float(p1.z) - origin.z);
-        for (uint32_t c = lane; c < nleaves; c += 32) {
+        for (uint32_t r0 = 0; r0 < nleaves; r0 += 32) {
             uint32_t first, cnt;
-            near_leaf(d, leaves, c, nleaves, qb, first, cnt);
-            for (uint32_t p = first; p < first + cnt; ++p) {
+            near_leaf(d, leaves, r0 + lane, nleaves, qb, first, cnt);
+            const uint32_t here = spread_candidates(first, cnt, pos, lane);
+            for (uint32_t c = lane; c < here; c += 32) {
+                const uint32_t p = pos[c];
                 if (FILTER && sweep_skip_f(d, p, origin, f1, target_ru)) continue;
                 const uint32_t slot = append_slot(&d.sc->pair_count);
                 if (slot < d.pair_capacity) {
