@@ -29,7 +29,7 @@
 //   direction     k_block_solve (blocks of one warp, a strand or five at a
 //                 time from a longest-first queue),
 //                 [float-float form: k_ff_factor, k_ff_residual, k_ff_correct],
-//                 k_steepest, k_scale, k_reduce_dir, k_final_dir
+//                 k_steepest, k_scale, k_reduce_dir, k_limit
 //   CCD           k_ccd (plain), k_ccd_collect + k_ccd_pairs (mixed)
 //   queries       k_contact, k_contact_query_records, k_gather
 //   root targets  k_root_tangents, k_root_transport, k_root_frames (thread
@@ -90,8 +90,8 @@ struct Mailbox {
     uint32_t pair_count;
     uint32_t refine_bits;
     uint32_t pad;
-    // The direction pass's values (every k_final_dir but the CCD pass of a
-    // pipelined iteration, which reduces the already limited direction).
+    // The direction as solved (k_reduce_dir); slope, dir_norm2 and
+    // max_translation are those of the limited one after k_limit.
     double dir_slope, dir_max_translation;
     int dir_solve_failed;
     int dir_pad;
@@ -110,9 +110,10 @@ struct Scalars {
     uint32_t near_count;  // elements queued for the warp-cooperative contact pass
     uint32_t ccd_near;    // elements queued for the warp-cooperative CCD pass
     uint32_t eval_done;   // blocks of k_reduce_eval finished (the last one reduces the partials)
+    uint32_t dir_done, ccd_done;  // the same for the direction's sums and the CCD pairs
     uint32_t pool_used;   // entries of the leaf pool handed out since the last cache rebuild
-    double trial_alpha;   // first line-search step from the last CCD bound (k_final_dir)
-    double max_translation;  // largest free-node translation of the last reduced direction (k_final_dir)
+    double trial_alpha;   // first line-search step from the last CCD bound (publish_ccd)
+    double max_translation;  // largest free-node translation of the last reduced direction
 };
 
 struct Partial {
@@ -137,7 +138,7 @@ struct View {
     uint32_t N, E, S, V, T, B;
     double *q, *q_old, *v, *q_base, *grad, *dir, *precond;
     double *inertia;  // inertia + damping diagonal of each node's block [N][6]
-    float *q32;       // FP32 copy of the node positions [N][3] (mixed contact filter)
+    float *q32, *e32;  // FP32 copies of the node positions and of positions + direction [N][3]
     double *rot, *jl, *node_energy, *node_kinetic;
     double *diag, *upper, *cprime, *dprime;
     double *as_i_g, *as_j_g, *as_i_h, *as_j_h, *as_i_f, *as_j_f;
@@ -205,6 +206,7 @@ struct View {
     dm::Weights w;
     double young, poisson, shear_corr;
     int has_collider;
+    struct Padding { double exact; float up, down; } contact_pad, ccd_pad;  // radius + offset + dhat, ... + min_gap
 };
 
 // Next free slot of a work list whose length is *count, for every lane that
@@ -245,35 +247,32 @@ __device__ __forceinline__ uint32_t escape_from(uint32_t i, uint32_t escape) { r
 // outward FP32 test failed it is false; only inside the rounding band is
 // the FP64 test evaluated.
 struct QueryBox {
-    V lo, hi;  // two opposite corners, or (make_query_f) the segment's ends
-    double pad;
     float olx, oly, olz, ohx, ohy, ohz, opad;  // outward-rounded box and padding
     float ilx, ily, ilz, ihx, ihy, ihz, ipad;  // inward-rounded box and padding
 };
 
-__device__ __forceinline__ QueryBox make_query(V lo, V hi, double pad)
+using Pad = View::Padding;  // with its roundings
+
+__device__ __forceinline__ QueryBox make_query(V lo, V hi, Pad pad)
 {
     QueryBox qb;
-    qb.lo = lo; qb.hi = hi; qb.pad = pad;
     qb.olx = __double2float_rd(lo.x); qb.oly = __double2float_rd(lo.y); qb.olz = __double2float_rd(lo.z);
     qb.ohx = __double2float_ru(hi.x); qb.ohy = __double2float_ru(hi.y); qb.ohz = __double2float_ru(hi.z);
-    qb.opad = __double2float_ru(pad);
+    qb.opad = pad.up;
     qb.ilx = __double2float_ru(lo.x); qb.ily = __double2float_ru(lo.y); qb.ilz = __double2float_ru(lo.z);
     qb.ihx = __double2float_rd(hi.x); qb.ihy = __double2float_rd(hi.y); qb.ihz = __double2float_rd(hi.z);
-    qb.ipad = __double2float_rd(pad);
+    qb.ipad = pad.down;
     return qb;
 }
 
-// The same box from FP32 copies of the segment's end points (lo32, hi32 =
+// The same box from FP32 copies of the points it spans (lo32, hi32 =
 // componentwise min / max of the rounded coordinates): rounding to nearest
 // moved each coordinate by at most 2^-24 of its magnitude, so widening by
 // 2^-23 of the magnitude (plus 1e-30) bounds the FP64 box from outside and
-// narrowing by the same bounds it from inside.  The FP64 ends p and q serve
-// the exact leaf test, which the FP32 bounds nearly always decide.
-__device__ __forceinline__ QueryBox make_query_f(const float lo32[3], const float hi32[3], V p, V q, double pad)
+// narrowing by the same bounds it from inside.
+__device__ __forceinline__ QueryBox make_query_f(const float lo32[3], const float hi32[3], Pad pad)
 {
     QueryBox qb;
-    qb.lo = p; qb.hi = q; qb.pad = pad;
     const float k = 1.1920929e-7f;  // 2^-23
     qb.olx = __fsub_rd(lo32[0], __fmaf_ru(fabsf(lo32[0]), k, 1e-30f));
     qb.oly = __fsub_rd(lo32[1], __fmaf_ru(fabsf(lo32[1]), k, 1e-30f));
@@ -287,8 +286,8 @@ __device__ __forceinline__ QueryBox make_query_f(const float lo32[3], const floa
     qb.ihx = __fsub_rd(hi32[0], __fmaf_ru(fabsf(hi32[0]), k, 1e-30f));
     qb.ihy = __fsub_rd(hi32[1], __fmaf_ru(fabsf(hi32[1]), k, 1e-30f));
     qb.ihz = __fsub_rd(hi32[2], __fmaf_ru(fabsf(hi32[2]), k, 1e-30f));
-    qb.opad = __double2float_ru(pad);
-    qb.ipad = __double2float_rd(pad);
+    qb.opad = pad.up;
+    qb.ipad = pad.down;
     return qb;
 }
 
@@ -298,7 +297,11 @@ __device__ __forceinline__ bool maybe_overlap(const QueryBox &q, float4 a, float
            a.y <= __fadd_ru(q.ohy, q.opad) && q.olz <= __fadd_ru(b.z, q.opad) && a.z <= __fadd_ru(q.ohz, q.opad);
 }
 
-__device__ __forceinline__ bool leaf_overlap_exact(const View &d, uint32_t node, float4 a, float4 b, const QueryBox &q)
+// box(lo, hi) gives the FP64 box, which the FP32 bounds nearly always make
+// unnecessary (an FP64 minimum costs several FP64 issue slots).
+template<class Box>
+__device__ __forceinline__ bool leaf_overlap_exact(const View &d, uint32_t node, float4 a, float4 b, const QueryBox &q, double pad,
+                                                   Box &&box)
 {
     const bool surely = q.ilx <= __fadd_rd(nextafterf(b.x, -INFINITY), q.ipad) &&
                         nextafterf(a.x, INFINITY) <= __fadd_rd(q.ihx, q.ipad) &&
@@ -307,8 +310,9 @@ __device__ __forceinline__ bool leaf_overlap_exact(const View &d, uint32_t node,
                         q.ilz <= __fadd_rd(nextafterf(b.z, -INFINITY), q.ipad) &&
                         nextafterf(a.z, INFINITY) <= __fadd_rd(q.ihz, q.ipad);
     if (surely) return true;
-    return dm::boxes_overlap(dm::vmin(q.lo, q.hi), dm::vmax(q.lo, q.hi), load3(d.blo + 3 * size_t(node)),
-                             load3(d.bhi + 3 * size_t(node)), q.pad);
+    V lo, hi;
+    box(lo, hi);
+    return dm::boxes_overlap(lo, hi, load3(d.blo + 3 * size_t(node)), load3(d.bhi + 3 * size_t(node)), pad);
 }
 
 // Stackless BVH walk in the reference's visiting order over packed 32-byte
@@ -319,7 +323,7 @@ __device__ __forceinline__ bool leaf_overlap_exact(const View &d, uint32_t node,
 // order are those of a walk over FP64 boxes; an FP64 comparison costs as much
 // as a multiply-add, twelve of them a node.  f receives the position of each
 // candidate in leaf order (index into border and tri32).
-template<class F> __device__ void bvh_positions_packed(const View &d, const QueryBox &q, F &&f)
+template<class Box, class F> __device__ void bvh_positions_packed(const View &d, const QueryBox &q, double pad, Box &&box, F &&f)
 {
     uint32_t i = 0;
     while (i < d.B) {
@@ -327,7 +331,7 @@ template<class F> __device__ void bvh_positions_packed(const View &d, const Quer
         const uint32_t escape = __float_as_uint(a.w), leaf = __float_as_uint(b.w);
         if (!maybe_overlap(q, a, b)) { i = escape_from(i, escape); continue; }
         if (leaf == 0) { ++i; continue; }
-        if (leaf_overlap_exact(d, i, a, b, q)) {
+        if (leaf_overlap_exact(d, i, a, b, q, pad, box)) {
             const uint32_t first = leaf >> 4, cnt = leaf & 15u;
             for (uint32_t k = first; k < first + cnt; ++k) f(k);
         }
@@ -335,9 +339,10 @@ template<class F> __device__ void bvh_positions_packed(const View &d, const Quer
     }
 }
 
-template<class F> __device__ void bvh_query_packed(const View &d, V lo, V hi, double pad, F &&f)
+template<class F> __device__ void bvh_query_packed(const View &d, V lo, V hi, Pad pad, F &&f)
 {
-    bvh_positions_packed(d, make_query(lo, hi, pad), [&](uint32_t k) { f(d.border[k]); });
+    bvh_positions_packed(d, make_query(lo, hi, pad), pad.exact, [&](V &l, V &h) { l = lo; h = hi; },
+                         [&](uint32_t k) { f(d.border[k]); });
 }
 
 constexpr int kCacheLeaves = 32;
@@ -348,7 +353,7 @@ constexpr uint8_t kCacheBig = 0xfe;     // cache_n of an element whose leaves li
 // Leaves whose FP32 outward box overlaps (lo, hi) padded by pad, in DFS
 // order; the first cap are written to out, and the return value is the
 // count of all of them.
-__device__ uint32_t collect_leaves(const View &d, V lo, V hi, double pad, uint32_t *out, uint32_t cap)
+__device__ uint32_t collect_leaves(const View &d, V lo, V hi, Pad pad, uint32_t *out, uint32_t cap)
 {
     const QueryBox q = make_query(lo, hi, pad);
     uint32_t i = 0, n = 0;
@@ -367,7 +372,7 @@ __device__ uint32_t collect_leaves(const View &d, V lo, V hi, double pad, uint32
 // Collects the leaves around (lo, hi) into the element's cache slots; returns
 // its cache_n.  More than kCacheLeaves, at a dense patch of the collider (a
 // mesh pole, a seam), go to the pool, which the warp passes take 32 at a time.
-__device__ __forceinline__ uint8_t leaves_to_cache(const View &d, uint32_t e, V lo, V hi, double pad)
+__device__ __forceinline__ uint8_t leaves_to_cache(const View &d, uint32_t e, V lo, V hi, Pad pad)
 {
     uint32_t *slots = d.cache_leaf + size_t(kCacheLeaves) * e;
     const uint32_t c = collect_leaves(d, lo, hi, pad, slots, kCacheLeaves);
@@ -552,7 +557,7 @@ __device__ bool sweep_element(const View &d, uint32_t e, SweepRecord *rec)
     const V p0 = load3(d.q + 6 * size_t(i)), p1 = load3(d.q + 6 * size_t(j));
     const double target = d.radius + d.offset + d.min_gap;
     bool failed = false;
-    bvh_query_packed(d, dm::vmin(p0, p1), dm::vmax(p0, p1), target, [&](uint32_t t) {
+    bvh_query_packed(d, dm::vmin(p0, p1), dm::vmax(p0, p1), d.ccd_pad, [&](uint32_t t) {
         if (failed) return;
         const V oa = load3(d.col_old + 3 * size_t(d.tri[3 * t])), ob = load3(d.col_old + 3 * size_t(d.tri[3 * t + 1])),
                 oc = load3(d.col_old + 3 * size_t(d.tri[3 * t + 2]));
@@ -744,7 +749,7 @@ __device__ __forceinline__ uint32_t closest_triangle_in(const View &d, V xi, V x
 // bound does not exceed that bound, in the same order, so the result (and
 // the first-found tie-break) equals the all-FP64 search.
 template<bool MIXED>
-__device__ __forceinline__ uint32_t closest_triangle(const View &d, V xi, V xj, double pad, uint32_t &cand,
+__device__ __forceinline__ uint32_t closest_triangle(const View &d, V xi, V xj, Pad pad, uint32_t &cand,
                                                      dm::ClosestPair &pair)
 {
     uint32_t closest = kNone;
@@ -780,7 +785,7 @@ template<bool MIXED> __global__ void __launch_bounds__(kBlock) k_contact(View d,
     pair.distance = 1.0e300; pair.t = 0.0; pair.bary = dm::v(1, 0, 0);
     if (d.has_collider && !d.fixed[i] && d.econtact[e]) {
         const V xi = load3(q + 6 * size_t(i)), xj = load3(q + 6 * size_t(j));
-        closest = closest_triangle<MIXED>(d, xi, xj, d.radius + d.offset + d.dhat, cand, pair);
+        closest = closest_triangle<MIXED>(d, xi, xj, d.contact_pad, cand, pair);
         if (closest != kNone) {
             flags |= kFlagClosest;
             gap = pair.distance - d.radius - d.offset;
@@ -901,7 +906,7 @@ __device__ __forceinline__ uint8_t refresh_leaves(const View &d, const double *q
     if (!force && nl != kCacheInvalid && within_cache_slack(c32, xi32, xj32)) return nl;
     const V xi = load3(q + 6 * size_t(i)), xj = load3(q + 6 * size_t(j));
     const V s3 = dm::v(kCacheSlack, kCacheSlack, kCacheSlack);
-    nl = leaves_to_cache(d, e, dm::vmin(xi, xj) - s3, dm::vmax(xi, xj) + s3, d.radius + d.offset + d.dhat);
+    nl = leaves_to_cache(d, e, dm::vmin(xi, xj) - s3, dm::vmax(xi, xj) + s3, d.contact_pad);
     c32[0] = xi32.x; c32[1] = xi32.y; c32[2] = xi32.z; c32[3] = xj32.x; c32[4] = xj32.y; c32[5] = xj32.z;
     return nl;
 }
@@ -935,15 +940,16 @@ __global__ void __launch_bounds__(kBlock) k_contact_filter(View d, const double 
 
 // Triangle range (first, cnt) of cached leaf k of a list of `count` when
 // its box passes the query's exact per-leaf test; cnt = 0 otherwise.
+template<class Box>
 __device__ __forceinline__ void near_leaf(const View &d, const uint32_t *leaves, uint32_t k, uint32_t count, const QueryBox &qb,
-                                          uint32_t &first, uint32_t &cnt)
+                                          double pad, Box &&box, uint32_t &first, uint32_t &cnt)
 {
     first = 0;
     cnt = 0;
     if (k >= count) return;
     const uint32_t node = leaves[k];
     const float4 a = __ldg(d.bnode + 2 * size_t(node)), b = __ldg(d.bnode + 2 * size_t(node) + 1);
-    if (maybe_overlap(qb, a, b) && leaf_overlap_exact(d, node, a, b, qb)) {
+    if (maybe_overlap(qb, a, b) && leaf_overlap_exact(d, node, a, b, qb, pad, box)) {
         const uint32_t leaf = __float_as_uint(b.w);
         first = leaf >> 4;
         cnt = leaf & 15u;
@@ -1019,16 +1025,18 @@ template<bool FILTER> __global__ void __launch_bounds__(kBlock) k_contact_near(V
     uint32_t *pos = lists[threadIdx.x >> 5];
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
     const uint32_t count = d.sc->near_count;
-    const double pad = d.radius + d.offset + d.dhat;
     for (uint32_t k = warp; k < count; k += nwarps) {
         const uint32_t e = d.near_list[k];
         const uint32_t i = d.ei[e], j = d.ej[e];
         const dm::F3 xi32 = dm::f3(d.q32[3 * size_t(i)], d.q32[3 * size_t(i) + 1], d.q32[3 * size_t(i) + 2]);
         const dm::F3 xj32 = dm::f3(d.q32[3 * size_t(j)], d.q32[3 * size_t(j) + 1], d.q32[3 * size_t(j) + 2]);
-        const V xi = load3(d.q + 6 * size_t(i)), xj = load3(d.q + 6 * size_t(j));
         const float lo32[3] = {fminf(xi32.x, xj32.x), fminf(xi32.y, xj32.y), fminf(xi32.z, xj32.z)};
         const float hi32[3] = {fmaxf(xi32.x, xj32.x), fmaxf(xi32.y, xj32.y), fmaxf(xi32.z, xj32.z)};
-        const QueryBox qb = make_query_f(lo32, hi32, xi, xj, pad);
+        const QueryBox qb = make_query_f(lo32, hi32, d.contact_pad);
+        auto box = [&](V &lo, V &hi) {
+            const V xi = load3(d.q + 6 * size_t(i)), xj = load3(d.q + 6 * size_t(j));
+            lo = dm::vmin(xi, xj); hi = dm::vmax(xi, xj);
+        };
         const dm::F3 origin = xi32, p0 = dm::f3(0.f, 0.f, 0.f);
         const dm::F3 p1 = dm::f3(xj32.x - origin.x, xj32.y - origin.y, xj32.z - origin.z);
         uint32_t nleaves = 0;
@@ -1043,7 +1051,7 @@ template<bool FILTER> __global__ void __launch_bounds__(kBlock) k_contact_near(V
         float ub = 3.0e38f, lb0 = 3.0e38f;
         for (uint32_t r0 = 0; r0 < nleaves; r0 += 32) {
             uint32_t first, cnt;
-            near_leaf(d, leaves, r0 + lane, nleaves, qb, first, cnt);
+            near_leaf(d, leaves, r0 + lane, nleaves, qb, d.contact_pad.exact, box, first, cnt);
             here = spread_candidates(first, cnt, pos, lane);
             if (FILTER)
                 for (uint32_t c = lane; c < here; c += 32) ub = fminf(ub, bounds(pos[c], lb0, tri0));
@@ -1075,7 +1083,7 @@ template<bool FILTER> __global__ void __launch_bounds__(kBlock) k_contact_near(V
             for (uint32_t r0 = 0; r0 < nleaves; r0 += 32) {
                 if (nleaves > 32) {
                     uint32_t first, cnt;
-                    near_leaf(d, leaves, r0 + lane, nleaves, qb, first, cnt);
+                    near_leaf(d, leaves, r0 + lane, nleaves, qb, d.contact_pad.exact, box, first, cnt);
                     here = spread_candidates(first, cnt, pos, lane);
                 }
                 for (uint32_t c0 = 0; c0 < here; c0 += 32) {
@@ -1158,8 +1166,8 @@ __device__ __forceinline__ uint32_t select_pair(const View &d, const double *q, 
     if (n == kSurvOverflow) {
         const uint32_t i = d.ei[e], j = d.ej[e];
         uint32_t cand = 0;
-        const uint32_t closest = closest_triangle<FILTER>(d, load3(q + 6 * size_t(i)), load3(q + 6 * size_t(j)),
-                                                          d.radius + d.offset + d.dhat, cand, pair);
+        const uint32_t closest = closest_triangle<FILTER>(d, load3(q + 6 * size_t(i)), load3(q + 6 * size_t(j)), d.contact_pad,
+                                                          cand, pair);
         d.c_cand[e] = cand;
         return closest;
     }
@@ -1214,7 +1222,7 @@ template<bool MIXED> __global__ void __launch_bounds__(kBlock) k_contact_query_r
     dm::ClosestPair pair;
     if (d.has_collider && !d.fixed[i] && d.econtact[e]) {
         const V xi = load3(q + 6 * size_t(i)), xj = load3(q + 6 * size_t(j));
-        closest = closest_triangle<MIXED>(d, xi, xj, d.radius + d.offset + d.dhat, cand, pair);
+        closest = closest_triangle<MIXED>(d, xi, xj, d.contact_pad, cand, pair);
         if (closest != kNone) {
             gap = pair.distance - d.radius - d.offset;
             active = gap > d.min_gap && gap < d.dhat ? 1u : 0u;
@@ -1833,32 +1841,41 @@ __global__ void __launch_bounds__(kBlock) k_scale(View d, double s)
     if (i < 6 * d.N) d.dir[i] *= s;
 }
 
-// The trust-radius limit applied on the device (pipelined iteration): the
-// same scale trust / max_translation as the host applies after reading the
-// reduction, when the direction's largest translation exceeds the radius.
-__global__ void __launch_bounds__(kBlock) k_scale_trust(View d, double trust)
+// The larger of two values >= 0, a NaN x ignored (as fmax does), compared as
+// bits.
+__device__ __forceinline__ double max_nonneg(double best, double x)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const double mt = d.sc->max_translation;
-    if (i < 6 * d.N && mt > trust) d.dir[i] *= trust / mt;
+    const unsigned long long b = (unsigned long long)__double_as_longlong(best), v = (unsigned long long)__double_as_longlong(x);
+    return v > b && v <= 0x7ff0000000000000ull ? x : best;
 }
 
-// g.d, |d|^2 and the largest free-node translation of d.
-__global__ void __launch_bounds__(kBlock) k_reduce_dir(View d)
+// Squared translation of a direction, rounded as the contracted dot product
+// x x + y y + z z is (the inner sum takes the first product into its
+// multiply-add); written out so that no other use of the products changes it.
+__device__ __forceinline__ double translation2(const double x[6])
 {
-    __shared__ double sh2[2][kBlock];
+    return __fma_rn(x[2], x[2], __fma_rn(x[0], x[0], __dmul_rn(x[1], x[1])));
+}
+
+// g.d, |d|^2 and the largest free-node translation of the direction over one
+// block's chunk of nodes, into the block's partial.  The root of the largest
+// square is the largest root: one square root a thread.
+__device__ void direction_partial(const View &d, double (*sh2)[kBlock])
+{
     uint32_t nb, ne;
     chunk(d.N, nb, ne);
     double gd = 0.0, dd = 0.0, mx = 0.0;
     for (uint32_t n = nb + threadIdx.x; n < ne; n += kBlock) {
+        double x[6];
+#pragma unroll
         for (int k = 0; k < 6; ++k) {
-            const double x = d.dir[6 * size_t(n) + k];
-            gd += d.grad[6 * size_t(n) + k] * x;
-            dd += x * x;
+            x[k] = d.dir[6 * size_t(n) + k];
+            gd += d.grad[6 * size_t(n) + k] * x[k];
+            dd += x[k] * x[k];
         }
-        if (!d.fixed[n]) mx = fmax(mx, dm::norm(load3(d.dir + 6 * size_t(n))));
+        if (!d.fixed[n]) mx = max_nonneg(mx, translation2(x));
     }
-    double sums[2] = {gd, dd}, maxs[1] = {mx};
+    double sums[2] = {gd, dd}, maxs[1] = {sqrt(mx)};
     block_tree<OpSum>(sums, sh2);
     block_tree<OpMax>(maxs, sh2);
     if (threadIdx.x == 0) {
@@ -1870,41 +1887,112 @@ __global__ void __launch_bounds__(kBlock) k_reduce_dir(View d)
     }
 }
 
-// ccd_pass: the CCD pass of a pipelined iteration, which leaves the
-// direction pass's values (dir_*) in the mailbox.
-__global__ void __launch_bounds__(kBlock) k_final_dir(View d, int ccd_pass)
+// True in the last block of the launch to get here, with the other blocks'
+// writes visible.
+__device__ bool last_block(uint32_t *done)
 {
-    __shared__ double sh2[2][kBlock];
+    __shared__ bool last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(done, 1u) == gridDim.x - 1;
+        if (last) *done = 0;
+    }
+    __syncthreads();
+    if (last) __threadfence();
+    return last;
+}
+
+// The partials of all blocks, in block order, to the mailbox and to device
+// memory.
+__device__ void direction_total(const View &d, double (*sh2)[kBlock])
+{
     double gd = 0, dd = 0, mx = 0;
     for (int b = threadIdx.x; b < kPartials; b += kBlock) {
-        const DirPartial p = d.dpartials[b];
-        gd += p.slope; dd += p.dnorm2; mx = fmax(mx, p.max_translation);
+        const DirPartial *p = d.dpartials + b;
+        gd += __ldcg(&p->slope); dd += __ldcg(&p->dnorm2); mx = fmax(mx, __ldcg(&p->max_translation));
     }
     double sums[2] = {gd, dd}, maxs[1] = {mx};
     block_tree<OpSum>(sums, sh2);
     block_tree<OpMax>(maxs, sh2);
-    gd = sums[0]; dd = sums[1]; mx = maxs[0];
     if (threadIdx.x == 0) {
-        d.mail->slope = gd; d.mail->dir_norm2 = dd; d.mail->max_translation = mx;
-        d.sc->max_translation = mx;
-        d.mail->ccd_bits = d.sc->ccd_bits;
-        d.mail->solve_failed = d.sc->solve_failed;
-        if (!ccd_pass) {
-            d.mail->dir_slope = gd; d.mail->dir_max_translation = mx; d.mail->dir_solve_failed = d.sc->solve_failed;
-        }
-        // The first line-search step as the host forms it: 0.9 x the CCD
-        // bound below 1, else 1 (no collider: 1).
-        const double lim = __longlong_as_double((long long)d.sc->ccd_bits);
-        d.sc->trial_alpha = d.has_collider ? (lim < 1.0 ? __dmul_rn(lim, 0.9) : lim) : 1.0;
-        d.mail->pair_count = d.sc->pair_count;
-        d.mail->refine_bits = d.sc->refine_bits;
-        d.sc->ccd_bits = 0x3ff0000000000000ULL;  // 1.0
+        d.mail->slope = sums[0]; d.mail->dir_norm2 = sums[1]; d.mail->max_translation = maxs[0];
+        d.sc->max_translation = maxs[0];
+    }
+}
+
+// The direction as solved: its sums (the last block to finish adds the
+// partials), and the flags of the solve.
+__global__ void __launch_bounds__(kBlock) k_reduce_dir(View d)
+{
+    __shared__ double sh2[2][kBlock];
+    direction_partial(d, sh2);
+    if (!last_block(&d.sc->dir_done)) return;
+    direction_total(d, sh2);
+    if (threadIdx.x == 0) {
+        Mailbox *m = d.mail;
+        m->dir_slope = m->slope; m->dir_max_translation = m->max_translation;
+        m->solve_failed = m->dir_solve_failed = d.sc->solve_failed;
+        m->refine_bits = d.sc->refine_bits;
         d.sc->solve_failed = 0;
-        d.sc->pair_count = 0;
         d.sc->solve_next = 0;
-        d.sc->ccd_near = 0;
         d.sc->refine_bits = 0;
     }
+}
+
+// Publishes the CCD bound and re-arms its counters; the first line-search step
+// is formed as the host does: 0.9 x the bound below 1, else 1.
+__device__ __forceinline__ void publish_ccd(const View &d)
+{
+    const double lim = __longlong_as_double((long long)__ldcg(&d.sc->ccd_bits));
+    d.mail->ccd_bits = (unsigned long long)__double_as_longlong(lim);
+    d.sc->trial_alpha = d.has_collider ? (lim < 1.0 ? __dmul_rn(lim, 0.9) : lim) : 1.0;
+    d.mail->pair_count = __ldcg(&d.sc->pair_count);
+    d.sc->ccd_bits = 0x3ff0000000000000ULL;  // 1.0
+    d.sc->pair_count = 0;
+    d.sc->ccd_near = 0;
+}
+
+__global__ void k_publish_ccd(View d)
+{
+    if (threadIdx.x == 0 && blockIdx.x == 0) publish_ccd(d);
+}
+
+// What lies between the direction and its CCD bound, in one pass over the
+// nodes: the trust-radius limit (scaled by trust / largest translation where
+// that is exceeded, as the host's k_scale does), the copy of the iterate, and
+// the FP32 end points of a full step.  The sums are taken again when the
+// limit changed the direction, or with `again` (the host changed it).
+// Without a collider the bound (1) is published here.
+__global__ void __launch_bounds__(kBlock) k_limit(View d, double trust, int again)
+{
+    __shared__ double sh2[2][kBlock];
+    const double mt = d.sc->max_translation;
+    const bool limited = mt > trust;
+    const double scale = limited ? trust / mt : 1.0;
+    uint32_t nb, ne;
+    chunk(d.N, nb, ne);
+    for (uint32_t n = nb + threadIdx.x; n < ne; n += kBlock) {
+        double2 *q = reinterpret_cast<double2 *>(d.q + 6 * size_t(n)), *base = reinterpret_cast<double2 *>(d.q_base + 6 * size_t(n));
+        double2 *dir = reinterpret_cast<double2 *>(d.dir + 6 * size_t(n));
+        const double2 qa = q[0], qb = q[1], qc = q[2];
+        double2 da = dir[0], db = dir[1];
+        base[0] = qa; base[1] = qb; base[2] = qc;
+        if (limited) {
+            double2 dc = dir[2];
+            da.x *= scale; da.y *= scale; db.x *= scale; db.y *= scale; dc.x *= scale; dc.y *= scale;
+            dir[0] = da; dir[1] = db; dir[2] = dc;
+        }
+        d.e32[3 * size_t(n)] = float(qa.x + da.x);
+        d.e32[3 * size_t(n) + 1] = float(qa.y + da.y);
+        d.e32[3 * size_t(n) + 2] = float(qb.x + db.x);
+    }
+    if (limited || again) {
+        __syncthreads();  // the chunk's scaled directions
+        direction_partial(d, sh2);
+        if (last_block(&d.sc->dir_done)) direction_total(d, sh2);
+    }
+    if (!d.has_collider && blockIdx.x == 0 && threadIdx.x == 0) publish_ccd(d);
 }
 
 // Line-search CCD bound (cuda_backend.cu:989-1000); the minimum over all
@@ -1923,7 +2011,7 @@ template<bool MIXED> __global__ void __launch_bounds__(kBlock) k_ccd(View d)
     const double target = d.radius + d.offset + d.min_gap;
     double local = 1.0;
     const dm::F3 f0 = dm::f3(0.f, 0.f, 0.f), f1 = dm::to_local(p1, p0);
-    bvh_query_packed(d, lo, hi, target, [&](uint32_t t) {
+    bvh_query_packed(d, lo, hi, d.ccd_pad, [&](uint32_t t) {
         const double speed = fmax(dm::gnorm(d0), dm::gnorm(d1));
         if (speed < 1e-30) return;
         const V a = tri_vertex(d, t, 0), b = tri_vertex(d, t, 1), c = tri_vertex(d, t, 2);
@@ -1972,25 +2060,41 @@ template<bool MIXED> __global__ void __launch_bounds__(kBlock) k_ccd(View d)
 struct SweptElement {
     QueryBox qb;
     dm::F3 origin, f1;
-    float target_ru, speed_ru;
-    bool moves;
+    float speed_ru;  // an upper bound of the larger end point displacement
 };
+
+__device__ __forceinline__ dm::F3 load3f(const float *p) { return dm::f3(p[0], p[1], p[2]); }
 
 __device__ __forceinline__ SweptElement swept_element(const View &d, uint32_t i, uint32_t j)
 {
     SweptElement w;
-    const V p0 = load3(d.q + 6 * size_t(i)), p1 = load3(d.q + 6 * size_t(j));
-    const V d0 = load3(d.dir + 6 * size_t(i)), d1 = load3(d.dir + 6 * size_t(j));
-    const double speed = fmax(dm::gnorm(d0), dm::gnorm(d1));
-    w.moves = !(speed < 1e-30);
-    const V e0 = p0 + d0, e1 = p1 + d1;
-    const double target = d.radius + d.offset + d.min_gap;
-    w.qb = make_query(dm::vmin(dm::vmin(p0, p1), dm::vmin(e0, e1)), dm::vmax(dm::vmax(p0, p1), dm::vmax(e0, e1)), target);
-    w.origin = dm::f3(d.q32[3 * size_t(i)], d.q32[3 * size_t(i) + 1], d.q32[3 * size_t(i) + 2]);
-    w.f1 = dm::f3(d.q32[3 * size_t(j)] - w.origin.x, d.q32[3 * size_t(j) + 1] - w.origin.y, d.q32[3 * size_t(j) + 2] - w.origin.z);
-    w.target_ru = __double2float_ru(target);
-    w.speed_ru = __fmul_ru(__double2float_ru(speed), 1.000002f);
+    const dm::F3 p0 = load3f(d.q32 + 3 * size_t(i)), p1 = load3f(d.q32 + 3 * size_t(j));
+    const dm::F3 e0 = load3f(d.e32 + 3 * size_t(i)), e1 = load3f(d.e32 + 3 * size_t(j));
+    const float lo32[3] = {fminf(fminf(p0.x, p1.x), fminf(e0.x, e1.x)), fminf(fminf(p0.y, p1.y), fminf(e0.y, e1.y)),
+                           fminf(fminf(p0.z, p1.z), fminf(e0.z, e1.z))};
+    const float hi32[3] = {fmaxf(fmaxf(p0.x, p1.x), fmaxf(e0.x, e1.x)), fmaxf(fmaxf(p0.y, p1.y), fmaxf(e0.y, e1.y)),
+                           fmaxf(fmaxf(p0.z, p1.z), fmaxf(e0.z, e1.z))};
+    w.qb = make_query_f(lo32, hi32, d.ccd_pad);
+    w.origin = p0;
+    w.f1 = dm::fsub(p1, p0);
+    // Either copy is within 2^-24 of a coordinate's magnitude, a difference of
+    // two within 2^-22 of the larger one.
+    auto bound = [](dm::F3 p, dm::F3 e) {
+        const float mag = fmaxf(fmaxf(fmaxf(fabsf(p.x), fabsf(p.y)), fabsf(p.z)), fmaxf(fmaxf(fabsf(e.x), fabsf(e.y)), fabsf(e.z)));
+        const dm::F3 v = dm::fsub(e, p);
+        return __fadd_ru(__fmul_ru(sqrtf(dm::fdot(v, v)), 1.00001f), __fmaf_ru(mag, 5.0e-7f, 1.0e-12f));
+    };
+    w.speed_ru = fmaxf(bound(p0, e0), bound(p1, e1));
     return w;
+}
+
+// The FP64 swept box.
+__device__ __forceinline__ void swept_box(const View &d, uint32_t i, uint32_t j, V &lo, V &hi)
+{
+    const V p0 = load3(d.q + 6 * size_t(i)), p1 = load3(d.q + 6 * size_t(j));
+    const V e0 = p0 + load3(d.dir + 6 * size_t(i)), e1 = p1 + load3(d.dir + 6 * size_t(j));
+    lo = dm::vmin(dm::vmin(p0, p1), dm::vmin(e0, e1));
+    hi = dm::vmax(dm::vmax(p0, p1), dm::vmax(e0, e1));
 }
 
 template<bool FILTER> __device__ __forceinline__ void list_swept_pair(const View &d, const SweptElement &w, uint32_t e, uint32_t p)
@@ -1999,7 +2103,7 @@ template<bool FILTER> __device__ __forceinline__ void list_swept_pair(const View
     if (FILTER) {
         float m;
         const float df = record_distance_f(d, p, w.origin, dm::f3(0.f, 0.f, 0.f), w.f1, m, t);
-        if (__fmul_rd(0.8f, __fsub_rd(__fsub_rd(df, m), w.target_ru)) >= w.speed_ru) return;
+        if (__fmul_rd(0.8f, __fsub_rd(__fsub_rd(df, m), d.ccd_pad.up)) >= w.speed_ru) return;
     } else {
         t = __float_as_uint(__ldg(d.tri32 + 3 * size_t(p)).w);
     }
@@ -2018,9 +2122,7 @@ template<bool FILTER> __global__ void __launch_bounds__(kBlock) k_ccd_collect(Vi
         const float *c = d.cache_x32 + 6 * size_t(e);
         const dm::F3 xi32 = dm::f3(d.q32[3 * size_t(i)], d.q32[3 * size_t(i) + 1], d.q32[3 * size_t(i) + 2]);
         const dm::F3 xj32 = dm::f3(d.q32[3 * size_t(j)], d.q32[3 * size_t(j) + 1], d.q32[3 * size_t(j) + 2]);
-        const V e0 = load3(d.q + 6 * size_t(i)) + load3(d.dir + 6 * size_t(i));
-        const V e1 = load3(d.q + 6 * size_t(j)) + load3(d.dir + 6 * size_t(j));
-        const dm::F3 a0 = dm::f3(float(e0.x), float(e0.y), float(e0.z)), a1 = dm::f3(float(e1.x), float(e1.y), float(e1.z));
+        const dm::F3 a0 = load3f(d.e32 + 3 * size_t(i)), a1 = load3f(d.e32 + 3 * size_t(j));
         if (within_cache_slack(c, xi32, xj32) && within_cache_slack(c, a0, a1)) {
             // k_ccd_near tests the cached leaves, one warp per element.
             if (nl > 0) d.near_list[append_slot(&d.sc->ccd_near)] = e;
@@ -2028,8 +2130,7 @@ template<bool FILTER> __global__ void __launch_bounds__(kBlock) k_ccd_collect(Vi
         }
     }
     const SweptElement w = swept_element(d, i, j);
-    if (!w.moves) return;
-    bvh_positions_packed(d, w.qb, [&](uint32_t p) { list_swept_pair<FILTER>(d, w, e, p); });
+    bvh_positions_packed(d, w.qb, d.ccd_pad.exact, [&](V &lo, V &hi) { swept_box(d, i, j, lo, hi); }, [&](uint32_t p) { list_swept_pair<FILTER>(d, w, e, p); });
 }
 
 // One warp per element queued by k_ccd_collect: its leaves are tested 32 at a
@@ -2046,11 +2147,12 @@ template<bool FILTER> __global__ void __launch_bounds__(kBlock) k_ccd_near(View 
         const uint32_t e = d.near_list[k];
         uint32_t nleaves = 0;
         const uint32_t *leaves = cached_leaves(d, e, d.cache_n[e], nleaves);
-        const SweptElement w = swept_element(d, d.ei[e], d.ej[e]);
-        if (!w.moves) continue;
+        const uint32_t i = d.ei[e], j = d.ej[e];
+        const SweptElement w = swept_element(d, i, j);
         for (uint32_t r0 = 0; r0 < nleaves; r0 += 32) {
             uint32_t first, cnt;
-            near_leaf(d, leaves, r0 + lane, nleaves, w.qb, first, cnt);
+            near_leaf(d, leaves, r0 + lane, nleaves, w.qb, d.ccd_pad.exact, [&](V &lo, V &hi) { swept_box(d, i, j, lo, hi); }, first,
+                      cnt);
             const uint32_t here = spread_candidates(first, cnt, pos, lane);
             for (uint32_t c = lane; c < here; c += 32) list_swept_pair<FILTER>(d, w, e, pos[c]);
         }
@@ -2099,8 +2201,8 @@ template<bool SWEEP> __global__ void __launch_bounds__(kPairBlock) k_advance_pai
             bool on = k < count;
             // Every limit a pair can still produce is >= 0.9 alpha, so it
             // stops as soon as that reaches the smallest limit found so far.
-            if (SWEEP) on = on && !(speed < 1e-30);
-            else on = on && __longlong_as_double(*reinterpret_cast<volatile long long *>(&d.sc->ccd_bits)) > 0.0;
+            on = on && !(speed < 1e-30);
+            if (!SWEEP) on = on && __longlong_as_double(*reinterpret_cast<volatile long long *>(&d.sc->ccd_bits)) > 0.0;
             const uint32_t active = __ballot_sync(0xffffffffu, on);
             sh_alpha[lane] = 0.0;
             if (lane == 0) sh_active = active;
@@ -2168,6 +2270,7 @@ template<bool SWEEP> __global__ void __launch_bounds__(kPairBlock) k_advance_pai
         }
         __syncthreads();
     }
+    if (!SWEEP && last_block(&d.sc->ccd_done) && threadIdx.x == 0) publish_ccd(d);
 }
 
 // ---- moving-collider sweep ------------------------------------------------
@@ -2188,7 +2291,7 @@ __global__ void __launch_bounds__(kBlock) k_sweep_collect(View d)
     const uint32_t i = d.ei[e], j = d.ej[e];
     if (d.fixed[i] || !d.econtact[e]) return;
     const V p0 = load3(d.q + 6 * size_t(i)), p1 = load3(d.q + 6 * size_t(j));
-    const uint8_t nl = leaves_to_cache(d, e, dm::vmin(p0, p1), dm::vmax(p0, p1), d.radius + d.offset + d.min_gap);
+    const uint8_t nl = leaves_to_cache(d, e, dm::vmin(p0, p1), dm::vmax(p0, p1), d.ccd_pad);
     if (nl == kCacheInvalid) {  // the leaf pool is full
         if (sweep_element(d, e, nullptr)) atomicMin(&d.sc->sweep_fail, e);
     } else if (nl > 0) {
@@ -2203,23 +2306,24 @@ template<bool FILTER> __global__ void __launch_bounds__(kBlock) k_sweep_near(Vie
     uint32_t *pos = lists[threadIdx.x >> 5];
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
     const uint32_t count = d.sc->ccd_near;
-    const double target = d.radius + d.offset + d.min_gap;
-    const float target_ru = __double2float_ru(target);
     for (uint32_t k = warp; k < count; k += nwarps) {
         const uint32_t e = d.near_list[k];
         uint32_t nleaves = 0;
         const uint32_t *leaves = cached_leaves(d, e, d.cache_n[e], nleaves);
         const V p0 = load3(d.q + 6 * size_t(d.ei[e])), p1 = load3(d.q + 6 * size_t(d.ej[e]));
-        const QueryBox qb = make_query(dm::vmin(p0, p1), dm::vmax(p0, p1), target);
-        const dm::F3 origin = dm::f3(float(p0.x), float(p0.y), float(p0.z));
-        const dm::F3 f1 = dm::f3(float(p1.x) - origin.x, float(p1.y) - origin.y, float(p1.z) - origin.z);
+        const dm::F3 origin = dm::f3(float(p0.x), float(p0.y), float(p0.z)), end = dm::f3(float(p1.x), float(p1.y), float(p1.z));
+        const dm::F3 f1 = dm::fsub(end, origin);
+        const float lo32[3] = {fminf(origin.x, end.x), fminf(origin.y, end.y), fminf(origin.z, end.z)};
+        const float hi32[3] = {fmaxf(origin.x, end.x), fmaxf(origin.y, end.y), fmaxf(origin.z, end.z)};
+        const QueryBox qb = make_query_f(lo32, hi32, d.ccd_pad);
+        auto box = [&](V &lo, V &hi) { lo = dm::vmin(p0, p1); hi = dm::vmax(p0, p1); };
         for (uint32_t r0 = 0; r0 < nleaves; r0 += 32) {
             uint32_t first, cnt;
-            near_leaf(d, leaves, r0 + lane, nleaves, qb, first, cnt);
+            near_leaf(d, leaves, r0 + lane, nleaves, qb, d.ccd_pad.exact, box, first, cnt);
             const uint32_t here = spread_candidates(first, cnt, pos, lane);
             for (uint32_t c = lane; c < here; c += 32) {
                 const uint32_t p = pos[c];
-                if (FILTER && sweep_skip_f(d, p, origin, f1, target_ru)) continue;
+                if (FILTER && sweep_skip_f(d, p, origin, f1, d.ccd_pad.up)) continue;
                 const uint32_t slot = append_slot(&d.sc->pair_count);
                 if (slot < d.pair_capacity) {
                     d.pair_elem[slot] = e;
@@ -2355,6 +2459,8 @@ __global__ void k_init_scalars(View d)
     d.sc->ccd_near = 0;
     d.sc->pool_used = 0;
     d.sc->eval_done = 0;
+    d.sc->dir_done = 0;
+    d.sc->ccd_done = 0;
 }
 
 __global__ void __launch_bounds__(kBlock) k_gather(const double *q, const uint32_t *map, uint32_t count, double *out)
@@ -2676,7 +2782,7 @@ void Engine::initialize(const Model &m, const KhsSolverDesc &desc, const KhsHair
     bytes += padded<uint32_t>(size_t(kCacheLeaves) * E) + padded<uint8_t>(E);
     const size_t leaf_pool = std::min<size_t>(std::max<size_t>(size_t(1) << 20, 4 * E), size_t(16) << 20);
     bytes += padded<uint32_t>(leaf_pool);
-    bytes += padded<float>(3 * N) + padded<float>(6 * E);
+    bytes += 2 * padded<float>(3 * N) + padded<float>(6 * E);
     bytes += padded<uint32_t>(E);
     bytes += 2 * padded<float2>(36 * N) + padded<float2>(6 * N) + padded<float>(N);
     bytes += 2 * padded<float4>(3 * T) + 2 * padded<uint32_t>(surv_capacity) + 2 * padded<uint32_t>(E) +
@@ -2696,7 +2802,7 @@ void Engine::initialize(const Model &m, const KhsSolverDesc &desc, const KhsHair
     v.q = a.take<double>(6 * N); v.q_old = a.take<double>(6 * N); v.v = a.take<double>(6 * N);
     v.q_base = a.take<double>(6 * N); v.grad = a.take<double>(6 * N); v.dir = a.take<double>(6 * N);
     v.precond = a.take<double>(6 * N); v.dprime = a.take<double>(6 * N); v.inertia = a.take<double>(6 * N);
-    v.q32 = a.take<float>(3 * N);
+    v.q32 = a.take<float>(3 * N); v.e32 = a.take<float>(3 * N);
     v.as_i_g = a.take<double>(6 * N); v.as_j_g = a.take<double>(6 * N);
     I.q_snap = a.take<double>(6 * N); I.v_snap = a.take<double>(6 * N);
     v.diag = a.take<double>(36 * N); v.upper = a.take<double>(36 * N); v.cprime = a.take<double>(36 * N);
@@ -2877,6 +2983,12 @@ void Engine::update_runtime(const KhsSolverDesc &desc, const KhsHairMaterial &ma
     v.radius = material.radius; v.offset = material.collider_offset; v.dhat = material.barrier_distance;
     v.kc = material.contact_stiffness; v.friction = material.friction; v.smoothing = material.friction_smoothing;
     v.damping = material.mass_damping; v.min_gap = desc.minimum_gap;
+    auto padding = [](double x) {
+        float near = float(x), inf = std::numeric_limits<float>::infinity();
+        return View::Padding{x, double(near) < x ? std::nextafter(near, inf) : near, double(near) > x ? std::nextafter(near, -inf) : near};
+    };
+    v.contact_pad = padding(v.radius + v.offset + v.dhat);
+    v.ccd_pad = padding(v.radius + v.offset + v.min_gap);
     v.gx = desc.gravity.x; v.gy = desc.gravity.y; v.gz = desc.gravity.z;
     v.young = material.young_modulus; v.poisson = material.poisson_ratio; v.shear_corr = material.shear_correction;
     v.w = dm::strain_weights(material.radius, material.young_modulus, material.poisson_ratio, material.shear_correction);
@@ -3112,7 +3224,6 @@ bool Engine::make_steepest()
     Impl &I = *d_;
     I.launch("k_steepest", k_steepest, grid_for(6 * size_t(I.v.N)), kBlock, I.v);
     I.launch("k_reduce_dir", k_reduce_dir, kPartials, kBlock, I.v);
-    I.launch("k_final_dir", k_final_dir, 1, kBlock, I.v, 0);
     I.check();
     I.sync();
     return limit_direction(I.mail_host->max_translation);
@@ -3225,7 +3336,6 @@ bool Engine::make_direction(KhsxSubstepRecord &rec, double grad_norm2)
             I.launch("k_ff_correct", k_ff_correct, I.ff_blocks, 128, I.v);
             ++sweeps;
             I.launch("k_reduce_dir", k_reduce_dir, kPartials, kBlock, I.v);
-            I.launch("k_final_dir", k_final_dir, 1, kBlock, I.v, 0);
             I.check();
             I.sync();
             if (mb.solve_failed) break;
@@ -3242,7 +3352,6 @@ bool Engine::make_direction(KhsxSubstepRecord &rec, double grad_norm2)
     if (fp64) {
         launch_block_solve();
         I.launch("k_reduce_dir", k_reduce_dir, kPartials, kBlock, I.v);
-        I.launch("k_final_dir", k_final_dir, 1, kBlock, I.v, 0);
         I.check();
         I.sync();
     }
@@ -3303,11 +3412,11 @@ KhsResult Engine::optimize_substep(double dt, KhsxSubstepRecord &rec)
         if (it == desc_.newton_iterations) break;
         progress_phase_.store(KHS_PHASE_LINEAR_SOLVE);
         // FP64 solve: the direction, its CCD bound and the first line-search
-        // trial (at the step k_final_dir leaves in device memory) are enqueued
+        // trial (at the step publish_ccd leaves in device memory) are enqueued
         // together, with one host synchronisation instead of three.  The
         // device runs the same kernels in the same order as step by step.
-        // The trust-radius limit is applied on the device (k_scale_trust, the
-        // host's scale when it applies, else nothing).  When the direction is
+        // The trust-radius limit is applied on the device (k_limit, the host's
+        // scale when it applies, else nothing).  When the direction is
         // not used as is (steepest fallback, CCD work-list overflow, step
         // below the minimum) the trial is discarded: the iterate is restored
         // and evaluated again, and the iteration goes on step by step.
@@ -3318,12 +3427,8 @@ KhsResult Engine::optimize_substep(double dt, KhsxSubstepRecord &rec)
         if (mode_ != KHSX_MODE_MIXED_FF) {
             launch_block_solve();
             I.launch("k_reduce_dir", k_reduce_dir, kPartials, kBlock, v);
-            I.launch("k_final_dir", k_final_dir, 1, kBlock, v, 0);
-            I.launch("k_scale", k_scale_trust, grid_for(6 * size_t(v.N)), kBlock, v, trust_radius_);
-            KHS_CUDA(cudaMemcpyAsync(v.q_base, v.q, 6 * size_t(v.N) * 8, cudaMemcpyDeviceToDevice, I.stream));
-            I.launch("k_reduce_dir", k_reduce_dir, kPartials, kBlock, v);
+            I.launch("k_limit", k_limit, kPartials, kBlock, v, trust_radius_, 0);
             if (v.has_collider) launch_ccd_bound();
-            I.launch("k_final_dir", k_final_dir, 1, kBlock, v, 1);
             first = evaluate(true, dt, -1.0, &v.sc->trial_alpha);
             const Mailbox &mb = *I.mail_host;
             const bool used = !mb.dir_solve_failed && mb.dir_slope < 0 && std::isfinite(mb.dir_slope);
@@ -3374,18 +3479,17 @@ KhsResult Engine::optimize_substep(double dt, KhsxSubstepRecord &rec)
                 alpha = first_alpha;
             } else {
                 // Slope of the (possibly scaled) direction, and the CCD bound.
-                I.launch("k_reduce_dir", k_reduce_dir, kPartials, kBlock, v);
+                I.launch("k_limit", k_limit, kPartials, kBlock, v, std::numeric_limits<double>::infinity(), 1);
                 if (v.has_collider) {
                     progress_phase_.store(KHS_PHASE_CCD);
                     launch_ccd_bound();
                 }
-                I.launch("k_final_dir", k_final_dir, 1, kBlock, v, 0);
                 I.check();
                 I.sync();
                 if (v.has_collider && I.mail_host->pair_count > v.pair_capacity) {
                     // Work list overflow: redo the bound with the per-element kernel.
                     I.launch("k_ccd", mode_ ? k_ccd<true> : k_ccd<false>, grid_for(v.E), kBlock, v);
-                    I.launch("k_final_dir", k_final_dir, 1, kBlock, v, 0);
+                    I.launch("k_publish_ccd", k_publish_ccd, 1, 1, v);
                     I.check();
                     I.sync();
                 }
