@@ -773,14 +773,44 @@ KHS_HD V gcross(V a, V b)
     return v(xs(xm(a.y, b.z), xm(a.z, b.y)), xs(xm(a.z, b.x), xm(a.x, b.z)), xs(xm(a.x, b.y), xm(a.y, b.x)));
 }
 
+// a / n rounded to nearest with r = 1 / n rounded to nearest: the quotient
+// a r, its exact remainder, and one correction by it, which Markstein
+// (Computation of elementary functions on the IBM RISC System/6000, 1990)
+// shows to round correctly when r does.  Three multiply-adds where a division
+// takes a dozen FP64 instructions, and several numerators share r.  The
+// division itself where the remainder or the quotient could leave the normal
+// range (a zero, tiny or huge a or n, a NaN).
+KHS_HD double div_by(double a, double n, double r)
+{
+    const int ea = int((bits_of(a) >> 52) & 0x7ff), en = int((bits_of(n) >> 52) & 0x7ff);
+    if (ea < 200 || ea > 1800 || en < 200 || en > 1800 || ea - en > 600 || en - ea > 600) return a / n;
+#if defined(__CUDA_ARCH__)
+    const double q = __dmul_rn(a, r);
+    return __fma_rn(__fma_rn(-q, n, a), r, q);
+#else
+    const double q = a * r;
+    return std::fma(std::fma(-q, n, a), r, q);
+#endif
+}
+
+// a / n for each component.
+KHS_HD V gdiv(V a, double n)
+{
+#if defined(__CUDA_ARCH__)
+    const double r = recip_any(n);
+    return v(div_by(a.x, n, r), div_by(a.y, n, r), div_by(a.z, n, r));
+#else
+    return v(a.x / n, a.y / n, a.z / n);
+#endif
+}
+
 // Unit vector with Eigen's normalized() semantics: a zero (or NaN) squared
 // norm leaves the vector unchanged; each component is divided.
 KHS_HD V gunit(V a)
 {
     const double n2 = gdot(a, a);
     if (!(n2 > 0.0)) return a;
-    const double n = sqrt(n2);
-    return v(a.x / n, a.y / n, a.z / n);
+    return gdiv(a, sqrt(n2));
 }
 
 // (1 - t) a + t b, each product and the sum rounded on its own.
@@ -847,7 +877,7 @@ KHS_HD Transport transport_between(V from, V to)
         t.kind = t.c > 0.0 ? 1 : 2;
         t.n = t.kind == 2 ? unit_orthogonal(a) : v(0.0, 0.0, 0.0);
     } else {
-        t.n = v(axis.x / t.s, axis.y / t.s, axis.z / t.s);
+        t.n = gdiv(axis, t.s);
     }
     return t;
 }
@@ -901,7 +931,7 @@ KHS_HD V rotation_vector(const M &r)
     if (!(n != 0.0)) return v(0.0, 0.0, 0.0);
     double angle = xm(2.0, atan2(n, fabs(q[3])));
     if (q[3] < 0.0) n = -n;
-    const V axis = v(q[0] / n, q[1] / n, q[2] / n);
+    const V axis = gdiv(v(q[0], q[1], q[2]), n);
     if (!gfinite(angle) || !gfinite(axis.x) || !gfinite(axis.y) || !gfinite(axis.z)) return v(0.0, 0.0, 0.0);
     if (angle > kPi) angle = xs(angle, xm(2.0, kPi));
     return gmul(axis, angle);

@@ -32,8 +32,8 @@
 //                 k_steepest, k_scale, k_reduce_dir, k_limit
 //   CCD           k_ccd (plain), k_ccd_collect + k_ccd_pairs (mixed)
 //   queries       k_contact, k_contact_query_records, k_gather
-//   root targets  k_root_tangents, k_root_transport, k_root_frames (thread
-//                 per strand), k_root_rotations: per call of
+//   root targets  k_root_tangents, k_root_transport, k_root_frames (three
+//                 lanes per strand), k_root_rotations: per call of
 //                 khsUpdateRootTargets / khsSetRootAnimationFrame
 // Reductions are two-level (fixed per-block trees, then one block over the
 // partials) and therefore deterministic.
@@ -2478,8 +2478,10 @@ __global__ void __launch_bounds__(kBlock) k_gather(const double *q, const uint32
 // Target positions and rotation vectors of every node for one set of
 // evaluated source points: positions and unit tangents, the tangent-only
 // part of each frame step (thread per node), the frame walk along each
-// strand (thread per strand, longest strands first), then the rotation
+// strand (three lanes per strand, longest strands first), then the rotation
 // vector of frame * reference^T (thread per node).
+
+constexpr int kRootStrands = 10;  // strands a warp in k_root_frames
 
 struct RootArgs {
     uint32_t N, S;
@@ -2534,24 +2536,86 @@ __global__ void __launch_bounds__(kBlock) k_root_transport(RootArgs a)
 
 // The sequential part (solver.cpp:435-443): each frame's first column is the
 // previous one carried by the minimal rotation between consecutive tangents.
-// One thread per strand, longest strands first.
-__global__ void __launch_bounds__(kBlock) k_root_frames(RootArgs a)
+// Three lanes a strand, one component each, ten strands a warp, longest
+// strands first; a warp a block, so that few strands spread over many SMs.
+// What bounds it is the FP64 chain of the longest strands: three normalisations
+// a node, each a dot product, a square root and a division; with a component a
+// lane a node takes about 130 FP64 instructions (270 with a thread a strand).
+// 4,000 strands of 16-160 nodes: 510 us, 2,041 with a thread a strand in
+// blocks of 256.
+struct Lanes3 {
+    int c, base;  // component, first lane of the strand
+    __device__ double at(double x, int k) const { return __shfl_sync(0xffffffffu, x, base + k); }
+    __device__ double next(double x) const { return at(x, c == 2 ? 0 : c + 1); }
+    __device__ double prev(double x) const { return at(x, c == 0 ? 2 : c - 1); }
+    __device__ double dot(double a, double b) const
+    {
+        const double m = dm::xm(a, b);
+        return dm::xa(dm::xa(at(m, 0), at(m, 1)), at(m, 2));
+    }
+    __device__ double cross(double a, double b) const
+    {
+        return dm::xs(dm::xm(next(a), prev(b)), dm::xm(prev(a), next(b)));
+    }
+    __device__ double unit(double a) const
+    {
+        const double n2 = dot(a, a);
+        if (!(n2 > 0.0)) return a;  // no shuffle below
+        const double n = sqrt(n2);
+        return dm::div_by(a, n, dm::recip_any(n));
+    }
+};
+
+// frame_from_d3 (khs_device_math.cuh) with a component a lane.
+__device__ __forceinline__ void frame_lanes(const Lanes3 &l, double d3, double hint, double &d1, double &d2)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.S) return;
-    const uint32_t s = a.sorder[i], first = a.sfirst[s], count = a.scount[s];
-    const double *r0 = a.ref + 9 * size_t(first);
+    d1 = dm::xs(hint, dm::xm(d3, l.dot(hint, d3)));
+    const bool flat = l.dot(d1, d1) < 1.0e-16;
+    if (__any_sync(0xffffffffu, flat)) {
+        const bool along_x = fabs(l.at(d3, 0)) < 0.8;
+        const double axis = l.c == (along_x ? 0 : 1) ? 1.0 : 0.0;
+        const double other = dm::xs(axis, dm::xm(d3, l.dot(axis, d3)));
+        if (flat) d1 = other;
+    }
+    d1 = l.unit(d1);
+    d2 = l.unit(l.cross(d3, d1));
+    d1 = l.unit(l.cross(d2, d3));
+}
+
+__global__ void __launch_bounds__(32) k_root_frames(RootArgs a)
+{
+    const int lane = threadIdx.x;
+    const int slot = min(lane / 3, kRootStrands - 1);  // lanes 30 and 31 shadow the last strand's first two
+    Lanes3 l;
+    l.c = lane < 3 * kRootStrands ? lane % 3 : lane - 3 * kRootStrands;
+    l.base = 3 * slot;
+    const uint32_t i = blockIdx.x * kRootStrands + slot;
+    const bool member = lane < 3 * kRootStrands && i < a.S;
+    const uint32_t s = a.sorder[min(i, a.S - 1)], first = a.sfirst[s], count = a.scount[s];
+    const uint32_t most = __reduce_max_sync(0xffffffffu, count);
     double *p = a.frame + 9 * size_t(first);
-    M f = dm::frame_from_d3(load3(p), dm::v(r0[0], r0[3], r0[6]));
-#pragma unroll
-    for (int c = 0; c < 9; ++c) p[c] = f.m[c];
-    for (uint32_t k = 1; k < count; ++k) {
-        p += 9;
-        dm::Transport tr;
-        tr.n = load3(p + 3); tr.s = p[6]; tr.c = p[7]; tr.kind = int(p[8]);
-        f = dm::frame_from_d3(load3(p), dm::transport_apply(tr, dm::v(f.m[0], f.m[3], f.m[6])));
-#pragma unroll
-        for (int c = 0; c < 9; ++c) p[c] = f.m[c];
+    double d3 = p[l.c], d1, d2, d3_next = 0.0, n = 0.0, sine = 0.0, cosine = 0.0, kind = 1.0;
+    // The next node's tangent and rotation, read while this node's frame is
+    // under way; a finished strand goes on with its last slot, unwritten.
+    auto fetch = [&](uint32_t k) {
+        const double *o = k < count ? p + 9 : p;
+        d3_next = o[l.c]; n = o[3 + l.c]; sine = o[6]; cosine = o[7]; kind = o[8];
+    };
+    fetch(1);
+    frame_lanes(l, d3, a.ref[9 * size_t(first) + 3 * l.c], d1, d2);
+    for (uint32_t k = 0;;) {
+        __syncwarp();  // every lane has read its share of the slot
+        if (member && k < count) { p[3 * l.c] = d1; p[3 * l.c + 1] = d2; p[3 * l.c + 2] = d3; }
+        if (++k >= most) break;
+        if (k < count) p += 9;
+        d3 = d3_next;
+        // transport_apply of the first column.
+        const double nd = l.dot(n, d1);
+        double hint = dm::xa(dm::xa(dm::xm(d1, cosine), dm::xm(l.cross(n, d1), sine)), dm::xm(dm::xm(n, nd), dm::xs(1.0, cosine)));
+        if (kind == 1.0 || k >= count) hint = d1;
+        else if (kind == 2.0) hint = dm::xs(dm::xm(dm::xm(n, 2.0), nd), d1);
+        fetch(k + 1);
+        frame_lanes(l, d3, hint, d1, d2);
     }
 }
 
@@ -3021,7 +3085,7 @@ KhsResult Engine::run_root_pass(const KhsVec3 *points, uint32_t count)
     KHS_CUDA(cudaMemsetAsync(I.root.bad, 0, sizeof(uint32_t), I.stream));
     I.launch("k_root_tangents", k_root_tangents, grid_for(N), kBlock, I.root);
     I.launch("k_root_transport", k_root_transport, grid_for(N), kBlock, I.root);
-    I.launch("k_root_frames", k_root_frames, grid_for(I.v.S), kBlock, I.root);
+    I.launch("k_root_frames", k_root_frames, grid_for(I.v.S, kRootStrands), 32, I.root);
     I.launch("k_root_rotations", k_root_rotations, grid_for(N), kBlock, I.root);
     I.check();
     uint32_t bad = 0;
