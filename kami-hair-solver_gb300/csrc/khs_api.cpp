@@ -269,27 +269,21 @@ struct KhsSolver {
         return KHS_OK;
     }
 
-    // Source points of new root targets: the solver must be built, the
-    // count must match the curves, every coordinate finite
-    // (solver.cpp:802-811).  The targets themselves are computed on the
-    // device by the engine.
-    KhsResult check_root_points(const KhsVec3 *p, uint32_t n, KhsResult bad_point, KhsResult bad_count)
+    // Source points of new root targets: the solver must be built and the
+    // count must match the curves (solver.cpp:802-811).  The engine computes
+    // the targets on the device and rejects non-finite points there.
+    KhsResult check_root_points(const KhsVec3 *p, uint32_t n)
     {
         if (!built || !engine || !p || n != input.points.size()) {
             error = "the root target point count does not match the source curves";
-            return bad_count;
+            return KHS_ERROR_INVALID_ARGUMENT;
         }
-        for (uint32_t i = 0; i < n; ++i)
-            if (!finite3(p[i])) {
-                error = "root targets have a non-finite coordinate";
-                return bad_point;
-            }
         return KHS_OK;
     }
 
     KhsResult update_roots(const KhsVec3 *p, uint32_t n)
     {
-        const KhsResult r = check_root_points(p, n, KHS_ERROR_INVALID_HAIR, KHS_ERROR_INVALID_ARGUMENT);
+        const KhsResult r = check_root_points(p, n);
         if (r != KHS_OK) return r;
         return from_engine(engine->set_pending_root_points(p, n));
     }
@@ -461,7 +455,7 @@ KHS_API KhsResult khsAllocateAnimation(KhsSolver *s, uint32_t frame_count)
 KHS_API KhsResult khsSetRootAnimationFrame(KhsSolver *s, uint32_t frame_index, const KhsVec3 *points, uint32_t point_count)
 {
     return guarded(s, [&] {
-        const KhsResult c = s->check_root_points(points, point_count, KHS_ERROR_INVALID_HAIR, KHS_ERROR_INVALID_ARGUMENT);
+        const KhsResult c = s->check_root_points(points, point_count);
         if (c != KHS_OK) return c;
         return s->from_engine(s->engine->set_root_animation_frame(frame_index, points, point_count));
     });
@@ -732,9 +726,14 @@ KHS_API KhsResult khsxComputeRootTargets(KhsSolver *s, const KhsVec3 *points, ui
                                          KhsVec3 *rotations, uint32_t node_capacity)
 {
     return guarded(s, [&] {
-        const KhsResult c = s->check_root_points(points, point_count, KHS_ERROR_INVALID_HAIR, KHS_ERROR_INVALID_ARGUMENT);
+        const KhsResult c = s->check_root_points(points, point_count);
         if (c != KHS_OK) return c;
         if (!positions || !rotations || node_capacity < s->model.nodes()) {
+            for (uint32_t i = 0; i < point_count; ++i)
+                if (!finite3(points[i])) {
+                    s->error = khs::kRootPointsNotFinite;
+                    return KHS_ERROR_INVALID_HAIR;
+                }
             s->error = "the root target output arrays are smaller than the internal node count";
             return KHS_ERROR_INVALID_ARGUMENT;
         }

@@ -2484,14 +2484,14 @@ __global__ void __launch_bounds__(kBlock) k_gather(const double *q, const uint32
 constexpr int kRootStrands = 10;  // strands a warp in k_root_frames
 
 struct RootArgs {
-    uint32_t N, S;
+    uint32_t N, S, P;
     const double *points;                    // [P][3] evaluated source points
     const uint32_t *bind_l, *bind_r;         // the two source points a node interpolates
     const double *bind_t;
     const uint32_t *node_strand, *sfirst, *scount, *sorder;
     const double *ref;                       // [N][9] reference frames
     double *x, *tangent, *frame, *rot;       // [N][3], [N][3], [N][9], [N][3]
-    uint32_t *bad;                           // nonzero after a degenerate tangent
+    uint32_t *bad;                           // bit 0: a degenerate tangent, bit 1: a non-finite point
 };
 
 __device__ __forceinline__ V root_position(const RootArgs &a, uint32_t n)
@@ -2500,10 +2500,18 @@ __device__ __forceinline__ V root_position(const RootArgs &a, uint32_t n)
 }
 
 // Central-difference tangents, one-sided at the strand ends
-// (solver.cpp:426-433); a squared length below 1e-24 fails the whole call.
+// (solver.cpp:426-433); a squared length below 1e-24 fails the whole call, and
+// so does a point that is not finite.
 __global__ void __launch_bounds__(kBlock) k_root_tangents(RootArgs a)
 {
     const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
+    if (n < a.P) {
+        bool finite = true;
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            finite = finite && (uint32_t(__double2hiint(a.points[3 * size_t(n) + k])) & 0x7ff00000u) != 0x7ff00000u;
+        if (!finite) atomicOr(a.bad, 2u);
+    }
     if (n >= a.N) return;
     const uint32_t s = a.node_strand[n], k = n - a.sfirst[s], count = a.scount[s];
     const V x = root_position(a, n);
@@ -3082,8 +3090,9 @@ KhsResult Engine::run_root_pass(const KhsVec3 *points, uint32_t count)
         I.root.bad = reinterpret_cast<uint32_t *>(base + off);
     }
     KHS_CUDA(cudaMemcpyAsync(const_cast<double *>(I.root.points), points, size_t(count) * 24, cudaMemcpyHostToDevice, I.stream));
+    I.root.P = count;
     KHS_CUDA(cudaMemsetAsync(I.root.bad, 0, sizeof(uint32_t), I.stream));
-    I.launch("k_root_tangents", k_root_tangents, grid_for(N), kBlock, I.root);
+    I.launch("k_root_tangents", k_root_tangents, grid_for(std::max<size_t>(N, count)), kBlock, I.root);
     I.launch("k_root_transport", k_root_transport, grid_for(N), kBlock, I.root);
     I.launch("k_root_frames", k_root_frames, grid_for(I.v.S, kRootStrands), 32, I.root);
     I.launch("k_root_rotations", k_root_rotations, grid_for(N), kBlock, I.root);
@@ -3091,6 +3100,10 @@ KhsResult Engine::run_root_pass(const KhsVec3 *points, uint32_t count)
     uint32_t bad = 0;
     KHS_CUDA(cudaMemcpyAsync(&bad, I.root.bad, sizeof(bad), cudaMemcpyDeviceToHost, I.stream));
     I.sync();
+    if (bad & 2u) {
+        error_ = kRootPointsNotFinite;  // rejected like other bad arguments: no failed phase
+        return KHS_ERROR_INVALID_HAIR;
+    }
     if (bad) return fail(KHS_ERROR_INVALID_HAIR, "cannot compute root directions from the root targets");
     return KHS_OK;
 }

@@ -30,6 +30,8 @@ struct KernelTiming {
     double milliseconds;
 };
 
+constexpr const char *kRootPointsNotFinite = "root targets have a non-finite coordinate";
+
 class Engine {
 public:
     Engine();
@@ -45,8 +47,8 @@ public:
     // Root targets of every node (positions and rotation vectors) for the
     // evaluated source points, computed on the device (solver.cpp:416-447):
     // into the pending targets of the next step, into an animation frame, or
-    // back to the host.  The points must be finite; a degenerate tangent
-    // gives KHS_ERROR_INVALID_HAIR and changes nothing.
+    // back to the host.  A non-finite point or a degenerate tangent gives
+    // KHS_ERROR_INVALID_HAIR and changes nothing.
     KhsResult set_pending_root_points(const KhsVec3 *points, uint32_t count);
     KhsResult root_targets_to_host(const KhsVec3 *points, uint32_t count, KhsVec3 *positions, KhsVec3 *rotations);
     void set_pending_collider(const std::vector<Vec> &vertices);

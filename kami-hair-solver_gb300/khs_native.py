@@ -548,8 +548,8 @@ class HairSolver:
         internal node, each (N, 3), for the evaluated source points."""
         pts = _vec3_buffer(points)
         n = self.build_stats().internal_node_count
-        pos = np.zeros((n, 3), dtype=np.float64)
-        rot = np.zeros((n, 3), dtype=np.float64)
+        pos = np.empty((n, 3), dtype=np.float64)
+        rot = np.empty((n, 3), dtype=np.float64)
         self._check(self._library.khsxComputeRootTargets(self._handle, _ptr(pts), len(pts), _ptr(pos), _ptr(rot), n))
         return pos, rot
 
