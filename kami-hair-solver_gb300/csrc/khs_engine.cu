@@ -18,9 +18,9 @@
 //                  bottom-up refit)
 //
 // Kernels (thread per node / element / BVH leaf unless noted):
-//   per substep   k_begin_substep, k_collider_interp, k_tri32, k_refit,
-//                 k_sweep(+record), k_precond, k_update_velocity,
-//                 k_friction(+apply)
+//   per substep   k_begin_substep, k_refit (eight lanes per leaf),
+//                 k_sweep_collect, k_sweep_near, k_advance_pairs,
+//                 k_sweep_record, k_update_velocity, k_friction(+apply)
 //   evaluation    k_node_eval, [mixed: k_contact_filter, k_contact_near (warp
 //                 per element with cached leaves), k_contact_exact (thread per
 //                 FP32 survivor), k_contact_select], k_elem_eval, k_node_sum
@@ -155,7 +155,10 @@ struct View {
     const uint32_t *tri;
     double *col_cur, *col_old;
     float *col32;  // FP32 copy of col_cur for the mixed form's filters
-    double *blo, *bhi;
+    double *blo, *bhi;  // leaves only: the FP64 boxes of the exact leaf test
+    // The tree over old and new positions, for the moving-collider sweep.
+    double *swept_lo, *swept_hi;
+    float4 *swept_node;
     // Mixed form: each BVH node packed in 32 bytes (FP32 outward-rounded box,
     // escape index, leaf range), the per-element contact result of the
     // separate contact pass, and the CCD (element, triangle) work list.
@@ -431,70 +434,147 @@ __device__ __forceinline__ float candidate_distance_f(const View &d, uint32_t t,
 
 // ---- per-substep set-up ---------------------------------------------------
 
-__global__ void __launch_bounds__(kBlock) k_begin_substep(View d, const double *root_a, const double *rot_a,
-                                                          const double *root_b, const double *rot_b, double f, double dt)
+// Start of a substep, thread per node and per collider vertex.  Uncontracted
+// lerps: the root targets and collider vertices feed the integer contact work,
+// so they round exactly like a host evaluation.
+struct SubstepTargets {
+    const double *root_a, *rot_a, *root_b, *rot_b;  // [N][3]
+    const double *col_a, *col_b;                    // [V][3]
+    double f, dt;
+};
+
+__global__ void __launch_bounds__(kBlock) k_begin_substep(View d, SubstepTargets s)
 {
     const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
+    const double f = s.f;
+    if (d.has_collider && n < d.V) {
+        const V cur = load3(d.col_cur + 3 * size_t(n));
+        store3(d.col_old + 3 * size_t(n), cur);
+        const V nv = dm::gadd(dm::gmul(load3(s.col_a + 3 * size_t(n)), 1.0 - f), dm::gmul(load3(s.col_b + 3 * size_t(n)), f));
+        store3(d.col_cur + 3 * size_t(n), nv);
+        d.col32[3 * size_t(n)] = float(nv.x); d.col32[3 * size_t(n) + 1] = float(nv.y); d.col32[3 * size_t(n) + 2] = float(nv.z);
+    }
     if (n >= d.N) return;
     double q[6];
 #pragma unroll
     for (int k = 0; k < 6; ++k) { q[k] = d.q[6 * size_t(n) + k]; d.q_old[6 * size_t(n) + k] = q[k]; }
     if (!d.fixed[n]) return;
-    // Uncontracted lerps: the root targets and collider vertices feed the
-    // integer contact work, so they round exactly like a host evaluation.
-    const V p = dm::gadd(dm::gmul(load3(root_a + 3 * size_t(n)), 1.0 - f), dm::gmul(load3(root_b + 3 * size_t(n)), f));
-    const V r = dm::gadd(dm::gmul(load3(rot_a + 3 * size_t(n)), 1.0 - f), dm::gmul(load3(rot_b + 3 * size_t(n)), f));
+    const V p = dm::gadd(dm::gmul(load3(s.root_a + 3 * size_t(n)), 1.0 - f), dm::gmul(load3(s.root_b + 3 * size_t(n)), f));
+    const V r = dm::gadd(dm::gmul(load3(s.rot_a + 3 * size_t(n)), 1.0 - f), dm::gmul(load3(s.rot_b + 3 * size_t(n)), f));
     const double vals[6] = {p.x, p.y, p.z, r.x, r.y, r.z};
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
         d.q[6 * size_t(n) + k] = vals[k];
-        d.v[6 * size_t(n) + k] = (vals[k] - q[k]) / dt;
+        d.v[6 * size_t(n) + k] = (vals[k] - q[k]) / s.dt;
     }
 }
 
-__global__ void __launch_bounds__(kBlock) k_collider_interp(View d, const double *a, const double *b, double f)
+// Minima and maxima of coordinates on order-preserving integers: an FP64
+// minimum costs several FP64 issue slots, 144 to 288 of them a leaf.  A NaN is
+// skipped, as fmin and fmax do.
+__device__ __forceinline__ long long order_key(double x)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= d.V) return;
-    const V cur = load3(d.col_cur + 3 * size_t(i));
-    store3(d.col_old + 3 * size_t(i), cur);
-    const V nv = dm::gadd(dm::gmul(load3(a + 3 * size_t(i)), 1.0 - f), dm::gmul(load3(b + 3 * size_t(i)), f));
-    store3(d.col_cur + 3 * size_t(i), nv);
-    d.col32[3 * size_t(i)] = float(nv.x); d.col32[3 * size_t(i) + 1] = float(nv.y); d.col32[3 * size_t(i) + 2] = float(nv.z);
+    const long long b = __double_as_longlong(x);
+    return b ^ ((b >> 63) & 0x7fffffffffffffffll);
 }
+__device__ __forceinline__ double from_key(long long k) { return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll)); }
 
-// The outward-rounded FP32 box of a packed node (its escape index and leaf
-// range, the .w words, are the build's).
-__device__ __forceinline__ void put_box(const View &d, uint32_t node, V lo, V hi)
+struct KeyBox {
+    long long lo[3], hi[3];
+    __device__ void clear()
+    {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) { lo[k] = order_key(1e300); hi[k] = order_key(-1e300); }
+    }
+    __device__ void add(V p)
+    {
+        const double x[3] = {p.x, p.y, p.z};
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const long long b = __double_as_longlong(x[k]), key = order_key(x[k]);
+            if ((b & 0x7fffffffffffffffll) > 0x7ff0000000000000ll) continue;
+            lo[k] = min(lo[k], key);
+            hi[k] = max(hi[k], key);
+        }
+    }
+    // Over the eight lanes of a leaf.
+    __device__ void reduce8()
+    {
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                lo[k] = min(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], o));
+                hi[k] = max(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], o));
+            }
+    }
+};
+
+// A leaf's FP64 box and its outward-rounded FP32 copy in the packed node,
+// whose .w words (escape index and leaf range) are the build's.
+__device__ __forceinline__ void put_leaf(float4 *bnode, double *blo, double *bhi, uint32_t node, const KeyBox &box)
 {
-    float4 *pn = d.bnode + 2 * size_t(node);
+    const V lo = dm::v(from_key(box.lo[0]), from_key(box.lo[1]), from_key(box.lo[2]));
+    const V hi = dm::v(from_key(box.hi[0]), from_key(box.hi[1]), from_key(box.hi[2]));
+    store3(blo + 3 * size_t(node), lo);
+    store3(bhi + 3 * size_t(node), hi);
+    float4 *pn = bnode + 2 * size_t(node);
     pn[0].x = __double2float_rd(lo.x); pn[0].y = __double2float_rd(lo.y); pn[0].z = __double2float_rd(lo.z);
     pn[1].x = __double2float_ru(hi.x); pn[1].y = __double2float_ru(hi.y); pn[1].z = __double2float_ru(hi.z);
 }
 
-// Bottom-up refit in one launch: each leaf thread computes its box and walks
-// up; the second child to arrive at a parent (atomic counter) merges the two
-// children, resets the counter for the next launch and continues.
-__global__ void __launch_bounds__(kBlock) k_refit(View d, int swept)
+// An inner node's FP32 box from its children's: rounding is monotone, so the
+// merge of the rounded boxes is the rounded merge.  Inner boxes are only ever
+// tested in FP32.
+__device__ __forceinline__ void merge_children(float4 *bnode, uint32_t p, uint32_t l, uint32_t r)
 {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= d.L) return;
-    uint32_t node = d.bleaves[k];
-    V lo = dm::v(1e300, 1e300, 1e300), hi = dm::v(-1e300, -1e300, -1e300);
-    const uint32_t first = d.bfirst[node], cnt = d.bcount[node];
-    for (uint32_t j = first; j < first + cnt; ++j) {
-        const uint32_t t = d.border[j];
+    const float4 la = __ldcg(bnode + 2 * size_t(l)), lb = __ldcg(bnode + 2 * size_t(l) + 1);
+    const float4 ra = __ldcg(bnode + 2 * size_t(r)), rb = __ldcg(bnode + 2 * size_t(r) + 1);
+    float4 *pn = bnode + 2 * size_t(p);
+    pn[0].x = fminf(la.x, ra.x); pn[0].y = fminf(la.y, ra.y); pn[0].z = fminf(la.z, ra.z);
+    pn[1].x = fmaxf(lb.x, rb.x); pn[1].y = fmaxf(lb.y, rb.y); pn[1].z = fmaxf(lb.z, rb.z);
+}
+
+// Bottom-up refit of both trees (at the new positions, and swept over old and
+// new ones) and the FP32 records of every triangle, in one launch: eight lanes
+// a leaf, a triangle each; the first one walks up, the second child to arrive
+// at a parent (atomic counter) merges the two children, resets the counter for
+// the next launch and continues.  Two launches with a thread a leaf, and a
+// third for the records, took 72 us a substep on 1,280 triangles and 230 on
+// 449,940; this one 24 and 127.
+constexpr int kLeafTriangles = 8;  // BVH leaves hold at most 8 triangles (cuda_backend.cu:305)
+__global__ void __launch_bounds__(kBlock) k_refit(View d)
+{
+    const uint32_t thread = blockIdx.x * blockDim.x + threadIdx.x, leaf = thread / kLeafTriangles, sub = thread % kLeafTriangles;
+    const bool live = leaf < d.L;
+    uint32_t node = 0;
+    KeyBox now, swept;
+    now.clear();
+    swept.clear();
+    if (live) {
+        node = d.bleaves[leaf];
+        const uint32_t p = d.bfirst[node] + sub;
+        if (sub < d.bcount[node]) {
+            const uint32_t t = d.border[p];
+            float4 *rec = d.tri32 + 3 * size_t(p), *rec_old = d.tri32_old + 3 * size_t(p);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const uint32_t vi = d.tri[3 * t + c];
-            const V a = load3(d.col_cur + 3 * size_t(vi));
-            lo = dm::vmin(lo, a); hi = dm::vmax(hi, a);
-            if (swept) { const V o = load3(d.col_old + 3 * size_t(vi)); lo = dm::vmin(lo, o); hi = dm::vmax(hi, o); }
+            for (int c = 0; c < 3; ++c) {
+                const uint32_t vi = d.tri[3 * t + c];
+                const V a = load3(d.col_cur + 3 * size_t(vi)), o = load3(d.col_old + 3 * size_t(vi));
+                const float w = c == 0 ? __uint_as_float(t) : 0.0f;
+                rec[c] = make_float4(float(a.x), float(a.y), float(a.z), w);
+                rec_old[c] = make_float4(float(o.x), float(o.y), float(o.z), w);
+                now.add(a);
+                swept.add(a);
+                swept.add(o);
+            }
         }
     }
-    store3(d.blo + 3 * size_t(node), lo);
-    store3(d.bhi + 3 * size_t(node), hi);
-    put_box(d, node, lo, hi);
+    now.reduce8();
+    swept.reduce8();
+    if (!live || sub != 0) return;
+    put_leaf(d.bnode, d.blo, d.bhi, node, now);
+    put_leaf(d.swept_node, d.swept_lo, d.swept_hi, node, swept);
     for (;;) {
         const int32_t p = d.bparent[node];
         if (p < 0) return;
@@ -502,16 +582,9 @@ __global__ void __launch_bounds__(kBlock) k_refit(View d, int swept)
         if (atomicAdd(&d.brefit[p], 1u) == 0) return;
         d.brefit[p] = 0;
         __threadfence();
-        const volatile double *blo = d.blo, *bhi = d.bhi;
         const uint32_t l = d.bleft[p], r = d.bright[p];
-        const V llo = dm::v(blo[3 * l], blo[3 * l + 1], blo[3 * l + 2]), rlo = dm::v(blo[3 * r], blo[3 * r + 1], blo[3 * r + 2]);
-        const V lhi = dm::v(bhi[3 * l], bhi[3 * l + 1], bhi[3 * l + 2]), rhi = dm::v(bhi[3 * r], bhi[3 * r + 1], bhi[3 * r + 2]);
-        const V plo = dm::vmin(llo, rlo), phi = dm::vmax(lhi, rhi);
-        store3(d.blo + 3 * size_t(p), plo);
-        store3(d.bhi + 3 * size_t(p), phi);
-        // Rounding is monotone, so rounding the merged FP64 box equals the
-        // merge of the rounded children.
-        put_box(d, p, plo, phi);
+        merge_children(d.bnode, uint32_t(p), l, r);
+        merge_children(d.swept_node, uint32_t(p), l, r);
         node = uint32_t(p);
     }
 }
@@ -821,26 +894,7 @@ template<bool MIXED> __global__ void __launch_bounds__(kBlock) k_contact(View d,
 // contacts that took 2.0 ms an evaluation; the pairs are few (7,000 there) and
 // independent.
 
-constexpr int kLeafTriangles = 8;  // BVH leaves hold at most 8 triangles (cuda_backend.cu:305)
 constexpr uint32_t kSurvOverflow = 0xffffffffu;  // surv_n: no room in a pool, k_contact_select searches
-
-// FP32 vertex records of every triangle in leaf order, of col_cur and of
-// col_old; run whenever they change (after k_collider_interp and at set-up).
-__global__ void __launch_bounds__(kBlock) k_tri32(View d)
-{
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= d.T) return;
-    const uint32_t t = d.border[p];
-    const V a = tri_vertex(d, t, 0), b = tri_vertex(d, t, 1), c = tri_vertex(d, t, 2);
-    d.tri32[3 * size_t(p)] = make_float4(float(a.x), float(a.y), float(a.z), __uint_as_float(t));
-    d.tri32[3 * size_t(p) + 1] = make_float4(float(b.x), float(b.y), float(b.z), 0.0f);
-    d.tri32[3 * size_t(p) + 2] = make_float4(float(c.x), float(c.y), float(c.z), 0.0f);
-    const V oa = load3(d.col_old + 3 * size_t(d.tri[3 * t])), ob = load3(d.col_old + 3 * size_t(d.tri[3 * t + 1])),
-            oc = load3(d.col_old + 3 * size_t(d.tri[3 * t + 2]));
-    d.tri32_old[3 * size_t(p)] = make_float4(float(oa.x), float(oa.y), float(oa.z), __uint_as_float(t));
-    d.tri32_old[3 * size_t(p) + 1] = make_float4(float(ob.x), float(ob.y), float(ob.z), 0.0f);
-    d.tri32_old[3 * size_t(p) + 2] = make_float4(float(oc.x), float(oc.y), float(oc.z), 0.0f);
-}
 
 // candidate_distance_f on the record at leaf-order position p (one 48-byte
 // record instead of an index triple and three vertex reads).
@@ -2844,7 +2898,7 @@ void Engine::initialize(const Model &m, const KhsSolverDesc &desc, const KhsHair
     bytes += 3 * padded<double>(E) + 2 * padded<uint32_t>(E) + padded<uint8_t>(E);
     bytes += 5 * padded<uint32_t>(S);
     bytes += padded<uint32_t>(3 * T) + 5 * padded<double>(3 * Vn) + padded<float>(3 * Vn);
-    bytes += padded<float4>(2 * B);
+    bytes += 2 * padded<float4>(2 * B);
     // Pairs of the contact pass: the mixed form keeps one or two candidates of
     // an element near the surface, the plain form all of them, hundreds at a
     // mesh pole; a full pool falls back to the search by one thread.
@@ -2859,7 +2913,7 @@ void Engine::initialize(const Model &m, const KhsSolverDesc &desc, const KhsHair
     bytes += 2 * padded<float2>(36 * N) + padded<float2>(6 * N) + padded<float>(N);
     bytes += 2 * padded<float4>(3 * T) + 2 * padded<uint32_t>(surv_capacity) + 2 * padded<uint32_t>(E) +
              padded<double>(5 * surv_capacity);
-    bytes += 2 * padded<double>(3 * B) + 4 * padded<uint32_t>(B) + padded<int32_t>(B) + 2 * padded<uint32_t>(B) +
+    bytes += 4 * padded<double>(3 * B) + 4 * padded<uint32_t>(B) + padded<int32_t>(B) + 2 * padded<uint32_t>(B) +
              padded<uint32_t>(L) + padded<uint32_t>(T);
     bytes += padded<Partial>(kPartials) + padded<DirPartial>(kPartials) + padded<Scalars>(1);
     bytes += padded<uint32_t>(O) + padded<double>(3 * std::max(N, O));
@@ -2902,7 +2956,9 @@ void Engine::initialize(const Model &m, const KhsSolverDesc &desc, const KhsHair
     v.col32 = a.take<float>(3 * Vn);
     I.col_frame_start = a.take<double>(3 * Vn); I.col_pending = a.take<double>(3 * Vn); I.col_a_copy = a.take<double>(3 * Vn);
     v.blo = a.take<double>(3 * B); v.bhi = a.take<double>(3 * B);
+    v.swept_lo = a.take<double>(3 * B); v.swept_hi = a.take<double>(3 * B);
     v.bnode = B ? a.take<float4>(2 * B) : nullptr;
+    v.swept_node = B ? a.take<float4>(2 * B) : nullptr;
     v.c_t = a.take<double>(E); v.c_dist = a.take<double>(E); v.c_bary = a.take<double>(3 * E);
     v.pair_elem = a.take<uint32_t>(pair_capacity); v.pair_tri = a.take<uint32_t>(pair_capacity);
     v.pair_capacity = uint32_t(pair_capacity);
@@ -3006,6 +3062,7 @@ void Engine::initialize(const Model &m, const KhsSolverDesc &desc, const KhsHair
             packed[2 * k + 1] = make_float4(hi32[3 * k], hi32[3 * k + 1], hi32[3 * k + 2], l_f);
         }
         up(v.bnode, packed.data(), 2 * B * sizeof(float4));
+        up(v.swept_node, packed.data(), 2 * B * sizeof(float4));  // its .w words are never written again
         up(bfirst, m.bvh.first.data(), B * 4); up(bcount, m.bvh.count.data(), B * 4);
         up(bparent, m.bvh.parent.data(), B * 4); up(bleft, m.bvh.left_child.data(), B * 4);
         up(bright, m.bvh.right_child.data(), B * 4); up(bleaves, m.bvh.leaves.data(), L * 4);
@@ -3021,7 +3078,7 @@ void Engine::initialize(const Model &m, const KhsSolverDesc &desc, const KhsHair
     KHS_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void **>(&v.sweep), I.sweep_host, 0));
     v.has_collider = T > 0 ? 1 : 0;
     I.launch("k_init_scalars", k_init_scalars, 1, 1, v);
-    if (T) I.launch("k_tri32", k_tri32, grid_for(T), kBlock, v);
+    if (T) I.launch("k_refit", k_refit, grid_for(size_t(kLeafTriangles) * v.L), kBlock, v);
     KHS_CUDA(cudaGetLastError());
     I.original_count = uint32_t(O);
     I.fixed_host = m.fixed;
@@ -3299,6 +3356,7 @@ bool Engine::limit_direction(double max_translation)
 bool Engine::make_steepest()
 {
     Impl &I = *d_;
+    I.launch("k_precond", k_precond, grid_for(I.v.N), kBlock, I.v, last_dt_);
     I.launch("k_steepest", k_steepest, grid_for(6 * size_t(I.v.N)), kBlock, I.v);
     I.launch("k_reduce_dir", k_reduce_dir, kPartials, kBlock, I.v);
     I.check();
@@ -3457,7 +3515,6 @@ KhsResult Engine::optimize_substep(double dt, KhsxSubstepRecord &rec)
     Impl &I = *d_;
     last_dt_ = dt;
     const View &v = I.v;
-    I.launch("k_precond", k_precond, grid_for(v.N), kBlock, v, dt);
     EvalStats current = evaluate(true, dt, -1.0);
     if (!current.feasible) return fail(KHS_ERROR_NOT_CONVERGED, "state is outside the barrier feasible region");
     const double initial = std::sqrt(current.grad_norm2);
@@ -3685,23 +3742,24 @@ KhsResult Engine::run_frame(double frame_dt, const double *root_a, const double 
             rec.substep = sub;
             rec.minimum_gap = std::numeric_limits<double>::infinity();
             const double f = double(sub) / substeps;
-            I.launch("k_begin_substep", k_begin_substep, grid_for(v.N), kBlock, v, root_a, rot_a, root_b, rot_b, f, dt);
+            const SubstepTargets targets{root_a, rot_a, root_b, rot_b, I.col_a_copy, col_b, f, dt};
+            I.launch("k_begin_substep", k_begin_substep, grid_for(std::max(v.N, v.has_collider ? v.V : 0u)), kBlock, v, targets);
             if (v.has_collider) {
-                I.launch("k_collider_interp", k_collider_interp, grid_for(v.V), kBlock, v, I.col_a_copy, col_b, f);
-                I.launch("k_tri32", k_tri32, grid_for(v.T), kBlock, v);
-                I.launch("k_refit", k_refit, grid_for(v.L), kBlock, v, 1);
+                I.launch("k_refit", k_refit, grid_for(size_t(kLeafTriangles) * v.L), kBlock, v);
+                View vs = v;  // walks the swept tree
+                vs.bnode = v.swept_node; vs.blo = v.swept_lo; vs.bhi = v.swept_hi;
                 progress_phase_.store(KHS_PHASE_CCD);
                 KHS_CUDA(cudaMemsetAsync(&v.sc->pool_used, 0, sizeof(uint32_t), I.stream));
-                I.launch("k_sweep_collect", k_sweep_collect, grid_for(v.E), kBlock, v);
-                I.launch("k_sweep_near", mode_ ? k_sweep_near<true> : k_sweep_near<false>, 152u * 8u, kBlock, v);
-                I.launch("k_sweep_pairs", k_advance_pairs<true>, kPairGrid, kPairBlock, v);
-                I.launch("k_sweep_record", k_sweep_record, 1, 1, v);
+                I.launch("k_sweep_collect", k_sweep_collect, grid_for(v.E), kBlock, vs);
+                I.launch("k_sweep_near", mode_ ? k_sweep_near<true> : k_sweep_near<false>, 152u * 8u, kBlock, vs);
+                I.launch("k_sweep_pairs", k_advance_pairs<true>, kPairGrid, kPairBlock, vs);
+                I.launch("k_sweep_record", k_sweep_record, 1, 1, vs);
                 I.check();
                 I.sync();
                 if (I.mail_host->pair_count > v.pair_capacity) {
                     // Pair list overflow: every element by one thread.
-                    I.launch("k_sweep", k_sweep, grid_for(v.E), kBlock, v);
-                    I.launch("k_sweep_record", k_sweep_record, 1, 1, v);
+                    I.launch("k_sweep", k_sweep, grid_for(v.E), kBlock, vs);
+                    I.launch("k_sweep_record", k_sweep_record, 1, 1, vs);
                     I.check();
                     I.sync();
                 }
@@ -3721,7 +3779,6 @@ KhsResult Engine::run_frame(double frame_dt, const double *root_a, const double 
                     crossed = true;
                     break;
                 }
-                I.launch("k_refit", k_refit, grid_for(v.L), kBlock, v, 0);
                 rebuild_cache_ = true;
             }
             progress_phase_.store(KHS_PHASE_ASSEMBLING);
