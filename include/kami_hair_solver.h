@@ -407,7 +407,8 @@ KHS_API KhsResult khsxSetSolveMode(KhsSolver *solver, uint32_t mode);
 KHS_API uint32_t khsxGetSolveMode(const KhsSolver *solver);
 
 /* Launch shape of the FP64 block-tridiagonal solve.  By default a rule on the
-   strands' lengths chooses it; this pins it: strands_per_warp 5 (6 lanes per
+   strands' lengths chooses it (also three warps for every strand, which only
+   the rule takes); this pins it: strands_per_warp 5 (6 lanes per
    strand), or 1 or 2 (a warp for every strand: the shortest sequential
    chain), blocks_per_sm 1-8 (four warps each); long_strands > 0 (with
    strands_per_warp 5 or 1) gives that many longest strands a warp each and

@@ -1,5 +1,5 @@
 // FP64 block-tridiagonal solve of the Gauss-Newton direction: the device
-// code of k_block_solve (khs_engine.cu), for a view D of the solver's arrays
+// code of k_block_solve and k_block_solve_team (khs_engine.cu), for a view D of the solver's arrays
 // (diag, upper, cprime [N][36]; grad, dprime, dir [N][6]; the strands' order
 // and ranges; sc->solve_failed).
 #pragma once
@@ -25,7 +25,10 @@ constexpr int kStrandsPerWarp = 5;  // solve_strands_five: 6 lanes per strand
 // cycles whatever the number of active lanes (76 with all four
 // sub-partitions busy), and a dependent one waits as long, so a strand's time
 // is its chain of nodes and the machine's throughput is instructions times 76
-// cycles.  Two layouts, one for each:
+// cycles.  Three layouts:
+// * solve_strand_team: one strand on three warps, the pivot chain on one and
+//   what follows it on the others, 4,000 cycles a node alone and 4,550 with
+//   608 strands;
 // * solve_strand_warp: one strand on a warp, one matrix entry per lane, 42
 //   FP64 instructions and 4,950 cycles a node alone, 3,200 of a
 //   sub-partition's cycles when the machine is full;
@@ -35,11 +38,11 @@ constexpr int kStrandsPerWarp = 5;  // solve_strands_five: 6 lanes per strand
 // (160-node strands.  The layouts they replace, with 6 H lanes a strand and
 // four warps on the longest, took 12,000 cycles a node on one warp, 8,800 on
 // four.)
-// Both take the pivot's reciprocal on the integer pipes (dm::recip_rn, equal
+// All take the pivot's reciprocal on the integer pipes (dm::recip_rn, equal
 // to the FP64 division) for every candidate of the column while the pivot
 // search runs.  Shuffles, reductions and FP64 instructions share a queue that
 // issues in order, so shuffles are counted like arithmetic.  Every entry goes
-// through the same operations in the same order in both layouts, so the
+// through the same operations in the same order in every layout, so the
 // results are identical bit for bit and the split between them changes no
 // result.
 
@@ -147,6 +150,57 @@ template<bool EXACT> __device__ __forceinline__ bool eliminate_node(WarpNode &w,
     return EXACT ? flag : __any_sync(FULL, flag);
 }
 
+// Back substitution d_n = d'_n - C_n d_{n+1} of one strand on a warp, every
+// lane of row r: a chain of six multiply-adds a node, shorter than a read from
+// L2, so the rows come through a ring of asynchronous copies (16 bytes a lane),
+// and from there to registers one node ahead.  C and d' are visible to the
+// warp.
+template<class D>
+__device__ __forceinline__ void substitute_back(const D &d, uint32_t begin, uint32_t len, BackRing &ring, int lane, int r)
+{
+    const unsigned FULL = 0xffffffffu;
+    const uint32_t last = begin + len - 1;
+    const double *src = lane < 18 ? d.cprime + 36 * size_t(last) + 2 * lane : d.dprime + 6 * size_t(last) + 2 * (lane - 18);
+    const int back = lane < 18 ? 36 : 6;
+    uint32_t asked = 0;
+    auto request = [&]() {
+        if (lane < 21 && asked < len) copy16_async(ring.row[asked % kRing] + 2 * lane, src);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        src -= back;
+        ++asked;
+    };
+    double next = 0.0, nv, nc[6];
+    auto take = [&](uint32_t done) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kRing - 2) : "memory");
+        __syncwarp();
+        const double *row = ring.row[done % kRing];
+        nv = row[36 + r];
+        const double2 *pair = reinterpret_cast<const double2 *>(row + 6 * r);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) { nc[2 * q] = pair[q].x; nc[2 * q + 1] = pair[q].y; }
+    };
+    for (int a = 0; a < kRing - 1; ++a) request();
+    take(0);
+    double *out = d.dir + 6 * size_t(last) + r;
+    for (uint32_t done = 0; done < len; ++done) {
+        double value = nv, crow[6];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) crow[q] = nc[q];
+        // The slot of kRing - 1 ahead is that of the row before this one,
+        // which every lane took before the __syncwarp of the last take.
+        request();
+        take(done + 1);  // past the last row: an old slot, unused
+        if (done > 0) {
+#pragma unroll
+            for (int q = 0; q < 6; ++q) value = __fma_rn(-crow[q], __shfl_sync(FULL, next, q), value);
+        }
+        if (lane < 6) *out = value;
+        out -= 6;
+        next = value;
+    }
+    __syncwarp();  // the ring is free for the next strand
+}
+
 // One strand on one warp.  Lane 6 g + r holds row r of column g + 1 of B_n
 // and U_n (g < 5) in b and u, and of an extra column in bx and ux: column 0
 // for g = 0, the right-hand side for g = 1 (the other lanes' extra entries
@@ -233,50 +287,186 @@ template<class D> __device__ __forceinline__ void solve_strand_warp(const D &d, 
     }
     if (failed) return;
     __syncwarp();  // C_n and d'_n written by the other lanes of this warp
-    // Back substitution d_n = d'_n - C_n d_{n+1}, every lane of row r: a chain
-    // of six multiply-adds a node, shorter than a read from L2, so the rows
-    // come through a ring of asynchronous copies (16 bytes a lane), and from
-    // there to registers one node ahead.
-    const uint32_t last = begin + len - 1;
-    const double *src = lane < 18 ? d.cprime + 36 * size_t(last) + 2 * lane : d.dprime + 6 * size_t(last) + 2 * (lane - 18);
-    const int back = lane < 18 ? 36 : 6;
-    uint32_t asked = 0;
-    auto request = [&]() {
-        if (lane < 21 && asked < len) copy16_async(ring.row[asked % kRing] + 2 * lane, src);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        src -= back;
-        ++asked;
-    };
-    double next = 0.0, nv, nc[6];
-    auto take = [&](uint32_t done) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(kRing - 2) : "memory");
-        __syncwarp();
-        const double *row = ring.row[done % kRing];
-        nv = row[36 + r];
-        const double2 *pair = reinterpret_cast<const double2 *>(row + 6 * r);
+    substitute_back(d, begin, len, ring, lane, r);
+}
+
+// One strand on a team of three warps (on three sub-partitions):
+// * the pivot warp holds B_n, row r of columns 1 ... 5 in lane 6 g + r and
+//   column 0 in the lanes g = 0 once more, adds the shift and runs the six
+//   pivot steps; the reciprocal of every candidate is taken beside the pivot
+//   search.  It publishes each step's row factors, pivot and reciprocal and
+//   goes on without waiting;
+// * two column warps hold one entry of [U_n | rhs_n] a lane (columns 0 ... 4;
+//   column 5 and the right-hand side), follow the published steps, scale the
+//   rows, store C_n and d'_n and form the same entries of the next Schur
+//   complement and right-hand side (column c of B_{n+1} needs column c of C_n
+//   only), which goes back to the pivot warp.
+// On one warp the updates of U sit in the pivot chain, since FP64 instructions
+// and shuffles issue in order, and each node's Schur complement waits for all
+// of them.  What bounds the team is the chain of six pivot steps (2,700 of the
+// 4,000 cycles a node), then the Schur complement (540), the scaling (160) and
+// the hand-overs.  It has more FP64 instructions in flight for the same
+// result, so it pays while a sub-partition has less work than the longest
+// chain: a solve of 100 strands of 16-160 nodes 384 -> 311 us, of 1,200 451 ->
+// 413, of 2,200 495 -> 513.
+struct TeamShared {
+    double B[36];      // B_n row-major, from the column warps
+    double fp[6][6];   // row factors a[r][col] / pivot of each step
+    double ip[6];      // pivot reciprocals
+    int pivot[6];      // pivot rows
+    int redo;          // the node is eliminated again with the exact search
+    BackRing ring;
+};
+
+// Named barriers of a team: 1 ... 6 the pivot steps (the pivot warp arrives,
+// the column warps wait), 7 all three warps.
+constexpr int kTeam = 96;
+__device__ __forceinline__ void team_wait(int id) { asm volatile("bar.sync %0, 96;" ::"r"(id) : "memory"); }
+__device__ __forceinline__ void team_arrive(int id) { asm volatile("bar.arrive %0, 96;" ::"r"(id) : "memory"); }
+
+// The six pivot steps on b and (column 0) bx.  The pivot search compares the
+// top 29 bits of the magnitudes with the row beside them, in one warp
+// reduction; EXACT compares all bits and checks the pivots.  Returns whether,
+// for !EXACT, some step needs EXACT (candidates equal in those bits, or a
+// pivot outside [1e-30, 2^1022)), which the column warps learn with the last
+// step, and for EXACT, whether a pivot failed.
+template<bool EXACT> __device__ __forceinline__ bool team_pivots(double b, double bx, TeamShared &sh, int lane, int g, int r)
+{
+    const unsigned FULL = 0xffffffffu;
+    bool flag = false;
 #pragma unroll
-        for (int q = 0; q < 3; ++q) { nc[2 * q] = pair[q].x; nc[2 * q + 1] = pair[q].y; }
-    };
-    for (int a = 0; a < kRing - 1; ++a) request();
-    take(0);
-    double *out = d.dir + 6 * size_t(last) + r;
-    for (uint32_t done = 0; done < len; ++done) {
-        double value = nv, crow[6];
-#pragma unroll
-        for (int q = 0; q < 6; ++q) crow[q] = nc[q];
-        // The slot of kRing - 1 ahead is that of the row before this one,
-        // which every lane took before the __syncwarp of the last take.
-        request();
-        take(done + 1);  // past the last row: an old slot, unused
-        if (done > 0) {
-#pragma unroll
-            for (int q = 0; q < 6; ++q) value = __fma_rn(-crow[q], __shfl_sync(FULL, next, q), value);
+    for (int col = 0; col < 6; ++col) {
+        const int base = col == 0 ? 0 : 6 * (col - 1);  // first lane of the pivot column
+        const double mine = col == 0 ? bx : b;
+        // The first row of the largest magnitude, among rows col ... 5.
+        const bool cand = lane >= base + col && lane < base + 6;
+        const unsigned hi = cand ? unsigned(__double2hiint(mine)) & 0x7fffffffu : 0u;
+        const unsigned key = EXACT ? hi : cand ? (hi & ~7u) | unsigned(5 - r) : 0u;
+        const unsigned best = __reduce_max_sync(FULL, key);
+        int pivot = 5 - int(best & 7u);
+        if (EXACT) {
+            const unsigned lo = cand && hi == best ? unsigned(__double2loint(mine)) : 0u;
+            const unsigned ml = __reduce_max_sync(FULL, lo);
+            pivot = 5 - int(__reduce_max_sync(FULL, cand && hi == best && lo == ml ? unsigned(5 - r) : 0u));
+            flag |= pivot_fails((unsigned long long)best << 32 | ml);
+        } else {
+            const unsigned off = (r != pivot) & cand ? key ^ best : 8u;
+            const unsigned low = best - 0x39b44850u;  // wraps below the least pivot
+            flag |= (off < 8u) | (low >= 0x7fd00000u - 0x39b44850u);
         }
-        if (lane < 6) *out = value;
-        out -= 6;
-        next = value;
+        const int partner = r == col ? pivot : (r == pivot ? col : r);
+        const double fcol = __shfl_sync(FULL, mine, base + partner);
+        double xb = 0.0;
+        if (col < 5) {
+            xb = __shfl_sync(FULL, b, 6 * g + pivot);
+            if (pivot != col) b = __shfl_sync(FULL, b, 6 * g + partner);
+        }
+        const double rc = EXACT ? dm::recip_rn(mine) : dm::recip_normal(mine);
+        if (col == 5 && !EXACT) flag = __any_sync(FULL, flag);
+        const double ip = __shfl_sync(FULL, rc, base + pivot);
+        const double fp = __dmul_rn(fcol, ip);
+        if (col < 5) b = r == col ? b : __fma_rn(-fp, xb, b);
+        // Lanes that hold the same value write the same word: no branch.
+        sh.fp[col][r] = fp;
+        sh.ip[col] = ip;
+        sh.pivot[col] = pivot;
+        if (col == 5) sh.redo = !EXACT && flag ? 1 : 0;
+        team_arrive(1 + col);
     }
-    __syncwarp();  // the ring is free for the next strand
+    return flag;
+}
+
+template<class D> __device__ __forceinline__ void team_pivot_warp(const D &d, uint32_t len, TeamShared &sh, int lane, int g, int r)
+{
+    const unsigned FULL = 0xffffffffu;
+    const bool wide = g < 5;
+    for (uint32_t t = 0; t < len; ++t) {
+        team_wait(7);  // B_t is in shared memory
+        double b = sh.B[6 * r + (wide ? g + 1 : 0)], bx = sh.B[6 * r];
+        {
+            const bool first = lane == 0, diagonal = first || (wide && r == g + 1);
+            const unsigned long long mag = (unsigned long long)__double_as_longlong(first ? bx : b) & 0x7fffffffffffffffull;
+            const unsigned hi = diagonal ? unsigned(mag >> 32) : 0u;
+            const unsigned mh = __reduce_max_sync(FULL, hi);
+            const unsigned ml = __reduce_max_sync(FULL, diagonal && hi == mh ? unsigned(mag) : 0u);
+            const double shifted = __dadd_rn(first ? bx : b, diagonal_shift((unsigned long long)mh << 32 | ml));
+            if (first) bx = shifted;
+            else if (diagonal) b = shifted;
+        }
+        if (team_pivots<false>(b, bx, sh, lane, g, r)) {
+            team_wait(7);  // the column warps have read every step
+            if (team_pivots<true>(b, bx, sh, lane, g, r) && lane == 0) atomicExch(&d.sc->solve_failed, 1);
+        }
+    }
+}
+
+// Column warp w (0 or 1).  Every lane reads through pointers of its own,
+// without conditions (a divergent one costs more than the read): lanes without
+// an entry read a neighbour's and nothing uses it.
+template<class D>
+__device__ __forceinline__ void team_column_warp(const D &d, uint32_t begin, uint32_t len, TeamShared &sh, int lane, int g, int r, int w)
+{
+    const unsigned FULL = 0xffffffffu;
+    const bool rhs = w == 1 && g == 1;                     // this lane holds the right-hand side
+    const bool entry = w == 0 ? g < 5 : g < 2;             // ... something at all
+    const int c = w == 0 ? (g < 5 ? g : 0) : 5;            // column of B and U
+    const double *pd = rhs ? d.grad + 6 * size_t(begin) + r : d.diag + 36 * size_t(begin) + 6 * r + c;
+    const double *pu = d.upper + 36 * size_t(begin) + 6 * r + c, *puc = d.upper + 36 * size_t(begin) + r;
+    double *pc = rhs ? d.dprime + 6 * size_t(begin) + r : d.cprime + 36 * size_t(begin) + 6 * r + c;
+    const int step = rhs ? 6 : 36, sign = rhs ? int(0x80000000) : 0;
+    double nd = *pd, nu = *pu, nuc[6];
+    double acc = __hiloint2double(__double2hiint(nd) ^ sign, __double2loint(nd));
+    for (uint32_t t = 0; t < len; ++t) {
+        const bool tip = t + 1 == len;  // U_n couples to nothing there
+        if (entry && !rhs) sh.B[6 * r + c] = acc;
+        const double start = rhs ? acc : tip ? 0.0 : nu;
+        team_wait(7);  // hand B_t over
+        if (!tip) {
+            // U_t's column r for the Schur complement, the next D and U.
+#pragma unroll
+            for (int q = 0; q < 6; ++q) nuc[q] = puc[6 * q];
+            pd += step; pu += 36; puc += 36;
+            nd = *pd; nu = *pu;
+        }
+        double u;
+        for (;;) {
+            u = start;
+#pragma unroll
+            for (int col = 0; col < 6; ++col) {
+                team_wait(1 + col);
+                const int pivot = sh.pivot[col];
+                const double fp = sh.fp[col][r];
+                const double x = __shfl_sync(FULL, u, 6 * g + pivot);
+                if (pivot != col) u = __shfl_sync(FULL, u, 6 * g + (r == col ? pivot : (r == pivot ? col : r)));
+                u = r == col ? u : __fma_rn(-fp, x, u);
+            }
+            if (sh.redo == 0) break;
+            team_wait(7);
+        }
+        const double scaled = __dmul_rn(u, sh.ip[r]);  // row r of C_t, or d'_t
+        if (entry) *pc = scaled;
+        pc += step;
+        if (!tip) {
+            // B = D - U_t^T C_t, rhs = -g - U_t^T d'_t
+            acc = __hiloint2double(__double2hiint(nd) ^ sign, __double2loint(nd));
+#pragma unroll
+            for (int q = 0; q < 6; ++q) acc = __fma_rn(-nuc[q], __shfl_sync(FULL, scaled, 6 * g + q), acc);
+        }
+    }
+}
+
+template<class D> __device__ __forceinline__ void solve_strand_team(const D &d, uint32_t k, TeamShared &sh)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int g = lane / 6, r = lane - 6 * g;
+    uint32_t begin, len;
+    strand_range(d, k, begin, len);
+    if (len == 0) return;
+    if (warp == 0) team_pivot_warp(d, len, sh, lane, g, r);
+    else team_column_warp(d, begin, len, sh, lane, g, r, warp - 1);
+    team_wait(7);  // C and d' are stored
+    if (warp != 0) return;
+    substitute_back(d, begin, len, sh.ring, lane, r);
 }
 
 // Five strands on one warp: lane 6 s + r holds row r of strand first + s of

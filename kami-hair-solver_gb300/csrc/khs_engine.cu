@@ -27,7 +27,8 @@
 //                 (thread per block entry), k_reduce_eval (both levels: the
 //                 last block to finish reduces the partials)
 //   direction     k_block_solve (blocks of one warp, a strand or five at a
-//                 time from a longest-first queue),
+//                 time from a longest-first queue) or k_block_solve_team
+//                 (three warps per strand),
 //                 [float-float form: k_ff_factor, k_ff_residual, k_ff_correct],
 //                 k_steepest, k_scale, k_reduce_dir, k_limit
 //   CCD           k_ccd (plain), k_ccd_collect + k_ccd_pairs (mixed)
@@ -1560,6 +1561,13 @@ __global__ void __launch_bounds__(32) k_block_solve(View d, uint32_t items)
     }
 }
 
+// Every strand on a team of three warps, longest first.
+__global__ void __launch_bounds__(kTeam) k_block_solve_team(View d)
+{
+    __shared__ __align__(16) TeamShared sh;
+    solve_strand_team(d, blockIdx.x, sh);
+}
+
 // ---- mixed form: float-float block solve with FP64 refinement -------------
 //
 // The same block Thomas recurrence as the FP64 solve (per strand, one lane
@@ -2744,6 +2752,7 @@ struct Engine::Impl {
     uint64_t launches = 0;
     // Launch shape of the FP64 block solve: work items, blocks of one warp.
     unsigned solve_items = 0, solve_blocks = 0;
+    bool solve_team = false;
     // Rollback ring: q and v of the last ring_frame.size() animation frames,
     // slot k holding frame ring_frame[k] (-1 = empty), [slots][2][N][6] FP64.
     double *ring = nullptr;
@@ -3365,8 +3374,9 @@ bool Engine::make_steepest()
 }
 
 // Work items of the FP64 block solve: the `alone` longest strands on a warp
-// each, the rest five to a warp, longest expected time first.  The split does
-// not change the result (k_block_solve).
+// each, the rest five to a warp, longest expected time first; by rule, or
+// every strand on a team of three warps.  None of it changes the result
+// (khs_block_solve.cuh).
 //
 // The rule's model, in cycles measured on GB300 (160-node strands on random
 // blocks): a node of a strand alone takes 4,950 with one warp on a
@@ -3380,6 +3390,13 @@ bool Engine::make_steepest()
 // solve, all by fives 992); 2,000 all alone (491, 1,159); the body scene's
 // 6,757 strands of 8-200 nodes with a quarter alone (575, all alone 654, all
 // by fives 1,650; 831 with the timed shapes this replaces).
+//
+// Teams are taken while the work on one warp a strand is at most 1.1 times
+// the longest chain, us a solve against the split: the body scene with 700 of
+// its strands 375 and 452, with 3,000 476 and 514 (work 0.6 of the chain);
+// 1,000 strands of 16-160 nodes 266 and 327, 1,800 467 and 490 (1.05), 2,200
+// 513 and 495 (1.3); 2,000 of 8-24 nodes 85 and 88 (1.4), 4,000 162 and 159
+// (2.8); all of the body scene 674 and 569 (1.4).
 void Engine::plan_block_solve(uint32_t alone, uint32_t blocks_per_sm)
 {
     Impl &I = *d_;
@@ -3387,11 +3404,13 @@ void Engine::plan_block_solve(uint32_t alone, uint32_t blocks_per_sm)
     const uint32_t S = uint32_t(len.size());
     int sms = 0;
     KHS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, kDevice));
-    constexpr double kAlone[2] = {4950.0, 6400.0}, kFive[2] = {14700.0, 20200.0};
+    constexpr double kAlone[2] = {4950.0, 6400.0}, kFive[2] = {14700.0, 20200.0}, kAloneWork = 3200.0, kFiveWork = 2020.0;
+    I.solve_team = false;
     if (alone == kSolveByRule) {
         std::vector<double> sum(S + 1, 0.0);
         for (uint32_t k = 0; k < S; ++k) sum[k + 1] = sum[k] + len[k];
         const double parts = 4.0 * sms;
+        I.solve_team = S && sum[S] * kAloneWork <= 1.1 * parts * len[0] * kAlone[0];
         double best = std::numeric_limits<double>::infinity();
         for (uint32_t step = 0; step <= 20; ++step) {
             const uint32_t w = uint32_t(uint64_t(S) * step / 20);
@@ -3404,7 +3423,7 @@ void Engine::plan_block_solve(uint32_t alone, uint32_t blocks_per_sm)
                 chain = std::max(chain, len[w] * node(kFive));
                 shortest = std::min(shortest, len[w + (S - w - 1) / kStrandsPerWarp * kStrandsPerWarp] * kFive[1]);
             }
-            const double work = (sum[w] * 3200.0 + (sum[S] - sum[w]) * 2020.0) / parts;
+            const double work = (sum[w] * kAloneWork + (sum[S] - sum[w]) * kFiveWork) / parts;
             const double time = std::max(chain, items > 2.0 * parts ? work + 0.5 * shortest : 0.0);
             if (time <= best) { best = time; alone = w; }
         }
@@ -3454,7 +3473,8 @@ KhsResult Engine::set_block_solve_tiers(uint32_t quads, uint32_t singles, uint32
 void Engine::launch_block_solve()
 {
     Impl &I = *d_;
-    I.launch("k_block_solve", k_block_solve, I.solve_blocks, 32, I.v, uint32_t(I.solve_items));
+    if (I.solve_team) I.launch("k_block_solve", k_block_solve_team, I.v.S, kTeam, I.v);
+    else I.launch("k_block_solve", k_block_solve, I.solve_blocks, 32, I.v, uint32_t(I.solve_items));
 }
 
 bool Engine::make_direction(KhsxSubstepRecord &rec, double grad_norm2)

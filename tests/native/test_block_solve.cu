@@ -1,9 +1,9 @@
-// Both layouts of the FP64 block solve (csrc/khs_block_solve.cuh) against the
+// The three layouts of the FP64 block solve (csrc/khs_block_solve.cuh) against the
 // same recurrence on the host, entry by entry with std::fma and IEEE division,
 // bit for bit: random blocks; blocks of small integers, where pivot candidates
 // tie exactly; candidates that differ only below the bits the warp's pivot
 // search compares first; pivots with reciprocals below the normal range; and
-// a singular block, which both layouts report.  Strand lengths around the
+// a singular block, which every layout reports.  Strand lengths around the
 // back substitution's ring.  Built and run by tests/test_gpu_block_solve.py.
 #include "khs_block_solve.cuh"
 
@@ -27,6 +27,11 @@ __global__ void __launch_bounds__(32) k_alone(Arrays d)
 {
     __shared__ __align__(16) BackRing ring;
     solve_strand_warp(d, blockIdx.x, ring);
+}
+__global__ void __launch_bounds__(kTeam) k_team(Arrays d)
+{
+    __shared__ __align__(16) TeamShared sh;
+    solve_strand_team(d, blockIdx.x, sh);
 }
 __global__ void __launch_bounds__(32) k_five(Arrays d) { solve_strands_five(d, kStrandsPerWarp * blockIdx.x); }
 
@@ -132,10 +137,11 @@ int main()
         a.diag = device(D); a.upper = device(U); a.grad = device(g);
         a.cprime = device(D); a.dprime = device(g);
         a.sorder = device(order); a.sfirst = device(first); a.scount = device(count); a.sfixed = device(fixed);
-        for (int five = 0; five < 2; ++five) {
+        for (int layout = 0; layout < 3; ++layout) {
             a.dir = device(std::vector<double>(x.size(), 0.0));
             a.sc = device(std::vector<Flags>(1, Flags{0}));
-            if (five) k_five<<<(27 + kStrandsPerWarp - 1) / kStrandsPerWarp, 32>>>(a);
+            if (layout == 2) k_team<<<27, kTeam>>>(a);
+            else if (layout == 1) k_five<<<(27 + kStrandsPerWarp - 1) / kStrandsPerWarp, 32>>>(a);
             else k_alone<<<27, 32>>>(a);
             if (cudaDeviceSynchronize() != cudaSuccess) { std::printf("CUDA error\n"); return 1; }
             std::vector<double> got(x.size());
@@ -146,7 +152,7 @@ int main()
             if (!failed)
                 for (size_t i = 0; i < x.size(); ++i) differ += std::memcmp(&got[i], &x[i], 8) != 0;
             const bool ok = differ == 0 && (f.solve_failed != 0) == failed;
-            std::printf("kind %d layout %d: %zu of %zu differ, failed %d / %d\n", kind, five, differ, x.size(), f.solve_failed, int(failed));
+            std::printf("kind %d layout %d: %zu of %zu differ, failed %d / %d\n", kind, layout, differ, x.size(), f.solve_failed, int(failed));
             if (!ok) ++bad;
         }
     }

@@ -1,4 +1,4 @@
-"""Both layouts of the FP64 block solve against the same recurrence on the
+"""The three layouts of the FP64 block solve against the same recurrence on the
 host, bit for bit (tests/native/test_block_solve.cu)."""
 import os
 import subprocess
