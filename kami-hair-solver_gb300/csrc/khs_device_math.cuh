@@ -293,12 +293,12 @@ struct ElementJacobian {
     M A2, S2i, S2j, Kki, Kkj;
 };
 
-// invL = 1 / L0.
-KHS_HD void element_strain_inv(const M &Ri, const M &Rj, V xi, V xj, double invL, V gamma0, V kappa0, double eps[6],
-                               ElementJacobian *J, const M *Jli, const M *Jlj)
+// What both ends of an element need of its strain (invL = 1 / L0): t, S = Ri^T
+// + Rj^T and, with a Jacobian, K.
+KHS_HD void element_strain_shared(const M &Ri, const M &Rj, V xi, V xj, double invL, V gamma0, V kappa0, double eps[6], V &t,
+                                  M &S, M *K)
 {
-    const V t = (xj - xi) * invL;
-    M S;  // Ri^T + Rj^T
+    t = (xj - xi) * invL;
 #pragma unroll
     for (int r = 0; r < 3; ++r)
 #pragma unroll
@@ -315,33 +315,43 @@ KHS_HD void element_strain_inv(const M &Ri, const M &Rj, V xi, V xj, double invL
     eps[3] = ax2.x * is * invL - kappa0.x;
     eps[4] = ax2.y * is * invL - kappa0.y;
     eps[5] = ax2.z * is * invL - kappa0.z;
-    if (!J) return;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) J->A2.m[k] = S.m[k] * invL;
-    // [t]x Jl: column k = t x Jl_col(k)
-    M TJi, TJj;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const V ci = cross(t, v(Jli->m[k], Jli->m[3 + k], Jli->m[6 + k]));
-        const V cj = cross(t, v(Jlj->m[k], Jlj->m[3 + k], Jlj->m[6 + k]));
-        TJi.m[k] = ci.x; TJi.m[3 + k] = ci.y; TJi.m[6 + k] = ci.z;
-        TJj.m[k] = cj.x; TJj.m[3 + k] = cj.y; TJj.m[6 + k] = cj.z;
-    }
-    J->S2i = mtmul(Ri, TJi);
-    J->S2j = mtmul(Rj, TJj);
+    if (!K) return;
     // K = ((tr Q) I - Q) / s + 2 c c^T / s^2 with c = ax2 / 2
-    M K;
     const double is2 = 0.5 * is * is;
     const double axv[3] = {ax2.x, ax2.y, ax2.z};
 #pragma unroll
     for (int r = 0; r < 3; ++r)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) K.m[3 * r + c] = ((r == c ? trQ : 0.0) - Q.m[3 * r + c]) * is + is2 * axv[r] * axv[c];
-    const M RJi = mtmul(Ri, *Jli), RJj = mtmul(Ri, *Jlj);
-    J->Kki = mmul(K, RJi);
-    J->Kkj = mmul(K, RJj);
+        for (int c = 0; c < 3; ++c) K->m[3 * r + c] = ((r == c ? trQ : 0.0) - Q.m[3 * r + c]) * is + is2 * axv[r] * axv[c];
+}
+
+// The Jacobian blocks of one end, with its rotation R and left Jacobian Jl
+// (scale: invL, negative for node i).
+KHS_HD void element_strain_end(const M &R, const M &Ri, const M &Jl, V t, const M &K, double scale, M &S2, M &Kk)
+{
+    M TJ;  // [t]x Jl: column k = t x Jl_col(k)
 #pragma unroll
-    for (int k = 0; k < 9; ++k) { J->Kki.m[k] *= -invL; J->Kkj.m[k] *= invL; }
+    for (int k = 0; k < 3; ++k) {
+        const V c = cross(t, v(Jl.m[k], Jl.m[3 + k], Jl.m[6 + k]));
+        TJ.m[k] = c.x; TJ.m[3 + k] = c.y; TJ.m[6 + k] = c.z;
+    }
+    S2 = mtmul(R, TJ);
+    Kk = mmul(K, mtmul(Ri, Jl));
+#pragma unroll
+    for (int k = 0; k < 9; ++k) Kk.m[k] *= scale;
+}
+
+KHS_HD void element_strain_inv(const M &Ri, const M &Rj, V xi, V xj, double invL, V gamma0, V kappa0, double eps[6],
+                               ElementJacobian *J, const M *Jli, const M *Jlj)
+{
+    V t;
+    M S, K;
+    element_strain_shared(Ri, Rj, xi, xj, invL, gamma0, kappa0, eps, t, S, J ? &K : nullptr);
+    if (!J) return;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) J->A2.m[k] = S.m[k] * invL;
+    element_strain_end(Ri, Ri, *Jli, t, K, -invL, J->S2i, J->Kki);
+    element_strain_end(Rj, Ri, *Jlj, t, K, invL, J->S2j, J->Kkj);
 }
 
 KHS_HD void element_strain(const M &Ri, const M &Rj, V xi, V xj, double L0, V gamma0, V kappa0, double eps[6],
@@ -452,6 +462,51 @@ KHS_HD void element_hessian(const ElementJacobian &J, const Weights &w, double L
     }
 }
 
+// One end's share of the gradient and the Hessian blocks, for two threads an
+// element: right 0 for node i, 1 for node j.  g: the node's gradient; H: its
+// diagonal block; x = A^T Wg Sg; WS, WK: the rows scaled for the mixed block.
+KHS_HD void element_end(bool right, const M &A2, const M &S2, const M &Kk, const double eps[6], const Weights &w, double L0,
+                        double g[6], double H[36], M &x, M &WS, M &WK)
+{
+    M WA;
+    const HalfWeights h = half_weights(w, L0);
+    const double hs[3] = {h.shear, h.shear, h.stretch}, hb[3] = {h.bend, h.bend, h.twist};
+    double se[3], ke[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) { se[k] = hs[k] * eps[k]; ke[k] = 2.0 * (hb[k] * eps[3 + k]); }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const double ax = A2.m[c] * se[0] + A2.m[3 + c] * se[1] + A2.m[6 + c] * se[2];
+        g[c] = right ? ax : -ax;
+        g[3 + c] = S2.m[c] * se[0] + S2.m[3 + c] * se[1] + S2.m[6 + c] * se[2] +
+                   Kk.m[c] * ke[0] + Kk.m[3 + c] * ke[1] + Kk.m[6 + c] * ke[2];
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const double gk = 0.5 * hs[k], kk = 2.0 * hb[k];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            WA.m[3 * k + c] = gk * A2.m[3 * k + c];
+            WS.m[3 * k + c] = gk * S2.m[3 * k + c];
+            WK.m[3 * k + c] = kk * Kk.m[3 * k + c];
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const double xc = dot3w(A2, r, WS, c);
+            x.m[3 * r + c] = xc;
+            H[6 * r + 3 + c] = H[6 * (3 + c) + r] = right ? xc : -xc;
+            if (c < r) continue;
+            const double p = dot3w(A2, r, WA, c);
+            const double rr = dot3w(S2, r, WS, c) + dot3w(Kk, r, WK, c);
+            H[6 * r + c] = H[6 * c + r] = p;
+            H[6 * (3 + r) + 3 + c] = H[6 * (3 + c) + 3 + r] = rr;
+        }
+    }
+}
+
 // ---- geometry (device flavour, cuda_backend.cu:200-223) ----------------
 //
 // The proximity tests decide integer outputs (candidate sets, closest
@@ -465,10 +520,12 @@ KHS_HD void element_hessian(const ElementJacobian &J, const Weights &w, double L
 KHS_HD double xm(double a, double b) { return __dmul_rn(a, b); }
 KHS_HD double xa(double a, double b) { return __dadd_rn(a, b); }
 KHS_HD double xs(double a, double b) { return __dsub_rn(a, b); }
+KHS_HD double xf(double a, double b, double c) { return __fma_rn(a, b, c); }
 #else
 KHS_HD double xm(double a, double b) { return a * b; }
 KHS_HD double xa(double a, double b) { return a + b; }
 KHS_HD double xs(double a, double b) { return a - b; }
+KHS_HD double xf(double a, double b, double c) { return fma(a, b, c); }
 #endif
 KHS_HD V gadd(V a, V b) { return v(xa(a.x, b.x), xa(a.y, b.y), xa(a.z, b.z)); }
 KHS_HD V gsub(V a, V b) { return v(xs(a.x, b.x), xs(a.y, b.y), xs(a.z, b.z)); }
@@ -726,27 +783,39 @@ KHS_HD bool boxes_overlap(V al, V au, V bl, V bu, double p)
            bl.z <= au.z + p;
 }
 
-// Log barrier b(g) = -kc (dh - g)^2 ln(g / dh) of the contact gap and its
-// gradient with respect to the two segment end points at fixed (t, bary)
-// (cuda_backend.cu:255-265: the distance is regularised by 1e-30 inside the
-// square root).  Returns the energy; g0, g1 get the gradients.
-KHS_HD double barrier_energy_gradient(V x0, V x1, double t, V body_point, double radius_offset, double dh, double kc,
-                                      double g0[3], double g1[3])
+// Offset of a segment's point at t from a triangle's point at the barycentric
+// weights.  Which products its sums take into a multiply-add is written out
+// here and in the barrier: left to the compiler it depends on what stands
+// around them, and stiff contacts carry a changed bit into the step counts.
+KHS_HD V contact_offset(V x0, V x1, double t, V a, V b, V c, V bary)
 {
-    const V p = x0 * (1.0 - t) + x1 * t;
-    const V diff = p - body_point;
-    const double dist = sqrt(dot(diff, diff) + 1e-30);
+    const double w = 1.0 - t;
+    auto one = [&](double p0, double p1, double va, double vb, double vc) {
+        const double p = xf(p1, t, xm(p0, w));
+        return xs(p, xf(vc, bary.z, xf(va, bary.x, xm(vb, bary.y))));
+    };
+    return v(one(x0.x, x1.x, a.x, b.x, c.x), one(x0.y, x1.y, a.y, b.y, c.y), one(x0.z, x1.z, a.z, b.z, c.z));
+}
+
+// Log barrier b(g) = -kc (dh - g)^2 ln(g / dh) of the contact gap and its
+// gradient with respect to the two segment end points at fixed (t, bary), from
+// their offset (cuda_backend.cu:255-265: the distance is regularised by 1e-30
+// inside the square root).  Returns the energy; g0, g1 get the gradients.
+KHS_HD double barrier_energy_gradient(V offset, double t, double radius_offset, double dh, double kc, double g0[3], double g1[3])
+{
+    const double dist = sqrt(xa(xf(offset.z, offset.z, xf(offset.x, offset.x, xm(offset.y, offset.y))), 1e-30));
     const double gap = dist - radius_offset;
     if (gap >= dh) {
         g0[0] = g0[1] = g0[2] = g1[0] = g1[1] = g1[2] = 0.0;
         return 0.0;
     }
-    const double aa = dh - gap, lg = log(gap / dh);
-    const double energy = -kc * aa * aa * lg;
-    const double db = kc * (2.0 * aa * lg - aa * aa / gap);  // d energy / d gap
+    const double aa = dh - gap, lg = log(gap / dh), w = 1.0 - t;
+    const double energy = xm(xm(xm(-kc, aa), aa), lg);
+    const double db = xm(kc, xs(xm(2.0 * aa, lg), xm(aa, aa) / gap));  // d energy / d gap
     const double s = db / dist;
-    g0[0] = s * diff.x * (1.0 - t); g0[1] = s * diff.y * (1.0 - t); g0[2] = s * diff.z * (1.0 - t);
-    g1[0] = s * diff.x * t; g1[1] = s * diff.y * t; g1[2] = s * diff.z * t;
+    const double f[3] = {xm(s, offset.x), xm(s, offset.y), xm(s, offset.z)};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) { g0[k] = xm(f[k], w); g1[k] = xm(f[k], t); }
     return energy;
 }
 

@@ -23,8 +23,9 @@
 //                 k_sweep_record, k_update_velocity, k_friction(+apply)
 //   evaluation    k_node_eval, [mixed: k_contact_filter, k_contact_near (warp
 //                 per element with cached leaves), k_contact_exact (thread per
-//                 FP32 survivor), k_contact_select], k_elem_eval, k_node_sum
-//                 (thread per block entry), k_reduce_eval (both levels: the
+//                 FP32 survivor), k_contact_select], k_elem_eval or k_elem_ends
+//                 (two threads per element), k_node_sum (thread per two
+//                 block entries), k_reduce_eval (both levels: the
 //                 last block to finish reduces the partials)
 //   direction     k_block_solve (blocks of one warp, a strand or five at a
 //                 time from a longest-first queue) or k_block_solve_team
@@ -165,6 +166,7 @@ struct View {
     const uint8_t *econtact;
     const double *L0, *invL, *gamma0, *kappa0;  // invL = 1 / L0
     double *e_el, *e_co, *c_gap;
+    double *push;  // the barrier's gradient and curvature [E][kPush] (element_barrier)
     uint32_t *c_cand, *c_tri;
     uint8_t *c_flags;
     const uint32_t *sfirst, *scount, *sfixed, *sorder;
@@ -867,7 +869,7 @@ __device__ __forceinline__ uint32_t closest_triangle(const View &d, V xi, V xj, 
 // Contact classification of every element at the state q: candidate count,
 // closest triangle with its closest pair, gap and flags.  The mixed form runs
 // this as its own low-register pass before the element energy (and for the
-// contact-query entry point); the plain form searches inside k_elem_eval.
+// contact-query entry point).
 template<bool MIXED> __global__ void __launch_bounds__(kBlock) k_contact(View d, const double *q)
 {
     follow_previous();
@@ -908,7 +910,7 @@ template<bool MIXED> __global__ void __launch_bounds__(kBlock) k_contact(View d,
 // does not exceed the smallest upper bound, in the plain form all stay.  They
 // go to a pool of (element, triangle) pairs.  k_contact_exact (thread per
 // pair): the FP64 closest pair.  k_contact_select (thread per element): the
-// first strictly closest of the element's pairs.  Candidates the mixed form
+// first strictly closest of the element's pairs, and its barrier.  Candidates the mixed form
 // drops are strictly farther in FP64 than the minimum, so either way the
 // result, tie-break included, equals k_contact's.
 //
@@ -939,7 +941,7 @@ __device__ __forceinline__ float record_distance_f(const View &d, uint32_t p, dm
     return df;
 }
 
-__device__ __forceinline__ void write_contact(const View &d, uint32_t e, uint32_t closest, const dm::ClosestPair &pair)
+__device__ __forceinline__ uint8_t write_contact(const View &d, uint32_t e, uint32_t closest, const dm::ClosestPair &pair)
 {
     uint8_t flags = 0;
     double gap = 0.0;
@@ -955,6 +957,8 @@ __device__ __forceinline__ void write_contact(const View &d, uint32_t e, uint32_
     d.c_t[e] = pair.t;
     d.c_dist[e] = pair.distance;
     store3(d.c_bary + 3 * size_t(e), pair.bary);
+    d.e_co[e] = 0.0;
+    return flags;
 }
 
 // Slack test of the leaf cache on the FP32 copies: below kCacheReach metres
@@ -1263,7 +1267,43 @@ __device__ __forceinline__ uint32_t select_pair(const View &d, const double *q, 
     return d.surv_tri[best];
 }
 
-template<bool FILTER> __global__ void __launch_bounds__(kBlock) k_contact_select(View d, const double *q)
+// The barrier of an active element (cuda_backend.cu:899-939), with a gradient
+// also what it adds, for k_node_sum: g0 and g1 to the gradients of the ends'
+// positions, curv dg dg^T (dg: node i, then node j) to the position parts of
+// the blocks.  In its own record, so that the element kernel, whose chain of
+// FP64 instructions bounds small scenes, runs beside the contact pass.
+// Within the element kernel the barrier's logarithm and divisions added 8 us to
+// an evaluation of 3,200 elements (39.0 us, then 30.7), and the element kernel
+// waited for the contact pass.
+constexpr int kPush = 13;  // g0, g1, curv, dg
+__device__ __forceinline__ void element_barrier(const View &d, const double *q, uint32_t e, uint32_t closest,
+                                                const dm::ClosestPair &pair, bool gradient)
+{
+    const V xi = load3(q + 6 * size_t(d.ei[e])), xj = load3(q + 6 * size_t(d.ej[e]));
+    const double gap = pair.distance - d.radius - d.offset;
+    const V offset = dm::contact_offset(xi, xj, pair.t, tri_vertex(d, closest, 0), tri_vertex(d, closest, 1),
+                                        tri_vertex(d, closest, 2), pair.bary);
+    double g0[3], g1[3];
+    const double energy = dm::barrier_energy_gradient(offset, pair.t, d.radius + d.offset, d.dhat, d.kc, g0, g1);
+    if (!isfinite(energy)) {
+        d.c_flags[e] |= kFlagInfeasible;
+        return;
+    }
+    d.c_flags[e] |= kFlagEnergy;
+    d.e_co[e] = energy;
+    if (!gradient) return;
+    double *push = d.push + kPush * size_t(e);
+    const V normal = offset * (1.0 / fmax(pair.distance, 1e-15));
+    const double aa = d.dhat - gap;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) { push[k] = g0[k]; push[3 + k] = g1[k]; }
+    push[6] = d.kc * (-2.0 * log(gap / d.dhat) + 4.0 * aa / gap + aa * aa / (gap * gap));
+    push[7] = normal.x * (1.0 - pair.t); push[8] = normal.y * (1.0 - pair.t); push[9] = normal.z * (1.0 - pair.t);
+    push[10] = normal.x * pair.t; push[11] = normal.y * pair.t; push[12] = normal.z * pair.t;
+}
+
+constexpr int kSelectBlock = 64;
+template<bool FILTER> __global__ void __launch_bounds__(kSelectBlock) k_contact_select(View d, const double *q, int gradient)
 {
     follow_previous();
     const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1276,7 +1316,7 @@ template<bool FILTER> __global__ void __launch_bounds__(kBlock) k_contact_select
     if (n == 0) return;
     dm::ClosestPair pair;
     const uint32_t closest = select_pair<FILTER>(d, q, e, n, pair);
-    write_contact(d, e, closest, pair);
+    if (write_contact(d, e, closest, pair) & kFlagActive) element_barrier(d, q, e, closest, pair, gradient);
 }
 
 // ---- contact query without allocation -------------------------------------
@@ -1319,8 +1359,7 @@ template<bool MIXED> __global__ void __launch_bounds__(kBlock) k_contact_query_r
     out[e] = r;
 }
 
-// Per element: elastic energy (+ gradient and GN blocks) and barrier contact
-// against the closest BVH candidate (cuda_backend.cu:899-939).
+// Per element: elastic energy (+ gradient and GN blocks) (cuda_backend.cu:899-939).
 __global__ void __launch_bounds__(kEvalBlock) k_elem_eval(View d, int gradient)
 {
     follow_previous();
@@ -1365,71 +1404,144 @@ __global__ void __launch_bounds__(kEvalBlock) k_elem_eval(View d, int gradient)
                                nullptr, nullptr, nullptr);
     }
     d.e_el[e] = dm::element_energy(eps, d.w, L0);
+}
 
-    uint32_t cand = 0, closest = kNone;
-    uint8_t flags = 0;
-    double gap = 0.0, ce = 0.0;
-    if (d.has_collider && !fi && d.econtact[e]) {
-        // Result of the contact pass at this same state.
-        dm::ClosestPair pair;
-        cand = d.c_cand[e]; closest = d.c_tri[e]; flags = d.c_flags[e]; gap = d.c_gap[e];
-        pair.t = d.c_t[e]; pair.distance = d.c_dist[e]; pair.bary = load3(d.c_bary + 3 * size_t(e));
-        if (closest != kNone) {
-            if (flags & kFlagActive) {
-                const V a = tri_vertex(d, closest, 0), b = tri_vertex(d, closest, 1), c = tri_vertex(d, closest, 2);
-                const V bp = a * pair.bary.x + b * pair.bary.y + c * pair.bary.z;
-                double g0[3], g1[3];
-                const double energy = dm::barrier_energy_gradient(xi, xj, pair.t, bp, d.radius + d.offset, d.dhat, d.kc, g0, g1);
-                if (!isfinite(energy)) flags |= kFlagInfeasible;
+// The gradient form with two threads an element: warp 0 of a block takes the
+// left ends of 32 elements, warp 1 the right ones.  What both need (the strain
+// and K) is evaluated twice; the mixed block, which needs both ends' rows, is
+// shared out through shared memory.  One thread an element is a chain of 720
+// FP64 instructions of 64 cycles, two a chain of 360, with 15% more of them in
+// all; so two are taken while every warp has a sub-partition to itself (two
+// blocks on each SM).  us a launch: 2,000 elements 30.7 -> 20.4, 6,200 30.6 ->
+// 22.5; beyond the line one thread is the faster: 15,500 34.8 against 38.9,
+// 66,000 106 against 115, 258,000 358 against 426.
+constexpr int kEndElements = 32, kEndBlock = 2 * kEndElements;
+__global__ void __launch_bounds__(kEndBlock) k_elem_ends(View d)
+{
+    follow_previous();
+    __shared__ double rows[2][18][kEndElements];  // S2, Kk of the left end; the scaled rows of the right one
+    const int lane = threadIdx.x & 31;
+    const bool right = threadIdx.x >= 32;
+    const uint32_t e = blockIdx.x * kEndElements + lane;
+    const bool on = e < d.E;
+    bool fij = false;
+    M WS, WK, S2, Kk;
+    double eps[6], L0 = 0.0, *Hij = nullptr;
+    if (on) {
+        const uint32_t i = d.ei[e], j = d.ej[e], n = right ? j : i;
+        const bool fi = d.fixed[i], fj = d.fixed[j], fixed = right ? fj : fi;
+        fij = fi || fj;
+        const V xi = load3(d.q + 6 * size_t(i)), xj = load3(d.q + 6 * size_t(j));
+        const M Ri = load9(d.rot + 9 * size_t(i)), Rj = load9(d.rot + 9 * size_t(j)), R = load9(d.rot + 9 * size_t(n));
+        const M Jl = load9(d.jl + 9 * size_t(n));
+        const double invL = d.invL[e];
+        L0 = d.L0[e];
+        V t;
+        M A2, S, K, x;
+        dm::element_strain_shared(Ri, Rj, xi, xj, invL, load3(d.gamma0 + 3 * size_t(e)), load3(d.kappa0 + 3 * size_t(e)), eps, t, S, &K);
+#pragma unroll
+        for (int k = 0; k < 9; ++k) A2.m[k] = S.m[k] * invL;
+        dm::element_strain_end(R, Ri, Jl, t, K, right ? invL : -invL, S2, Kk);
+        double g[6], H[36];
+        dm::element_end(right, A2, S2, Kk, eps, d.w, L0, g, H, x, WS, WK);
+        double2 *g2 = reinterpret_cast<double2 *>((right ? d.as_j_g : d.as_i_g) + 6 * size_t(n));
+        double2 *H2 = reinterpret_cast<double2 *>((right ? d.as_j_h : d.as_i_h) + 36 * size_t(n));
+#pragma unroll
+        for (int k = 0; k < 3; ++k) g2[k] = fixed ? make_double2(0.0, 0.0) : make_double2(g[2 * k], g[2 * k + 1]);
+#pragma unroll
+        for (int k = 0; k < 18; ++k) H2[k] = fixed ? make_double2(0.0, 0.0) : make_double2(H[2 * k], H[2 * k + 1]);
+        // Top left (-P) and bottom left (Xi^T) of the mixed block with the left
+        // end, top right (-Xj) with the right one.
+        Hij = d.upper + 36 * size_t(i);
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                if (right) Hij[6 * r + 3 + c] = fij ? 0.0 : -x.m[3 * r + c];
                 else {
-                    flags |= kFlagEnergy;
-                    ce = energy;
-                    if (gradient) {
-#pragma unroll
-                        for (int k = 0; k < 3; ++k) { gi[k] += g0[k]; gj[k] += g1[k]; }
-                        const V normal = (xi * (1.0 - pair.t) + xj * pair.t - bp) * (1.0 / fmax(pair.distance, 1e-15));
-                        const double aa = d.dhat - gap;
-                        const double curv = d.kc * (-2.0 * log(gap / d.dhat) + 4.0 * aa / gap + aa * aa / (gap * gap));
-                        const double dg[6] = {normal.x * (1.0 - pair.t), normal.y * (1.0 - pair.t), normal.z * (1.0 - pair.t),
-                                              normal.x * pair.t, normal.y * pair.t, normal.z * pair.t};
-#pragma unroll
-                        for (int r = 0; r < 3; ++r)
-#pragma unroll
-                            for (int c2 = 0; c2 < 3; ++c2) {
-                                Hii[6 * r + c2] += curv * dg[r] * dg[c2];
-                                Hjj[6 * r + c2] += curv * dg[3 + r] * dg[3 + c2];
-                                Hij[6 * r + c2] += curv * dg[r] * dg[3 + c2];
-                            }
-                    }
+                    Hij[6 * r + c] = fij ? 0.0 : -H[6 * r + c];
+                    Hij[6 * (3 + r) + c] = fij ? 0.0 : x.m[3 * c + r];
                 }
             }
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            rows[right][k][lane] = right ? WS.m[k] : S2.m[k];
+            rows[right][9 + k][lane] = right ? WK.m[k] : Kk.m[k];
         }
     }
-    d.e_co[e] = ce;
-    d.c_cand[e] = cand;
-    d.c_tri[e] = closest;
-    d.c_flags[e] = flags;
-    d.c_gap[e] = gap;
+    __syncthreads();
+    if (!on) return;
+    // Bottom right: four entries with the left end (and the energy), five with
+    // the right one.
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        M &a = right ? S2 : WS, &b = right ? Kk : WK;
+        a.m[k] = rows[!right][k][lane];
+        b.m[k] = rows[!right][9 + k][lane];
+    }
+    auto mixed = [&](int k) {
+        const int r = k / 3, c = k % 3;
+        Hij[6 * (3 + r) + 3 + c] = fij ? 0.0 : dm::dot3w(S2, r, WS, c) + dm::dot3w(Kk, r, WK, c);
+    };
+    if (right) {
+#pragma unroll
+        for (int k = 4; k < 9; ++k) mixed(k);
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) mixed(k);
+        d.e_el[e] = dm::element_energy(eps, d.w, L0);
+    }
 }
 
 // Node sums in a fixed order: inertia, then the element on the left (this
 // node as its right end), then the element on the right.
-// One thread per entry (36 N diagonal-block entries, then 6 N gradient
-// entries) so every access is coalesced.  Diagonal block = inertia diagonal
+// One thread per two entries (18 N of the diagonal blocks, then 3 N of the
+// gradient) so every access is coalesced; memory bounds it (265,000 nodes: 293
+// MB, 57 us).  Diagonal block = inertia diagonal
 // + the contribution of the element whose right node is n + that of the
-// element whose left node is n, in that order.
+// element whose left node is n, in that order, each with what its barrier adds
+// to the position part (element_barrier), as does the coupling block.
+__device__ __forceinline__ const double *pushed(const View &d, int32_t e)
+{
+    return e >= 0 && (d.c_flags[e] & kFlagEnergy) ? d.push + kPush * size_t(e) : nullptr;
+}
+
 __global__ void __launch_bounds__(kBlock) k_node_sum(View d)
 {
     follow_previous();
     const size_t idx = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    const size_t nh = 36 * size_t(d.N);
+    const size_t nh = 18 * size_t(d.N);
     if (idx < nh) {
-        const size_t n = idx / 36, k = idx % 36;
-        const double base = (k % 7 == 0) ? d.inertia[6 * n + k / 7] : 0.0;
-        d.diag[idx] = (base + d.as_j_h[idx]) + d.as_i_h[idx];
-    } else if (idx < nh + 6 * size_t(d.N)) {
-        const size_t i = idx - nh;
-        d.grad[i] = (d.grad[i] + d.as_j_g[i]) + d.as_i_g[i];
+        const size_t n = idx / 18;
+        const int k = int(idx % 18), r = k / 3, c = 2 * (k % 3);  // entries (r, c) and (r, c + 1)
+        const bool position = r < 3 && c < 3;
+        const int32_t left = position ? d.elem_left[n] : -1, right = position ? d.elem_right[n] : -1;
+        double2 hj = reinterpret_cast<const double2 *>(d.as_j_h)[idx], hi = reinterpret_cast<const double2 *>(d.as_i_h)[idx];
+        double2 sum = make_double2(0.0, 0.0);
+        if (r == c) sum.x = d.inertia[6 * n + r];
+        if (r == c + 1) sum.y = d.inertia[6 * n + r];
+        if (const double *p = pushed(d, left)) {
+            const double cr = p[6] * p[10 + r];
+            hj.x += cr * p[10 + c];
+            if (c == 0) hj.y += cr * p[11];
+        }
+        if (const double *p = pushed(d, right)) {
+            const double cr = p[6] * p[7 + r];
+            double2 &u = reinterpret_cast<double2 *>(d.upper)[idx];
+            hi.x += cr * p[7 + c];
+            u.x += cr * p[10 + c];
+            if (c == 0) { hi.y += cr * p[8]; u.y += cr * p[11]; }
+        }
+        reinterpret_cast<double2 *>(d.diag)[idx] = make_double2((sum.x + hj.x) + hi.x, (sum.y + hj.y) + hi.y);
+    } else if (idx < nh + 3 * size_t(d.N)) {
+        const size_t i = idx - nh, n = i / 3;
+        const int k = 2 * int(i % 3);
+        const int32_t left = k < 3 ? d.elem_left[n] : -1, right = k < 3 ? d.elem_right[n] : -1;
+        double2 gj = reinterpret_cast<const double2 *>(d.as_j_g)[i], gi = reinterpret_cast<const double2 *>(d.as_i_g)[i];
+        double2 &g = reinterpret_cast<double2 *>(d.grad)[i];
+        if (const double *p = pushed(d, left)) { gj.x += p[3 + k]; if (k == 0) gj.y += p[4]; }
+        if (const double *p = pushed(d, right)) { gi.x += p[k]; if (k == 0) gi.y += p[1]; }
+        g = make_double2((g.x + gj.x) + gi.x, (g.y + gj.y) + gi.y);
     }
 }
 
@@ -1455,10 +1567,10 @@ template<class Op, class T> __device__ __forceinline__ T warp_tree(const T *sh, 
 // The block's sums: every thread brings its values, a warp of its own reduces
 // each kind.  All kinds on the first warp, and fmin on the FP64 pipe, put some
 // 45 FP64 instructions of 64 cycles in a row there: k_reduce_eval took 18.3 us
-// on 2,000 elements and takes 12.2, k_reduce_dir 15.2 and 10.6.  EVAL: five FP64 sums, the
-// smallest gap's key and three counts; else two FP64 sums and the largest
-// square as bits.  Thread 0 finds the results in element 0 of each row; the
-// rows may be used again after a barrier.
+// on 2,000 elements and takes 12.2, k_reduce_dir 15.2 and 10.6.  An evaluation
+// has five FP64 sums, the smallest gap's key and three counts, a direction two
+// FP64 sums and the largest square as bits.  Thread 0 finds the results in
+// element 0 of each row; the rows may be used again after a barrier.
 constexpr int kEvalSums = 5, kEvalCounts = 3, kDirSums = 2;
 struct EvalRows {
     double sum[kEvalSums][kBlock];
@@ -1512,7 +1624,8 @@ __device__ __forceinline__ void block_sums(DirRows &r, const double (&s)[kDirSum
 // A NaN orders above everything, so it loses every minimum as it does in fmin.
 __device__ __forceinline__ long long gap_key(double x)
 {
-    return isnan(x) ? 0x7fffffffffffffffll : order_key(x);
+    const bool nan = (__double_as_longlong(x) & 0x7fffffffffffffffll) > 0x7ff0000000000000ll;
+    return nan ? 0x7fffffffffffffffll : order_key(x);
 }
 constexpr long long kInfKey = 0x7ff0000000000000ll;
 
@@ -2852,6 +2965,7 @@ struct Engine::Impl {
     // Launch shape of the FP64 block solve: work items, blocks of one warp.
     unsigned solve_items = 0, solve_blocks = 0;
     bool solve_team = false;
+    uint32_t sms = 152;
     // Rollback ring: q and v of the last ring_frame.size() animation frames,
     // slot k holding frame ring_frame[k] (-1 = empty), [slots][2][N][6] FP64.
     double *ring = nullptr;
@@ -2905,11 +3019,11 @@ struct Engine::Impl {
         kstats.push_back({name, 0, 0.0});
         return kstats.size() - 1;
     }
-    cudaStream_t joined = nullptr;  // stream that has waited for the other one since its last launch
+    cudaStream_t ordinary = nullptr;  // stream whose next launch waits in the ordinary way
     void wait_for(cudaStream_t s, cudaEvent_t e)
     {
         KHS_CUDA(cudaStreamWaitEvent(s, e, 0));
-        joined = s;
+        ordinary = s;
     }
     // A launch on stream s (the solver's stream, or the side stream, which
     // is only used while kernels are not timed one by one).
@@ -2935,8 +3049,8 @@ struct Engine::Impl {
         config.blockDim = dim3(block);
         config.stream = s;
         config.attrs = &early;
-        config.numAttrs = s == joined ? 0 : 1;
-        if (s == joined) joined = nullptr;
+        config.numAttrs = s == ordinary ? 0 : 1;
+        if (s == ordinary) ordinary = nullptr;
         KHS_CUDA(cudaLaunchKernelEx(&config, kernel, args...));
     }
     template<class K, class... A> void launch(const char *name, K kernel, unsigned grid, unsigned block, A... args)
@@ -3025,7 +3139,7 @@ void Engine::initialize(const Model &m, const KhsSolverDesc &desc, const KhsHair
     bytes += 4 * padded<double>(3 * N);      // root cur/pending x r
     bytes += 3 * padded<uint32_t>(N) + padded<double>(N);  // root bindings, node strand
     bytes += 3 * padded<uint32_t>(E) + padded<uint8_t>(E) + 2 * padded<double>(E) + 2 * padded<double>(3 * E);
-    bytes += 3 * padded<double>(E) + 2 * padded<uint32_t>(E) + padded<uint8_t>(E);
+    bytes += 3 * padded<double>(E) + 2 * padded<uint32_t>(E) + padded<uint8_t>(E) + padded<double>(kPush * E);
     bytes += 5 * padded<uint32_t>(S);
     bytes += padded<uint32_t>(3 * T) + 5 * padded<double>(3 * Vn) + padded<float>(3 * Vn);
     bytes += 2 * padded<float4>(2 * B);
@@ -3078,6 +3192,7 @@ void Engine::initialize(const Model &m, const KhsSolverDesc &desc, const KhsHair
     uint8_t *ec = a.take<uint8_t>(E);
     double *L0 = a.take<double>(E), *invL = a.take<double>(E), *g0 = a.take<double>(3 * E), *k0 = a.take<double>(3 * E);
     v.e_el = a.take<double>(E); v.e_co = a.take<double>(E); v.c_gap = a.take<double>(E);
+    v.push = a.take<double>(kPush * E);
     v.c_cand = a.take<uint32_t>(E); v.c_tri = a.take<uint32_t>(E); v.c_flags = a.take<uint8_t>(E);
     uint32_t *sf = a.take<uint32_t>(S), *sc = a.take<uint32_t>(S), *sx = a.take<uint32_t>(S), *so = a.take<uint32_t>(S);
     v.solve_items = a.take<uint32_t>(S);
@@ -3435,7 +3550,8 @@ EvalStats Engine::evaluate(bool gradient, double dt, double alpha, const double 
     if (v.has_collider) {
         // The contact passes read only q and its FP32 copy: once k_positions
         // has written them, the passes run on a second stream beside the node
-        // kernel (on one stream while kernels are timed one by one).  The same kernels see the same inputs either way.
+        // and element kernels (on one stream while kernels are timed one by
+        // one).  The same kernels see the same inputs either way.
         I.launch("k_positions", k_positions, grid_for(v.N), kBlock, v, trial ? 1 : 0, a, alpha_dev);
         const bool side = !I.profiling;
         const cudaStream_t cs = side ? I.side : I.stream;
@@ -3449,19 +3565,20 @@ EvalStats Engine::evaluate(bool gradient, double dt, double alpha, const double 
                     k_contact_filter, grid_for(v.E), kBlock, v, q, rebuild_cache_ ? 1 : 0);
         I.launch_on(cs, "k_contact_near", mode_ ? k_contact_near<true> : k_contact_near<false>, 152 * 8, kBlock, v);
         I.launch_on(cs, "k_contact_exact", k_contact_exact, kPairGrid, kPairBlock, v, q);
-        I.launch_on(cs, "k_contact_select", mode_ ? k_contact_select<true> : k_contact_select<false>, grid_for(v.E),
-                    kBlock, v, q);
+        I.launch_on(cs, "k_contact_select", mode_ ? k_contact_select<true> : k_contact_select<false>,
+                    grid_for(v.E, kSelectBlock), kSelectBlock, v, q, gradient ? 1 : 0);
         if (side) KHS_CUDA(cudaEventRecord(I.join, I.side));
-        I.launch(gradient ? "k_node_eval_grad" : "k_node_eval_energy", k_node_eval, grid_for(v.N, kEvalBlock), kEvalBlock, v,
-                 gradient ? 1 : 0, trial ? 1 : 0, a, dt, alpha_dev, 1);
-        if (side) I.wait_for(I.stream, I.join);
-    } else {
-        I.launch(gradient ? "k_node_eval_grad" : "k_node_eval_energy", k_node_eval, grid_for(v.N, kEvalBlock), kEvalBlock, v,
-                 gradient ? 1 : 0, trial ? 1 : 0, a, dt, alpha_dev, 0);
     }
+    I.launch(gradient ? "k_node_eval_grad" : "k_node_eval_energy", k_node_eval, grid_for(v.N, kEvalBlock), kEvalBlock, v,
+             gradient ? 1 : 0, trial ? 1 : 0, a, dt, alpha_dev, v.has_collider);
     rebuild_cache_ = false;
-    I.launch(gradient ? "k_elem_eval_grad" : "k_elem_eval_energy", k_elem_eval, grid_for(v.E, kEvalBlock), kEvalBlock, v, gradient ? 1 : 0);
-    if (gradient) I.launch("k_node_sum", k_node_sum, grid_for(42 * size_t(v.N)), kBlock, v);
+    // Brought up early, the element kernel's blocks would take the registers that
+    // the contact passes need (1,000 strands: 186.5 ms a frame, so 181.1).
+    if (v.has_collider) I.ordinary = I.stream;
+    if (gradient && v.E <= kEndElements * 2 * I.sms) I.launch("k_elem_eval_grad", k_elem_ends, grid_for(v.E, kEndElements), kEndBlock, v);
+    else I.launch(gradient ? "k_elem_eval_grad" : "k_elem_eval_energy", k_elem_eval, grid_for(v.E, kEvalBlock), kEvalBlock, v, gradient ? 1 : 0);
+    if (v.has_collider && !I.profiling) I.wait_for(I.stream, I.join);
+    if (gradient) I.launch("k_node_sum", k_node_sum, grid_for(21 * size_t(v.N)), kBlock, v);
     I.launch("k_reduce_eval", k_reduce_eval, kPartials, kBlock, v, gradient ? 1 : 0);
     I.check();
     I.sync();
@@ -3525,6 +3642,7 @@ void Engine::plan_block_solve(uint32_t alone, uint32_t blocks_per_sm)
     const uint32_t S = uint32_t(len.size());
     int sms = 0;
     KHS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, kDevice));
+    I.sms = uint32_t(sms);
     constexpr double kAlone[2] = {4950.0, 6400.0}, kFive[2] = {14700.0, 20200.0}, kAloneWork = 3200.0, kFiveWork = 2020.0;
     I.solve_team = false;
     if (alone == kSolveByRule) {
