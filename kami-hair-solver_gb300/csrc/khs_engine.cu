@@ -131,6 +131,7 @@ struct Scalars {
     uint32_t pool_used;   // entries of the leaf pool handed out since the last cache rebuild
     double trial_alpha;   // first line-search step from the last CCD bound (publish_ccd)
     double max_translation;  // largest free-node translation of the last reduced direction
+    uint32_t wide_count;  // elements queued for k_contact_near that take a block each
 };
 
 struct Partial {
@@ -208,7 +209,7 @@ struct View {
     uint32_t *surv_elem, *surv_tri;
     uint32_t surv_capacity;
     uint32_t *surv_off, *surv_n;
-    uint32_t *near_list;  // elements with cached leaves, one warp each in k_contact_near
+    uint32_t *near_list;  // elements with cached leaves, one warp each in k_contact_near (from the end: a block each)
     double *surv_res;
     const uint32_t *solve_items;  // work items of the block solve, at most one per strand
     const uint32_t *bfirst, *bcount, *border, *bleaves;
@@ -904,7 +905,8 @@ template<bool MIXED> __global__ void __launch_bounds__(kBlock) k_contact(View d,
 //
 // k_contact_filter (thread per element): the element's cached leaves are still
 // valid, or are collected again; elements with leaves are queued.
-// k_contact_near (warp per queued element): lane l tests leaf l exactly, so
+// k_contact_near (warp per queued element, a block per element with many
+// leaves): lane l tests leaf l exactly, so
 // the candidates are counted in traversal order; in the mixed form an FP32
 // filter over the triangle records keeps every candidate whose lower bound
 // does not exceed the smallest upper bound, in the plain form all stay.  They
@@ -992,6 +994,13 @@ __device__ __forceinline__ uint8_t refresh_leaves(const View &d, const double *q
     return nl;
 }
 
+// Queues an element with leaves for k_contact_near.
+__device__ __forceinline__ void queue_near(const View &d, uint32_t e, uint8_t nl)
+{
+    if (nl == kCacheBig) d.near_list[d.E - 1 - atomicAdd(&d.sc->wide_count, 1u)] = e;
+    else d.near_list[append_slot(&d.sc->near_count)] = e;
+}
+
 // cache 1: collect every element's leaves (the first evaluation of a
 // substep); 0: only where the element has left its slack.
 __global__ void __launch_bounds__(kBlock) k_contact_filter(View d, const double *q, int cache)
@@ -1007,7 +1016,7 @@ __global__ void __launch_bounds__(kBlock) k_contact_filter(View d, const double 
             return;
         }
         if (nl > 0) {
-            d.near_list[append_slot(&d.sc->near_count)] = e;
+            queue_near(d, e, nl);
             return;
         }
     } else if (cache == 1 && !d.fixed[j] && d.econtact[e]) {
@@ -1093,23 +1102,40 @@ __device__ __forceinline__ uint32_t spread_candidates(uint32_t first, uint32_t c
     return __shfl_sync(0xffffffffu, incl, 31);
 }
 
-// One warp per element queued by k_contact_filter: the leaves are tested 32 at
-// a time, lane by lane, their candidates taken 32 at a time, lane by lane: with
-// FILTER once for the smallest upper bound, once to count the survivors, and
-// once to write the pairs, in traversal order (leaf, then triangle), so the
-// first-found tie-break is kept.  With at most 32 candidates, the common case,
-// the first round's bounds are kept instead.
-template<bool FILTER> __global__ void __launch_bounds__(kBlock) k_contact_near(View d)
+// The leaves of an element queued by k_contact_filter are tested 32 at a time,
+// lane by lane, their candidates taken 32 at a time, lane by lane: with FILTER
+// once for the smallest upper bound, once to count the survivors, and once to
+// write the pairs, in traversal order (leaf, then triangle), so the first-found
+// tie-break is kept.  With at most 32 candidates, the common case, the first
+// round's bounds are kept instead.  An element has a warp; one with more than
+// kCacheLeaves leaves (a mesh pole), queued at the list's other end, has a
+// block, whose warps take runs of its leaves: the longest list of a pole bound
+// the launch at 67 us with one warp, 26 with eight.
+constexpr int kNearWarps = kBlock / 32;
+// Four blocks an SM are resident.  Where their warps have several elements each,
+// that many blocks spread the work better than twice as many (a frame of 1,000
+// strands, 68,000 elements: 177.6 ms against 181.5); beside a half-empty
+// element kernel, twice as many start sooner (27,000: 66.7 against 67.5).
+inline unsigned near_grid(uint32_t E) { return E > 40000u ? 152u * 4u : 152u * 8u; }
+template<bool FILTER> __global__ void __launch_bounds__(kBlock, 4) k_contact_near(View d)
 {
     follow_previous();
-    __shared__ uint32_t lists[kBlock / 32][kNearList];
+    __shared__ uint32_t lists[kNearWarps][kNearList];
+    __shared__ uint32_t totals[kNearWarps], counts[kNearWarps], slot;
+    __shared__ float ubs[kNearWarps];
     const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    uint32_t *pos = lists[threadIdx.x >> 5];
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
-    const uint32_t count = d.sc->near_count;
-    for (uint32_t k = warp; k < count; k += nwarps) {
-        const uint32_t e = d.near_list[k];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint32_t *pos = lists[w];
+    const uint32_t nwide = d.sc->wide_count, count = d.sc->near_count;
+    // Wide elements block by block, the others warp by warp from the next
+    // block on.
+    uint32_t kw = blockIdx.x, k = (blockIdx.x + gridDim.x - nwide % gridDim.x) % gridDim.x * kNearWarps + w;
+    for (;;) {
+        const bool wide = kw < nwide;
+        if (!wide && k >= count) break;
+        const uint32_t e = wide ? d.near_list[d.E - 1 - kw] : d.near_list[k];
+        if (wide) kw += gridDim.x;
+        else k += gridDim.x * kNearWarps;
         const uint32_t i = d.ei[e], j = d.ej[e];
         const dm::F3 xi32 = dm::f3(d.q32[3 * size_t(i)], d.q32[3 * size_t(i) + 1], d.q32[3 * size_t(i) + 2]);
         const dm::F3 xj32 = dm::f3(d.q32[3 * size_t(j)], d.q32[3 * size_t(j) + 1], d.q32[3 * size_t(j) + 2]);
@@ -1124,74 +1150,89 @@ template<bool FILTER> __global__ void __launch_bounds__(kBlock) k_contact_near(V
         const dm::F3 p1 = dm::f3(xj32.x - origin.x, xj32.y - origin.y, xj32.z - origin.z);
         uint32_t nleaves = 0;
         const uint32_t *leaves = cached_leaves(d, e, d.cache_n[e], nleaves);
-        auto bounds = [&](uint32_t p, float &lb, uint32_t &t) {  // returns the upper bound
-            float m;
-            const float df = record_distance_f(d, p, origin, p0, p1, m, t);
-            lb = df - m;
-            return df + m;
-        };
-        uint32_t total = 0, here = 0, tri0 = 0;
-        float ub = 3.0e38f, lb0 = 3.0e38f;
-        for (uint32_t r0 = 0; r0 < nleaves; r0 += 32) {
-            uint32_t first, cnt;
-            near_leaf(d, leaves, r0 + lane, nleaves, qb, d.contact_pad.exact, box, first, cnt);
-            here = spread_candidates(first, cnt, pos, lane);
-            if (FILTER)
-                for (uint32_t c = lane; c < here; c += 32) ub = fminf(ub, bounds(pos[c], lb0, tri0));
-            total += here;
-        }
-        if (FILTER) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) ub = fminf(ub, __shfl_xor_sync(FULL, ub, o));
-        }
-        if (nleaves <= 32 && total <= 32) {
-            const bool stays = uint32_t(lane) < total && !(FILTER && lb0 > ub);
-            const uint32_t mask = __ballot_sync(FULL, stays);
-            const uint32_t base = near_claim(d, e, total, __popc(mask), lane);
-            if (base != kNone && stays) {
-                if (!FILTER) tri0 = __float_as_uint(__ldg(d.tri32 + 3 * size_t(pos[lane])).w);
-                put_pair(d, base + __popc(mask & ((1u << lane) - 1u)), e, tri0);
-            }
-            continue;
-        }
-        // More candidates: count the survivors, then write them.
-        uint32_t n = total, at = 0;
-        for (int pass = FILTER ? 0 : 1; pass < 2; ++pass) {
-            if (pass == 1) {
-                at = near_claim(d, e, total, n, lane);
-                if (at == kNone) break;
-            } else {
-                n = 0;
-            }
-            for (uint32_t r0 = 0; r0 < nleaves; r0 += 32) {
-                if (nleaves > 32) {
+        const uint32_t begin = wide ? uint32_t(uint64_t(nleaves) * w / kNearWarps) : 0;
+        const uint32_t end = wide ? uint32_t(uint64_t(nleaves) * (w + 1) / kNearWarps) : nleaves;
+        uint32_t total = 0, n = 0, at = 0, here = 0, t = 0;
+        float ub = 3.0e38f, lb = 3.0e38f;
+        for (int pass = 0; pass < 3; ++pass) {  // bounds, count, write
+            if (pass == 1 && !FILTER) n = total;
+            for (uint32_t r0 = begin; r0 < end && !(pass == 1 && !FILTER); r0 += 32) {
+                if (pass == 0 || end - begin > 32) {
                     uint32_t first, cnt;
-                    near_leaf(d, leaves, r0 + lane, nleaves, qb, d.contact_pad.exact, box, first, cnt);
+                    near_leaf(d, leaves, r0 + lane, end, qb, d.contact_pad.exact, box, first, cnt);
                     here = spread_candidates(first, cnt, pos, lane);
                 }
+                if (pass == 0) total += here;
+                if (pass == 0 && !FILTER) continue;
                 for (uint32_t c0 = 0; c0 < here; c0 += 32) {
                     const uint32_t c = c0 + lane;
                     bool stays = c < here;
-                    uint32_t t = 0;
                     if (stays) {
-                        float lb;
                         if (FILTER) {
-                            bounds(pos[c], lb, t);
+                            float m;
+                            const float df = record_distance_f(d, pos[c], origin, p0, p1, m, t);
+                            lb = df - m;
+                            if (pass == 0) ub = fminf(ub, df + m);
                             stays = !(lb > ub);
                         } else {
                             t = __float_as_uint(__ldg(d.tri32 + 3 * size_t(pos[c])).w);
                         }
                     }
+                    if (pass == 0) continue;
                     const uint32_t mask = __ballot_sync(FULL, stays);
-                    if (pass == 0) {
-                        n += __popc(mask);
-                    } else {
+                    if (pass == 1) n += __popc(mask);
+                    else {
                         if (stays) put_pair(d, at + __popc(mask & ((1u << lane) - 1u)), e, t);
                         at += __popc(mask);
                     }
                 }
             }
+            if (pass == 0) {
+                if (FILTER) {
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) ub = fminf(ub, __shfl_xor_sync(FULL, ub, o));
+                }
+                if (wide) {
+                    if (lane == 0) { totals[w] = total; ubs[w] = ub; }
+                    __syncthreads();
+#pragma unroll
+                    for (int o = 0; o < kNearWarps; ++o) ub = fminf(ub, ubs[o]);
+                } else if (total <= 32) {
+                    const bool stays = uint32_t(lane) < total && !(FILTER && lb > ub);
+                    const uint32_t mask = __ballot_sync(FULL, stays);
+                    const uint32_t base = near_claim(d, e, total, __popc(mask), lane);
+                    if (base != kNone && stays) {
+                        if (!FILTER) t = __float_as_uint(__ldg(d.tri32 + 3 * size_t(pos[lane])).w);
+                        put_pair(d, base + __popc(mask & ((1u << lane) - 1u)), e, t);
+                    }
+                    break;
+                }
+            } else if (pass == 1) {
+                uint32_t before = 0;
+                if (wide) {
+                    if (lane == 0) counts[w] = n;
+                    __syncthreads();
+                    uint32_t every = 0, all = 0;
+#pragma unroll
+                    for (int o = 0; o < kNearWarps; ++o) {
+                        every += totals[o];
+                        before += o < w ? counts[o] : 0;
+                        all += counts[o];
+                    }
+                    if (w == 0) {
+                        at = near_claim(d, e, every, all, lane);
+                        if (lane == 0) slot = at;
+                    }
+                    __syncthreads();
+                    at = slot;
+                } else {
+                    at = near_claim(d, e, total, n, lane);
+                }
+                if (at == kNone) break;
+                at += before;
+            }
         }
+        if (wide) __syncthreads();  // the shared values are read
     }
 }
 
@@ -1310,6 +1351,7 @@ template<bool FILTER> __global__ void __launch_bounds__(kSelectBlock) k_contact_
     if (e == 0) {  // k_contact_near and k_contact_exact, their only readers, have completed
         d.sc->surv_count = 0;
         d.sc->near_count = 0;
+        d.sc->wide_count = 0;
     }
     if (e >= d.E) return;
     const uint32_t n = d.surv_n[e];
@@ -2643,7 +2685,7 @@ __global__ void __launch_bounds__(kBlock) k_friction_collect(View d)
     if (!friction_root(d, e, i, j)) return;
     const uint8_t nl = refresh_leaves(d, d.q, e, i, j, false);
     d.surv_n[e] = nl == kCacheInvalid ? kSurvOverflow : 0;
-    if (nl != kCacheInvalid && nl > 0) d.near_list[append_slot(&d.sc->near_count)] = e;
+    if (nl != kCacheInvalid && nl > 0) queue_near(d, e, nl);
 }
 
 // Coulomb friction impulse (cuda_backend.cu:941-964); each element writes
@@ -2655,6 +2697,7 @@ template<bool FILTER> __global__ void __launch_bounds__(kBlock) k_friction(View 
     if (e == 0) {  // k_contact_near and k_contact_exact, their only readers, have completed
         d.sc->surv_count = 0;
         d.sc->near_count = 0;
+        d.sc->wide_count = 0;
     }
     if (e >= d.E) return;
     const uint32_t i = d.ei[e], j = d.ej[e];
@@ -2725,6 +2768,7 @@ __global__ void k_init_scalars(View d)
     d.sc->solve_next = 0;
     d.sc->refine_bits = 0;
     d.sc->near_count = 0;
+    d.sc->wide_count = 0;
     d.sc->ccd_near = 0;
     d.sc->pool_used = 0;
     d.sc->eval_done = 0;
@@ -3563,7 +3607,7 @@ EvalStats Engine::evaluate(bool gradient, double dt, double alpha, const double 
         if (rebuild_cache_) KHS_CUDA(cudaMemsetAsync(&v.sc->pool_used, 0, sizeof(uint32_t), cs));
         I.launch_on(cs, rebuild_cache_ ? "k_contact_filter_rebuild" : trial ? "k_contact_filter_trial" : "k_contact_filter",
                     k_contact_filter, grid_for(v.E), kBlock, v, q, rebuild_cache_ ? 1 : 0);
-        I.launch_on(cs, "k_contact_near", mode_ ? k_contact_near<true> : k_contact_near<false>, 152 * 8, kBlock, v);
+        I.launch_on(cs, "k_contact_near", mode_ ? k_contact_near<true> : k_contact_near<false>, near_grid(v.E), kBlock, v);
         I.launch_on(cs, "k_contact_exact", k_contact_exact, kPairGrid, kPairBlock, v, q);
         I.launch_on(cs, "k_contact_select", mode_ ? k_contact_select<true> : k_contact_select<false>,
                     grid_for(v.E, kSelectBlock), kSelectBlock, v, q, gradient ? 1 : 0);
@@ -4053,7 +4097,7 @@ KhsResult Engine::run_frame(double frame_dt, const double *root_a, const double 
             }
             if (v.has_collider && material_.friction > 0.0) {
                 I.launch("k_friction_collect", k_friction_collect, grid_for(v.E), kBlock, v);
-                I.launch("k_contact_near", mode_ ? k_contact_near<true> : k_contact_near<false>, 152 * 8, kBlock, v);
+                I.launch("k_contact_near", mode_ ? k_contact_near<true> : k_contact_near<false>, near_grid(v.E), kBlock, v);
                 I.launch("k_contact_exact", k_contact_exact, kPairGrid, kPairBlock, v, v.q);
                 I.launch("k_friction", mode_ ? k_friction<true> : k_friction<false>, grid_for(v.E), kBlock, v, dt);
                 I.launch("k_friction_apply", k_friction_apply, grid_for(v.N), kBlock, v);
