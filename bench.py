@@ -83,16 +83,17 @@ MEASURED_PEAKS = REPO / "MEASURED_PEAKS.json"
 # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) of the
 # dominant kernels from one ncu capture of this workload; see profiles/.
 # (k_block_solve's traffic does not depend on the contact state.)
-NCU_TRAFFIC_BYTES: dict[str, float] = {"k_block_solve": 195.529728e6 + 69.514496e6,
-                                      "k_elem_eval_grad": 89.102592e6 + 211.5456e6}
+NCU_TRAFFIC_BYTES: dict[str, float] = {"k_block_solve": 178.00e6 + 63.42e6,
+                                      "k_elem_eval_grad": 73.49e6 + 195.42e6}
 
 # FP64 operations per unit that the element and node kernels execute (dadd +
 # dmul + 2 dfma, thread level, predicated-on), counted by ncu on the body
-# scene (profiles/fp64_op_counts_body_scene.md).  The reference method
+# scene, the energy forms on 80 strands among contacts
+# (profiles/fp64_op_counts_body_scene.md).  The reference method
 # differentiates with Dual<12>; these count this implementation's
 # closed-form arithmetic, which is the work the FP64 pipe has to do.
-COUNTED_FLOPS = {"k_elem_eval_grad": 1089.0, "k_elem_eval_energy": 152.0,
-                 "k_node_eval_grad": 365.0, "k_node_eval_energy": 256.0}
+COUNTED_FLOPS = {"k_elem_eval_grad": 1048.0, "k_elem_eval_energy": 122.0,
+                 "k_node_eval_grad": 312.0, "k_node_eval_energy": 233.0}
 
 
 def algorithmic(name: str, nodes: int, free_nodes: int, elements: int, candidates: float):

@@ -1,7 +1,7 @@
-// FP64 block-tridiagonal solve of the Gauss-Newton direction: the device
-// code of k_block_solve and k_block_solve_team (khs_engine.cu), for a view D of the solver's arrays
-// (diag, upper, cprime [N][36]; grad, dprime, dir [N][6]; the strands' order
-// and ranges; sc->solve_failed).
+// FP64 block-tridiagonal solve of the Gauss-Newton direction: the device code
+// of k_block_solve and k_block_solve_team (khs_engine.cu), for a view D of the
+// solver's arrays (diag, upper, cprime [N][36]; grad, dprime, dir [N][6]; the
+// strands' order and ranges; sc->solve_failed).
 #pragma once
 
 #include "khs_device_math.cuh"

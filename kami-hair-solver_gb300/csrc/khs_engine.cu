@@ -21,18 +21,20 @@
 //   per substep   k_begin_substep, k_refit (eight lanes per leaf),
 //                 k_sweep_collect, k_sweep_near, k_advance_pairs,
 //                 k_sweep_record, k_update_velocity, k_friction(+apply)
-//   evaluation    k_node_eval, [mixed: k_contact_filter, k_contact_near (warp
-//                 per element with cached leaves), k_contact_exact (thread per
-//                 FP32 survivor), k_contact_select], k_elem_eval or k_elem_ends
-//                 (two threads per element), k_node_sum (thread per two
-//                 block entries), k_reduce_eval (both levels: the
-//                 last block to finish reduces the partials)
+//   evaluation    k_positions, k_node_eval, k_contact_filter, k_contact_near
+//                 (warp per element with cached leaves, block where they are
+//                 many), k_contact_exact (five warps to 32 pairs),
+//                 k_contact_select, k_elem_eval or k_elem_ends (two threads
+//                 per element), k_node_sum (thread per two block entries),
+//                 k_reduce_eval (both levels: the last block to finish
+//                 reduces the partials)
 //   direction     k_block_solve (blocks of one warp, a strand or five at a
 //                 time from a longest-first queue) or k_block_solve_team
 //                 (three warps per strand),
 //                 [float-float form: k_ff_factor, k_ff_residual, k_ff_correct],
 //                 k_steepest, k_scale, k_reduce_dir, k_limit
-//   CCD           k_ccd (plain), k_ccd_collect + k_ccd_pairs (mixed)
+//   CCD           k_ccd_collect, k_ccd_near, k_advance_pairs; k_ccd where the
+//                 pair list is full
 //   queries       k_contact, k_contact_query_records, k_gather
 //   root targets  k_root_tangents, k_root_transport, k_root_frames (three
 //                 lanes per strand), k_root_rotations: per call of
@@ -868,9 +870,8 @@ __device__ __forceinline__ uint32_t closest_triangle(const View &d, V xi, V xj, 
 // Contact classification of every element at a caller-provided state
 // (positions of q_probe); used to check the integer contact work.
 // Contact classification of every element at the state q: candidate count,
-// closest triangle with its closest pair, gap and flags.  The mixed form runs
-// this as its own low-register pass before the element energy (and for the
-// contact-query entry point).
+// closest triangle with its closest pair, gap and flags, by one thread an
+// element (the contact-query entry point).
 template<bool MIXED> __global__ void __launch_bounds__(kBlock) k_contact(View d, const double *q)
 {
     follow_previous();
@@ -912,7 +913,8 @@ template<bool MIXED> __global__ void __launch_bounds__(kBlock) k_contact(View d,
 // does not exceed the smallest upper bound, in the plain form all stay.  They
 // go to a pool of (element, triangle) pairs.  k_contact_exact (thread per
 // pair): the FP64 closest pair.  k_contact_select (thread per element): the
-// first strictly closest of the element's pairs, and its barrier.  Candidates the mixed form
+// first strictly closest of the element's pairs, and its barrier.  Candidates
+// the mixed form
 // drops are strictly farther in FP64 than the minimum, so either way the
 // result, tie-break included, equals k_contact's.
 //
