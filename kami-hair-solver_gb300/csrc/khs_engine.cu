@@ -914,9 +914,8 @@ template<bool MIXED> __global__ void __launch_bounds__(kBlock) k_contact(View d,
 // go to a pool of (element, triangle) pairs.  k_contact_exact (thread per
 // pair): the FP64 closest pair.  k_contact_select (thread per element): the
 // first strictly closest of the element's pairs, and its barrier.  Candidates
-// the mixed form
-// drops are strictly farther in FP64 than the minimum, so either way the
-// result, tie-break included, equals k_contact's.
+// the mixed form drops are strictly farther in FP64 than the minimum, so either
+// way the result, tie-break included, equals k_contact's.
 //
 // The plain form used to search inside the element kernel, one thread walking
 // the FP64 boxes and evaluating every candidate in turn: on 80 strands among
