@@ -4174,7 +4174,7 @@ void Engine::push_output(uint32_t frame)
     double *dst = I.out_dev + k * per;
     // The slot's previous copy must have finished before the gather
     // overwrites it; an event never recorded does not wait.
-    KHS_CUDA(cudaStreamWaitEvent(I.stream, I.out_copied[k], 0));
+    I.wait_for(I.stream, I.out_copied[k]);
     I.launch("k_gather", k_gather, grid_for(I.original_count), kBlock, I.v.q, I.mapping_dev, I.original_count, dst);
     KHS_CUDA(cudaEventRecord(I.out_gathered[k], I.stream));
     KHS_CUDA(cudaStreamWaitEvent(I.copy_stream, I.out_gathered[k], 0));
