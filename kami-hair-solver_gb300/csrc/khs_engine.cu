@@ -105,10 +105,9 @@ struct Mailbox {
     int solve_failed;
     double slope, dir_norm2, max_translation;
     unsigned long long ccd_bits;
+    unsigned long long pair_count;
     uint32_t sweep_fail;
-    uint32_t pair_count;
     uint32_t refine_bits;
-    uint32_t pad;
     // The direction as solved (k_reduce_dir); slope, dir_norm2 and
     // max_translation are those of the limited one after k_limit.
     double dir_slope, dir_max_translation;
@@ -120,17 +119,21 @@ struct Mailbox {
 // the host-mapped mailbox and reset them for the next use.
 struct Scalars {
     unsigned long long ccd_bits;
+    // Room asked for in the bounded lists, in 64 bits: a full list goes on
+    // counting (claim_range, append_slot), with elements asking again at every
+    // evaluation of a substep, and a count that came round would hand out
+    // ranges in use.
+    unsigned long long pair_count;
+    unsigned long long surv_count;  // pairs of the contact pass's FP64 pool
+    unsigned long long pool_used;   // entries of the leaf pool, since the last cache rebuild
     uint32_t sweep_fail;
     int solve_failed;
-    uint32_t pair_count;
-    uint32_t surv_count;  // pairs of the contact pass's FP64 pool handed out
     uint32_t solve_next;  // next strand group of the block-solve work queue
     uint32_t refine_bits; // largest relative refinement correction (FP32 bits)
     uint32_t near_count;  // elements queued for the warp-cooperative contact pass
     uint32_t ccd_near;    // elements queued for the warp-cooperative CCD pass
     uint32_t eval_done;   // blocks of k_reduce_eval finished (the last one reduces the partials)
     uint32_t dir_done, ccd_done;  // the same for the direction's sums and the CCD pairs
-    uint32_t pool_used;   // entries of the leaf pool handed out since the last cache rebuild
     double trial_alpha;   // first line-search step from the last CCD bound (publish_ccd)
     double max_translation;  // largest free-node translation of the last reduced direction
     uint32_t wide_count;  // elements queued for k_contact_near that take a block each
@@ -238,13 +241,21 @@ struct View {
 // atomic (a per-lane atomic on one address serialises at L2 when tens of
 // thousands of elements append in one launch).  Slot order within a list is
 // not meaningful to any of its consumers.
-__device__ __forceinline__ uint32_t append_slot(uint32_t *count)
+template<class T> __device__ __forceinline__ T append_slot(T *count)
 {
     namespace cg = cooperative_groups;
     const cg::coalesced_group g = cg::coalesced_threads();
-    uint32_t base = 0;
-    if (g.thread_rank() == 0) base = atomicAdd(count, g.size());
+    T base = 0;
+    if (g.thread_rank() == 0) base = atomicAdd(count, T(g.size()));
     return g.shfl(base, 0) + g.thread_rank();
+}
+
+// n entries of a list of `capacity` entries, *used of which were asked for so
+// far: their offset, or kNone without room.
+__device__ __forceinline__ uint32_t claim_range(unsigned long long *used, uint32_t n, uint32_t capacity)
+{
+    const unsigned long long off = atomicAdd(used, (unsigned long long)n);
+    return off + n <= capacity ? uint32_t(off) : kNone;
 }
 
 __device__ __forceinline__ V load3(const double *p) { return dm::v(p[0], p[1], p[2]); }
@@ -402,9 +413,9 @@ __device__ __forceinline__ uint8_t leaves_to_cache(const View &d, uint32_t e, V 
     const uint32_t c = collect_leaves(d, lo, hi, pad, slots, kCacheLeaves);
     uint8_t nl = uint8_t(c);
     if (c > uint32_t(kCacheLeaves)) {
-        const uint32_t off = atomicAdd(&d.sc->pool_used, c);
+        const uint32_t off = claim_range(&d.sc->pool_used, c, d.leaf_pool_capacity);
         nl = kCacheInvalid;
-        if (size_t(off) + c <= d.leaf_pool_capacity) {
+        if (off != kNone) {
             collect_leaves(d, lo, hi, pad, d.leaf_pool + off, c);
             slots[0] = off;
             slots[1] = c;
@@ -1071,11 +1082,8 @@ __device__ __forceinline__ uint32_t near_claim(const View &d, uint32_t e, uint32
             pair.distance = 1.0e300; pair.t = 0.0; pair.bary = dm::v(1, 0, 0);
             write_contact(d, e, kNone, pair);
         } else {
-            off = atomicAdd(&d.sc->surv_count, n);
-            if (uint64_t(off) + n > d.surv_capacity) {
-                off = kNone;
-                held = kSurvOverflow;
-            }
+            off = claim_range(&d.sc->surv_count, n, d.surv_capacity);
+            if (off == kNone) held = kSurvOverflow;
             d.surv_off[e] = off;
         }
         d.surv_n[e] = held;
@@ -1256,7 +1264,7 @@ __global__ void __launch_bounds__(kPairBlock) k_contact_exact(View d, const doub
     follow_previous();
     __shared__ double sh[kPairWarps][5][32];
     const int part = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t count = min(d.sc->surv_count, d.surv_capacity);
+    const uint32_t count = uint32_t(min(d.sc->surv_count, (unsigned long long)d.surv_capacity));
     for (uint32_t base = 32 * blockIdx.x; base < count; base += 32 * gridDim.x) {
         const uint32_t k = base + lane;
         if (k < count) {
@@ -2408,7 +2416,7 @@ template<bool FILTER> __device__ __forceinline__ void list_swept_pair(const View
     } else {
         t = __float_as_uint(__ldg(d.tri32 + 3 * size_t(p)).w);
     }
-    const uint32_t slot = append_slot(&d.sc->pair_count);
+    const unsigned long long slot = append_slot(&d.sc->pair_count);
     if (slot < d.pair_capacity) { d.pair_elem[slot] = e; d.pair_tri[slot] = t; }
 }
 
@@ -2474,7 +2482,7 @@ template<bool SWEEP> __global__ void __launch_bounds__(kPairBlock) k_advance_pai
     __shared__ double sh_d2[kPairWarps][32], sh_alpha[32];
     __shared__ uint32_t sh_active;
     const int part = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t count = min(d.sc->pair_count, d.pair_capacity);
+    const uint32_t count = uint32_t(min(d.sc->pair_count, (unsigned long long)d.pair_capacity));
     const double target = d.radius + d.offset + d.min_gap;
     for (uint32_t base = 32 * blockIdx.x; base < count; base += 32 * gridDim.x) {
         const uint32_t k = base + lane;
@@ -2630,7 +2638,7 @@ template<bool FILTER> __global__ void __launch_bounds__(kBlock) k_sweep_near(Vie
             for (uint32_t c = lane; c < here; c += 32) {
                 const uint32_t p = pos[c];
                 if (FILTER && sweep_skip_f(d, p, origin, f1, d.ccd_pad.up)) continue;
-                const uint32_t slot = append_slot(&d.sc->pair_count);
+                const unsigned long long slot = append_slot(&d.sc->pair_count);
                 if (slot < d.pair_capacity) {
                     d.pair_elem[slot] = e;
                     d.pair_tri[slot] = __float_as_uint(__ldg(d.tri32 + 3 * size_t(p)).w);
@@ -3605,7 +3613,7 @@ EvalStats Engine::evaluate(bool gradient, double dt, double alpha, const double 
             I.wait_for(I.side, I.fork);
         }
         const double *q = v.q;
-        if (rebuild_cache_) KHS_CUDA(cudaMemsetAsync(&v.sc->pool_used, 0, sizeof(uint32_t), cs));
+        if (rebuild_cache_) KHS_CUDA(cudaMemsetAsync(&v.sc->pool_used, 0, sizeof(v.sc->pool_used), cs));
         I.launch_on(cs, rebuild_cache_ ? "k_contact_filter_rebuild" : trial ? "k_contact_filter_trial" : "k_contact_filter",
                     k_contact_filter, grid_for(v.E), kBlock, v, q, rebuild_cache_ ? 1 : 0);
         I.launch_on(cs, "k_contact_near", mode_ ? k_contact_near<true> : k_contact_near<false>, near_grid(v.E), kBlock, v);
@@ -4053,7 +4061,7 @@ KhsResult Engine::run_frame(double frame_dt, const double *root_a, const double 
                 View vs = v;  // walks the swept tree
                 vs.bnode = v.swept_node; vs.blo = v.swept_lo; vs.bhi = v.swept_hi;
                 progress_phase_.store(KHS_PHASE_CCD);
-                KHS_CUDA(cudaMemsetAsync(&v.sc->pool_used, 0, sizeof(uint32_t), I.stream));
+                KHS_CUDA(cudaMemsetAsync(&v.sc->pool_used, 0, sizeof(v.sc->pool_used), I.stream));
                 I.launch("k_sweep_collect", k_sweep_collect, grid_for(v.E), kBlock, vs);
                 I.launch("k_sweep_near", mode_ ? k_sweep_near<true> : k_sweep_near<false>, 152u * 8u, kBlock, vs);
                 I.launch("k_sweep_pairs", k_advance_pairs<true>, kPairGrid, kPairBlock, vs);
