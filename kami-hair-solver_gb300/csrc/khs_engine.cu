@@ -178,19 +178,19 @@ struct View {
     const uint32_t *sfirst, *scount, *sfixed, *sorder;
     const uint32_t *tri;
     double *col_cur, *col_old;
-    float *col32;  // FP32 copy of col_cur for the mixed form's filters
+    float *col32;  // FP32 copy of col_cur for the FP32 search by one thread (closest_triangle)
     double *blo, *bhi;  // leaves only: the FP64 boxes of the exact leaf test
     // The tree over old and new positions, for the moving-collider sweep.
     double *swept_lo, *swept_hi;
     float4 *swept_node;
-    // Mixed form: each BVH node packed in 32 bytes (FP32 outward-rounded box,
+    // Each BVH node packed in 32 bytes (FP32 outward-rounded box,
     // escape index, leaf range), the per-element contact result of the
     // separate contact pass, and the CCD (element, triangle) work list.
     float4 *bnode;
     double *c_t, *c_bary, *c_dist;
     uint32_t *pair_elem, *pair_tri;
     uint32_t pair_capacity;
-    // Per-substep leaf cache of the mixed contact pass: the leaves (DFS
+    // Per-substep leaf cache of the contact pass: the leaves (DFS
     // order) whose FP32 box overlaps the element box grown by kCacheSlack,
     // and the element's node positions when they were collected.
     uint32_t *cache_leaf;
@@ -573,8 +573,8 @@ __device__ __forceinline__ void merge_children(float4 *bnode, uint32_t p, uint32
 // a leaf, a triangle each; the first one walks up, the second child to arrive
 // at a parent (atomic counter) merges the two children, resets the counter for
 // the next launch and continues.  Two launches with a thread a leaf, and a
-// third for the records, took 72 us a substep on 1,280 triangles and 230 on
-// 449,940; this one 24 and 127.
+// third for the records, took 90 us a substep on 1,280 triangles and 204 on
+// 449,940; this one 25 and 127.
 constexpr int kLeafTriangles = 8;  // BVH leaves hold at most 8 triangles (cuda_backend.cu:305)
 __global__ void __launch_bounds__(kBlock) k_refit(View d)
 {
@@ -878,8 +878,6 @@ __device__ __forceinline__ uint32_t closest_triangle(const View &d, V xi, V xj, 
     return closest_triangle_in(d, xi, xj, cand, pair, [&](auto &&fn) { bvh_query_packed(d, lo, hi, pad, fn); });
 }
 
-// Contact classification of every element at a caller-provided state
-// (positions of q_probe); used to check the integer contact work.
 // Contact classification of every element at the state q: candidate count,
 // closest triangle with its closest pair, gap and flags, by one thread an
 // element (the contact-query entry point).
@@ -3683,11 +3681,12 @@ bool Engine::make_steepest()
 // by fives 1,650; 831 with the timed shapes this replaces).
 //
 // Teams are taken while the work on one warp a strand is at most 1.1 times
-// the longest chain, us a solve against the split: the body scene with 700 of
-// its strands 375 and 452, with 3,000 476 and 514 (work 0.6 of the chain);
-// 1,000 strands of 16-160 nodes 266 and 327, 1,800 467 and 490 (1.05), 2,200
-// 513 and 495 (1.3); 2,000 of 8-24 nodes 85 and 88 (1.4), 4,000 162 and 159
-// (2.8); all of the body scene 674 and 569 (1.4).
+// the longest chain, us a solve against a warp each: the body scene with 700 of
+// its strands 376 and 458, with 3,000 476 and 530 (work 0.6 of the chain);
+// 1,000 strands of 20-120 nodes 291 and 343, of 16-160 nodes 380 and 457, 1,800
+// of these 467 and 490 (1.05); against the best split beyond the line, 2,200
+// of 16-160 nodes 513 and 495 (1.3), 2,000 of 8-24 nodes 84 and 87 (1.4), 4,000
+// 162 and 161 (2.8), all of the body scene 674 and 568 (1.4).
 void Engine::plan_block_solve(uint32_t alone, uint32_t blocks_per_sm)
 {
     Impl &I = *d_;
